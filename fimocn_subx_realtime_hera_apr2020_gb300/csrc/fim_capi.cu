@@ -85,8 +85,7 @@ struct fim_ctx {
   // scratch (sized for all members)
   void *antifx = nullptr, *delp_lo = nullptr, *p_plus = nullptr, *p_mnus = nullptr, *r_plus = nullptr,
        *r_mnus = nullptr;
-  void *t_antiflx = nullptr, *t_trmin = nullptr, *t_trmax = nullptr, *t_trcr_lo = nullptr, *t_rp = nullptr,
-       *t_rm = nullptr;
+  void *t_antiflx = nullptr, *t_sp = nullptr, *t_sm = nullptr, *t_trcr_lo = nullptr, *t_trold = nullptr;
   int tchunk = 0;
   void *f_trcr_lo = nullptr, *f_sp = nullptr, *f_sm = nullptr, *f_trold = nullptr, *f_rp = nullptr,
        *f_rm = nullptr, *f_af = nullptr;
@@ -391,23 +390,39 @@ int ensure_cnuity(fim_ctx* c, int members) {
   return FIM_OK;
 }
 
+// scratch of trcadv with the caller's edge values (the per-routine entry, and
+// the step without hi_order_flux_comp)
 int ensure_trcadv(fim_ctx* c, int members) {
-  if (c->t_antiflx) return FIM_OK;
+  if (c->t_trold) return FIM_OK;
+  {
+    const int e = c->prec == FIM_PREC_F64 ? prepare_tracers<double>(c->ftab) : prepare_tracers<float>(c->ftab);
+    if (e) return set_err(c, FIM_ECUDA, "tracer kernel attributes", (cudaError_t)e);
+  }
   const size_t NL = (size_t)c->N * c->L;
-  // bound the tracer chunk so the six scratch fields take at most ~12 GB
-  size_t per_tracer = NL * members * 11 * c->esz;
+  // per tracer of a chunk: six antidiffusive fluxes, S+, S-, trcr_lo and the
+  // old tracer; chunks of at most ~12 GB
+  size_t per_tracer = NL * members * 10 * c->esz;
   int tch = c->T;
   while (tch > 1 && per_tracer * tch > (size_t)12 << 30) tch = (tch + 1) / 2;
   c->tchunk = tch;
   const size_t n = NL * members * tch;
   int rc;
   if ((rc = ensure(c, &c->t_antiflx, n * 6))) return rc;
-  if ((rc = ensure(c, &c->t_trmin, n))) return rc;
-  if ((rc = ensure(c, &c->t_trmax, n))) return rc;
+  if ((rc = ensure(c, &c->t_sp, n))) return rc;
+  if ((rc = ensure(c, &c->t_sm, n))) return rc;
   if ((rc = ensure(c, &c->t_trcr_lo, n))) return rc;
-  if ((rc = ensure(c, &c->t_rp, n))) return rc;
-  if ((rc = ensure(c, &c->t_rm, n))) return rc;
+  if ((rc = ensure(c, &c->t_trold, n))) return rc;
   return FIM_OK;
+}
+
+// tracer kernels with the caller's edge values: the widest level vectors,
+// four threads a cell
+template <typename R>
+TrcFusedScratch<R> trcadv_scratch(fim_ctx* c) {
+  TrcFusedScratch<R> w{(R*)c->t_trcr_lo, (R*)c->t_sp, (R*)c->t_sm, (R*)c->t_trold, nullptr, nullptr,
+                       (R*)c->t_antiflx, c->tchunk, 0, 4, c->ftab};
+  w.edges = true;
+  return w;
 }
 
 // The strides of a state's fields in the step: with the fused tracer
@@ -662,9 +677,8 @@ int trcadv_impl(fim_ctx* c, const R* trcr_edg, R* tracr, R* trcdp, R* trc_tdcy, 
   const R* dp = s.map(delp, NL, 0);
   if (s.rc) return s.rc;
   if ((rc = push_sp(c))) return rc;
-  TrcadvScratch<R> w{(R*)c->t_antiflx, (R*)c->t_trmin, (R*)c->t_trmax, (R*)c->t_trcr_lo, (R*)c->t_rp, (R*)c->t_rm,
-                     c->tchunk};
-  launch_trcadv<R>(make_launch(c, 1), grid_of<R>(c), c->str, w, te, tr, td, tt, tl, mf, dp);
+  launch_tracers_fused<R>(make_launch(c, 1), grid_of<R>(c), c->str, trcadv_scratch<R>(c), const_cast<R*>(te), tr, td,
+                          tt, tl, mf, dp);
   if ((rc = check_launch(c, "trcadv"))) return rc;
   return s.finish();
 }
@@ -1186,11 +1200,9 @@ int enqueue_step(fim_ctx* c, fim_state* st, StepIo* io = nullptr) {
                               P(FIM_TRC_TDCY), P(FIM_TRL_TDCY), P(FIM_MASSFX),
                               P(FIM_DP3D), io ? &io->hook : nullptr);
     } else {
-      TrcadvScratch<R> tw{(R*)c->t_antiflx, (R*)c->t_trmin, (R*)c->t_trmax, (R*)c->t_trcr_lo, (R*)c->t_rp,
-                          (R*)c->t_rm, c->tchunk};
       if (io) io_chunk_hook(io, 0, 0, c->T);
-      launch_trcadv<R>(lg, g, s, tw, P(FIM_TRC_EDG), P(FIM_TR3D), P(FIM_TRDP),
-                       P(FIM_TRC_TDCY), P(FIM_TRL_TDCY), P(FIM_MASSFX), P(FIM_DP3D));
+      launch_tracers_fused<R>(lg, g, s, trcadv_scratch<R>(c), P(FIM_TRC_EDG), P(FIM_TR3D), P(FIM_TRDP),
+                              P(FIM_TRC_TDCY), P(FIM_TRL_TDCY), P(FIM_MASSFX), P(FIM_DP3D));
       if (io) io_chunk_hook(io, 1, 0, c->T);
     }
     if (io && io->rc) return io->rc;

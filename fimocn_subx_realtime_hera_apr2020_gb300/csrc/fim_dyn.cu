@@ -1,5 +1,5 @@
 // Horizontal stencil kernels of the FIM dynamics step: edgvar1, edgvar3,
-// cnuity1..5, trcadv1..3, del4prep/dissip/momtum1.
+// cnuity1..5, del4prep/dissip/momtum1 (trcadv1..3: fim_trc.cu).
 //
 // Layout is the reference's (level index fastest), so one thread per
 // (level, cell) gives fully coalesced loads along k for own and neighbour
@@ -834,158 +834,6 @@ void launch_massadv(const Launch& l, const Grid<R>& g, const Strides& s, const C
 }
 
 // --------------------------------------------------------------------------
-// trcadv1 (trcadv_compute.F90:55-135) for tracers t0..t0+gridDim.z-1.
-template <typename R>
-__global__ void __launch_bounds__(kBlock) k_trcadv1(Grid<R> g, Strides s, const StepParams* __restrict__ sp, int t0,
-    const R* __restrict__ massfx, const R* __restrict__ trc_edg, const R* __restrict__ tracr,
-    const R* __restrict__ trcdp, R* __restrict__ trl_tdcy, const R* __restrict__ delp,
-    R* __restrict__ antiflx, R* __restrict__ trmin, R* __restrict__ trmax, R* __restrict__ trcr_lo, size_t sc_stride) {
-  int i, k;
-  if (!cell_level(g.N, g.L, i, k)) return;
-  const int L = g.L, N = g.N;
-  const size_t m = blockIdx.y;
-  sp += m;
-  if (!sp->active) return;
-  const int tz = blockIdx.z, t = t0 + tz;
-  const size_t NL = (size_t)N * L;
-  massfx += m * s.mf; delp += m * s.cell;
-  trc_edg += m * s.tredg + (size_t)t * 6 * NL;
-  tracr += m * s.tr + (size_t)t * NL;
-  trcdp += m * s.tr + (size_t)t * NL;
-  trl_tdcy += m * s.trab + (size_t)t * 3 * NL;
-  const size_t so = (m * gridDim.z + tz) * sc_stride;
-  antiflx += so * 6; trmin += so; trmax += so; trcr_lo += so;
-  const int nf = sp->nf, of = sp->of, vof = sp->vof;
-  const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
-  const R thshld = R(1.e-11), half = R(0.5);
-  const R* mfn = massfx + (size_t)nf * N * 6 * L;
-  const int np = g.nprox[i];
-  const size_t c = (size_t)i * L + k;
-  const R tri = tracr[c];
-  if (np < 6) antiflx[((size_t)i * 6 + 5) * L + k] = R(0);
-  R sumlo = R(0);
-  for (int e = 0; e < np; e++) {
-    const int ipx = g.prox[i * 6 + e], edx = g.proxs[i * 6 + e];
-    const size_t o = ((size_t)i * 6 + e) * L + k;
-    const R mf = mfn[o], mx = mfn[((size_t)ipx * 6 + edx) * L + k];
-    const R flx_hi = mf * trc_edg[o];
-    const R lo = half * ((mf + rabs(mf)) * tri - (mx + rabs(mx)) * tracr[(size_t)ipx * L + k]);
-    antiflx[o] = flx_hi - lo;
-    sumlo = sumlo + lo;
-  }
-  const R tn = -sumlo * g.rarea[i];
-  trl_tdcy[(size_t)nf * NL + c] = tn;
-  const R trcdp_lo = trcdp[c] + ab1 * tn + ab2 * trl_tdcy[(size_t)of * NL + c] + ab3 * trl_tdcy[(size_t)vof * NL + c];
-  const int* pr = g.prox + i * 6;
-  R mx = tri, mn = tri;
-#pragma unroll
-  for (int e = 0; e < 6; e++) {
-    const R x = tracr[(size_t)pr[e] * L + k];
-    mx = rmax(mx, x);
-    mn = rmin(mn, x);
-  }
-  mx = rmax(R(0), mx);
-  mn = rmax(R(0), mn);
-  trmax[c] = mx;
-  trmin[c] = mn;
-  trcr_lo[c] = rmax(mn, rmin(mx, fdiv(trcdp_lo, rmax(thshld, delp[c]))));
-}
-
-// trcadv2 (trcadv_compute.F90:171-235)
-template <typename R>
-__global__ void __launch_bounds__(kBlock) k_trcadv2(Grid<R> g, Strides s, const StepParams* __restrict__ sp, int t0,
-    const R* __restrict__ trc_tdcy, const R* __restrict__ delp, const R* __restrict__ antiflx,
-    R* __restrict__ trmin, R* __restrict__ trmax, const R* __restrict__ trcr_lo, R* __restrict__ r_plus,
-    R* __restrict__ r_mnus, size_t sc_stride) {
-  int i, k;
-  if (!cell_level(g.N, g.L, i, k)) return;
-  const int L = g.L, N = g.N;
-  const size_t m = blockIdx.y;
-  sp += m;
-  if (!sp->active) return;
-  const int tz = blockIdx.z, t = t0 + tz;
-  const size_t NL = (size_t)N * L;
-  delp += m * s.cell;
-  trc_tdcy += m * s.trab + (size_t)t * 3 * NL;
-  const size_t so = (m * gridDim.z + tz) * sc_stride;
-  antiflx += so * 6; trmin += so; trmax += so; trcr_lo += so; r_plus += so; r_mnus += so;
-  const int of = sp->of, vof = sp->vof;
-  const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
-  const R thshld = R(1.e-11);
-  const int np = g.nprox[i];
-  const size_t c = (size_t)i * L + k;
-  R s_plus = R(0), s_mnus = R(0);
-  for (int e = 0; e < np; e++) {
-    const R a = antiflx[((size_t)i * 6 + e) * L + k];
-    s_plus = s_plus - rmin(R(0), a);
-    s_mnus = s_mnus + rmax(R(0), a);
-  }
-  const R lo = trcr_lo[c];
-  R mx = rmax(trmax[c], lo), mn = rmin(trmin[c], lo);
-  const int* pr = g.prox + i * 6;
-#pragma unroll
-  for (int e = 0; e < 6; e++) {
-    const R x = trcr_lo[(size_t)pr[e] * L + k];
-    mx = rmax(mx, x);
-    mn = rmin(mn, x);
-  }
-  mx = rmax(R(0), mx);
-  mn = rmax(R(0), mn);
-  trmax[c] = mx;
-  trmin[c] = mn;
-  const R dp = delp[c];
-  const R to = trc_tdcy[(size_t)of * NL + c], tv = trc_tdcy[(size_t)vof * NL + c];
-  const R rab1 = R(1) / ab1;  // one reciprocal, as k_tr_lim
-  const R q_plus = ((mx - lo) * dp - (ab2 * rmin(R(0), to) + ab3 * rmax(R(0), tv))) * rab1 * g.area[i];
-  const R q_mnus = ((lo - mn) * dp + (ab2 * rmax(R(0), to) + ab3 * rmin(R(0), tv))) * rab1 * g.area[i];
-  r_plus[c] = rmax(R(0), rmin(R(1), fdiv(q_plus, rmax(s_plus, thshld))));
-  r_mnus[c] = rmax(R(0), rmin(R(1), fdiv(q_mnus, rmax(s_mnus, thshld))));
-}
-
-// trcadv3 (trcadv_compute.F90:270-309)
-template <typename R>
-__global__ void __launch_bounds__(kBlock) k_trcadv3(Grid<R> g, Strides s, const StepParams* __restrict__ sp, int t0,
-    R* __restrict__ trc_tdcy, const R* __restrict__ trl_tdcy, R* __restrict__ trcdp, R* __restrict__ tracr,
-    const R* __restrict__ delp, const R* __restrict__ antiflx, const R* __restrict__ r_mnus,
-    const R* __restrict__ r_plus, const R* __restrict__ trmin, const R* __restrict__ trmax, size_t sc_stride) {
-  int i, k;
-  if (!cell_level(g.N, g.L, i, k)) return;
-  const int L = g.L, N = g.N;
-  const size_t m = blockIdx.y;
-  sp += m;
-  if (!sp->active) return;
-  const int tz = blockIdx.z, t = t0 + tz;
-  const size_t NL = (size_t)N * L;
-  delp += m * s.cell;
-  trc_tdcy += m * s.trab + (size_t)t * 3 * NL;
-  trl_tdcy += m * s.trab + (size_t)t * 3 * NL;
-  trcdp += m * s.tr + (size_t)t * NL;
-  tracr += m * s.tr + (size_t)t * NL;
-  const size_t so = (m * gridDim.z + tz) * sc_stride;
-  antiflx += so * 6; trmin += so; trmax += so; r_plus += so; r_mnus += so;
-  const int nf = sp->nf, of = sp->of, vof = sp->vof;
-  const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
-  const R thshld = R(1.e-11);
-  const int np = g.nprox[i];
-  const size_t c = (size_t)i * L + k;
-  const R rp = r_plus[c], rm = r_mnus[c];
-  R at = R(0);
-  for (int e = 0; e < np; e++) {
-    const int px = g.prox[i * 6 + e];
-    R a = antiflx[((size_t)i * 6 + e) * L + k];
-    if (a >= R(0)) a = a * rmin(rm, r_plus[(size_t)px * L + k]);
-    else a = a * rmin(rp, r_mnus[(size_t)px * L + k]);
-    at = at + a;
-  }
-  at = -at * g.rarea[i];
-  const R tn = trl_tdcy[(size_t)nf * NL + c] + at;
-  trc_tdcy[(size_t)nf * NL + c] = tn;
-  const R td = trcdp[c] + ab1 * tn + ab2 * trc_tdcy[(size_t)of * NL + c] + ab3 * trc_tdcy[(size_t)vof * NL + c];
-  trcdp[c] = td;
-  tracr[c] = rmax(trmin[c], rmin(trmax[c], fdiv(td, rmax(thshld, delp[c]))));
-}
-
-// --------------------------------------------------------------------------
 // del4prep (momtum_compute.F90:16-95) on u+grndspd, v; writes prepared fields.
 template <typename R>
 __global__ void __launch_bounds__(kBlock) k_del4prep(Grid<R> g, Strides s, const R* __restrict__ u,
@@ -1342,29 +1190,6 @@ void launch_cnuity(const Launch& l, const Grid<R>& g, const Strides& s, const Cn
 }
 
 template <typename R>
-void launch_trcadv(const Launch& l, const Grid<R>& g, const Strides& s, const TrcadvScratch<R>& w,
-                   const R* trc_edg, R* tracr, R* trcdp, R* trc_tdcy, R* trl_tdcy, const R* massfx,
-                   const R* delp) {
-  const size_t scs = (size_t)g.N * g.L;
-  for (int t0 = 0; t0 < g.T; t0 += w.tchunk) {
-    const int nt = (g.T - t0 < w.tchunk) ? g.T - t0 : w.tchunk;
-    dim3 grid(blocks_for((long long)g.N * g.L), l.members, nt);
-    FIM_KBEGIN(l, "k_trcadv1");
-    k_trcadv1<R><<<grid, kBlock, 0, l.stream>>>(g, s, l.sp, t0, massfx, trc_edg, tracr, trcdp, trl_tdcy, delp,
-                                                 w.antiflx, w.trmin, w.trmax, w.trcr_lo, scs);
-    FIM_KEND(l);
-    FIM_KBEGIN(l, "k_trcadv2");
-    k_trcadv2<R><<<grid, kBlock, 0, l.stream>>>(g, s, l.sp, t0, trc_tdcy, delp, w.antiflx, w.trmin, w.trmax,
-                                                 w.trcr_lo, w.r_plus, w.r_mnus, scs);
-    FIM_KEND(l);
-    FIM_KBEGIN(l, "k_trcadv3");
-    k_trcadv3<R><<<grid, kBlock, 0, l.stream>>>(g, s, l.sp, t0, trc_tdcy, trl_tdcy, trcdp, tracr, delp,
-                                                 w.antiflx, w.r_mnus, w.r_plus, w.trmin, w.trmax, scs);
-    FIM_KEND(l);
-  }
-}
-
-template <typename R>
 void launch_momtum(const Launch& l, const Grid<R>& g, const Strides& s, const Knobs& kn, const MomtumScratch<R>& w,
                    R* u, R* v, const R* exner, R* relvor, const R* u_edg, const R* v_edg,
                    const R* trc_edg, const R* mont_edg, const R* uvsq_edg, R* u_tndcy, R* v_tndcy,
@@ -1424,8 +1249,6 @@ void launch_step_begin(const Launch& l, StepParams* sp) {
   template void launch_massadv<R>(const Launch&, const Grid<R>&, const Strides&, const CnuityScratch<R>&,     \
                                   const R*, const R*, const R*, const R*, R*, const R*, R*, R*, R*, R*, R*,   \
                                   R*);                                                                       \
-  template void launch_trcadv<R>(const Launch&, const Grid<R>&, const Strides&, const TrcadvScratch<R>&,      \
-                                 const R*, R*, R*, R*, R*, const R*, const R*);                               \
   template void launch_momtum<R>(const Launch&, const Grid<R>&, const Strides&, const Knobs&,                 \
                                  const MomtumScratch<R>&, R*, R*, const R*, R*, const R*, const R*, const R*, \
                                  const R*, const R*, R*, R*, const R*, const float2*, const R*);

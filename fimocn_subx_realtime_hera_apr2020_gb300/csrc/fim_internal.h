@@ -385,12 +385,6 @@ template <typename R>
 void launch_massadv(const Launch&, const Grid<R>&, const Strides&, const CnuityScratch<R>&, const R* u,
                     const R* v, const R* u_edg, const R* v_edg, R* dp_edg, const R* lp_edg, R* delp, R* pres,
                     R* exner, R* dp_tndcy, R* massfx, R* omega);
-template <typename R>
-struct TrcadvScratch { R *antiflx, *trmin, *trmax, *trcr_lo, *r_plus, *r_mnus; int tchunk; };
-template <typename R>
-void launch_trcadv(const Launch&, const Grid<R>&, const Strides&, const TrcadvScratch<R>&,
-                   const R* trc_edg, R* tracr, R* trcdp, R* trc_tdcy, R* trl_tdcy, const R* massfx,
-                   const R* delp);
 // Cell patches of the fused tracer kernels (fim_trc.cu).  A patch is a set
 // of interior cells; its frame lists them first, then every other cell one
 // neighbour step away (ring 1), then two steps away (ring 2), so a block can
@@ -428,6 +422,7 @@ struct TrcFusedScratch {
   int vk;  // levels per thread (0: widest the layout admits)
   int gc;  // threads per cell and level tile: the tile is vk * gc levels
   FrameTab ft;
+  bool edges = false;  // trc_edg holds every tracer's edge values (the per-routine trcadv); 4 threads a cell
 };
 // one-time launch attributes (shared-memory size) of the tracer kernels for
 // these patches; returns a cudaError_t value

@@ -20,15 +20,20 @@
 //             limiters of their two cells, AB3 update of tracer x thickness,
 //             new tracer.
 //
+// The per-routine trcadv runs the same two kernels with the caller's edge
+// values (EV): 38 words a cell-level and tracer at 16-byte accesses where one
+// thread a cell-level took about 60 at 4 (glvl 7, nvl 64, 11 tracers, FP32:
+// 8.04 -> 3.00 ms; FP64, glvl 5, nvl 37, 5 tracers: 0.82 -> 0.56 ms).
+//
 // The edge values (six per cell-level and tracer) and R+/R- never reach HBM:
 // per cell-level and tracer the pair reads and writes 32 words (10 of them
 // the step's own state traffic), where edge values written and read back and
 // R+/R- stored cost 46.  The old tracer is copied because k_trf_hi overwrites
 // the tracer in place while the blocks of neighbouring patches still read it.
 //
-// Every value is formed from the same operands in the same order as the
-// per-routine kernels (k_edgvar3_own, k_trcadv1..3), so the fused step is
-// bit-identical to the routine sequence.  nprox is 5 or 6 (checked when the
+// Every value is formed from the same operands in the same order as in the
+// per-routine entries (k_edgvar3_own/_avg, then these kernels with EV), so the
+// fused step is bit-identical to the routine sequence.  nprox is 5 or 6 (checked when the
 // context is created), so only slot 5 of a cell can be missing: the tests
 // "e < nprox" are written (e < 5 || e < np) and cost nothing for slots 0..4.
 #include "fim_internal.h"
@@ -42,23 +47,121 @@ namespace {
 
 template <typename R> __device__ __forceinline__ R tmax(R a, R b) { return a > b ? a : b; }
 template <typename R> __device__ __forceinline__ R tmin(R a, R b) { return a < b ? a : b; }
-template <typename R> __device__ __forceinline__ R tabs(R a) { return a < R(0) ? -a : a; }
-// max/min of three (exact; FP32 uses the three-input instructions)
-template <typename R> __device__ __forceinline__ R tmax3(R a, R b, R c) { return tmax(a, tmax(b, c)); }
-template <typename R> __device__ __forceinline__ R tmin3(R a, R b, R c) { return tmin(a, tmin(b, c)); }
-template <> __device__ __forceinline__ float tmax3<float>(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
+
+// Bounds, signs and quotients of the transport.  FP32 takes the min/max
+// instructions.  GB300 issues 2 FP64 lanes a clock and SM against 64 integer
+// ones, so the FP64 build compares on the integer pipe (a double's bits with
+// the magnitude of negative values complemented order as int64) and divides
+// with the fewest FP64 operations.  A NaN operand does not enter a bound or a
+// sign split here; it reaches the cell's result through the fluxes and the
+// AB3 sums, whose final clip (tmin/tmax) keeps it.
+// At glvl 6 / nvl 64 / 11 tracers this took the FP64 k_trf_lo from 9.56 to
+// 6.1 ms and k_trf_hi from 8.15 to 2.86 ms a step (FP32: 2% of k_trf_hi).
+template <typename R> struct Bound;
+template <> struct Bound<float> {
+  float v;
+  __device__ __forceinline__ static Bound of(float x) { return {x}; }
+  __device__ __forceinline__ float value() const { return v; }
+  __device__ __forceinline__ void up(Bound a) { v = fmaxf(v, a.v); }
+  __device__ __forceinline__ void down(Bound a) { v = fminf(v, a.v); }
+  // with two values at once (three-input instructions)
+  __device__ __forceinline__ void up(Bound a, Bound b) { asm("max.f32 %0, %0, %1, %2;" : "+f"(v) : "f"(a.v), "f"(b.v)); }
+  __device__ __forceinline__ void down(Bound a, Bound b) { asm("min.f32 %0, %0, %1, %2;" : "+f"(v) : "f"(a.v), "f"(b.v)); }
+  __device__ __forceinline__ float at_least_zero() const { return fmaxf(v, 0.f); }
+};
+template <> struct Bound<double> {
+  long long v;
+  __device__ __forceinline__ static long long flip(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffll); }
+  __device__ __forceinline__ static Bound of(double x) { return {flip(__double_as_longlong(x))}; }
+  __device__ __forceinline__ double value() const { return __longlong_as_double(flip(v)); }
+  __device__ __forceinline__ void up(Bound a) { v = a.v > v ? a.v : v; }
+  __device__ __forceinline__ void down(Bound a) { v = a.v < v ? a.v : v; }
+  __device__ __forceinline__ void up(Bound a, Bound b) { up(a); up(b); }
+  __device__ __forceinline__ void down(Bound a, Bound b) { down(a); down(b); }
+  __device__ __forceinline__ double at_least_zero() const { return __longlong_as_double(v > 0 ? v : 0); }
+};
+
+// the positive / negative part of x
+__device__ __forceinline__ float pos(float x) { return fmaxf(x, 0.f); }
+__device__ __forceinline__ float neg(float x) { return fminf(x, 0.f); }
+__device__ __forceinline__ double pos(double x) { return __double2hiint(x) < 0 ? 0. : x; }
+__device__ __forceinline__ double neg(double x) { return __double2hiint(x) < 0 ? x : 0.; }
+// the smaller of two values >= 0
+__device__ __forceinline__ float min0(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ double min0(double a, double b) {
+  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  return __longlong_as_double(x < y ? x : y);
 }
-template <> __device__ __forceinline__ float tmin3<float>(float a, float b, float c) {
-  float r;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
+// max(a, b) of values >= 0
+__device__ __forceinline__ float floor_at(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double floor_at(double a, double b) {
+  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  return __longlong_as_double(x > y ? x : y);
 }
-// product rounded on its own (never contracted into a following add)
+__device__ __forceinline__ bool negative(float x) { return x < 0.f; }
+__device__ __forceinline__ bool negative(double x) { return __double2hiint(x) < 0; }
+
+// products and sums whose contraction is pinned: the same value must come out
+// of every instantiation (the per-routine and the fused kernels, every shape)
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// low-order flux a tri - b trx of the two sides' outflows a, b >= 0.  The
+// two sides hold the same mass flux with opposite signs, up to rounding, so
+// one of the products is zero but for fluxes of a rounding error's size: FP64
+// forms the other one only.
+__device__ __forceinline__ float donor(float mf, float mfx, float tri, float trx) {
+  return fma_rn(pos(mf), tri, -mul_rn(pos(mfx), trx));
+}
+__device__ __forceinline__ double donor(double mf, double mfx, double tri, double trx) {
+  const bool out = __double2hiint(mf) >= 0;
+  const double b = pos(mfx);
+  double lo = mul_rn(out ? mf : -b, out ? tri : trx);
+  if (out && __double_as_longlong(b) != 0ll) lo = fma_rn(mf, tri, -mul_rn(b, trx));
+  return lo;
+}
+
+// S+ -= min(0, a), S- += max(0, a); FP64: one addition, to the sum a's sign names
+__device__ __forceinline__ void split_sum(float a, float& sp, float& sm) {
+  sp = sp - neg(a);
+  sm = sm + pos(a);
+}
+__device__ __forceinline__ void split_sum(double a, double& sp, double& sm) {
+  const bool n = negative(a);
+  const double t = (n ? sp : sm) + fabs(a);
+  sp = n ? t : sp;
+  sm = n ? sm : t;
+}
+
+// a / b with rb = 1 / b formed once: the product and, in FP64, one residual
+// correction (Markstein), correctly rounded but for rare last-bit cases; a
+// result that is not finite is divided as written
+__device__ __forceinline__ float quot(float a, float b, float rb) { return a * rb; }
+__device__ __forceinline__ double quot(double a, double b, double rb) {
+  const double q0 = a * rb;
+  double q = fma(fma(-b, q0, a), rb, q0);
+  if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) q = a / b;
+  return q;
+}
+
+// max(0, min(1, a / b)), b > 0
+__device__ __forceinline__ float ratio01(float a, float b) { return __saturatef(__fdividef(a, b)); }
+__device__ __forceinline__ double ratio01(double a, double b) {
+  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  if (x <= 0) return 0.;
+  if (x >= y) return 1.;
+  // 0 < a < b: reciprocal by one third-order step from the hardware's
+  // approximation (e^3 < 2^-57), the quotient by one residual correction
+  if (y >= 0x7e00000000000000ll) return a / b;
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+  const double e = fma(-b, r, 1.);
+  r = fma(r, fma(e, e, e), r);
+  const double q = a * r;
+  return fma(fma(-b, q, a), r, q);
+}
 
 // asynchronous global -> shared copy of B = 4, 8 or 16 bytes (16: through L2 only)
 template <int B>
@@ -91,7 +194,8 @@ __device__ __forceinline__ int nb_at(uint2 nb, int e) {
 //       slots, then the ring edges' neighbour sides); the patch cells'
 //       low-order AB3 slots of and vof and tracer x thickness, x 2 buffers
 //       [3][SC][LK]; least-squares coefficients, 36 per patch cell (row
-//       stride 36), then 6 per ring edge.
+//       stride 36), then 6 per ring edge.  With the caller's edge values
+//       (EV) neither edge values nor coefficients are held.
 //   hi: old-tracer and trcr_lo frames [S2][LK]; the ring-1 frame's AB3 slots
 //       of and vof, S+ and S- [4][S1][LK]; R+, R- [S1][LK]; the patch cells'
 //       antidiffusive fluxes [SC][6][LK], low-order tendency and tracer x
@@ -102,16 +206,16 @@ struct PatchLayout {
   size_t TO, TL, opq, Rp, Rm, af, tlt, tdb, dpf, arf;  // hi
   size_t r_elems, tab, bytes;
   template <typename R>
-  __host__ __device__ static PatchLayout make(const FrameTab& f, int LK, bool hi) {
+  __host__ __device__ static PatchLayout make(const FrameTab& f, int LK, bool hi, bool ev = false) {
     PatchLayout p{};
     const size_t S2 = f.S2, S1 = f.S1, SC = f.SC, SE = f.SE, SR = f.SR;
     size_t o = 0;
     if (!hi) {
       p.trs = o; o += 2 * S2 * LK;
-      p.E = o; o += SE * LK;
+      p.E = o; o += ev ? 0 : SE * LK;
       p.mf = o; o += SE * LK;
       p.ops = o; o += 2 * 3 * SC * LK;
-      p.hf = o; o += SC * 36 + SR * 6;
+      p.hf = o; o += ev ? 0 : SC * 36 + SR * 6;
     } else {
       p.TO = o; o += S2 * LK;
       p.TL = o; o += S2 * LK;
@@ -163,16 +267,18 @@ __device__ __forceinline__ FrameSm load_tables(const Grid<R>& g, const FrameTab&
 }
 
 // least-squares coefficients of the patch cells (all 36) and of the ring
-// edges (the row of the edge's slot) into hf; needs the tables in place
+// edges (the row of the edge's slot), halved, into hf; needs the tables in
+// place.  The edge values are kept halved (exactly), so that the average of
+// an edge's two sides is one addition.
 template <typename R>
 __device__ __forceinline__ void load_coefs(const Grid<R>& g, const FrameSm& fs, R* hf, int C, int nre) {
   for (int q = threadIdx.x; q < C * 36; q += blockDim.x) {
     const int x = q / 36;
-    hf[q] = g.hfcoef[(size_t)fs.cells[x] * 36 + (q - x * 36)];
+    hf[q] = R(0.5) * g.hfcoef[(size_t)fs.cells[x] * 36 + (q - x * 36)];
   }
   for (int q = threadIdx.x; q < nre * 6; q += blockDim.x) {
     const int r = q / 6, code = fs.red[r];
-    hf[C * 36 + q] = g.hfcoef[(size_t)fs.cells[code >> 3] * 36 + (code & 7) * 6 + (q - r * 6)];
+    hf[C * 36 + q] = R(0.5) * g.hfcoef[(size_t)fs.cells[code >> 3] * 36 + (code & 7) * 6 + (q - r * 6)];
   }
 }
 
@@ -238,9 +344,9 @@ __device__ __forceinline__ void coef6(const R* hf, R (&h)[6]) {
   }
 }
 
-// own-side least-squares edge value of every slot ie of a patch cell
-// (k_edgvar3_own's arithmetic): val = bc + sum_e hfcoef(e, ie) (tr_e - bc),
-// d[e] = tr_e - bc (0 past nprox); hf = the cell's 36 coefficients
+// half the own-side least-squares edge value of every slot ie of a patch cell
+// (k_edgvar3_own's arithmetic, halved): val = bc + sum_e hfcoef(e, ie) (tr_e -
+// bc), d[e] = tr_e - bc (0 past nprox); hf = the cell's 36 halved coefficients
 template <typename R, int VK, int LK>
 __device__ __forceinline__ void own_values(const R* hf, int x, int v, const R (&bc)[VK], const R (&d)[6][VK],
                                            int np, R* E) {
@@ -249,17 +355,17 @@ __device__ __forceinline__ void own_values(const R* hf, int x, int v, const R (&
     R h[6];
     coef6<R>(hf + ie * 6, h);
     R val[VK];
-    FOR_V val[j] = bc[j];
+    FOR_V val[j] = mul_rn(R(0.5), bc[j]);
 #pragma unroll
     for (int e = 0; e < 6; e++) {
-      FOR_V val[j] = (e < 5 || e < np) ? val[j] + d[e][j] * h[e] : val[j];
+      FOR_V val[j] = (e < 5 || e < np) ? fma_rn(d[e][j], h[e], val[j]) : val[j];
     }
     FOR_V val[j] = (ie < 5 || ie < np) ? val[j] : R(0);
     stv<VK>(E + erow(x, ie) * LK + v, val);
   }
 }
 
-// the value on slot p of ring-1 cell y (its side of the edge it shares with a
+// half the value on slot p of ring-1 cell y (its side of the edge it shares with a
 // patch cell), into edge-value row 6C + r; hf = that slot's 6 coefficients
 template <typename R, int VK, int LK>
 __device__ __forceinline__ void ring_value(const R* T, const FrameSm& fs, const R* hf, int code, int row, int v,
@@ -270,26 +376,26 @@ __device__ __forceinline__ void ring_value(const R* T, const FrameSm& fs, const 
   R bc[VK], val[VK], h[6];
   coef6<R>(hf, h);
   ldv<VK>(T + y * LK + v, bc);
-  FOR_V val[j] = bc[j];
+  FOR_V val[j] = mul_rn(R(0.5), bc[j]);
 #pragma unroll
   for (int e = 0; e < 6; e++) {
     R d[VK];
     ldv<VK>(T + nb_at(nb, e) * LK + v, d);
     FOR_V d[j] = (e < 5 || e < np) ? d[j] - bc[j] : R(0);
-    FOR_V val[j] = (e < 5 || e < np) ? val[j] + d[j] * h[e] : val[j];
+    FOR_V val[j] = (e < 5 || e < np) ? fma_rn(d[j], h[e], val[j]) : val[j];
   }
   stv<VK>(E + row * LK + v, val);
 }
 
 // The thread's patch cell and levels (one per thread: the block has SC * GC
-// threads), with the layer thickness, which it keeps in registers for the
-// whole tracer loop.
+// threads), with the layer thickness (at least the threshold) and its
+// reciprocal, which it keeps in registers for the whole tracer loop.
 template <typename R, int VK>
 struct CellItem {
   bool on;
   int i, x, v, k, c, np;
   R rar;
-  R dp[VK];
+  R dp[VK], rdp[VK];
   template <int GC>
   __device__ __forceinline__ void load(const Grid<R>& g, const Strides& s, const FrameSm& fs, size_t m,
                                        const R* delp, int C, int k0, int lk) {
@@ -304,11 +410,20 @@ struct CellItem {
     np = fs.np[x];
     rar = g.rarea[i];
     ldv<VK>(delp + m * s.cell + c, dp);
+    FOR_V {
+      dp[j] = tmax(R(1.e-11), dp[j]);
+      rdp[j] = fdiv(R(1), dp[j]);
+    }
   }
 };
 
-// trcadv1 + the S+/S- sums of trcadv2 + copy of the old tracer, per patch
-template <typename R, int VK, int GC>
+// trcadv1 + the S+/S- sums of trcadv2 + copy of the old tracer, per patch.
+// EV: the edge values of every tracer are the caller's (trc_edg of the
+// per-routine trcadv, or edgvar1's without hi_order_flux_comp); a thread
+// loads its cell's six rows before it waits for the staged operands, and the
+// member's own tracer count does not apply.  EV = false forms them on chip
+// (theta's are edgvar1's).
+template <typename R, int VK, int GC, bool EV>
 __global__ void __launch_bounds__(64 * GC, 8 / GC) k_trf_lo(Grid<R> g, Strides s, FrameTab ft,
     const StepParams* __restrict__ sp, int t0, int nt, const R* __restrict__ massfx, const R* __restrict__ trc_edg,
     const R* __restrict__ tracr, const R* __restrict__ trcdp, R* __restrict__ trl_tdcy, const R* __restrict__ delp,
@@ -320,7 +435,7 @@ __global__ void __launch_bounds__(64 * GC, 8 / GC) k_trf_lo(Grid<R> g, Strides s
   if (!sp->active) return;
   // the member's tracers in this chunk (fim_member_set_tracers); the
   // scratch keeps the chunk's layout
-  const int ntm = min(nt, sp->ntr - t0);
+  const int ntm = EV ? nt : min(nt, sp->ntr - t0);
   if (ntm <= 0) return;
   const int L = g.L, N = g.N;
   const int nlc = (L + LK - 1) / LK;
@@ -330,7 +445,7 @@ __global__ void __launch_bounds__(64 * GC, 8 / GC) k_trf_lo(Grid<R> g, Strides s
   const int4 cn = ft.cnt[tile];
   const int C = cn.x, n1 = cn.y, n2 = cn.z, nre = cn.w;
   extern __shared__ __align__(16) unsigned char fsm[];
-  const PatchLayout lay = PatchLayout::make<R>(ft, LK, false);
+  const PatchLayout lay = PatchLayout::make<R>(ft, LK, false, EV);
   R* const sr = reinterpret_cast<R*>(fsm);
   R* const trs = sr + lay.trs;
   R* const E = sr + lay.E;
@@ -339,13 +454,12 @@ __global__ void __launch_bounds__(64 * GC, 8 / GC) k_trf_lo(Grid<R> g, Strides s
   R* const hf = sr + lay.hf;
   const FrameSm fs = load_tables<R>(g, ft, fsm, lay.tab, tile, C, n1, n2, nre);
   __syncthreads();
-  load_coefs<R>(g, fs, hf, C, nre);
+  if (!EV) load_coefs<R>(g, fs, hf, C, nre);
   const size_t NL = (size_t)N * L;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
   const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
-  const R thshld = R(1.e-11), half = R(0.5);
   const R* mfn = massfx + m * s.mf + (size_t)nf * 6 * NL;
-  const R* te0 = trc_edg + m * s.tredg;  // theta (t = 0): edgvar1's edge values
+  const R* te0 = trc_edg + m * s.tredg;  // EV: tracer t's at t * 6 NL; else theta's (edgvar1)
   // this step's tracer t: its frame, and the patch cells' AB3 slots of/vof
   // and tracer x thickness
   RowPlan<R, VK, GC> rp;
@@ -382,11 +496,19 @@ __global__ void __launch_bounds__(64 * GC, 8 / GC) k_trf_lo(Grid<R> g, Strides s
   ci.template load<GC>(g, s, fs, m, delp, C, k0, lk);
   for (int tz = 0; tz < ntm; tz++) {
     const int t = t0 + tz, b = tz & 1;
+    R ter[6][VK];  // EV: the edge values of the thread's cell, in flight over the wait
+    if constexpr (EV) {
+      if (ci.on) {
+        const R* te = te0 + (size_t)t * 6 * NL;
+#pragma unroll
+        for (int e = 0; e < 6; e++) ldv<VK>(te + (ci.i * 6 + e) * L + ci.k, ter[e]);
+      }
+    }
     stage_wait();
     __syncthreads();
     if (tz + 1 < ntm) stage(t + 1, b ^ 1);
     const R* T = trs + b * ft.S2 * LK;
-    if (t != 0) {
+    if (!EV && t != 0) {
       // edge values: the six of the thread's patch cell, then the ring cells'
       // sides of the patch's boundary edges
       if (ci.on) {
@@ -409,21 +531,28 @@ __global__ void __launch_bounds__(64 * GC, 8 / GC) k_trf_lo(Grid<R> g, Strides s
     if (!ci.on) continue;
     const int x = ci.x, v = ci.v, i = ci.i, c = ci.c;
     const uint2 nb = fs.nbr[x];
-    R tri[VK], sumlo[VK], sp_[VK], sm_[VK], mx[VK], mn[VK];
+    R tri[VK], sumlo[VK], sp_[VK], sm_[VK];
+    Bound<R> mx[VK], mn[VK];
     ldv<VK>(T + x * LK + v, tri);
-    FOR_V { sumlo[j] = R(0); sp_[j] = R(0); sm_[j] = R(0); mx[j] = tri[j]; mn[j] = tri[j]; }
+    FOR_V { sumlo[j] = R(0); sp_[j] = R(0); sm_[j] = R(0); mx[j] = mn[j] = Bound<R>::of(tri[j]); }
 #pragma unroll
     for (int e = 0; e < 6; e++) {
       R trx[VK];
       ldv<VK>(T + nb_at(nb, e) * LK + v, trx);
-      FOR_V { mx[j] = tmax(mx[j], trx[j]); mn[j] = tmin(mn[j], trx[j]); }
+      FOR_V {
+        const Bound<R> bx = Bound<R>::of(trx[j]);
+        mx[j].up(bx);
+        mn[j].down(bx);
+      }
       if (e < 5 || e < ci.np) {
         R tev[VK];
-        if (t != 0) {
+        if constexpr (EV) {
+          FOR_V tev[j] = ter[e][j];
+        } else if (t != 0) {
           R tem[VK];
           ldv<VK>(E + erow(x, e) * LK + v, tev);
           ldv<VK>(E + fs.mir[x * 6 + e] * LK + v, tem);
-          FOR_V tev[j] = half * (tev[j] + tem[j]);
+          FOR_V tev[j] = tev[j] + tem[j];
         } else {
           ldv<VK>(te0 + (i * 6 + e) * L + ci.k, tev);
         }
@@ -432,13 +561,10 @@ __global__ void __launch_bounds__(64 * GC, 8 / GC) k_trf_lo(Grid<R> g, Strides s
         ldv<VK>(MF + erow(x, e) * LK + v, mfo);
         ldv<VK>(MF + fs.mir[x * 6 + e] * LK + v, mfm);
         FOR_V {
-          const R mf = mfo[j], mfx = mfm[j];
-          const R hi = mf * tev[j];
-          const R lo = half * ((mf + tabs(mf)) * tri[j] - (mfx + tabs(mfx)) * trx[j]);
-          anti[j] = hi - lo;
+          const R lo = donor(mfo[j], mfm[j], tri[j], trx[j]);
+          anti[j] = fma_rn(mfo[j], tev[j], -lo);
           sumlo[j] = sumlo[j] + lo;
-          sp_[j] = sp_[j] - tmin(R(0), anti[j]);
-          sm_[j] = sm_[j] + tmax(R(0), anti[j]);
+          split_sum(anti[j], sp_[j], sm_[j]);
         }
         stv<VK>(antifx + (m * nt + tz) * 6 * sc + (size_t)(i * 6 + e) * L + ci.k, anti);
       }
@@ -453,8 +579,8 @@ __global__ void __launch_bounds__(64 * GC, 8 / GC) k_trf_lo(Grid<R> g, Strides s
     const size_t q = (m * nt + tz) * sc + c;
     FOR_V {
       const R lo = td[j] + ab1 * tn[j] + ab2 * tlo[j] + ab3 * tlv[j];
-      const R hx = tmax(R(0), mx[j]), hn = tmax(R(0), mn[j]);
-      out[j] = tmax(hn, tmin(hx, fdiv(lo, tmax(thshld, ci.dp[j]))));
+      const R hx = mx[j].at_least_zero(), hn = mn[j].at_least_zero();
+      out[j] = tmax(hn, tmin(hx, quot(lo, ci.dp[j], ci.rdp[j])));
     }
     stv<VK>(trcr_lo + q, out);
     stv<VK>(s_plus + q, sp_);
@@ -474,27 +600,36 @@ struct TrOut {
   int tbase;
 };
 
-// R+/R- of trcadv2 (k_trcadv2's arithmetic) for frame cell xe at levels ve,
-// from the staged old tracer and trcr_lo, AB3 slots, S+/S- and thickness; the
-// bounds (before the clamp at zero) and the slots of/vof are returned for
-// trcadv3
+// R+/R- of trcadv2 for frame cell xe at levels ve, from the staged old tracer
+// and trcr_lo, AB3 slots, S+/S- and thickness (arf = area / ab1); the bounds
+// (clamped at zero) and the slots of/vof are returned for trcadv3
 template <typename R, int VK, int LK>
 __device__ __forceinline__ void limiters(const FrameSm& fs, const R* TO, const R* TL, const R* opq, const R* dpf,
-                                         const R* arf, int S1, int xe, int ve, R ab2, R ab3, R rab1,
-                                         R* Rp, R* Rm, R (&mx)[VK], R (&mn)[VK], R (&tof)[VK], R (&tvf)[VK]) {
+                                         const R* arf, int S1, int xe, int ve, R ab2, R ab3,
+                                         R* Rp, R* Rm, R (&hx)[VK], R (&hn)[VK], R (&tof)[VK], R (&tvf)[VK]) {
   const R thshld = R(1.e-11);
   const uint2 nb = fs.nbr[xe];
   const int o = xe * LK + ve;
   R lc[VK], tc0[VK];
+  Bound<R> mx[VK], mn[VK];
   ldv<VK>(TL + o, lc);
   ldv<VK>(TO + o, tc0);
-  FOR_V { mx[j] = tmax(tc0[j], lc[j]); mn[j] = tmin(tc0[j], lc[j]); }
+  FOR_V {
+    mx[j] = mn[j] = Bound<R>::of(lc[j]);
+    const Bound<R> b = Bound<R>::of(tc0[j]);
+    mx[j].up(b);
+    mn[j].down(b);
+  }
 #pragma unroll
   for (int e = 0; e < 6; e++) {
     R aa[VK], bb[VK];
     ldv<VK>(TO + nb_at(nb, e) * LK + ve, aa);
     ldv<VK>(TL + nb_at(nb, e) * LK + ve, bb);
-    FOR_V { mx[j] = tmax3(mx[j], aa[j], bb[j]); mn[j] = tmin3(mn[j], aa[j], bb[j]); }
+    FOR_V {
+      const Bound<R> a = Bound<R>::of(aa[j]), b = Bound<R>::of(bb[j]);
+      mx[j].up(a, b);
+      mn[j].down(a, b);
+    }
   }
   R dp[VK], spl[VK], smn[VK], rp[VK], rm[VK];
   ldv<VK>(opq + o, tof);
@@ -504,11 +639,12 @@ __device__ __forceinline__ void limiters(const FrameSm& fs, const R* TO, const R
   ldv<VK>(dpf + o, dp);
   const R ar = arf[xe];
   FOR_V {
-    const R hx = tmax(R(0), mx[j]), hn = tmax(R(0), mn[j]);
-    const R q_plus = ((hx - lc[j]) * dp[j] - (ab2 * tmin(R(0), tof[j]) + ab3 * tmax(R(0), tvf[j]))) * rab1 * ar;
-    const R q_mnus = ((lc[j] - hn) * dp[j] + (ab2 * tmax(R(0), tof[j]) + ab3 * tmin(R(0), tvf[j]))) * rab1 * ar;
-    rp[j] = tmax(R(0), tmin(R(1), fdiv(q_plus, tmax(spl[j], thshld))));
-    rm[j] = tmax(R(0), tmin(R(1), fdiv(q_mnus, tmax(smn[j], thshld))));
+    hx[j] = mx[j].at_least_zero();
+    hn[j] = mn[j].at_least_zero();
+    const R q_plus = ((hx[j] - lc[j]) * dp[j] - (ab2 * neg(tof[j]) + ab3 * pos(tvf[j]))) * ar;
+    const R q_mnus = ((lc[j] - hn[j]) * dp[j] + (ab2 * pos(tof[j]) + ab3 * neg(tvf[j]))) * ar;
+    rp[j] = ratio01(q_plus, floor_at(spl[j], thshld));
+    rm[j] = ratio01(q_mnus, floor_at(smn[j], thshld));
   }
   stv<VK>(Rp + o, rp);
   stv<VK>(Rm + o, rm);
@@ -528,7 +664,8 @@ __global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameT
     const StepParams* __restrict__ sp, int t0, int nt, const R* __restrict__ trl_tdcy, const R* trcdp,
     R* __restrict__ trc_tdcy, const R* __restrict__ delp, const R* __restrict__ trold,
     const R* __restrict__ trcr_lo, const R* __restrict__ s_plus, const R* __restrict__ s_mnus,
-    const R* __restrict__ antifx, TrOut<R> out, size_t sc) {
+    const R* __restrict__ antifx, TrOut<R> out, size_t sc, int all) {
+  // all: every tracer of the chunk, whatever the member's own count
   // trcdp (read) and out.trdp (written) are the same array in the step
   constexpr int LK = VK * GC;
   const size_t m = blockIdx.y;
@@ -536,7 +673,7 @@ __global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameT
   if (!sp->active) return;
   // the member's tracers in this chunk (fim_member_set_tracers); the
   // scratch keeps the chunk's layout
-  const int ntm = min(nt, sp->ntr - t0);
+  const int ntm = all ? nt : min(nt, sp->ntr - t0);
   if (ntm <= 0) return;
   const int L = g.L, N = g.N;
   const int nlc = (L + LK - 1) / LK;
@@ -560,12 +697,11 @@ __global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameT
   R* const arf = sr + lay.arf;
   const FrameSm fs = load_tables<R>(g, ft, fsm, lay.tab, tile, C, n1, n2, nre);
   __syncthreads();
-  for (int x = threadIdx.x; x < n1; x += blockDim.x) arf[x] = g.area[fs.cells[x]];
   const size_t NL = (size_t)N * L;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
   const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
-  const R rab1 = R(1) / ab1;  // Q+/Q- divide by ab1: one reciprocal (as k_trcadv2)
-  const R thshld = R(1.e-11);
+  const R rab1 = R(1) / ab1;  // Q+/Q- divide by ab1: one factor a cell
+  for (int x = threadIdx.x; x < n1; x += blockDim.x) arf[x] = g.area[fs.cells[x]] * rab1;
   // the limiters' operands of tracer t0 + tz
   RowPlan<R, VK, GC> rp;
   rp.init(fs, ft.SC, n2, lk, L);
@@ -600,6 +736,18 @@ __global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameT
   stage_lim(0);
   const int x = threadIdx.x / GC, v = (threadIdx.x - x * GC) * VK;
   const bool on = x < C && v < lk;
+  // FP64: the thickness (at least the threshold) and its reciprocal, once a
+  // block (FP32 has no registers left and divides in three instructions)
+  R dpk[VK], rdp[VK];
+  if constexpr (sizeof(R) == 8) {
+    if (on) {
+      ldv<VK>(delp + m * s.cell + (size_t)fs.cells[x] * L + k0 + v, dpk);
+      FOR_V {
+        dpk[j] = tmax(R(1.e-11), dpk[j]);
+        rdp[j] = R(1) / dpk[j];
+      }
+    }
+  }
   for (int tz = 0; tz < ntm; tz++) {
     const int t = t0 + tz;
     stage_wait();
@@ -607,13 +755,13 @@ __global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameT
     stage_clip(tz);
     // R+/R- of the thread's patch cell (its bounds and slots kept for
     // trcadv3), then of the ring-1 cells
-    R mx[VK], mn[VK], tof[VK], tvf[VK];
-    if (on) limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, x, v, ab2, ab3, rab1, Rp, Rm, mx, mn, tof, tvf);
+    R hx[VK], hn[VK], tof[VK], tvf[VK];
+    if (on) limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, x, v, ab2, ab3, Rp, Rm, hx, hn, tof, tvf);
     for (int it = threadIdx.x; it < (n1 - C) * GC; it += blockDim.x) {
       const int xe = C + it / GC, ve = (it % GC) * VK;
       if (ve >= lk) continue;
       R mx2[VK], mn2[VK], tof2[VK], tvf2[VK];
-      limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, xe, ve, ab2, ab3, rab1, Rp, Rm, mx2, mn2, tof2, tvf2);
+      limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, xe, ve, ab2, ab3, Rp, Rm, mx2, mn2, tof2, tvf2);
     }
     stage_wait();
     __syncthreads();
@@ -636,10 +784,8 @@ __global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameT
         ldv<VK>(Rp + y * LK + v, rpx);
         ldv<VK>(Rm + y * LK + v, rmx);
         FOR_V {
-          R aa = a[j];
-          if (aa >= R(0)) aa = aa * tmin(rmc[j], rpx[j]);
-          else aa = aa * tmin(rpc[j], rmx[j]);
-          at[j] = at[j] + aa;
+          const bool in = negative(a[j]);
+          at[j] = fma_rn(a[j], min0(in ? rpc[j] : rmc[j], in ? rmx[j] : rpx[j]), at[j]);
         }
       }
     }
@@ -654,15 +800,15 @@ __global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameT
     const size_t ob = m * out.mstride + (size_t)(t - out.tbase) * NL + c;
     FOR_V {
       tdv[j] = tdv[j] + ab1 * tn[j] + ab2 * tof[j] + ab3 * tvf[j];
-      const R hx = tmax(R(0), mx[j]), hn = tmax(R(0), mn[j]);
-      res[j] = tmax(hn, tmin(hx, fdiv(tdv[j], tmax(thshld, dp[j]))));
+      const R q = sizeof(R) == 8 ? quot(tdv[j], dpk[j], rdp[j]) : fdiv(tdv[j], tmax(R(1.e-11), dp[j]));
+      res[j] = tmax(hn[j], tmin(hx[j], q));
     }
     stv<VK>(out.trdp + ob, tdv);
     stv<VK>(out.tr + ob, res);
   }
 }
 
-template <typename R, int VK, int GC>
+template <typename R, int VK, int GC, bool EV>
 void trf_chunks(const Launch& l, const Grid<R>& g, const Strides& s, const TrcFusedScratch<R>& w, R* trc_edg,
                 R* tracr, R* trcdp, R* trc_tdcy, R* trl_tdcy, const R* massfx, const R* delp, bool probe,
                 const ChunkHook* hook) {
@@ -670,22 +816,24 @@ void trf_chunks(const Launch& l, const Grid<R>& g, const Strides& s, const TrcFu
   const FrameTab& ft = w.ft;
   const size_t sc = (size_t)g.N * g.L;
   const int nlc = (g.L + LK - 1) / LK;
-  const size_t sm_lo = PatchLayout::make<R>(ft, LK, false).bytes, sm_hi = PatchLayout::make<R>(ft, LK, true).bytes;
+  const size_t sm_lo = PatchLayout::make<R>(ft, LK, false, EV).bytes,
+               sm_hi = PatchLayout::make<R>(ft, LK, true).bytes;
   dim3 grid((unsigned)(ft.ntile * nlc), l.members);
   const int tb = ft.SC * GC;
   for (int t0 = 0; t0 < g.T; t0 += w.tchunk) {
     const int nt = (g.T - t0 < w.tchunk) ? g.T - t0 : w.tchunk;
     if (hook && hook->fn) hook->fn(hook->arg, 0, t0, nt);
     FIM_KBEGIN(l, "k_trf_lo");
-    k_trf_lo<R, VK, GC><<<grid, tb, sm_lo, l.stream>>>(g, s, ft, l.sp, t0, nt, massfx, trc_edg, tracr, trcdp,
-                                                        trl_tdcy, delp, w.trcr_lo, w.s_plus, w.s_mnus, w.trold,
-                                                        w.antifx, sc);
+    k_trf_lo<R, VK, GC, EV><<<grid, tb, sm_lo, l.stream>>>(g, s, ft, l.sp, t0, nt, massfx, trc_edg, tracr, trcdp,
+                                                            trl_tdcy, delp, w.trcr_lo, w.s_plus, w.s_mnus, w.trold,
+                                                            w.antifx, sc);
     FIM_KEND(l);
     // the probe sends the new tracer and tracer x thickness to scratch
     const TrOut<R> out = probe ? TrOut<R>{w.r_plus, w.r_mnus, (size_t)nt * sc, t0} : TrOut<R>{trcdp, tracr, s.tr, 0};
     FIM_KBEGIN(l, "k_trf_hi");
     k_trf_hi<R, VK, GC><<<grid, tb, sm_hi, l.stream>>>(g, s, ft, l.sp, t0, nt, trl_tdcy, trcdp, trc_tdcy, delp,
-                                                        w.trold, w.trcr_lo, w.s_plus, w.s_mnus, w.antifx, out, sc);
+                                                        w.trold, w.trcr_lo, w.s_plus, w.s_mnus, w.antifx, out, sc,
+                                                        EV ? 1 : 0);
     FIM_KEND(l);
     if (probe) return;  // the first chunk only
     if (hook && hook->fn) hook->fn(hook->arg, 1, t0, nt);
@@ -709,8 +857,12 @@ void fused_dispatch(const Launch& l, const Grid<R>& g, const Strides& s, const T
   const bool g4 = w.gc >= 4;
 #define FIM_TRF(VKV)                                                                                            \
   do {                                                                                                          \
-    if (g4) trf_chunks<R, VKV, 4>(l, g, s, w, trc_edg, tracr, trcdp, trc_tdcy, trl_tdcy, massfx, delp, probe, hook); \
-    else trf_chunks<R, VKV, 2>(l, g, s, w, trc_edg, tracr, trcdp, trc_tdcy, trl_tdcy, massfx, delp, probe, hook);    \
+    if (w.edges)                                                                                                \
+      trf_chunks<R, VKV, 4, true>(l, g, s, w, trc_edg, tracr, trcdp, trc_tdcy, trl_tdcy, massfx, delp, probe, hook);  \
+    else if (g4)                                                                                                \
+      trf_chunks<R, VKV, 4, false>(l, g, s, w, trc_edg, tracr, trcdp, trc_tdcy, trl_tdcy, massfx, delp, probe, hook); \
+    else                                                                                                        \
+      trf_chunks<R, VKV, 2, false>(l, g, s, w, trc_edg, tracr, trcdp, trc_tdcy, trl_tdcy, massfx, delp, probe, hook); \
   } while (0)
   if (vk == 4) FIM_TRF((sizeof(R) == 4 ? 4 : 2));
   else if (vk == 2) FIM_TRF(2);
@@ -722,7 +874,13 @@ template <typename R, int VK, int GC>
 int prepare_one(const FrameTab& ft) {
   constexpr int LK = VK * GC;
   const size_t lo = PatchLayout::make<R>(ft, LK, false).bytes, hi = PatchLayout::make<R>(ft, LK, true).bytes;
-  cudaError_t e = cudaFuncSetAttribute(k_trf_lo<R, VK, GC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lo);
+  cudaError_t e =
+      cudaFuncSetAttribute(k_trf_lo<R, VK, GC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lo);
+  if constexpr (GC == 4) {
+    const size_t ev = PatchLayout::make<R>(ft, LK, false, true).bytes;
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_trf_lo<R, VK, GC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ev);
+  }
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_trf_hi<R, VK, GC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hi);
   return (int)e;
