@@ -597,7 +597,7 @@ int edgvar_impl(fim_ctx* c, int which, const R* u_vel, const R* v_vel, const R* 
     s.bufs.push_back(w);
     launch_edgvar2<R>(l, g, c->str, du, dv, due, dve, dqe, w);
   } else {
-    launch_edgvar3<R>(l, g, c->str, ddp, dtr, dde, dte, c->kn.hi_order ? c->T : 1);
+    launch_edgvar3<R>(l, g, c->str, ddp, dtr, dde, dte, c->kn.hi_order ? c->T : 1, c->ftab);
   }
   if ((rc = check_launch(c, which == 1 ? "edgvar1" : which == 2 ? "edgvar2" : "edgvar3"))) return rc;
   return s.finish();
@@ -1155,7 +1155,7 @@ int enqueue_step(fim_ctx* c, fim_state* st, StepIo* io = nullptr) {
       // the pass.  The tracers' edge values are formed on chip by the tracer
       // kernels
       launch_edgvar3<R>(lg, g, s, P(FIM_DP3D), P(FIM_TR3D), P(FIM_DP_EDG), P(FIM_TRC_EDG),
-                        1, c->cfg.flux_conserv_schm != 1);
+                        1, c->ftab, c->cfg.flux_conserv_schm != 1);
     }
     CnuityScratch<R> cw{(R*)c->antifx, (R*)c->delp_lo, (R*)c->p_plus, (R*)c->p_mnus, (R*)c->r_plus, (R*)c->r_mnus};
     if (io && (rc = io_wait(*io, io->up_ev[kIoC]))) return rc;
@@ -1519,7 +1519,8 @@ int fim_ctx_create(const fim_grid_desc* g, const fim_config* cfg, fim_ctx** out)
   int rc = build_grid<double>(c, g, rarea, corio, grnd, dfflen, biharw, smoo, prox, proxs, nprox);
   if (!rc && c->prec == FIM_PREC_F32)
     rc = build_grid<float>(c, g, rarea, corio, grnd, dfflen, biharw, smoo, prox, proxs, nprox);
-  if (!rc && c->kn.hi_order) rc = build_patches(c, prox, proxs, nprox);
+  if (!rc) rc = build_patches(c, prox, proxs, nprox);
+  if (!rc && c->prec == FIM_PREC_F32 && prepare_edges<float>(c->ftab)) rc = FIM_ECUDA;
   if (!rc) rc = dalloc(c, (void**)&c->d_sp, sizeof(StepParams) * c->M);
   if (!rc) rc = dalloc(c, (void**)&c->d_flags, sizeof(int) * c->M);
   if (!rc) {

@@ -31,15 +31,30 @@ __device__ __forceinline__ bool cell_level(int N, int L, int& i, int& k) {
 
 inline unsigned blocks_for(long long n, int b = kBlock) { return (unsigned)((n + b - 1) / b); }
 
-// |(a, b)|: IEEE sqrt in FP64; in the FP32-mixed build x * rsqrt(x), a few
-// ulp from the rounded root and about a third of its instructions (edgvar1
-// forms 30 magnitudes a level)
-template <typename R>
-__device__ __forceinline__ R vmag(R a, R b) { return sqrt(a * a + b * b); }
-template <>
-__device__ __forceinline__ float vmag<float>(float a, float b) {
+// 1 / sqrt(x) of a squared speed.  FP64 (2 lanes a clock and SM on GB300, so
+// operations count): one third-order step r (1 + e/2 + 3 e^2/8), e = 1 - x r^2,
+// from the hardware's approximation, whose error cubed is below rounding.
+__device__ __forceinline__ float inv_root(float x) { return rsqrtf(x); }
+__device__ __forceinline__ double inv_root(double x) {
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-(x * r), r, 1.);
+  return fma(r, e * fma(.375, e, .5), r);
+}
+
+// |(a, b)|: IEEE sqrt in FP64; x * rsqrt(x) in FP32, a few ulp from the
+// rounded root and about a third of its instructions
+__device__ __forceinline__ double vmag(double a, double b) { return sqrt(a * a + b * b); }
+__device__ __forceinline__ float vmag(float a, float b) {
   const float x = a * a + b * b;
   return x > 0.f ? x * rsqrtf(x) : 0.f;
+}
+
+// four table entries of an edge (cs or sn): 16-byte loads
+__device__ __forceinline__ void ld4(const float* p, float (&r)[4]) { ldv<4>(p, r); }
+__device__ __forceinline__ void ld4(const double* p, double (&r)[4]) {
+  const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
+  r[0] = a.x; r[1] = a.y; r[2] = b.x; r[3] = b.y;
 }
 
 // --------------------------------------------------------------------------
@@ -48,8 +63,46 @@ __device__ __forceinline__ float vmag<float>(float a, float b) {
 // into the edge frame, equal-weight interpolate with magnitude correction;
 // mid-layer pressure, Montgomery potential, kinetic energy and tracer 1 (all
 // tracers and dp when hi_order == 0) on the cell's own edges.
+//
+// A thread loads each of its cell's six neighbours once and keeps what the
+// three edges that see it share: the wind, the float-float difference of the
+// Montgomery potential, theta; in FP64, where operations bound the kernel,
+// also the wind's magnitude (a rotation keeps it; the FP32 build forms it from
+// the rotated components, because the thickness tendencies, differences of
+// large fluxes, show the last bit of the edge winds).  FP64 folds the edge
+// wind's common factors: with U, V six times the interpolated components and
+// M the interpolated magnitude, u m_2 / max(eps, m_1) = U M / sqrt(U^2 + V^2).
+// The winds and the scalars are formed one after the other, so their operands
+// share registers: 64 a thread, four blocks an SM (three: 1.53 ms, five,
+// spilling: 1.88 ms).  At glvl 8 / nvl 64 in FP32 1.41 ms, 4,880 GB/s of its
+// 41 words, where loading each neighbour for each of its edges took 1.98 ms;
+// glvl 6 in FP64 3.08 -> 1.81 ms.
+#define FIM_TRAIL(x) (e == 0 ? (five ? x[4][j] : x[5][j]) : x[e == 0 ? 0 : e - 1][j])
+#define FIM_LEAD(x) (e == 5 ? x[0][j] : e == 4 ? (five ? x[0][j] : x[5][j]) : x[e == 5 ? 0 : e + 1][j])
+// (2 (a + b) + c + d) / 6 on the live edges of a cell: x0 the cell's value, x
+// its neighbours'; written to rows of o
 template <typename R, int VK>
-__global__ void __launch_bounds__(kBlock) k_edgvar1(Grid<R> g, Strides s, int hi_order,
+__device__ __forceinline__ void edge_means(bool five, int L, const R (&x0)[VK], const R (&x)[6][VK], R* o) {
+  const R divby6 = R(1) / R(6), two = R(2);
+#pragma unroll
+  for (int e = 0; e < 6; e++) {
+    if (e == 5 && five) continue;
+    R out[VK];
+    FOR_V out[j] = (two * (x0[j] + x[e][j]) + FIM_TRAIL(x) + FIM_LEAD(x)) * divby6;
+    stv<VK>(o + (size_t)e * L, out);
+  }
+}
+// a cell field's values at the cell and its six prox slots (all valid cells)
+template <typename R, int VK>
+__device__ __forceinline__ void around(const R* f, int L, int i, int k, const int (&nb)[6], R (&x0)[VK],
+                                       R (&x)[6][VK]) {
+  ldv<VK>(f + (size_t)i * L + k, x0);
+#pragma unroll
+  for (int e = 0; e < 6; e++) ldv<VK>(f + (size_t)nb[e] * L + k, x[e]);
+}
+
+template <typename R, int VK>
+__global__ void __launch_bounds__(kBlock, 4) k_edgvar1(Grid<R> g, Strides s, int hi_order,
     const R* __restrict__ u, const R* __restrict__ v, const R* __restrict__ delp,
     const R* __restrict__ pres, const R* __restrict__ montg, const R* __restrict__ tracr,
     R* __restrict__ u_edg, R* __restrict__ v_edg, R* __restrict__ dp_edg, R* __restrict__ lp_edg,
@@ -59,112 +112,136 @@ __global__ void __launch_bounds__(kBlock) k_edgvar1(Grid<R> g, Strides s, int hi
   if (!cell_levels<VK>(g.N, g.L, i, k)) return;
   const int L = g.L, N = g.N, L1 = L + 1;
   const size_t m = blockIdx.y;
-  if (mpf) mpf += m * s.cell;
   const size_t c = (size_t)i * L + k;
-  if (thold) {
-    // the potential temperature of this step's edge values, for momtum1
-    R th[VK];
-    ldv<VK>(tracr + m * s.tr + c, th);
-    stv<VK>(thold + m * s.cell + c, th);
+  const bool five = g.nprox[i] < 6;
+  int nb[6];
+#pragma unroll
+  for (int e = 0; e < 6; e++) nb[e] = g.prox[i * 6 + e];
+  const size_t oe = (size_t)i * 6 * L + k;
+  // the wind
+  {
+    R u0[VK], v0[VK], ux[6][VK], vx[6][VK];
+    around<R, VK>(u + m * s.cell, L, i, k, nb, u0, ux);
+    around<R, VK>(v + m * s.cell, L, i, k, nb, v0, vx);
+    R m0[VK], mx[6][VK];
+    if constexpr (sizeof(R) == 8) {
+      FOR_V {
+        m0[j] = vmag(u0[j], v0[j]);
+#pragma unroll
+        for (int e = 0; e < 6; e++) mx[e][j] = vmag(ux[e][j], vx[e][j]);
+      }
+    }
+    const R divby6 = R(1) / R(6), eps = R(0.001), two = R(2), half = R(0.5);
+    R* pu = u_edg + m * s.edge + oe;
+    R* pv = v_edg + m * s.edge + oe;
+    R* pq = uvsq_edg + m * s.edge + oe;
+#pragma unroll
+    for (int e = 0; e < 6; e++) {
+      if (e == 5 && five) continue;
+      R cs[4], sn[4];
+      ld4(g.cs + (i * 6 + e) * 4, cs);
+      ld4(g.sn + (i * 6 + e) * 4, sn);
+      R ue[VK], ve[VK], uv[VK];
+      FOR_V {
+        const R ut = FIM_TRAIL(ux), vt = FIM_TRAIL(vx), ul = FIM_LEAD(ux), vl = FIM_LEAD(vx);
+        if constexpr (sizeof(R) == 8) {
+          R un = cs[0] * u0[j] + sn[0] * v0[j] + cs[1] * ux[e][j] + sn[1] * vx[e][j];
+          R vn = cs[0] * v0[j] - sn[0] * u0[j] + cs[1] * vx[e][j] - sn[1] * ux[e][j];
+          un = two * un + cs[2] * ut + sn[2] * vt + cs[3] * ul + sn[3] * vl;
+          vn = two * vn + cs[2] * vt - sn[2] * ut + cs[3] * vl - sn[3] * ul;
+          const R sq = un * un + vn * vn;
+          const R ms = (two * (m0[j] + mx[e][j]) + FIM_TRAIL(mx) + FIM_LEAD(mx)) * divby6;
+          const R q = sq > R(36) * eps * eps ? ms * inv_root(sq) : ms * (R(1) / (R(6) * eps));
+          ue[j] = un * q;
+          ve[j] = vn * q;
+        } else {
+          const R u3trl = cs[2] * ut + sn[2] * vt, v3trl = -sn[2] * ut + cs[2] * vt;
+          const R u1ldg = cs[0] * u0[j] + sn[0] * v0[j], v1ldg = -sn[0] * u0[j] + cs[0] * v0[j];
+          const R u2ldg = cs[1] * ux[e][j] + sn[1] * vx[e][j], v2ldg = -sn[1] * ux[e][j] + cs[1] * vx[e][j];
+          const R u3ldg = cs[3] * ul + sn[3] * vl, v3ldg = -sn[3] * ul + cs[3] * vl;
+          const R uu = (two * (u1ldg + u2ldg) + u3trl + u3ldg) * divby6;
+          const R vv = (two * (v1ldg + v2ldg) + v3trl + v3ldg) * divby6;
+          const R m_1 = vmag(uu, vv);
+          const R m_2 = (two * (vmag(u1ldg, v1ldg) + vmag(u2ldg, v2ldg)) + vmag(u3trl, v3trl) + vmag(u3ldg, v3ldg)) *
+                        divby6;
+          const R q = fdiv(m_2, rmax(eps, m_1));  // one division for both components
+          ue[j] = uu * q;
+          ve[j] = vv * q;
+        }
+        uv[j] = half * (ue[j] * ue[j] + ve[j] * ve[j]);
+      }
+      stv<VK>(pu + (size_t)e * L, ue);
+      stv<VK>(pv + (size_t)e * L, ve);
+      stv<VK>(pq + (size_t)e * L, uv);
+    }
   }
-  u += m * s.cell; v += m * s.cell; delp += m * s.cell; pres += m * s.intf;
-  montg += m * s.cell; tracr += m * s.tr;
-  u_edg += m * s.edge; v_edg += m * s.edge; dp_edg += m * s.edge; lp_edg += m * s.edge;
-  mont_edg += m * s.edge; uvsq_edg += m * s.edge; trc_edg += m * s.tredg;
-  const R divby6 = R(1) / R(6), eps = R(0.001), two = R(2), half = R(0.5);
-  const int np = g.nprox[i];
-  const int* pr = g.prox + i * 6;
-  R u1[VK], v1[VK], p1a[VK], p1b[VK], m1[VK];
-  ldv<VK>(u + c, u1);
-  ldv<VK>(v + c, v1);
-  ldv<VK>(montg + c, m1);
-  FOR_V { p1a[j] = pres[(size_t)i * L1 + k + j]; p1b[j] = pres[(size_t)i * L1 + k + j + 1]; }
-  for (int e = 0; e < np; e++) {
-    const int i2 = pr[e], i3t = pr[e == 0 ? np - 1 : e - 1], i3l = pr[e == np - 1 ? 0 : e + 1];
-    const R* cs = g.cs + (i * 6 + e) * 4;
-    const R* sn = g.sn + (i * 6 + e) * 4;
-    R ut[VK], vt[VK], u2[VK], v2[VK], ul[VK], vl[VK];
-    ldv<VK>(u + (size_t)i3t * L + k, ut);
-    ldv<VK>(v + (size_t)i3t * L + k, vt);
-    ldv<VK>(u + (size_t)i2 * L + k, u2);
-    ldv<VK>(v + (size_t)i2 * L + k, v2);
-    ldv<VK>(u + (size_t)i3l * L + k, ul);
-    ldv<VK>(v + (size_t)i3l * L + k, vl);
-    R ue[VK], ve[VK], lp[VK], mo[VK], uv[VK];
-    FOR_V {
-      const R u3trl = cs[2] * ut[j] + sn[2] * vt[j], v3trl = -sn[2] * ut[j] + cs[2] * vt[j];
-      const R u1ldg = cs[0] * u1[j] + sn[0] * v1[j], v1ldg = -sn[0] * u1[j] + cs[0] * v1[j];
-      const R u2ldg = cs[1] * u2[j] + sn[1] * v2[j], v2ldg = -sn[1] * u2[j] + cs[1] * v2[j];
-      const R u3ldg = cs[3] * ul[j] + sn[3] * vl[j], v3ldg = -sn[3] * ul[j] + cs[3] * vl[j];
-      R uu = (two * (u1ldg + u2ldg) + u3trl + u3ldg) * divby6;
-      R vv = (two * (v1ldg + v2ldg) + v3trl + v3ldg) * divby6;
-      const R m_1ldg = vmag(u1ldg, v1ldg);
-      const R m_2ldg = vmag(u2ldg, v2ldg);
-      const R m_3trl = vmag(u3trl, v3trl);
-      const R m_3ldg = vmag(u3ldg, v3ldg);
-      const R m_1 = vmag(uu, vv);
-      const R m_2 = (two * (m_1ldg + m_2ldg) + m_3trl + m_3ldg) * divby6;
-      const R q = fdiv(m_2, rmax(eps, m_1));  // one division for both components
-      uu = uu * q;
-      vv = vv * q;
-      ue[j] = uu;
-      ve[j] = vv;
-      uv[j] = half * (uu * uu + vv * vv);
-      const size_t kk = (size_t)k + j;
-      lp[j] = (p1a[j] + p1b[j] + pres[(size_t)i2 * L1 + kk] + pres[(size_t)i2 * L1 + kk + 1] +
-               half * (pres[(size_t)i3t * L1 + kk] + pres[(size_t)i3t * L1 + kk + 1] +
-                       pres[(size_t)i3l * L1 + kk] + pres[(size_t)i3l * L1 + kk + 1])) * divby6;
+  // mid-layer pressure
+  {
+    const R divby6 = R(1) / R(6), half = R(0.5);
+    const R* pm = pres + m * s.intf;
+    R p0[VK], pa[6][VK], pb[6][VK];
+    FOR_V p0[j] = pm[(size_t)i * L1 + k + j] + pm[(size_t)i * L1 + k + j + 1];
+#pragma unroll
+    for (int e = 0; e < 6; e++) {
+      const R* pe = pm + (size_t)nb[e] * L1 + k;
+      R a = pe[0];
+      FOR_V {
+        const R b = pe[j + 1];
+        pa[e][j] = a;
+        pb[e][j] = b;
+        a = b;
+      }
     }
-    const size_t o = ((size_t)i * 6 + e) * L + k;
-    stv<VK>(u_edg + o, ue);
-    stv<VK>(v_edg + o, ve);
-    stv<VK>(lp_edg + o, lp);
-    stv<VK>(uvsq_edg + o, uv);
-    if (!hi_order) {
-      R d1[VK], d2[VK], dt[VK], dl[VK], de[VK];
-      ldv<VK>(delp + c, d1);
-      ldv<VK>(delp + (size_t)i2 * L + k, d2);
-      ldv<VK>(delp + (size_t)i3t * L + k, dt);
-      ldv<VK>(delp + (size_t)i3l * L + k, dl);
-      FOR_V de[j] = (two * (d1[j] + d2[j]) + dt[j] + dl[j]) * divby6;
-      stv<VK>(dp_edg + o, de);
+    R* o = lp_edg + m * s.edge + oe;
+#pragma unroll
+    for (int e = 0; e < 6; e++) {
+      if (e == 5 && five) continue;
+      R lp[VK];
+      FOR_V lp[j] = (p0[j] + pa[e][j] + pb[e][j] + half * (FIM_TRAIL(pa) + FIM_TRAIL(pb) + FIM_LEAD(pa) + FIM_LEAD(pb))) *
+                    divby6;
+      stv<VK>(o + (size_t)e * L, lp);
     }
+  }
+  // Montgomery potential
+  {
+    R x0[VK], x[6][VK];
     if (mpf) {
       // edge minus cell value from float-float differences (no cancellation)
+      const float2* mp = mpf + m * s.cell;
+      float2 mc[VK];
       FOR_V {
-        const size_t kk = (size_t)k + j;
-        const float2 mc = mpf[(size_t)i * L + kk];
-        mo[j] = R((2.f * ff_diff(mpf[(size_t)i2 * L + kk], mc) + ff_diff(mpf[(size_t)i3t * L + kk], mc) +
-                   ff_diff(mpf[(size_t)i3l * L + kk], mc)) * (1.f / 6.f));
+        mc[j] = mp[c + j];
+        x0[j] = R(0);
       }
+#pragma unroll
+      for (int e = 0; e < 6; e++) FOR_V x[e][j] = R(ff_diff(mp[(size_t)nb[e] * L + k + j], mc[j]));
     } else {
-      R m2[VK], mt[VK], ml[VK];
-      ldv<VK>(montg + (size_t)i2 * L + k, m2);
-      ldv<VK>(montg + (size_t)i3t * L + k, mt);
-      ldv<VK>(montg + (size_t)i3l * L + k, ml);
-      FOR_V mo[j] = (two * (m1[j] + m2[j]) + mt[j] + ml[j]) * divby6;
+      around<R, VK>(montg + m * s.cell, L, i, k, nb, x0, x);
     }
-    stv<VK>(mont_edg + o, mo);
+    edge_means<R, VK>(five, L, x0, x, mont_edg + m * s.edge + oe);
+  }
+  if (!hi_order) {
+    R x0[VK], x[6][VK];
+    around<R, VK>(delp + m * s.cell, L, i, k, nb, x0, x);
+    edge_means<R, VK>(five, L, x0, x, dp_edg + m * s.edge + oe);
   }
   const int ntr = hi_order ? 1 : g.T;
   for (int t = 0; t < ntr; t++) {
-    const R* tr = tracr + (size_t)t * N * L;
-    R* te = trc_edg + (size_t)t * N * 6 * L;
-    R z[VK], t1[VK];
-    FOR_V z[j] = R(0);
-    stv<VK>(te + ((size_t)i * 6 + 5) * L + k, z);
-    ldv<VK>(tr + c, t1);
-    for (int e = 0; e < np; e++) {
-      const int i2 = pr[e], i3t = pr[e == 0 ? np - 1 : e - 1], i3l = pr[e == np - 1 ? 0 : e + 1];
-      R t2[VK], tt[VK], tl[VK], out[VK];
-      ldv<VK>(tr + (size_t)i2 * L + k, t2);
-      ldv<VK>(tr + (size_t)i3t * L + k, tt);
-      ldv<VK>(tr + (size_t)i3l * L + k, tl);
-      FOR_V out[j] = (two * (t1[j] + t2[j]) + tt[j] + tl[j]) * divby6;
-      stv<VK>(te + ((size_t)i * 6 + e) * L + k, out);
+    R x0[VK], x[6][VK];
+    around<R, VK>(tracr + m * s.tr + (size_t)t * N * L, L, i, k, nb, x0, x);
+    // the potential temperature of this step's edge values, for momtum1
+    if (t == 0 && thold) stv<VK>(thold + m * s.cell + c, x0);
+    R* te = trc_edg + m * s.tredg + (size_t)t * N * 6 * L + oe;
+    edge_means<R, VK>(five, L, x0, x, te);
+    if (five) {
+      R z[VK];
+      FOR_V z[j] = R(0);
+      stv<VK>(te + (size_t)5 * L, z);
     }
   }
 }
+#undef FIM_TRAIL
+#undef FIM_LEAD
 
 // --------------------------------------------------------------------------
 // edgvar2 (edgvar2.F90:24-319, hiOrderUVComp; the MORE_VARS block is compiled
@@ -1107,10 +1184,11 @@ void launch_edgvar1(const Launch& l, const Grid<R>& g, const Strides& s, int hi_
                     const R* v, const R* delp, const R* pres, const R* montg, const R* tracr,
                     R* u_edg, R* v_edg, R* dp_edg, R* lp_edg, R* mont_edg, R* uvsq_edg, R* trc_edg,
                     const float2* mpf, R* thold) {
-  // 8-byte accesses: at 4 levels a thread the kernel holds ~100 registers and
-  // runs at half the occupancy, which costs more than the wider accesses gain
+  // FP32: 8-byte accesses; at 4 levels a thread the neighbours' values take
+  // twice the registers and half the occupancy (glvl 8: 1.47 against 1.41 ms),
+  // at one level a thread half the bytes a load (1.87 ms)
   const int vk = pick_vk<R>(g.L, {u, v, delp, montg, tracr, u_edg, v_edg, dp_edg, lp_edg, mont_edg, uvsq_edg,
-                                  trc_edg, thold}, 2);
+                                  trc_edg, thold}, sizeof(R) == 8 ? 1 : 2);
   FIM_KBEGIN(l, "k_edgvar1");
   FIM_VK_DISPATCH(R, vk, (k_edgvar1<R, VK><<<dim3(blocks_for((long long)g.N * (g.L / VK)), l.members), kBlock, 0,
                                              l.stream>>>(g, s, hi_order, u, v, delp, pres, montg, tracr, u_edg,
@@ -1121,7 +1199,11 @@ void launch_edgvar1(const Launch& l, const Grid<R>& g, const Strides& s, int hi_
 
 template <typename R>
 void launch_edgvar3(const Launch& l, const Grid<R>& g, const Strides& s, const R* delp, const R* tracr,
-                    R* dp_edg, R* trc_edg, int nfields, bool average) {
+                    R* dp_edg, R* trc_edg, int nfields, const FrameTab& ft, bool average) {
+  if (sizeof(R) == 4 && average) {
+    launch_edges_patch<R>(l, g, s, ft, nfields, delp, tracr, dp_edg, trc_edg);
+    return;
+  }
   const int vk = pick_vk<R>(g.L, {delp, tracr, dp_edg, trc_edg});
   FIM_KBEGIN(l, "k_edgvar3_own");
   FIM_VK_DISPATCH(R, vk, (k_edgvar3_own<R, VK><<<dim3(blocks_for((long long)g.N * (g.L / VK)), l.members, nfields),
@@ -1242,7 +1324,7 @@ void launch_step_begin(const Launch& l, StepParams* sp) {
   template void launch_edgvar2<R>(const Launch&, const Grid<R>&, const Strides&, const R*, const R*, R*, R*,  \
                                   R*, R*);                                                                    \
   template void launch_edgvar3<R>(const Launch&, const Grid<R>&, const Strides&, const R*, const R*, R*, R*,  \
-                                  int, bool);                                                                \
+                                  int, const FrameTab&, bool);                                                                \
   template void launch_cnuity<R>(const Launch&, const Grid<R>&, const Strides&, const CnuityScratch<R>&,      \
                                  const R*, const R*, const R*, const R*, const R*, const R*, R*, R*, R*, R*,  \
                                  R*, R*, R*);                                                                 \

@@ -368,12 +368,6 @@ void launch_edgvar1(const Launch&, const Grid<R>&, const Strides&, int hi_order,
                     const R* v, const R* delp, const R* pres, const R* montg, const R* tracr,
                     R* u_edg, R* v_edg, R* dp_edg, R* lp_edg, R* mont_edg, R* uvsq_edg, R* trc_edg,
                     const float2* mpf = nullptr, R* thold = nullptr);
-// nfields: 1 = dp only, T = dp and tracers 2..ntra (edgvar3's full output);
-// average = false leaves the own-side values (k_cnuity12 averages the layer
-// thickness's itself)
-template <typename R>
-void launch_edgvar3(const Launch&, const Grid<R>&, const Strides&, const R* delp, const R* tracr,
-                    R* dp_edg, R* trc_edg, int nfields, bool average = true);
 template <typename R>
 struct CnuityScratch { R *antifx, *delp_lo, *p_plus, *p_mnus, *r_plus, *r_mnus; };
 template <typename R>
@@ -424,6 +418,20 @@ struct TrcFusedScratch {
   FrameTab ft;
   bool edges = false;  // trc_edg holds every tracer's edge values (the per-routine trcadv); 4 threads a cell
 };
+// nfields: 1 = dp only, T = dp and tracers 2..ntra (edgvar3's full output);
+// average = false leaves the own-side values (k_cnuity12 averages the layer
+// thickness's itself); ft: the context's cell patches
+template <typename R>
+void launch_edgvar3(const Launch&, const Grid<R>&, const Strides&, const R* delp, const R* tracr,
+                    R* dp_edg, R* trc_edg, int nfields, const FrameTab& ft, bool average = true);
+// edgvar3 with the two-sided average on cell patches (fim_trc.cu; FP32: the
+// FP64 build is bound by its FP64 operations, which recomputing the ring
+// cells' sides would add to); prepare_edges: its one-time launch attributes
+template <typename R>
+int prepare_edges(const FrameTab& ft);
+template <typename R>
+void launch_edges_patch(const Launch&, const Grid<R>&, const Strides&, const FrameTab&, int nfields, const R* delp,
+                        const R* tracr, R* dp_edg, R* trc_edg);
 // one-time launch attributes (shared-memory size) of the tracer kernels for
 // these patches; returns a cudaError_t value
 template <typename R>

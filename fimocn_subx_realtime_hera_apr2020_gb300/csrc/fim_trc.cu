@@ -228,10 +228,27 @@ struct PatchLayout {
       p.dpf = o; o += S1 * LK;
       p.arf = o; o += S1;
     }
+    return p.tables<R>(f, o);
+  }
+  // edges: field frame x 2 buffers [S2][LK]; edge values [SE][LK];
+  // least-squares coefficients as in lo
+  template <typename R>
+  __host__ __device__ static PatchLayout edges(const FrameTab& f, int LK) {
+    PatchLayout p{};
+    size_t o = 0;
+    p.trs = o; o += (size_t)2 * f.S2 * LK;
+    p.E = o; o += (size_t)f.SE * LK;
+    p.hf = o; o += (size_t)f.SC * 36 + f.SR * 6;
+    return p.tables<R>(f, o);
+  }
+  // the patch tables after o elements of R
+  template <typename R>
+  __host__ __device__ PatchLayout tables(const FrameTab& f, size_t o) const {
+    PatchLayout p = *this;
     p.r_elems = o;
     size_t b = (o * sizeof(R) + 15) & ~(size_t)15;
     p.tab = b;
-    b += S2 * 4 + S1 * 8 + SC * 6 * 2 + SR * 2 + S1;
+    b += (size_t)f.S2 * 4 + f.S1 * 8 + f.SC * 6 * 2 + f.SR * 2 + f.S1;
     p.bytes = (b + 15) & ~(size_t)15;
     return p;
   }
@@ -344,6 +361,23 @@ __device__ __forceinline__ void coef6(const R* hf, R (&h)[6]) {
   }
 }
 
+// the twelve coefficients of two slots of a patch cell (a 16-byte boundary:
+// 16-byte shared loads)
+__device__ __forceinline__ void coef12(const float* hf, float (&h)[12]) {
+#pragma unroll
+  for (int u = 0; u < 3; u++) {
+    const float4 w = reinterpret_cast<const float4*>(hf)[u];
+    h[4 * u] = w.x; h[4 * u + 1] = w.y; h[4 * u + 2] = w.z; h[4 * u + 3] = w.w;
+  }
+}
+__device__ __forceinline__ void coef12(const double* hf, double (&h)[12]) {
+#pragma unroll
+  for (int u = 0; u < 6; u++) {
+    const double2 w = reinterpret_cast<const double2*>(hf)[u];
+    h[2 * u] = w.x; h[2 * u + 1] = w.y;
+  }
+}
+
 // half the own-side least-squares edge value of every slot ie of a patch cell
 // (k_edgvar3_own's arithmetic, halved): val = bc + sum_e hfcoef(e, ie) (tr_e -
 // bc), d[e] = tr_e - bc (0 past nprox); hf = the cell's 36 halved coefficients
@@ -351,17 +385,21 @@ template <typename R, int VK, int LK>
 __device__ __forceinline__ void own_values(const R* hf, int x, int v, const R (&bc)[VK], const R (&d)[6][VK],
                                            int np, R* E) {
 #pragma unroll
-  for (int ie = 0; ie < 6; ie++) {
-    R h[6];
-    coef6<R>(hf + ie * 6, h);
-    R val[VK];
-    FOR_V val[j] = mul_rn(R(0.5), bc[j]);
+  for (int i2 = 0; i2 < 6; i2 += 2) {
+    R h[12];
+    coef12(hf + i2 * 6, h);
 #pragma unroll
-    for (int e = 0; e < 6; e++) {
-      FOR_V val[j] = (e < 5 || e < np) ? fma_rn(d[e][j], h[e], val[j]) : val[j];
+    for (int q = 0; q < 2; q++) {
+      const int ie = i2 + q;
+      R val[VK];
+      FOR_V val[j] = mul_rn(R(0.5), bc[j]);
+#pragma unroll
+      for (int e = 0; e < 6; e++) {
+        FOR_V val[j] = (e < 5 || e < np) ? fma_rn(d[e][j], h[q * 6 + e], val[j]) : val[j];
+      }
+      FOR_V val[j] = (ie < 5 || ie < np) ? val[j] : R(0);
+      stv<VK>(E + erow(x, ie) * LK + v, val);
     }
-    FOR_V val[j] = (ie < 5 || ie < np) ? val[j] : R(0);
-    stv<VK>(E + erow(x, ie) * LK + v, val);
   }
 }
 
@@ -808,6 +846,97 @@ __global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameT
   }
 }
 
+// edgvar3 (edgvar3.F90:66-133) of several fields per patch: the own-side
+// values of the patch cells and the ring cells' sides of its boundary edges in
+// shared memory, then the two-sided average 0.5 own + 0.5 other side of every
+// slot of the patch cells (0 in a pentagon's sixth).  Field 0 is the layer
+// thickness, field f tracer f.  One read and six writes a value, where storing
+// the own-side values and averaging them in a second pass (k_edgvar3_own,
+// k_edgvar3_avg) moves 19.  Held by the shared-memory pipe (77% busy: 1,400
+// wavefronts a patch, 16 levels and field), three blocks an SM (80 registers;
+// two 0.98 ms, four 0.91 ms): at glvl 7 / nvl 64, dp and 10 tracers, 0.89 ms
+// against 0.65 + 0.90 ms for the two passes.  blockIdx.z takes every
+// gridDim.z-th field, so small grids fill the chip.
+template <typename R, int VK, int GC>
+__global__ void __launch_bounds__(64 * GC, 3) k_edgvar3_patch(Grid<R> g, Strides s, FrameTab ft, int nfields,
+    const R* __restrict__ delp, const R* __restrict__ tracr, R* __restrict__ dp_edg, R* __restrict__ trc_edg) {
+  constexpr int LK = VK * GC;
+  const size_t m = blockIdx.y;
+  const int L = g.L, N = g.N;
+  const int nlc = (L + LK - 1) / LK;
+  const int tile = blockIdx.x / nlc;
+  const int k0 = (blockIdx.x - tile * nlc) * LK;
+  const int lk = min(LK, L - k0);
+  const int4 cn = ft.cnt[tile];
+  const int C = cn.x, n1 = cn.y, n2 = cn.z, nre = cn.w;
+  extern __shared__ __align__(16) unsigned char fsm[];
+  const PatchLayout lay = PatchLayout::edges<R>(ft, LK);
+  R* const sr = reinterpret_cast<R*>(fsm);
+  R* const trs = sr + lay.trs;
+  R* const E = sr + lay.E;
+  R* const hf = sr + lay.hf;
+  const FrameSm fs = load_tables<R>(g, ft, fsm, lay.tab, tile, C, n1, n2, nre);
+  __syncthreads();
+  const size_t NL = (size_t)N * L;
+  RowPlan<R, VK, GC> rp;
+  rp.init(fs, ft.SC, n2, lk, L);
+  auto stage = [&](int f, int b) {
+    const R* src = f == 0 ? delp + m * s.cell : tracr + m * s.tr + (size_t)f * NL;
+    rp.copy(trs + b * ft.S2 * LK, src + k0, fs, ft.SC, n2, lk, L);
+    stage_commit();
+  };
+  int f = blockIdx.z;
+  stage(f, 0);
+  load_coefs<R>(g, fs, hf, C, nre);
+  const int x = threadIdx.x / GC, v = (threadIdx.x - x * GC) * VK;
+  const bool on = x < C && v < lk;
+  const int i = on ? fs.cells[x] : 0, np = on ? fs.np[x] : 0;
+  for (int b = 0; f < nfields; f += gridDim.z, b ^= 1) {
+    stage_wait();
+    __syncthreads();
+    if (f + (int)gridDim.z < nfields) stage(f + gridDim.z, b ^ 1);
+    const R* T = trs + b * ft.S2 * LK;
+    if (on) {
+      const uint2 nb = fs.nbr[x];
+      R bc[VK], d[6][VK];
+      ldv<VK>(T + x * LK + v, bc);
+#pragma unroll
+      for (int e = 0; e < 6; e++) {
+        ldv<VK>(T + nb_at(nb, e) * LK + v, d[e]);
+        FOR_V d[e][j] = (e < 5 || e < np) ? d[e][j] - bc[j] : R(0);
+      }
+      own_values<R, VK, LK>(hf + x * 36, x, v, bc, d, np, E);
+    }
+    for (int it = threadIdx.x; it < nre * GC; it += blockDim.x) {
+      const int r = it / GC, ve = (it - r * GC) * VK;
+      if (ve < lk) ring_value<R, VK, LK>(T, fs, hf + C * 36 + r * 6, fs.red[r], 6 * C + r, ve, E);
+    }
+    __syncthreads();
+    if (!on) continue;
+    R* dst = (f == 0 ? dp_edg + m * s.edge : trc_edg + m * s.tredg + (size_t)f * 6 * NL) + (size_t)i * 6 * L + k0 + v;
+#pragma unroll
+    for (int e = 0; e < 6; e++) {
+      R a[VK], o[VK];
+      ldv<VK>(E + erow(x, e) * LK + v, a);
+      ldv<VK>(E + fs.mir[x * 6 + e] * LK + v, o);
+      FOR_V a[j] = a[j] + o[j];
+      stv<VK>(dst + e * L, a);
+    }
+  }
+}
+
+template <typename R, int VK>
+void edges_launch(const Launch& l, const Grid<R>& g, const Strides& s, const FrameTab& ft, int nfields,
+                  const R* delp, const R* tracr, R* dp_edg, R* trc_edg) {
+  constexpr int GC = 4, LK = VK * GC;
+  const unsigned nb = (unsigned)(ft.ntile * ((g.L + LK - 1) / LK));
+  // enough blocks for two waves of three an SM, at most one field a block
+  const unsigned want = 912u / (nb * l.members) + 1u;
+  const unsigned nz = want < (unsigned)nfields ? want : (unsigned)nfields;
+  k_edgvar3_patch<R, VK, GC><<<dim3(nb, l.members, nz), ft.SC * GC, PatchLayout::edges<R>(ft, LK).bytes, l.stream>>>(
+      g, s, ft, nfields, delp, tracr, dp_edg, trc_edg);
+}
+
 template <typename R, int VK, int GC, bool EV>
 void trf_chunks(const Launch& l, const Grid<R>& g, const Strides& s, const TrcFusedScratch<R>& w, R* trc_edg,
                 R* tracr, R* trcdp, R* trc_tdcy, R* trl_tdcy, const R* massfx, const R* delp, bool probe,
@@ -870,23 +999,50 @@ void fused_dispatch(const Launch& l, const Grid<R>& g, const Strides& s, const T
 #undef FIM_TRF
 }
 
+// The attribute belongs to the kernel, not to a context: it is raised to the
+// architecture's limit, so that contexts of different grids do not lower it
+// for each other.
+template <typename K>
+cudaError_t allow_smem(K kernel, size_t bytes) {
+  constexpr int kLimit = 227 * 1024;
+  if (bytes > (size_t)kLimit) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit);
+}
+
 template <typename R, int VK, int GC>
 int prepare_one(const FrameTab& ft) {
   constexpr int LK = VK * GC;
-  const size_t lo = PatchLayout::make<R>(ft, LK, false).bytes, hi = PatchLayout::make<R>(ft, LK, true).bytes;
-  cudaError_t e =
-      cudaFuncSetAttribute(k_trf_lo<R, VK, GC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lo);
-  if constexpr (GC == 4) {
-    const size_t ev = PatchLayout::make<R>(ft, LK, false, true).bytes;
+  cudaError_t e = allow_smem(k_trf_lo<R, VK, GC, false>, PatchLayout::make<R>(ft, LK, false).bytes);
+  if constexpr (GC == 4)
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_trf_lo<R, VK, GC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ev);
-  }
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_trf_hi<R, VK, GC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hi);
+      e = allow_smem(k_trf_lo<R, VK, GC, true>, PatchLayout::make<R>(ft, LK, false, true).bytes);
+  if (e == cudaSuccess) e = allow_smem(k_trf_hi<R, VK, GC>, PatchLayout::make<R>(ft, LK, true).bytes);
   return (int)e;
 }
 
 }  // namespace
+
+template <typename R>
+int prepare_edges(const FrameTab& ft) {
+  cudaError_t e = cudaSuccess;
+  if constexpr (sizeof(R) == 4) {
+    e = allow_smem(k_edgvar3_patch<R, 1, 4>, PatchLayout::edges<R>(ft, 4).bytes);
+    if (e == cudaSuccess) e = allow_smem(k_edgvar3_patch<R, 2, 4>, PatchLayout::edges<R>(ft, 8).bytes);
+    if (e == cudaSuccess) e = allow_smem(k_edgvar3_patch<R, 4, 4>, PatchLayout::edges<R>(ft, 16).bytes);
+  }
+  return (int)e;
+}
+
+template <typename R>
+void launch_edges_patch(const Launch& l, const Grid<R>& g, const Strides& s, const FrameTab& ft, int nfields,
+                        const R* delp, const R* tracr, R* dp_edg, R* trc_edg) {
+  if constexpr (sizeof(R) == 4) {
+    const int vk = pick_vk<R>(g.L, {delp, tracr, dp_edg, trc_edg});
+    FIM_KBEGIN(l, "k_edgvar3_patch");
+    FIM_VK_DISPATCH(R, vk, (edges_launch<R, VK>(l, g, s, ft, nfields, delp, tracr, dp_edg, trc_edg)));
+    FIM_KEND(l);
+  }
+}
 
 // ---- cell patches ---------------------------------------------------------
 
@@ -1130,6 +1286,9 @@ int tune_tracers(const Launch& l, const Grid<R>& g, const Strides& s, const TrcF
   template void launch_tracers_fused<R>(const Launch&, const Grid<R>&, const Strides&,                       \
                                         const TrcFusedScratch<R>&, R*, R*, R*, R*, R*, const R*, const R*,   \
                                         const ChunkHook*);                                                    \
+  template int prepare_edges<R>(const FrameTab&);                                                             \
+  template void launch_edges_patch<R>(const Launch&, const Grid<R>&, const Strides&, const FrameTab&, int,   \
+                                      const R*, const R*, R*, R*);                                           \
   template int prepare_tracers<R>(const FrameTab&);                                                           \
   template int tune_tracers<R>(const Launch&, const Grid<R>&, const Strides&, const TrcFusedScratch<R>&, R*, \
                                R*, R*, R*, R*, const R*, const R*, int*, int*, float*);
