@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(kColBlock) k_remap(Grid<R> g, Strides s, Knobs
 // the serial pcwise by rounding.
 constexpr int kWarpsInflate = 4;
 constexpr int kWarpsRemapV = 4;
-constexpr int kColsPerWarp = 8;
+constexpr int kColsPerWarp = 8;  // at most; see remap_columns
 
 // pcwise's massless-layer fill moves y(k) by (y(k+-1) - y(k)) * 1e-22 / fco(k):
 // below the rounding of either precision unless fco(k) is under ~1e-4.
@@ -601,6 +601,17 @@ template <typename R>
 __device__ __forceinline__ R plm_slope(R fm, R f, R fp) {
   const R b = ((fp - fm) * (fm + fp - R(2) * f) > R(0)) ? f - fm : fp - f;
   return (f <= cmin(fm, fp) || f >= cmax(fm, fp)) ? R(0) : b;
+}
+
+// FP64: monotonicity and the slope's sign by integer comparisons (a zero
+// curvature takes the upper difference, as the product test does)
+__device__ __forceinline__ double plm_slope(double fm, double f, double fp) {
+  const long long km = f64_key(fm), k = f64_key(f), kp = f64_key(fp);
+  const bool rise = km < k && k < kp, fall = km > k && k > kp;
+  if (!rise && !fall) return 0.;
+  const double c = fma(-2., f, fm + fp);
+  const bool lower = c != 0. && f64_neg(c) == fall;
+  return (lower ? f : fp) - (lower ? fm : f);
 }
 
 // asynchronous global -> shared copy of B = 4, 8 or 16 bytes
@@ -621,6 +632,19 @@ __device__ __forceinline__ R warp_sum(R v) {
   return v;
 }
 
+// sums of two values over a segment of W lanes: the halves of the segment take
+// one value each, so a step is one addition for both; a's sum ends in the
+// lower half's lanes and is returned everywhere, b's likewise
+template <typename R, int W = 32>
+__device__ __forceinline__ void warp_sum2(int lane, R& a, R& b) {
+  const bool up = lane >= W / 2;
+  const R give = up ? a : b, keep = up ? b : a;
+  R t = keep + __shfl_xor_sync(0xffffffffu, give, W / 2, W);
+#pragma unroll
+  for (int off = W / 4; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off, W);
+  a = __shfl_sync(0xffffffffu, t, 0, W);
+  b = __shfl_sync(0xffffffffu, t, W / 2, W);
+}
 
 // Value entering each lane of a recurrence x <- a x + b whose per-lane
 // composed map is (a, b): from the lanes below (up) or above (down); the
@@ -667,6 +691,10 @@ static_assert(sizeof(RemapV<float, 1, 1>) % 16 == 0 && sizeof(RemapV<double, 1, 
                   sizeof(RemapV<float, 4, 2>) % 16 == 0,
               "ring slots of consecutive warps stay 16-byte aligned");
 
+// x / cp, the division as the reference writes it
+__device__ __forceinline__ float by_cp(float x) { return x / float(kCp); }
+__device__ __forceinline__ double by_cp(double x) { return f64_quot(x, kCp, 1. / kCp); }
+
 // pcwise's coordinate quantities for one lane's levels and interfaces
 template <typename R, int VL>
 struct LaneGeo {
@@ -675,6 +703,12 @@ struct LaneGeo {
   unsigned up;                 // bit v: interface kb+v takes layer kb+v as donor
   bool thin;                   // (whole warp) some layer is thin enough for the fill to matter
 };
+
+// 1 / x and a / b of thicknesses (x > 0, at least 1e-22; 0 <= a <= b)
+__device__ __forceinline__ float recip(float x) { return fdiv(1.f, x); }
+__device__ __forceinline__ double recip(double x) { return f64_recip(x); }
+__device__ __forceinline__ float over(float a, float b) { return fdiv(a, b); }
+__device__ __forceinline__ double over(double a, double b) { return f64_quot(a, b, f64_recip(b)); }
 
 template <typename R>
 __device__ __forceinline__ R coord_thick(bool flip, const R* x, int k) {
@@ -698,8 +732,8 @@ __device__ __forceinline__ void lane_geo(int L, int lane, const R* xo, const R* 
       thin = thin || fo < fill_thin<R>();
     }
     G.fo[v] = fo;
-    G.rfo[v] = fdiv(R(1), fo + small);
-    G.rfn[v] = fdiv(R(1), fn + small);
+    if constexpr (sizeof(R) == 4) G.rfo[v] = fdiv(R(1), fo + small);
+    G.rfn[v] = recip(fn + small);
     R nd = R(0), hh = R(0);
     if (k >= 1 && k <= L - 1) {
       const R d = flip ? (-xn[k]) - (-xo[k]) : xn[k] - xo[k];
@@ -707,8 +741,8 @@ __device__ __forceinline__ void lane_geo(int L, int lane, const R* xo, const R* 
         const R fl = coord_thick(flip, xo, d > R(0) ? k : k - 1);
         if (fl > R(0)) {
           const R dd = d > R(0) ? d : -d;
-          const R dsl = cmin(R(0) + fl, dd) - cmin(R(0), dd);
-          const R dx = fdiv(dsl, fl);
+          const R dsl = cmin(fl, dd);
+          const R dx = over(dsl, fl);
           const R hx = d > R(0) ? dx - R(1) : R(1) - dx;
           if (dsl != R(0)) {
             nd = -d;
@@ -726,6 +760,12 @@ __device__ __forceinline__ void lane_geo(int L, int lane, const R* xo, const R* 
   // shuffles, so both columns of a paired warp must take it together (the
   // fill is the reference's own step, exact for columns without thin layers)
   G.thin = __any_sync(0xffffffffu, thin);
+  if constexpr (sizeof(R) == 8) {  // read by the fill only
+    if (G.thin) {
+#pragma unroll
+      for (int v = 0; v < VL; v++) G.rfo[v] = R(1) / (G.fo[v] + small);
+    }
+  }
 }
 
 // pcwise (PLM, miglim = 1) of NF fields sharing one coordinate, lane =
@@ -850,7 +890,8 @@ __device__ __forceinline__ bool pcwise_v(int L, int lane, R (&y)[NF][VL], const 
       }
     }
     if (sizeof(R) == 8) {
-      const R dif = warp_sum<R, W>(bfore[h] - after), scl = warp_sum<R, W>(colscl[h]);
+      R dif = bfore[h] - after, scl = colscl[h];
+      warp_sum2<R, W>(lane, dif, scl);
       bad |= cabs(dif) > cmax(R(1.e-33), col_tol<R>(1.e-11) * scl);
     }
   }
@@ -967,7 +1008,7 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
     const StepParams* __restrict__ sp, const R* __restrict__ targt, const R* __restrict__ exsmo,
     R* __restrict__ us3d, R* __restrict__ vs3d, R* __restrict__ tr3d, R* __restrict__ sdot,
     R* __restrict__ ex3d, R* __restrict__ dp3d, R* __restrict__ pr3d, int* __restrict__ flags, int bnd,
-    int vec, R* __restrict__ trdp) {
+    int vec, R* __restrict__ trdp, int cpw) {
   constexpr int H = 32 / WL;  // columns in hand per warp
   using SW = RemapV<R, VL, H>;
   constexpr int D = SW::D;
@@ -978,9 +1019,8 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
   extern __shared__ __align__(16) unsigned char smraw[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int N = g.N, L = g.L, L1 = L + 1, T = g.T;
-  const int c0 = (blockIdx.x * kWarpsRemapV + wib) * kColsPerWarp;
-  if (c0 >= N) return;
-  const int ncol = (N - c0 < kColsPerWarp) ? N - c0 : kColsPerWarp;
+  const int c0 = (blockIdx.x * kWarpsRemapV + wib) * cpw;
+  const int ncol = N - c0 < cpw ? max(N - c0, 0) : cpw;
   const size_t m = blockIdx.y;
   sp += m;
   if (!sp->active || (bnd && sp->its <= 1)) return;
@@ -989,7 +1029,7 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
   ex3d += m * s.intf; dp3d += m * s.cell; pr3d += m * s.intf;
   if (trdp) trdp += m * s.tr;
   const int its = sp->its - bnd;
-  const R cp = R(kCp), rd = R(kRd), p1000 = R(kP1000), small = R(1.e-6);
+  const R p1000 = R(kP1000), small = R(1.e-6);
   // hystat's floors of tracers 2 and 3 (hystat.F90:90-93) when trdp is formed here
   const R qvmin = R(kQvmin), qwmin = R(kQwmin);
   const int hw = lane / WL, ls = lane - hw * WL;  // column in hand, lane within it
@@ -1077,7 +1117,7 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
           en = sl * en + (R(1) - sl) * eo;
         }
         S.exnew[hw][k] = en;
-        S.pk1col[hw][k] = eo * S.prcol[hw][k] / cp;
+        S.pk1col[hw][k] = by_cp(eo * S.prcol[hw][k]);
       }
       __syncwarp();
       // miglim = 1: exnew(2..nvl) between the neighbouring old interfaces
@@ -1090,9 +1130,9 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
         // interfaces then reproduce the old ones exactly, so the layer
         // thicknesses keep summing to the unchanged column mass
         const R en = S.exnew[hw][k];
-        const R pn = p1000 * pow(en / cp, cp / rd);
+        const R pn = p1000 * pow_cp_rd(by_cp(en));
         S.prnew[hw][k] = pn;
-        S.pk1new[hw][k] = en * pn / cp;
+        S.pk1new[hw][k] = by_cp(en * pn);
       }
       __syncwarp();
       for (int k = ls; k < L; k += WL) S.dpcol[hw][k] = S.prnew[hw][k] - S.prnew[hw][k + 1];
@@ -1112,7 +1152,7 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
 #pragma unroll
       for (int v = 0; v < VL; v++) {
         dpv[v] = kb + v < L ? S.dpcol[hw][kb + v] : R(0);
-        qqv[v] = fdiv(R(1), dpv[v] + small);
+        qqv[v] = sizeof(R) == 4 || kn.thktop == 0. ? fdiv(R(1), dpv[v] + small) : R(0);
       }
       __syncwarp();
     } else if (j == 1) {
@@ -1247,20 +1287,27 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
     if (++qs == D) qs = 0;
   }
   cp_async_wait<0>();
-  __syncwarp();
+  __syncthreads();
   // theta redistribution among neighbouring layers (hybgen.F90:648-667),
-  // lane = column: pairs (k-1, k) from the bottom up, each pair seeing the
-  // upper layer of the pair below as already adjusted
-  if (lane < ncol && L >= 3) {
-    R* th = S.thb[lane];
-    const R* dk = S.dkb[lane];
-    const R fl = S.flo[lane];
-    R thb = th[L - 1];
+  // lane = column over the block's columns: pairs (k-1, k) from the bottom up,
+  // each pair seeing the upper layer of the pair below as already adjusted.
+  // One warp sweeps for all four: the sweep's instructions cost the same for
+  // 8 columns as for 32 (a fifth of the FP64 kernel when each warp swept its
+  // own).
+  static_assert(kWarpsRemapV * kColsPerWarp <= 32, "one lane a column of the block");
+  const int sw = lane / kColsPerWarp, sc = lane - sw * kColsPerWarp;
+  if (wib == 0 && L >= 3 && sc < cpw && (blockIdx.x * kWarpsRemapV + sw) * cpw + sc < N) {
+    SW& Q = reinterpret_cast<SW*>(smraw)[sw];
+    R* th = Q.thb[sc];
+    const R* dk = Q.dkb[sc];
+    const R fl = Q.flo[sc];
+    R thb = th[L - 1], dkup = cmax(dk[L - 1], fl);
+    R dev = (thb - S.tg[L - 1]) * dkup;
     for (int k = L; k >= 3; k--) {
       const R tha = th[k - 2];
-      const R dplo = cmax(dk[k - 2], fl), dpup = cmax(dk[k - 1], fl);
+      const R dplo = cmax(dk[k - 2], fl), dpup = dkup;
       const R devilo = (tha - S.tg[k - 2]) * dplo;
-      const R deviup = (thb - S.tg[k - 1]) * dpup;
+      const R deviup = dev;
       R na = tha, nbv = thb;
       if (deviup > R(0) && devilo < R(0)) {
         const R cc = cmin(deviup, -devilo);
@@ -1273,15 +1320,17 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
       }
       th[k - 1] = nbv;
       thb = na;
+      dkup = dplo;
+      dev = (thb - S.tg[k - 2]) * dkup;
     }
     th[1] = thb;
     {
       R clout = R(0);
       for (int k = 0; k < L; k++) clout = clout + th[k] * dk[k];
-      if (cabs(clout - S.colin[lane]) > cmax(R(1.e-33), col_tol<R>(2.e-6) * S.colscl[lane])) bad = true;
+      if (cabs(clout - Q.colin[sc]) > cmax(R(1.e-33), col_tol<R>(2.e-6) * Q.colscl[sc])) bad = true;
     }
   }
-  __syncwarp();
+  __syncthreads();
   for (int cc = hw; cc < ncol; cc += H) {
     R y[VL];
 #pragma unroll
@@ -1309,6 +1358,29 @@ inline int remap_vl(int L) { return L <= 32 ? 1 : L <= 64 ? 2 : 4; }
 // each ring item, scan and shuffle then serves two columns
 template <typename R>
 inline bool remap_paired(int L) { return sizeof(R) == 4 && L > 32 && L <= 64; }
+
+// Columns a warp of k_remap_v takes in turn.  Many columns a warp amortise its
+// start (the first copies, the theta sweep); few leave small grids no nearly
+// empty last round of blocks.  FP64 (two blocks an SM by shared memory): the
+// rounds of 2 x 152 blocks times (columns + 1/2) follow the measured times at
+// glvl 6 / nvl 64 (8 columns 3.07 ms, 6: 2.81, 4: 2.90, 2: 2.98) and glvl 5 / nvl 38
+// (6: 0.59, 4: 0.60, 2: 0.55).  FP32: all blocks of a small grid are resident and
+// share their SM, blocks an SM times (columns + 3): glvl 5 / nvl 38 8: 62 us,
+// 6: 51, 4: 69; glvl 8 / nvl 64 8: 2.95 ms, 6: 3.01, 4: 3.12.
+template <typename R>
+int remap_columns(int N, int members, bool paired) {
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long slots = sizeof(R) == 8 ? 2 * sms : sms;
+  long long best = -1;
+  int cols = kColsPerWarp;
+  for (int c = kColsPerWarp; c >= (paired ? 4 : 3); c -= paired ? 2 : 1) {
+    const long long nb = (long long)nblocks(N, kWarpsRemapV * c) * members;
+    const long long cost = (nb + slots - 1) / slots * (sizeof(R) == 8 ? 2 * c + 1 : 2 * c + 6);
+    if (best < 0 || cost < best) { best = cost; cols = c; }
+  }
+  return cols;
+}
 
 template <typename R>
 int prepare_hybgen(int L) {
@@ -1744,7 +1816,8 @@ bool launch_hybgen(const Launch& l, const Grid<R>& g, const Strides& s, const Kn
                                                                                             w.exsmo2, l.boundary);
       FIM_KEND(l);
     }
-    dim3 gw(nblocks(g.N, kWarpsRemapV * kColsPerWarp), l.members);
+    const int cpw = remap_columns<R>(g.N, l.members, remap_paired<R>(g.L));
+    dim3 gw(nblocks(g.N, kWarpsRemapV * cpw), l.members);
     const bool paired = remap_paired<R>(g.L);
     const int vl = paired ? 4 : remap_vl(g.L);
     const int cb = (int)(vl * sizeof(R) < 16 ? vl * sizeof(R) : 16);
@@ -1754,7 +1827,7 @@ bool launch_hybgen(const Launch& l, const Grid<R>& g, const Strides& s, const Kn
     FIM_KBEGIN(l, "k_remap");
 #define FIM_REMAP_V(VL, WL)                                                                                  \
   k_remap_v<R, VL, WL><<<gw, 32 * kWarpsRemapV, remap_v_smem<R, VL, WL>(), l.stream>>>(                       \
-      g, s, kn, l.sp, targt, ex_in, us3d, vs3d, tr3d, sdot, ex3d, dp3d, pr3d, l.flags, l.boundary, vec, trdp)
+      g, s, kn, l.sp, targt, ex_in, us3d, vs3d, tr3d, sdot, ex3d, dp3d, pr3d, l.flags, l.boundary, vec, trdp, cpw)
     if (paired) {
       if constexpr (sizeof(R) == 4) FIM_REMAP_V(4, 16);
     } else if (vl == 1) FIM_REMAP_V(1, 32);

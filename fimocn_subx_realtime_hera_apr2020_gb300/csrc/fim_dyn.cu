@@ -31,16 +31,9 @@ __device__ __forceinline__ bool cell_level(int N, int L, int& i, int& k) {
 
 inline unsigned blocks_for(long long n, int b = kBlock) { return (unsigned)((n + b - 1) / b); }
 
-// 1 / sqrt(x) of a squared speed.  FP64 (2 lanes a clock and SM on GB300, so
-// operations count): one third-order step r (1 + e/2 + 3 e^2/8), e = 1 - x r^2,
-// from the hardware's approximation, whose error cubed is below rounding.
+// 1 / sqrt(x) of a squared speed
 __device__ __forceinline__ float inv_root(float x) { return rsqrtf(x); }
-__device__ __forceinline__ double inv_root(double x) {
-  double r;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-(x * r), r, 1.);
-  return fma(r, e * fma(.375, e, .5), r);
-}
+__device__ __forceinline__ double inv_root(double x) { return f64_rsqrt(x); }
 
 // |(a, b)|: IEEE sqrt in FP64; x * rsqrt(x) in FP32, a few ulp from the
 // rounded root and about a third of its instructions
@@ -668,26 +661,38 @@ __global__ void __launch_bounds__(kBlock) k_cnuity_coop(Grid<R> g, Strides s, co
                         flags);
 }
 
-// cnuity5 (cnuity_compute.F90:408-445) for 32 columns per warp, 32 levels
-// (top-down) at a time.  The layer thickness and pressure tendency of each
-// level are formed with lane = level, one column at a time (128-byte rows),
-// into a shared tile; the top-down pressure sum and the omega flux-convergence
-// integral run with lane = column up the tile in the reference's order (FP64,
-// or float-float in the FP32-mixed build); the Exner function and the
-// v.grad(p) term are formed with lane = level again.
-template <typename R>
-constexpr int kC5Warps = sizeof(R) == 4 ? 4 : 2;
-template <typename R>
-__global__ void __launch_bounds__(32 * kC5Warps<R>) k_cnuity5(Grid<R> g, Strides s,
+// a / b with rb = 1 / b: FP32 divides as written
+__device__ __forceinline__ float quot_by(float a, float b, float) { return a / b; }
+__device__ __forceinline__ double quot_by(double a, double b, double rb) { return f64_quot(a, b, rb); }
+
+// cnuity5 (cnuity_compute.F90:408-445), 32 columns a block.  The layer
+// thickness and pressure tendency of every level are formed with thread =
+// (column, VK levels) into shared tiles; the top-down pressure sum (warp 0) and
+// the omega flux-convergence integral (warp 1) run with lane = column up the
+// tiles in the reference's order (FP64, or float-float in the FP32-mixed
+// build); the Exner function and the v.grad(p) term are formed with thread =
+// (column, VK levels) again.  The sums are a serial chain of ~nvl steps, so the
+// block's other warps and its neighbours on the SM cover it: one warp doing
+// all three parts of its 32 columns, 32 levels at a time, left two to four warps
+// an SM in flight on small grids.  FP32, nvl 64: glvl 8 0.84 -> 0.44 ms (5,340
+// GB/s of its 14 words), glvl 5 / nvl 38 78 -> 14 us (4 levels a thread; one:
+// 0.65 ms and 18 us).  FP64, glvl 6: 0.70 -> 0.39 ms, with the power of
+// fim_internal.h; one level a thread, bound by the FP64 pipe.
+constexpr int kC5Cols = 32;
+constexpr int kC5Block = 256;
+template <typename R, int VK>
+__global__ void __launch_bounds__(kC5Block, 4) k_cnuity5(Grid<R> g, Strides s,
     const StepParams* __restrict__ sp, R* __restrict__ pres, R* __restrict__ delp, R* __restrict__ exner,
     const R* __restrict__ dp_tndcy, R* __restrict__ omega, const R* __restrict__ lp_edg, const R* __restrict__ u,
     const R* __restrict__ v, int ab3_delp) {
-  __shared__ R tiles[kC5Warps<R>][2][32][33];
+  extern __shared__ __align__(16) unsigned char c5sm[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int N = g.N, L = g.L, L1 = L + 1;
-  const int i0 = (blockIdx.x * kC5Warps<R> + wib) * 32;
-  if (i0 >= N) return;
-  const int ncol = N - i0 < 32 ? N - i0 : 32;
+  const int N = g.N, L = g.L, L1 = L + 1, LV = L / VK;
+  const int LS = L | 1;  // odd row stride: lane = column reads are conflict-free
+  R* const tp = reinterpret_cast<R*>(c5sm);  // thickness in, pressure out
+  R* const tw = tp + kC5Cols * LS;           // layer pressure tendency in, omega's first terms out
+  const int i0 = blockIdx.x * kC5Cols;
+  const int ncol = N - i0 < kC5Cols ? N - i0 : kC5Cols;
   const size_t m = blockIdx.y;
   sp += m;
   if (!sp->active) return;
@@ -695,88 +700,123 @@ __global__ void __launch_bounds__(32 * kC5Warps<R>) k_cnuity5(Grid<R> g, Strides
   omega += m * s.cell; lp_edg += m * s.edge; u += m * s.cell; v += m * s.cell;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
   const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3), dt = R(sp->dt);
-  const R cp = R(kCp), p1000 = R(kP1000), rdcp = R(kRd) / R(kCp);
+  const R cp = R(kCp), p1000 = R(kP1000), rdt = R(1) / dt;
   const size_t NL = (size_t)N * L;
-  R (*tp)[33] = tiles[wib][0];  // thickness in, pressure out
-  R (*tw)[33] = tiles[wib][1];  // layer pressure tendency in, omega's first terms out
-  const bool live = lane < ncol;
-  // the top-down sums of column i0 + lane
-  FF2 pf{0.f, 0.f}, cf{0.f, 0.f};
-  double pd = 0.0, cd = 0.0;
-  if (live) {
-    const R ptop = pres[(size_t)(i0 + lane) * L1 + L];
-    pf = FF2{(float)ptop, 0.f};
-    pd = (double)ptop;
-  }
-  for (int base = 0; base < L; base += 32) {
-    const int j = base + lane;
-    const bool act = j < L;
-    const int k = L - 1 - j;
-    const int nq = L - base < 32 ? L - base : 32;
-#pragma unroll 4
-    for (int r = 0; r < 32; r++)
-      if (r < ncol && act) {
-        const size_t c = (size_t)(i0 + r) * L + k;
-        const R tnf = dp_tndcy[(size_t)nf * NL + c], tof = dp_tndcy[(size_t)of * NL + c],
-                tvf = dp_tndcy[(size_t)vof * NL + c];
-        R d;
-        if (ab3_delp) {
-          // massflux_newdepth's AB3 thickness update (massadv_compute.F90:85-91)
-          R dn = delp[c] + ab1 * tnf + ab2 * tof + ab3 * tvf;
-          dn = dn > R(0) ? dn : R(0);
-          delp[c] = dn;
-          d = dn;
-        } else {
-          d = delp[c];
-        }
-        tp[r][lane] = d;
-        tw[r][lane] = (ab1 * tnf + ab2 * tof + ab3 * tvf) / dt;
+#pragma unroll 2
+  for (int it = threadIdx.x; it < ncol * LV; it += kC5Block) {
+    const int r = it / LV, k = (it - r * LV) * VK;
+    const size_t c = (size_t)(i0 + r) * L + k;
+    R tnf[VK], tof[VK], tvf[VK], d[VK];
+    ldv<VK>(dp_tndcy + (size_t)nf * NL + c, tnf);
+    ldv<VK>(dp_tndcy + (size_t)of * NL + c, tof);
+    ldv<VK>(dp_tndcy + (size_t)vof * NL + c, tvf);
+    ldv<VK>(delp + c, d);
+    if (ab3_delp) {
+      // massflux_newdepth's AB3 thickness update (massadv_compute.F90:85-91)
+      FOR_V {
+        const R dn = d[j] + ab1 * tnf[j] + ab2 * tof[j] + ab3 * tvf[j];
+        d[j] = dn > R(0) ? dn : R(0);
       }
-    __syncwarp();
-    if (live) {
-      for (int q = 0; q < nq; q++) {
-        const R d = tp[lane][q], lyr = tw[lane][q];
-        if constexpr (sizeof(R) == 4) {
-          pf = ff_add(pf, FF2{d, 0.f});
-          tp[lane][q] = pf.hi;
-          // omega = (integral of the layers above) + half of this layer
-          tw[lane][q] = R(cf.hi + cf.lo) + R(0.5) * lyr;
+      stv<VK>(delp + c, d);
+    }
+    FOR_V {
+      tp[r * LS + k + j] = d[j];
+      tw[r * LS + k + j] = quot_by(ab1 * tnf[j] + ab2 * tof[j] + ab3 * tvf[j], dt, rdt);
+    }
+  }
+  __syncthreads();
+  if (lane < ncol) {
+    if (wib == 0) {
+      R* t = tp + lane * LS;
+      const R ptop = pres[(size_t)(i0 + lane) * L1 + L];
+      if constexpr (sizeof(R) == 4) {
+        FF2 pf{(float)ptop, 0.f};
+#pragma unroll 4
+        for (int k = L - 1; k >= 0; k--) {
+          pf = ff_add(pf, FF2{t[k], 0.f});
+          t[k] = pf.hi;
+        }
+      } else {
+        double pd = (double)ptop;
+#pragma unroll 4
+        for (int k = L - 1; k >= 0; k--) {
+          pd = pd + (double)t[k];
+          t[k] = R(pd);
+        }
+      }
+    } else if (wib == 1) {
+      // omega = (integral of the layers above) + half of this layer
+      R* t = tw + lane * LS;
+      if constexpr (sizeof(R) == 4) {
+        FF2 cf{0.f, 0.f};
+#pragma unroll 4
+        for (int k = L - 1; k >= 0; k--) {
+          const R lyr = t[k];
+          t[k] = R(cf.hi + cf.lo) + R(0.5) * lyr;
           cf = ff_add(cf, FF2{lyr, 0.f});
-        } else {
-          pd = pd + (double)d;
-          tp[lane][q] = R(pd);
-          tw[lane][q] = R(cd + 0.5 * (double)lyr);
-          cd = cd + (double)lyr;
+        }
+      } else {
+        double cd = 0.0;
+#pragma unroll 4
+        for (int k = L - 1; k >= 0; k--) {
+          const double lyr = (double)t[k];
+          t[k] = R(cd + 0.5 * lyr);
+          cd = cd + lyr;
         }
       }
     }
-    __syncwarp();
-#pragma unroll 2
-    for (int r = 0; r < 32; r++)
-      if (r < ncol && act) {
-        const int i = i0 + r;
-        const size_t c = (size_t)i * L + k;
-        const R pr = tp[r][lane];
-        pres[(size_t)i * L1 + k] = pr;
-        exner[(size_t)i * L1 + k] = cp * pow(pr / p1000, rdcp);
-        // pressure gradient over the cell's edges (all six slots hold valid
-        // rows; a pentagon's slot 5 is left out)
-        const int np = g.nprox[i];
-        R lp[6];
-#pragma unroll
-        for (int e = 0; e < 6; e++) lp[e] = lp_edg[((size_t)i * 6 + e) * L + k];
-        R dpdx = R(0), dpdy = R(0);
-#pragma unroll
-        for (int e = 0; e < 6; e++)
-          if (e < np) {
-            const R* sv = g.svc + (i * 6 + e) * 2;
-            dpdx = dpdx + lp[e] * sv[1];
-            dpdy = dpdy - lp[e] * sv[0];
-          }
-        omega[c] = tw[r][lane] + (u[c] * dpdx + v[c] * dpdy) * g.rarea[i];
-      }
-    __syncwarp();
   }
+  __syncthreads();
+  for (int it = threadIdx.x; it < ncol * LV; it += kC5Block) {
+    const int r = it / LV, k = (it - r * LV) * VK;
+    const int i = i0 + r;
+    const size_t c = (size_t)i * L + k;
+    // pressure gradient over the cell's edges (all six slots hold valid
+    // rows; a pentagon's slot 5 is left out)
+    const int np = g.nprox[i];
+    R lp[6][VK], uu[VK], vv[VK], om[VK];
+#pragma unroll
+    for (int e = 0; e < 6; e++) ldv<VK>(lp_edg + ((size_t)i * 6 + e) * L + k, lp[e]);
+    ldv<VK>(u + c, uu);
+    ldv<VK>(v + c, vv);
+    R dpdx[VK], dpdy[VK];
+    FOR_V {
+      const R pr = tp[r * LS + k + j];
+      pres[(size_t)i * L1 + k + j] = pr;
+      exner[(size_t)i * L1 + k + j] = cp * pow_rd_cp(quot_by(pr, p1000, R(1) / R(kP1000)));
+      dpdx[j] = R(0);
+      dpdy[j] = R(0);
+    }
+#pragma unroll
+    for (int e = 0; e < 6; e++)
+      if (e < np) {
+        const R* sv = g.svc + (i * 6 + e) * 2;
+        FOR_V {
+          dpdx[j] = dpdx[j] + lp[e][j] * sv[1];
+          dpdy[j] = dpdy[j] - lp[e][j] * sv[0];
+        }
+      }
+    const R rar = g.rarea[i];
+    FOR_V om[j] = tw[r * LS + k + j] + (uu[j] * dpdx[j] + vv[j] * dpdy[j]) * rar;
+    stv<VK>(omega + c, om);
+  }
+}
+
+template <typename R>
+void launch_cnuity5(const Launch& l, const Grid<R>& g, const Strides& s, R* pres, R* delp, R* exner,
+                    const R* dp_tndcy, R* omega, const R* lp_edg, const R* u, const R* v, int ab3_delp) {
+  const int vk = pick_vk<R>(g.L, {delp, dp_tndcy, omega, lp_edg, u, v}, sizeof(R) == 8 ? 1 : 0);
+  const size_t smem = (size_t)2 * kC5Cols * (g.L | 1) * sizeof(R);
+  const dim3 grid((unsigned)((g.N + kC5Cols - 1) / kC5Cols), l.members);
+  FIM_KBEGIN(l, "k_cnuity5");
+  FIM_VK_DISPATCH(R, vk, ({
+    if (smem > (size_t)48 * 1024)  // FP64 columns of more than 95 levels
+      cudaFuncSetAttribute(k_cnuity5<R, VK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)(2 * kC5Cols * (kMaxL | 1) * sizeof(R)));
+    k_cnuity5<R, VK><<<grid, kC5Block, smem, l.stream>>>(g, s, l.sp, pres, delp, exner, dp_tndcy, omega, lp_edg, u, v,
+                                                         ab3_delp);
+  }));
+  FIM_KEND(l);
 }
 
 // --------------------------------------------------------------------------
@@ -903,11 +943,7 @@ void launch_massadv(const Launch& l, const Grid<R>& g, const Strides& s, const C
   k_massadv_flux<R><<<grid, kBlock, 0, l.stream>>>(g, s, l.sp, u_edg, v_edg, dp_edg, delp, w.r_plus, w.r_mnus,
                                                     massfx, dp_tndcy);
   FIM_KEND(l);
-  dim3 gw((unsigned)((g.N + 32 * kC5Warps<R> - 1) / (32 * kC5Warps<R>)), l.members);
-  FIM_KBEGIN(l, "k_cnuity5");
-  k_cnuity5<R><<<gw, 32 * kC5Warps<R>, 0, l.stream>>>(g, s, l.sp, pres, delp, exner, dp_tndcy, omega, lp_edg, u,
-                                                      v, 1);
-  FIM_KEND(l);
+  launch_cnuity5<R>(l, g, s, pres, delp, exner, dp_tndcy, omega, lp_edg, u, v, 1);
 }
 
 // --------------------------------------------------------------------------
@@ -1264,11 +1300,7 @@ void launch_cnuity(const Launch& l, const Grid<R>& g, const Strides& s, const Cn
                                                          dplo_tndcy, dp_tndcy, delp, l.flags)));
   FIM_KEND(l);
   }
-  dim3 gw((unsigned)((g.N + 32 * kC5Warps<R> - 1) / (32 * kC5Warps<R>)), l.members);
-  FIM_KBEGIN(l, "k_cnuity5");
-  k_cnuity5<R><<<gw, 32 * kC5Warps<R>, 0, l.stream>>>(g, s, l.sp, pres, delp, exner, dp_tndcy, omega, lp_edg, u,
-                                                      v, 0);
-  FIM_KEND(l);
+  launch_cnuity5<R>(l, g, s, pres, delp, exner, dp_tndcy, omega, lp_edg, u, v, 0);
 }
 
 template <typename R>

@@ -321,6 +321,93 @@ inline int pick_vk(int L, std::initializer_list<const void*> ptrs, int want = 0)
     }                                                         \
   } while (0)
 
+// ---- FP64 with few FP64 operations ------------------------------------------
+// GB300 issues 2 FP64 lanes a clock and SM (against 128 FP32 and 64 integer
+// ones), so the FP64 build is bound by its FP64 operations.  Comparisons run
+// on the integer pipe (a double's bits, the magnitude of negative values
+// complemented, order as int64), reciprocals and powers by few steps from the
+// hardware's FP32-accurate approximations.
+__device__ __forceinline__ long long f64_key(double x) {
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ bool f64_neg(double x) { return __double2hiint(x) < 0; }
+// 1 / b, b normal and below 2^1000: one third-order step from the
+// approximation (its error cubed is below rounding)
+__device__ __forceinline__ double f64_recip(double b) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+  const double e = fma(-b, r, 1.);
+  return fma(r, fma(e, e, e), r);
+}
+// a / b with rb = 1 / b: the product and one residual correction (Markstein),
+// correctly rounded but for rare last-bit cases (finite results)
+__device__ __forceinline__ double f64_quot(double a, double b, double rb) {
+  const double q = a * rb;
+  return fma(fma(-b, q, a), rb, q);
+}
+// 1 / sqrt(x), x normal: one third-order step r (1 + e/2 + 3 e^2/8)
+__device__ __forceinline__ double f64_rsqrt(double x) {
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-(x * r), r, 1.);
+  return fma(r, e * fma(.375, e, .5), r);
+}
+// ln(x) to ~1e-13 absolute, 2^-20 < x < 2^20: x = 2^n m, m in [0.71, 1.42),
+// ln m = 2 (s + s^3/3 + s^5/5 + ...), s = (m - 1) / (m + 1), |s| < 0.172
+__device__ __forceinline__ double f64_ln13(double x) {
+  const int hi = __double2hiint(x);
+  const int n = (hi - 0x3fe6a09e) >> 20;
+  const double m = __hiloint2double(hi - (n << 20), __double2loint(x));
+  const double s = (m - 1.) * f64_recip(m + 1.), z = s * s;
+  double p = 2. / 15.;
+  p = fma(p, z, 2. / 13.);
+  p = fma(p, z, 2. / 11.);
+  p = fma(p, z, 2. / 9.);
+  p = fma(p, z, 2. / 7.);
+  p = fma(p, z, 2. / 5.);
+  p = fma(p, z, 2. / 3.);
+  p = fma(p, z, 2.);
+  return fma(s, p, (double)n * 0.69314718055994530942);
+}
+// x^(cp/rd) and x^(rd/cp), the Exner function's powers.  cp/rd = 3.5 + d and
+// rd/cp = 2/7 + d' with |d| < 1e-4, |d'| < 1e-5, so the root is taken by
+// Newton-type steps with its rounding kept in a second term, and x^d =
+// exp(d ln x) needs ln x to 1e-12 only.  About 40 FP64 operations and within
+// an ulp of the rounded power, where pow takes several times as many.
+__device__ __forceinline__ double f64_expm1_small(double y) {  // |y| < 2e-3
+  return fma(y * y, fma(y, fma(y, 1. / 24., 1. / 6.), .5), y);
+}
+__device__ __forceinline__ bool f64_pow_range(double x) {
+  return __double2hiint(x) >= 0x3eb00000 && __double2hiint(x) < 0x41300000;  // 2^-20 <= x < 2^20
+}
+__device__ __forceinline__ double pow_cp_rd(double x) {
+  constexpr double a = kCp / kRd, d = a - 3.5;
+  if (!f64_pow_range(x)) return pow(x, a);
+  // sqrt(x) = sh + sl
+  const double r = f64_rsqrt(x), sh = x * r, sl = fma(-sh, sh, x) * (.5 * r);
+  // x^3 = qh + ql, their product bh + bl
+  const double ph = x * x, pl = fma(x, x, -ph);
+  const double qh = ph * x, ql = fma(ph, x, -qh) + pl * x;
+  const double bh = qh * sh, bl = fma(qh, sh, -bh) + (qh * sl + ql * sh);
+  return bh + fma(bh, f64_expm1_small(d * f64_ln13(x)), bl);
+}
+__device__ __forceinline__ double pow_rd_cp(double x) {
+  // 2/7 = hi + lo
+  constexpr double b = kRd / kCp, h27 = 2. / 7., l27 = 1. / 63050394783186944.;  // 2/7 - h27 = 2^-54 2/7
+  constexpr double d = (b - h27) - l27;
+  if (!f64_pow_range(x)) return pow(x, b);
+  // v = x^(2/7) to FP32 accuracy, exact in FP64; v (1 - e)^(-1/7), e = 1 - v^7 / x^2
+  const double v = (double)exp2f(0.2857142857f * log2f((float)x));
+  const double rx = f64_recip(x), v2 = v * v;
+  const double e = fma(-((v2 * v2) * (v2 * v)) * rx, rx, 1.);
+  const double c = fma(e * e, 4. / 49., e * (1. / 7.));
+  const double g = f64_expm1_small(d * f64_ln13(x));
+  return fma(v, fma(c, g, c + g), v);
+}
+__device__ __forceinline__ float pow_cp_rd(float x) { return pow(x, float(kCp) / float(kRd)); }
+__device__ __forceinline__ float pow_rd_cp(float x) { return pow(x, float(kRd) / float(kCp)); }
+
 // ---- float-float arithmetic (FP32-mixed build) ----------------------------
 // A value hi + lo with |lo| <= ulp(hi)/2 carries ~48 significant bits on the
 // FP32 pipes, which GB300 runs at 64x its FP64 rate.  two_sum and two_prod are
