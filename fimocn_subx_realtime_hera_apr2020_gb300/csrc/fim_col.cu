@@ -597,10 +597,9 @@ template <typename R>
 __device__ __forceinline__ R fill_thin() { return R(1.2e-4); }
 
 // PLM slope of a layer from its filled value f and its neighbours' fm, fp
-template <typename R>
-__device__ __forceinline__ R plm_slope(R fm, R f, R fp) {
-  const R b = ((fp - fm) * (fm + fp - R(2) * f) > R(0)) ? f - fm : fp - f;
-  return (f <= cmin(fm, fp) || f >= cmax(fm, fp)) ? R(0) : b;
+__device__ __forceinline__ float plm_slope(float fm, float f, float fp) {
+  const float b = ((fp - fm) * (fm + fp - 2.f * f) > 0.f) ? f - fm : fp - f;
+  return (f <= fminf(fm, fp) || f >= fmaxf(fm, fp)) ? 0.f : b;
 }
 
 // FP64: monotonicity and the slope's sign by integer comparisons (a zero
@@ -695,6 +694,18 @@ static_assert(sizeof(RemapV<float, 1, 1>) % 16 == 0 && sizeof(RemapV<double, 1, 
 __device__ __forceinline__ float by_cp(float x) { return x / float(kCp); }
 __device__ __forceinline__ double by_cp(double x) { return f64_quot(x, kCp, 1. / kCp); }
 
+// Level kb + v of a column of L levels held VL a lane by W lanes: with FULL the
+// column fills the lanes (L == W VL), so that the tests cost nothing but for
+// the first and last lane's end levels.
+template <int VL, int W, bool FULL>
+struct Lv {
+  int L, lane;
+  __device__ __forceinline__ int k(int v) const { return lane * VL + v; }
+  __device__ __forceinline__ bool in(int v) const { return FULL || k(v) < L; }
+  __device__ __forceinline__ bool first(int v) const { return FULL ? v == 0 && lane == 0 : k(v) == 0; }
+  __device__ __forceinline__ bool last(int v) const { return FULL ? v == VL - 1 && lane == W - 1 : k(v) == L - 1; }
+};
+
 // pcwise's coordinate quantities for one lane's levels and interfaces
 template <typename R, int VL>
 struct LaneGeo {
@@ -715,18 +726,19 @@ __device__ __forceinline__ R coord_thick(bool flip, const R* x, int k) {
   return flip ? cmax(R(0), (-x[k + 1]) - (-x[k])) : cmax(R(0), x[k + 1] - x[k]);
 }
 
-template <typename R, int VL, int W = 32>
+template <typename R, int VL, int W, bool FULL>
 __device__ __forceinline__ void lane_geo(int L, int lane, const R* xo, const R* xn, LaneGeo<R, VL>& G) {
   const R small = R(1.e-22);
   const bool flip = !(xo[0] < xo[L]);
   const int kb = lane * VL;
+  const Lv<VL, W, FULL> lv{L, lane};
   bool thin = false;
   unsigned up = 0u;
 #pragma unroll
   for (int v = 0; v < VL; v++) {
     const int k = kb + v;
     R fo = R(0), fn = R(0);
-    if (k < L) {
+    if (lv.in(v)) {
       fo = coord_thick(flip, xo, k);
       fn = coord_thick(flip, xn, k);
       thin = thin || fo < fill_thin<R>();
@@ -735,7 +747,7 @@ __device__ __forceinline__ void lane_geo(int L, int lane, const R* xo, const R* 
     if constexpr (sizeof(R) == 4) G.rfo[v] = fdiv(R(1), fo + small);
     G.rfn[v] = recip(fn + small);
     R nd = R(0), hh = R(0);
-    if (k >= 1 && k <= L - 1) {
+    if (lv.in(v) && !lv.first(v)) {
       const R d = flip ? (-xn[k]) - (-xo[k]) : xn[k] - xo[k];
       if (d != R(0)) {
         const R fl = coord_thick(flip, xo, d > R(0) ? k : k - 1);
@@ -776,10 +788,10 @@ __device__ __forceinline__ void lane_geo(int L, int lane, const R* xo, const R* 
 // sums and cost 0.49 ms a step at glvl 8 (a tenth of the remap), so it runs
 // in the FP64 build, and the FP32-mixed build keeps the two physical column
 // checks (restp_1d's, and remap_1d's theta integral).
-template <typename R, int VL, int NF, int W = 32>
+template <typename R, int VL, int NF, int W, bool FULL>
 __device__ __forceinline__ bool pcwise_v(int L, int lane, R (&y)[NF][VL], const LaneGeo<R, VL>& G) {
   const R small = R(1.e-22);
-  const int kb = lane * VL;
+  const Lv<VL, W, FULL> lv{L, lane};
   R bfore[NF], colscl[NF];
   if (sizeof(R) == 8) {
 #pragma unroll
@@ -788,7 +800,7 @@ __device__ __forceinline__ bool pcwise_v(int L, int lane, R (&y)[NF][VL], const 
       colscl[h] = R(0);
 #pragma unroll
       for (int v = 0; v < VL; v++)
-        if (kb + v < L) {
+        if (lv.in(v)) {
           bfore[h] += y[h][v] * G.fo[v];
           colscl[h] += cabs(y[h][v] * G.fo[v]);
         }
@@ -803,11 +815,10 @@ __device__ __forceinline__ bool pcwise_v(int L, int lane, R (&y)[NF][VL], const 
       R a = R(1), b = R(0);
 #pragma unroll
       for (int v = VL - 1; v >= 0; v--) {
-        const int k = kb + v;
-        if (k == L - 1) {
+        if (lv.last(v)) {
           a = R(0);
           b = y[h][v];
-        } else if (k < L) {
+        } else if (lv.in(v)) {
           const R A = small * G.rfo[v];
           b = A * b + y[h][v] * G.fo[v] * G.rfo[v];
           a = A * a;
@@ -816,9 +827,8 @@ __device__ __forceinline__ bool pcwise_v(int L, int lane, R (&y)[NF][VL], const 
       R x = affine_entry_down<R, W>(lane, a, b);
 #pragma unroll
       for (int v = VL - 1; v >= 0; v--) {
-        const int k = kb + v;
-        if (k == L - 1) x = y[h][v];
-        else if (k < L) x = (y[h][v] * G.fo[v] + x * small) * G.rfo[v];
+        if (lv.last(v)) x = y[h][v];
+        else if (lv.in(v)) x = (y[h][v] * G.fo[v] + x * small) * G.rfo[v];
         nb[h][v] = x;
       }
     }
@@ -828,11 +838,10 @@ __device__ __forceinline__ bool pcwise_v(int L, int lane, R (&y)[NF][VL], const 
       R a = R(1), b = R(0);
 #pragma unroll
       for (int v = 0; v < VL; v++) {
-        const int k = kb + v;
-        if (k == 0) {
+        if (lv.first(v)) {
           a = R(0);
           b = nb[h][v];
-        } else if (k < L) {
+        } else if (lv.in(v)) {
           const R A = small * G.rfo[v];
           b = A * b + nb[h][v] * G.fo[v] * G.rfo[v];
           a = A * a;
@@ -841,9 +850,8 @@ __device__ __forceinline__ bool pcwise_v(int L, int lane, R (&y)[NF][VL], const 
       R x = affine_entry_up<R, W>(lane, a, b);
 #pragma unroll
       for (int v = 0; v < VL; v++) {
-        const int k = kb + v;
-        if (k == 0) x = nb[h][v];
-        else if (k < L) x = (nb[h][v] * G.fo[v] + x * small) * G.rfo[v];
+        if (lv.first(v)) x = nb[h][v];
+        else if (lv.in(v)) x = (nb[h][v] * G.fo[v] + x * small) * G.rfo[v];
         yf[h][v] = x;
       }
     }
@@ -862,10 +870,9 @@ __device__ __forceinline__ bool pcwise_v(int L, int lane, R (&y)[NF][VL], const 
     R bk[VL];
 #pragma unroll
     for (int v = 0; v < VL; v++) {
-      const int k = kb + v;
       const R fm = v > 0 ? yf[h][v - 1] : ym;
       const R fp = v < VL - 1 ? yf[h][v + 1] : yp;
-      bk[v] = (k >= 1 && k <= L - 2) ? plm_slope(fm, yf[h][v], fp) : R(0);
+      bk[v] = lv.in(v) && !lv.first(v) && !lv.last(v) ? plm_slope(fm, yf[h][v], fp) : R(0);
     }
     // interface fluxes; one donor layer: vertfx = -dz * (fcdx * slab) / slab = -dz * fcdx
     const R bm = __shfl_up_sync(0xffffffffu, bk[VL - 1], 1, W);
@@ -881,9 +888,8 @@ __device__ __forceinline__ bool pcwise_v(int L, int lane, R (&y)[NF][VL], const 
     R after = R(0);
 #pragma unroll
     for (int v = 0; v < VL; v++) {
-      const int k = kb + v;
-      if (k < L) {
-        const R vn = (k + 1 < L) ? (v < VL - 1 ? fl[v + 1] : fnext) : R(0);
+      if (lv.in(v)) {
+        const R vn = !lv.last(v) ? (v < VL - 1 ? fl[v + 1] : fnext) : R(0);
         const R amount = yf[h][v] * G.fo[v] - (vn - fl[v]);
         after += amount;
         y[h][v] = (amount + yf[h][v] * small) * G.rfn[v];
@@ -900,7 +906,7 @@ __device__ __forceinline__ bool pcwise_v(int L, int lane, R (&y)[NF][VL], const 
 
 // remap_1d's fill of thin layers from above for tracers 2..ntra (thktop = 0):
 // y(k) = (y(k) dp(k) + y(k-1) small) / (dp(k) + small), k = 3..nvl
-template <typename R, int VL, int NF, int W = 32>
+template <typename R, int VL, int NF, int W, bool FULL>
 __device__ __forceinline__ void fill_from_above(int L, int lane, R (&y)[NF][VL], const R (&dpv)[VL],
                                                 const R (&qqv)[VL]) {
   const R small = R(1.e-6);
@@ -962,6 +968,17 @@ __device__ __forceinline__ void store_levels(R* dst, int L, int kb, int vec, con
   }
 }
 
+// one lane's levels from shared memory (n of the VL lie in the column)
+template <typename R, int VL, bool FULL>
+__device__ __forceinline__ void ld_levels(const R* p, int n, R (&y)[VL]) {
+  if constexpr (FULL && VL * sizeof(R) <= 16) {
+    ldv<VL>(p, y);
+  } else {
+#pragma unroll
+    for (int v = 0; v < VL; v++) y[v] = FULL || v < n ? p[v] : R(0);
+  }
+}
+
 // tracer t (0-based, >= 1) of column i leaving the remap when tracer x
 // thickness is formed here: hystat's floor for tracers 2 and 3 (applied to y,
 // which the caller then stores), then trdp = y * dp (hystat.F90:90-101)
@@ -1003,7 +1020,7 @@ __global__ void __launch_bounds__(32 * kWarpsInflate) k_inflate(Grid<R> g, Strid
 // vec: every field column starts on a min(16, VL*sizeof(R))-byte boundary
 // and nvl is a multiple of VL (the copies and stores are then VL wide)
 // WL: lanes per column (32, or 16 with two columns per warp in hand)
-template <typename R, int VL, int WL>
+template <typename R, int VL, int WL, bool FULL>
 __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Strides s, Knobs kn,
     const StepParams* __restrict__ sp, const R* __restrict__ targt, const R* __restrict__ exsmo,
     R* __restrict__ us3d, R* __restrict__ vs3d, R* __restrict__ tr3d, R* __restrict__ sdot,
@@ -1100,9 +1117,7 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
       }
     } else {
 #pragma unroll
-      for (int h = 0; h < 3; h++)
-#pragma unroll
-        for (int v = 0; v < VL; v++) y[h][v] = kb + v < L ? S.ring[qs][hw][h][kb + v] : R(0);
+      for (int h = 0; h < 3; h++) ld_levels<R, VL, FULL>(&S.ring[qs][hw][h][kb], L - kb, y[h]);
     }
     __syncwarp();
     issue(ic, ij, qs);   // D items ahead, into the slot just read
@@ -1148,10 +1163,10 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
       for (int k = ls; k < L; k += WL) S.dkb[cs][k] = S.pk1new[hw][k] - S.pk1new[hw][k + 1];
       if (trdp)
         for (int k = ls; k < L; k += WL) S.dpb[cs][k] = S.dpcol[hw][k];
-      lane_geo<R, VL, WL>(L, ls, S.prcol[hw], S.prnew[hw], gp);
+      lane_geo<R, VL, WL, FULL>(L, ls, S.prcol[hw], S.prnew[hw], gp);
+      ld_levels<R, VL, FULL>(&S.dpcol[hw][kb], L - kb, dpv);
 #pragma unroll
       for (int v = 0; v < VL; v++) {
-        dpv[v] = kb + v < L ? S.dpcol[hw][kb + v] : R(0);
         qqv[v] = sizeof(R) == 4 || kn.thktop == 0. ? fdiv(R(1), dpv[v] + small) : R(0);
       }
       __syncwarp();
@@ -1159,12 +1174,12 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
       // theta in p^(kappa+1), held for the redistribution after the last column
       {
         LaneGeo<R, VL> gk;
-        lane_geo<R, VL, WL>(L, ls, S.pk1col[hw], S.pk1new[hw], gk);
+        lane_geo<R, VL, WL, FULL>(L, ls, S.pk1col[hw], S.pk1new[hw], gk);
         {
           R colin = R(0), colscl = R(0);
 #pragma unroll
           for (int v = 0; v < VL; v++)
-            if (kb + v < L) {
+            if (FULL || kb + v < L) {
               const R w = y[0][v] * (S.pk1col[hw][kb + v] - S.pk1col[hw][kb + v + 1]);
               colin += w;
               colscl += cabs(w);
@@ -1179,11 +1194,15 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
         R t[1][VL];
 #pragma unroll
         for (int v = 0; v < VL; v++) t[0][v] = y[0][v];
-        const bool bt = pcwise_v<R, VL, 1, WL>(L, ls, t, gk);
+        const bool bt = pcwise_v<R, VL, 1, WL, FULL>(L, ls, t, gk);
         bad |= valid && bt;
+        if constexpr (FULL) {
+          st_lane<R, VL>(&S.thb[cs][kb], t[0]);
+        } else {
 #pragma unroll
-        for (int v = 0; v < VL; v++)
-          if (kb + v < L) S.thb[cs][kb + v] = t[0][v];
+          for (int v = 0; v < VL; v++)
+            if (kb + v < L) S.thb[cs][kb + v] = t[0][v];
+        }
       }
       // u, v in pressure
       if constexpr (NT == 3) {
@@ -1193,7 +1212,7 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
           uv[0][v] = y[1][v];
           uv[1][v] = y[2][v];
         }
-        const bool bu = pcwise_v<R, VL, 2, WL>(L, ls, uv, gp);
+        const bool bu = pcwise_v<R, VL, 2, WL, FULL>(L, ls, uv, gp);
         bad |= valid && bu;
         if (valid) {
           store_levels<R, VL>(us3d + (size_t)i * L, L, kb, vec, uv[0]);
@@ -1205,7 +1224,7 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
           R t[1][VL];
 #pragma unroll
           for (int v = 0; v < VL; v++) t[0][v] = y[h][v];
-          const bool bu = pcwise_v<R, VL, 1, WL>(L, ls, t, gp);
+          const bool bu = pcwise_v<R, VL, 1, WL, FULL>(L, ls, t, gp);
           bad |= valid && bu;
           if (valid) store_levels<R, VL>(field(h, i), L, kb, vec, t[0]);
         }
@@ -1214,9 +1233,9 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
       // tracers 2..ntra in pressure
       const int o0 = 3 * (j - 1);
       if constexpr (NT == 3) {
-        const bool bq = pcwise_v<R, VL, 3, WL>(L, ls, y, gp);
+        const bool bq = pcwise_v<R, VL, 3, WL, FULL>(L, ls, y, gp);
         bad |= valid && bq;
-        if (kn.thktop == 0.) fill_from_above<R, VL, 3, WL>(L, ls, y, dpv, qqv);
+        if (kn.thktop == 0.) fill_from_above<R, VL, 3, WL, FULL>(L, ls, y, dpv, qqv);
 #pragma unroll
         for (int h = 0; h < 3; h++)
           if (valid && o0 + h < F) {
@@ -1230,9 +1249,9 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
             R t[1][VL];
 #pragma unroll
             for (int v = 0; v < VL; v++) t[0][v] = y[h][v];
-            const bool bq = pcwise_v<R, VL, 1, WL>(L, ls, t, gp);
+            const bool bq = pcwise_v<R, VL, 1, WL, FULL>(L, ls, t, gp);
             bad |= valid && bq;
-            if (kn.thktop == 0.) fill_from_above<R, VL, 1, WL>(L, ls, t, dpv, qqv);
+            if (kn.thktop == 0.) fill_from_above<R, VL, 1, WL, FULL>(L, ls, t, dpv, qqv);
             if (valid) {
               if (trdp) tracer_out<R, VL>(o0 + h - 2, qvmin, qwmin, dpv, t[0], trdp, (size_t)N * L, i, L, kb, vec);
               store_levels<R, VL>(field(o0 + h, i), L, kb, vec, t[0]);
@@ -1333,8 +1352,7 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
   __syncthreads();
   for (int cc = hw; cc < ncol; cc += H) {
     R y[VL];
-#pragma unroll
-    for (int v = 0; v < VL; v++) y[v] = kb + v < L ? S.thb[cc][kb + v] : R(0);
+    ld_levels<R, VL, FULL>(&S.thb[cc][kb], L - kb, y);
     store_levels<R, VL>(tr3d + (size_t)(c0 + cc) * L, L, kb, vec, y);
     if (trdp) {
       R z[VL];
@@ -1382,23 +1400,25 @@ int remap_columns(int N, int members, bool paired) {
   return cols;
 }
 
+template <typename R, int VL, int WL>
+cudaError_t remap_v_attr() {
+  const int bytes = (int)remap_v_smem<R, VL, WL>();
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_remap_v<R, VL, WL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return e != cudaSuccess ? e
+                          : cudaFuncSetAttribute(k_remap_v<R, VL, WL, false>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 template <typename R>
 int prepare_hybgen(int L) {
   cudaError_t e = cudaSuccess;
   const int vl = remap_vl(L);
   if (remap_paired<R>(L)) {
-    if constexpr (sizeof(R) == 4)
-      e = cudaFuncSetAttribute(k_remap_v<R, 4, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)remap_v_smem<R, 4, 16>());
-  } else if (vl == 1)
-    e = cudaFuncSetAttribute(k_remap_v<R, 1, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)remap_v_smem<R, 1, 32>());
-  else if (vl == 2)
-    e = cudaFuncSetAttribute(k_remap_v<R, 2, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)remap_v_smem<R, 2, 32>());
-  else
-    e = cudaFuncSetAttribute(k_remap_v<R, 4, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)remap_v_smem<R, 4, 32>());
+    if constexpr (sizeof(R) == 4) e = remap_v_attr<R, 4, 16>();
+  } else if (vl == 1) e = remap_v_attr<R, 1, 32>();
+  else if (vl == 2) e = remap_v_attr<R, 2, 32>();
+  else e = remap_v_attr<R, 4, 32>();
   if (e == cudaSuccess) {
     if (L <= 64)
       e = cudaFuncSetAttribute(k_inflate<R, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1825,15 +1845,20 @@ bool launch_hybgen(const Launch& l, const Grid<R>& g, const Strides& s, const Kn
     for (const void* p : {(const void*)us3d, (const void*)vs3d, (const void*)tr3d})
       if ((uintptr_t)p % cb != 0) vec = 0;
     FIM_KBEGIN(l, "k_remap");
+    // a column that fills its lanes, copied 16 bytes at a time, needs no level tests
 #define FIM_REMAP_V(VL, WL)                                                                                  \
-  k_remap_v<R, VL, WL><<<gw, 32 * kWarpsRemapV, remap_v_smem<R, VL, WL>(), l.stream>>>(                       \
+  if (vec && g.L == VL * WL) FIM_REMAP_VF(VL, WL, true);                                                     \
+  else FIM_REMAP_VF(VL, WL, false)
+#define FIM_REMAP_VF(VL, WL, FULL)                                                                           \
+  k_remap_v<R, VL, WL, FULL><<<gw, 32 * kWarpsRemapV, remap_v_smem<R, VL, WL>(), l.stream>>>(                 \
       g, s, kn, l.sp, targt, ex_in, us3d, vs3d, tr3d, sdot, ex3d, dp3d, pr3d, l.flags, l.boundary, vec, trdp, cpw)
     if (paired) {
-      if constexpr (sizeof(R) == 4) FIM_REMAP_V(4, 16);
-    } else if (vl == 1) FIM_REMAP_V(1, 32);
-    else if (vl == 2) FIM_REMAP_V(2, 32);
-    else FIM_REMAP_V(4, 32);
+      if constexpr (sizeof(R) == 4) { FIM_REMAP_V(4, 16); }
+    } else if (vl == 1) { FIM_REMAP_V(1, 32); }
+    else if (vl == 2) { FIM_REMAP_V(2, 32); }
+    else { FIM_REMAP_V(4, 32); }
 #undef FIM_REMAP_V
+#undef FIM_REMAP_VF
     trdp_done = trdp != nullptr;
   } else if (g.L <= 64) {
     FIM_KBEGIN(l, "k_remap");
