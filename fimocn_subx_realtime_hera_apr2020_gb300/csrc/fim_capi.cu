@@ -62,8 +62,7 @@ struct fim_ctx {
   int graph_gen = 0;
   // fim_step_io's copy streams (host to device, device to host) and events
   cudaStream_t io_in = nullptr, io_out = nullptr;
-  // the branch of a step that forms the budget sums beside momtum (they share
-  // no written data), forked from and joined to the step's stream
+  // the branch of a step (enqueue_step), forked from and joined to its stream
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int prio = 0;  // priority of the streams above (fim_config.stream_priority, clamped)
@@ -1128,8 +1127,24 @@ int enqueue_step(fim_ctx* c, fim_state* st, StepIo* io = nullptr) {
                    F<R>(st, FIM_TR3D), F<R>(st, FIM_TRDP), F<R>(st, FIM_PSRF), F<R>(st, FIM_PTDCY), st->mpf,
                    trdp_done);
   if (io && (rc = io_download(*io, kIoA, 0, 0))) return rc;
-  // one member group and no host transfers: the budget sums run beside momtum
-  const bool branch = !io && c->G == c->M && c->aux;
+  // Without host transfers (whose copies order the stages) two parts of a
+  // group's dynamics run on a branch beside the main chain, since they share
+  // no written data with it: edgvar3's layer-thickness edges beside edgvar1,
+  // and pressure, Exner function and omega (cnuity5), dissip and momtum beside
+  // the tracer transport.  A small grid's kernels do not fill the chip, so the
+  // branch hides behind the chain (glvl 5 / nvl 38: BR_SMALL); at glvl 8 they do and
+  // it costs nothing (BR_LARGE).  Per-kernel timing keeps one chain.
+  const bool branch = !io && !c->prof.on && c->aux;
+  auto fork = [&]() -> int {
+    CK(cudaEventRecord(c->ev_fork, c->stream), "step fork");
+    CK(cudaStreamWaitEvent(c->aux, c->ev_fork, 0), "step fork");
+    return FIM_OK;
+  };
+  auto join = [&]() -> int {
+    CK(cudaEventRecord(c->ev_join, c->aux), "step join");
+    CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0), "step join");
+    return FIM_OK;
+  };
   // the dynamics of the step, one member group at a time; the edge work
   // fields and the scratch hold one group, the prognostic fields all members
   for (int m0 = 0; m0 < M; m0 += c->G) {
@@ -1142,6 +1157,9 @@ int enqueue_step(fim_ctx* c, fim_state* st, StepIo* io = nullptr) {
       return (R*)st->f[f] + (st->slots[f] == M ? (size_t)m0 * st->count[f] : (size_t)0);
     };
     float2* mpf = st->mpf ? st->mpf + (size_t)m0 * st->count[FIM_MP3D] : nullptr;
+    Launch lb2 = lg;  // the branch's launches
+    if (branch) lb2.stream = c->aux;
+    if (branch && c->kn.hi_order && (rc = fork())) return rc;
     launch_edgvar1<R>(lg, g, s, c->kn.hi_order, P(FIM_US3D), P(FIM_VS3D), P(FIM_DP3D),
                       P(FIM_PR3D), P(FIM_MP3D), P(FIM_TR3D), P(FIM_U_EDG),
                       P(FIM_V_EDG), P(FIM_DP_EDG), P(FIM_LP_EDG), P(FIM_MONT_EDG),
@@ -1154,8 +1172,9 @@ int enqueue_step(fim_ctx* c, fim_state* st, StepIo* io = nullptr) {
       // used (k_cnuity12); mass_adv reads the averaged dp edges, so it keeps
       // the pass.  The tracers' edge values are formed on chip by the tracer
       // kernels
-      launch_edgvar3<R>(lg, g, s, P(FIM_DP3D), P(FIM_TR3D), P(FIM_DP_EDG), P(FIM_TRC_EDG),
+      launch_edgvar3<R>(lb2, g, s, P(FIM_DP3D), P(FIM_TR3D), P(FIM_DP_EDG), P(FIM_TRC_EDG),
                         1, c->ftab, c->cfg.flux_conserv_schm != 1);
+      if (branch && (rc = join())) return rc;
     }
     CnuityScratch<R> cw{(R*)c->antifx, (R*)c->delp_lo, (R*)c->p_plus, (R*)c->p_mnus, (R*)c->r_plus, (R*)c->r_mnus};
     if (io && (rc = io_wait(*io, io->up_ev[kIoC]))) return rc;
@@ -1163,11 +1182,17 @@ int enqueue_step(fim_ctx* c, fim_state* st, StepIo* io = nullptr) {
       launch_cnuity<R>(lg, g, s, cw, P(FIM_US3D), P(FIM_VS3D), P(FIM_U_EDG), P(FIM_V_EDG),
                        P(FIM_DP_EDG), P(FIM_LP_EDG), P(FIM_DP3D), P(FIM_PR3D),
                        P(FIM_EX3D), P(FIM_DP_TDCY), P(FIM_DPL_TDCY), P(FIM_MASSFX),
-                       P(FIM_WS3D));
+                       P(FIM_WS3D), !branch);
     else
       launch_massadv<R>(lg, g, s, cw, P(FIM_US3D), P(FIM_VS3D), P(FIM_U_EDG), P(FIM_V_EDG),
                         P(FIM_DP_EDG), P(FIM_LP_EDG), P(FIM_DP3D), P(FIM_PR3D),
                         P(FIM_EX3D), P(FIM_DP_TDCY), P(FIM_MASSFX), P(FIM_WS3D));
+    if (branch) {
+      if ((rc = fork())) return rc;
+      if (c->cfg.flux_conserv_schm == 1)
+        launch_cnuity5<R>(lb2, g, s, P(FIM_PR3D), P(FIM_DP3D), P(FIM_EX3D), P(FIM_DP_TDCY), P(FIM_WS3D),
+                          P(FIM_LP_EDG), P(FIM_US3D), P(FIM_VS3D), 0);
+    }
     if (c->TB > 0) {
       // class-B transport (dyn_run.F90:388-403); transp2/transp0 act at steps
       // with mod(its, dtratio) == 0, decided per member on the device
@@ -1177,21 +1202,23 @@ int enqueue_step(fim_ctx* c, fim_state* st, StepIo* io = nullptr) {
       launch_transp0<R>(lg, g, s, c->dtratio, P(FIM_CUMUFX), P(FIM_DP3D), P(FIM_DPINIT));
     }
     if (io && (rc = io_download(*io, kIoC, 0, 0))) return rc;
-    // momtum reads theta's edge values (edgvar1), the edge winds and the new
-    // thicknesses, none of which the tracer transport writes, and writes
-    // nothing it reads: with host transfers it runs first, so the step ends on
-    // the tracer chunks whose results stream out as they finish
-    auto momentum = [&]() -> int {
+    // momtum reads theta's edge values (edgvar1), the edge winds, the Exner
+    // function and the new thicknesses, none of which the tracer transport
+    // writes, and writes nothing it reads: with host transfers it runs first,
+    // so the step ends on the tracer chunks whose results stream out as they
+    // finish
+    auto momentum = [&](const Launch& lm) -> int {
       if (io && (rc = io_wait(*io, io->up_ev[kIoU]))) return rc;
       MomtumScratch<R> mw{(R*)c->du, (R*)c->dv, (R*)c->wu, (R*)c->wv};
-      launch_momtum<R>(lg, g, s, c->kn, mw, P(FIM_US3D), P(FIM_VS3D), P(FIM_EX3D),
+      launch_momtum<R>(lm, g, s, c->kn, mw, P(FIM_US3D), P(FIM_VS3D), P(FIM_EX3D),
                        P(FIM_RELVOR), P(FIM_U_EDG), P(FIM_V_EDG), P(FIM_TRC_EDG),
                        P(FIM_MONT_EDG), P(FIM_UVSQ_EDG), P(FIM_U_TDCY), P(FIM_V_TDCY),
                        P(FIM_DP3D), mpf, (const R*)st->thold);
       if (io && (rc = io_download(*io, kIoU, 0, 0))) return rc;
       return FIM_OK;
     };
-    if (io && (rc = momentum())) return rc;
+    if (io && (rc = momentum(lg))) return rc;
+    if (branch && (rc = momentum(lb2))) return rc;
     if (c->kn.hi_order) {
       TrcFusedScratch<R> fw{(R*)c->f_trcr_lo, (R*)c->f_sp, (R*)c->f_sm, (R*)c->f_trold, (R*)c->f_rp, (R*)c->f_rm,
                             (R*)c->f_af,
@@ -1206,29 +1233,14 @@ int enqueue_step(fim_ctx* c, fim_state* st, StepIo* io = nullptr) {
       if (io) io_chunk_hook(io, 1, 0, c->T);
     }
     if (io && io->rc) return io->rc;
-    if (branch) {
-      // budgets of the state the step returns, on the branch stream beside
-      // momtum: they read the thicknesses and tracers, which momtum does not
-      // write, and momtum reads nothing they write
-      CK(cudaEventRecord(c->ev_fork, c->stream), "step fork");
-      CK(cudaStreamWaitEvent(c->aux, c->ev_fork, 0), "step fork");
-      Launch la = l;
-      la.stream = c->aux;
-      launch_globsum<R>(la, g, s, c->T + c->TB, F<R>(st, FIM_DP3D), F<R>(st, FIM_TR3D), (const R*)nullptr,
-                        (const R*)nullptr, F<R>(st, FIM_PR3D), F<R>(st, FIM_EX3D), (const R*)nullptr,
-                        c->gs_partial, st->sums);
-      CK(cudaEventRecord(c->ev_join, c->aux), "step join");
-    }
-    if (!io && (rc = momentum())) return rc;
+    if (branch) rc = join();
+    else if (!io) rc = momentum(lg);
+    if (rc) return rc;
   }
-  if (branch) {
-    CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0), "step join");
-  } else {
-    // budgets of the state the step returns
-    launch_globsum<R>(l, g, s, c->T + c->TB, F<R>(st, FIM_DP3D), F<R>(st, FIM_TR3D), (const R*)nullptr,
-                      (const R*)nullptr,
-                      F<R>(st, FIM_PR3D), F<R>(st, FIM_EX3D), (const R*)nullptr, c->gs_partial, st->sums);
-  }
+  // budgets of the state the step returns
+  launch_globsum<R>(l, g, s, c->T + c->TB, F<R>(st, FIM_DP3D), F<R>(st, FIM_TR3D), (const R*)nullptr,
+                    (const R*)nullptr,
+                    F<R>(st, FIM_PR3D), F<R>(st, FIM_EX3D), (const R*)nullptr, c->gs_partial, st->sums);
   if (io && (rc = io_download(*io, kIoE, 0, 0))) return rc;
   return FIM_OK;
 }

@@ -8,6 +8,7 @@
 // globsum accumulates per thread (FP64, or float-float compensated sums in the
 // FP32 build, whose error is that of an FP64 sum) and reduces per block into a
 // deterministic partial buffer.
+#include <algorithm>
 #include <cstdint>
 
 #include "fim_internal.h"
@@ -1620,7 +1621,7 @@ constexpr int kMaxT = 32;
 constexpr int kGsCol = kMaxT + 1;
 constexpr int kGsSlots = kMaxT + 5;
 
-// Level sums: a block takes one chunk of kGsChunkPer(VK) cell-levels and a
+// Level sums: a block takes one chunk of 256 VK iters cell-levels and a
 // group of kGsGroup consecutive slots q (0: area x dp, 1..ntr: area x dp x
 // tracer q-1): it reads the chunk's thicknesses and cell areas once for the
 // group and one tracer array per slot.  The group holding slot 0 also forms
@@ -1629,9 +1630,19 @@ constexpr int kGsSlots = kMaxT + 5;
 // and the partials are per (chunk, slot): the sums are deterministic and do
 // not depend on the grouping.
 constexpr int kGsGroup = 7;
-constexpr int kGsIter = 16;
-template <int VK>
-__host__ __device__ constexpr int kGsChunkPer() { return kBlock2 * VK * kGsIter; }
+// Iterations of a block: 16 where that leaves at least four blocks an SM, fewer
+// for small grids (glvl 5 / nvl 38: 24 blocks of 16 took GS_OLD us, 380 of one
+// GS_NEW us).  A function of the grid alone: the sums do not depend on the
+// tracers or members beside them.
+inline int gs_iters(long long NL, int vk) {
+  int it = 16;
+  while (it > 1 && NL / ((long long)kBlock2 * vk * it) < 608) it /= 2;
+  return it;
+}
+inline int gs_chunks(long long NL, int vk) {
+  const long long per = (long long)kBlock2 * vk * gs_iters(NL, vk);
+  return (int)((NL + per - 1) / per);
+}
 
 template <typename R, int VK> struct GsVec;
 template <typename R> struct GsVec<R, 1> {
@@ -1650,11 +1661,40 @@ template <> struct GsVec<double, 2> {
   }
 };
 
+// One step of a warp's sums of 2 n values: the lanes with bit `off` set keep
+// the upper n values' sums of their pair, the others the lower.
+template <int n>
+__device__ __forceinline__ void tree_step(int lane, int off, double* v) {
+  const bool up = lane & off;
+#pragma unroll
+  for (int i = 0; i < n; i++) {
+    const double give = up ? v[i] : v[n + i], keep = up ? v[n + i] : v[i];
+    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+  }
+}
+// sums of eight values over a warp: v[0] of a lane ends as the sum of value
+// warp_tree8's result (the same in each four lanes)
+__device__ __forceinline__ int warp_tree8(int lane, double (&v)[8]) {
+  tree_step<4>(lane, 16, v);
+  tree_step<2>(lane, 8, v);
+  tree_step<1>(lane, 4, v);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  return (lane & 16 ? 4 : 0) + (lane & 8 ? 2 : 0) + (lane & 4 ? 1 : 0);
+}
+__device__ __forceinline__ int warp_tree4(int lane, double (&v)[4]) {
+  tree_step<2>(lane, 16, v);
+  tree_step<1>(lane, 8, v);
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+  return (lane & 16 ? 2 : 0) + (lane & 8 ? 1 : 0);
+}
+
 template <typename R, int VK>
 __global__ void __launch_bounds__(kBlock2) k_globsum_levels(Grid<R> g, Strides s, const StepParams* __restrict__ sp,
     int T, const R* __restrict__ dp3d, const R* __restrict__ tr, const R* __restrict__ rn2d, const R* __restrict__ rc2d,
     const R* __restrict__ pr3d, const R* __restrict__ ex3d, const R* __restrict__ qf2d,
-    double* __restrict__ partial, int nchunk) {
+    double* __restrict__ partial, int nchunk, int iters) {
   const int N = g.N, L = g.L, L1 = L + 1;
   const size_t m = blockIdx.y;
   sp += m;
@@ -1665,7 +1705,7 @@ __global__ void __launch_bounds__(kBlock2) k_globsum_levels(Grid<R> g, Strides s
   dp3d += m * s.cell; tr += m * s.tr; pr3d += m * s.intf; ex3d += m * s.intf;
   // N * L < 2^31 (checked on the host): 32-bit cell-level indices
   const unsigned NL = (unsigned)N * (unsigned)L;
-  constexpr int CH = kGsChunkPer<VK>();
+  const unsigned CH = kBlock2 * VK * (unsigned)iters;
   const unsigned e0 = (unsigned)chunk * CH;
   Acc<R> acc[kGsGroup];
   // the group's arrays: slot 0 reads the thicknesses again (an L1 hit) and
@@ -1695,9 +1735,9 @@ __global__ void __launch_bounds__(kBlock2) k_globsum_levels(Grid<R> g, Strides s
       }
   };
   if (e0 + CH <= NL) {
-    for (int it = 0; it < kGsIter; it++) sum_at(e0 + ((unsigned)it * kBlock2 + threadIdx.x) * VK);
+    for (int it = 0; it < iters; it++) sum_at(e0 + ((unsigned)it * kBlock2 + threadIdx.x) * VK);
   } else {
-    for (int it = 0; it < kGsIter; it++) {
+    for (int it = 0; it < iters; it++) {
       const unsigned idx = e0 + ((unsigned)it * kBlock2 + threadIdx.x) * VK;
       if (idx < NL) sum_at(idx);
     }
@@ -1720,49 +1760,52 @@ __global__ void __launch_bounds__(kBlock2) k_globsum_levels(Grid<R> g, Strides s
       col[3] += a * den * qf * dt / (1.25 * 2.5e6);
     }
   }
-  __shared__ double red[kBlock2 / 32];
+  // block sums: each warp's tree over its lanes (pairs 16, 8, 4, 2, 1 apart,
+  // the slots of a group in different lanes from the first pair on, so a step
+  // adds for all of them), then over the warps in order
+  __shared__ double red[kBlock2 / 32][kGsGroup + 5];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < kGsGroup; u++) v[u] = acc[u].value();
+    v[7] = 0.;
+    const int u = warp_tree8(lane, v);
+    if ((lane & 3) == 0 && u < kGsGroup) red[wib][u] = v[0];
+  }
+  if (q0 == 0) {
+    const int w = warp_tree4(lane, col);
+    if ((lane & 7) == 0) red[wib][kGsGroup + w] = col[0];
+  }
+  __syncthreads();
   double* out = partial + (m * nchunk + chunk) * kGsSlots;
-  const int nout = nq + (q0 == 0 ? 4 : 0);
-#pragma unroll
-  for (int u = 0; u < kGsGroup + 4; u++) {
-    if (u >= nout) break;  // uniform across the block
-    double v = 0.;
-#pragma unroll
-    for (int w = 0; w < kGsGroup; w++)
-      if (w == u) v = acc[w].value();
-#pragma unroll
-    for (int w = 0; w < 4; w++)
-      if (u == nq + w) v = col[w];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if (lane == 0) red[wib] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < kBlock2 / 32; w++) t += red[w];
-      out[u < nq ? q0 + u : kGsCol + (u - nq)] = t;
-    }
-    __syncthreads();
+  const int u = threadIdx.x;
+  if (u < nq || (q0 == 0 && u >= kGsGroup && u < kGsGroup + 4)) {
+    double t = 0.0;
+    for (int w = 0; w < kBlock2 / 32; w++) t += red[w][u];
+    out[u < nq ? q0 + u : kGsCol + (u - kGsGroup)] = t;
   }
 }
 
-// Final reduction of the block partials; one warp per output slot.
+// Final reduction of the block partials; one warp per output slot, a block per
+// member and eight slots.
 template <typename R>
-__global__ void k_globsum_final(const StepParams* __restrict__ sp, int T, const double* __restrict__ partial,
+__global__ void __launch_bounds__(kBlock2) k_globsum_final(const StepParams* __restrict__ sp, int T, const double* __restrict__ partial,
                                 int nblk, double* __restrict__ sums) {
   const size_t m = blockIdx.x;
   sp += m;
   if (!sp->active) return;
   const int lane = threadIdx.x & 31;
   double* out = sums + m * (8 + T);
-  for (int j = threadIdx.x >> 5; j < T + 5; j += blockDim.x >> 5) {
+  const int j = blockIdx.y * (kBlock2 / 32) + (threadIdx.x >> 5);
+  if (j < T + 5) {
     const int q = j <= T ? j : kGsCol + (j - T - 1);
     double t = 0.;
+#pragma unroll 8
     for (int b = lane; b < nblk; b += 32) t += partial[(m * nblk + b) * kGsSlots + q];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
-    if (lane != 0) continue;
+    if (lane != 0) return;
     if (q == 0) {
       out[0] = t / kGrvity;
     } else if (q <= T) {
@@ -1890,11 +1933,12 @@ void launch_hystat(const Launch& l, const Grid<R>& g, const Strides& s, R* ph3d,
   FIM_KEND(l);
 }
 
-// partial buffer: the most chunks any layout uses (1 level a thread)
+// partial buffer: the most chunks any layout uses
 size_t globsum_partials(int N, int L, int T, int members) {
   (void)T;
-  const long long NL = (long long)N * L;
-  return (size_t)members * (size_t)((NL + kGsChunkPer<1>() - 1) / kGsChunkPer<1>()) * kGsSlots;
+  int n = 0;
+  for (int vk : {1, 2, 4}) n = std::max(n, gs_chunks((long long)N * L, vk));
+  return (size_t)members * (size_t)n * kGsSlots;
 }
 
 template <typename R>
@@ -1906,19 +1950,18 @@ void launch_globsum(const Launch& l, const Grid<R>& g, const Strides& s, int ntr
   const bool vec = g.L % VK == 0 && (uintptr_t)dp3d % (VK * sizeof(R)) == 0 && (uintptr_t)tr % (VK * sizeof(R)) == 0;
   const long long NL = (long long)g.N * g.L;
   const unsigned ngrp = (unsigned)(ntr + kGsGroup) / kGsGroup;
-  int nchunk;
+  const int vk = vec ? VK : 1, nchunk = gs_chunks(NL, vk), iters = gs_iters(NL, vk);
   if (vec) {
-    nchunk = (int)((NL + kGsChunkPer<VK>() - 1) / kGsChunkPer<VK>());
     k_globsum_levels<R, VK><<<dim3((unsigned)nchunk * ngrp, l.members), kBlock2, 0, l.stream>>>(
-        g, s, l.sp, ntr, dp3d, tr, rn2d, rc2d, pr3d, ex3d, qf2d, partial, nchunk);
+        g, s, l.sp, ntr, dp3d, tr, rn2d, rc2d, pr3d, ex3d, qf2d, partial, nchunk, iters);
   } else {
-    nchunk = (int)((NL + kGsChunkPer<1>() - 1) / kGsChunkPer<1>());
     k_globsum_levels<R, 1><<<dim3((unsigned)nchunk * ngrp, l.members), kBlock2, 0, l.stream>>>(
-        g, s, l.sp, ntr, dp3d, tr, rn2d, rc2d, pr3d, ex3d, qf2d, partial, nchunk);
+        g, s, l.sp, ntr, dp3d, tr, rn2d, rc2d, pr3d, ex3d, qf2d, partial, nchunk, iters);
   }
   FIM_KEND(l);
   FIM_KBEGIN(l, "k_globsum_final");
-  k_globsum_final<R><<<l.members, kBlock2, 0, l.stream>>>(l.sp, ntr, partial, nchunk, sums);
+  k_globsum_final<R><<<dim3(l.members, (unsigned)((ntr + 5 + kBlock2 / 32 - 1) / (kBlock2 / 32))), kBlock2, 0,
+                       l.stream>>>(l.sp, ntr, partial, nchunk, sums);
   FIM_KEND(l);
 }
 

@@ -1255,7 +1255,7 @@ void launch_edgvar3(const Launch& l, const Grid<R>& g, const Strides& s, const R
 template <typename R>
 void launch_cnuity(const Launch& l, const Grid<R>& g, const Strides& s, const CnuityScratch<R>& w, const R* u,
                    const R* v, const R* u_edg, const R* v_edg, const R* dp_edg, const R* lp_edg,
-                   R* delp, R* pres, R* exner, R* dp_tndcy, R* dplo_tndcy, R* massfx, R* omega) {
+                   R* delp, R* pres, R* exner, R* dp_tndcy, R* dplo_tndcy, R* massfx, R* omega, bool columns) {
   const int vk = pick_vk<R>(g.L, {u_edg, v_edg, dp_edg, delp, massfx, dplo_tndcy, dp_tndcy, w.antifx, w.delp_lo,
                                   w.p_plus, w.p_mnus, w.r_plus, w.r_mnus});
   if (l.coop) {
@@ -1300,7 +1300,7 @@ void launch_cnuity(const Launch& l, const Grid<R>& g, const Strides& s, const Cn
                                                          dplo_tndcy, dp_tndcy, delp, l.flags)));
   FIM_KEND(l);
   }
-  launch_cnuity5<R>(l, g, s, pres, delp, exner, dp_tndcy, omega, lp_edg, u, v, 0);
+  if (columns) launch_cnuity5<R>(l, g, s, pres, delp, exner, dp_tndcy, omega, lp_edg, u, v, 0);
 }
 
 template <typename R>
@@ -1359,7 +1359,9 @@ void launch_step_begin(const Launch& l, StepParams* sp) {
                                   int, const FrameTab&, bool);                                                                \
   template void launch_cnuity<R>(const Launch&, const Grid<R>&, const Strides&, const CnuityScratch<R>&,      \
                                  const R*, const R*, const R*, const R*, const R*, const R*, R*, R*, R*, R*,  \
-                                 R*, R*, R*);                                                                 \
+                                 R*, R*, R*, bool);                                                                 \
+  template void launch_cnuity5<R>(const Launch&, const Grid<R>&, const Strides&, R*, R*, R*, const R*, R*,    \
+                                  const R*, const R*, const R*, int);                                         \
   template void launch_massadv<R>(const Launch&, const Grid<R>&, const Strides&, const CnuityScratch<R>&,     \
                                   const R*, const R*, const R*, const R*, R*, const R*, R*, R*, R*, R*, R*,   \
                                   R*);                                                                       \

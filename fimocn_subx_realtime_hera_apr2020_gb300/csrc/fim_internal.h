@@ -460,7 +460,12 @@ struct CnuityScratch { R *antifx, *delp_lo, *p_plus, *p_mnus, *r_plus, *r_mnus; 
 template <typename R>
 void launch_cnuity(const Launch&, const Grid<R>&, const Strides&, const CnuityScratch<R>&, const R* u,
                    const R* v, const R* u_edg, const R* v_edg, const R* dp_edg, const R* lp_edg,
-                   R* delp, R* pres, R* exner, R* dp_tndcy, R* dplo_tndcy, R* massfx, R* omega);
+                   R* delp, R* pres, R* exner, R* dp_tndcy, R* dplo_tndcy, R* massfx, R* omega,
+                   bool columns = true);
+// cnuity5 (launch_cnuity runs it too when columns is set)
+template <typename R>
+void launch_cnuity5(const Launch&, const Grid<R>&, const Strides&, R* pres, R* delp, R* exner, const R* dp_tndcy,
+                    R* omega, const R* lp_edg, const R* u, const R* v, int ab3_delp);
 // flux_conserv_schm = 2 (the bounds use the r_plus/r_mnus scratch slots)
 template <typename R>
 void launch_massadv(const Launch&, const Grid<R>&, const Strides&, const CnuityScratch<R>&, const R* u,

@@ -638,12 +638,18 @@ struct TrOut {
   int tbase;
 };
 
+// q / ab1 x area: FP64 holds the factor once a cell; FP32 keeps two products
+// (theta's last bits decide branches of hybgen in the next step)
+__device__ __forceinline__ float per_ab1(float q, float rab1, float area) { return q * rab1 * area; }
+__device__ __forceinline__ double per_ab1(double q, double, double f) { return q * f; }
+
 // R+/R- of trcadv2 for frame cell xe at levels ve, from the staged old tracer
-// and trcr_lo, AB3 slots, S+/S- and thickness (arf = area / ab1); the bounds
+// and trcr_lo, AB3 slots, S+/S- and thickness (arf: the cell areas, in FP64
+// over ab1); the bounds
 // (clamped at zero) and the slots of/vof are returned for trcadv3
 template <typename R, int VK, int LK>
 __device__ __forceinline__ void limiters(const FrameSm& fs, const R* TO, const R* TL, const R* opq, const R* dpf,
-                                         const R* arf, int S1, int xe, int ve, R ab2, R ab3,
+                                         const R* arf, int S1, int xe, int ve, R ab2, R ab3, R rab1,
                                          R* Rp, R* Rm, R (&hx)[VK], R (&hn)[VK], R (&tof)[VK], R (&tvf)[VK]) {
   const R thshld = R(1.e-11);
   const uint2 nb = fs.nbr[xe];
@@ -679,8 +685,8 @@ __device__ __forceinline__ void limiters(const FrameSm& fs, const R* TO, const R
   FOR_V {
     hx[j] = mx[j].at_least_zero();
     hn[j] = mn[j].at_least_zero();
-    const R q_plus = ((hx[j] - lc[j]) * dp[j] - (ab2 * neg(tof[j]) + ab3 * pos(tvf[j]))) * ar;
-    const R q_mnus = ((lc[j] - hn[j]) * dp[j] + (ab2 * pos(tof[j]) + ab3 * neg(tvf[j]))) * ar;
+    const R q_plus = per_ab1((hx[j] - lc[j]) * dp[j] - (ab2 * neg(tof[j]) + ab3 * pos(tvf[j])), rab1, ar);
+    const R q_mnus = per_ab1((lc[j] - hn[j]) * dp[j] + (ab2 * pos(tof[j]) + ab3 * neg(tvf[j])), rab1, ar);
     rp[j] = ratio01(q_plus, floor_at(spl[j], thshld));
     rm[j] = ratio01(q_mnus, floor_at(smn[j], thshld));
   }
@@ -738,8 +744,8 @@ __global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameT
   const size_t NL = (size_t)N * L;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
   const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
-  const R rab1 = R(1) / ab1;  // Q+/Q- divide by ab1: one factor a cell
-  for (int x = threadIdx.x; x < n1; x += blockDim.x) arf[x] = g.area[fs.cells[x]] * rab1;
+  const R rab1 = R(1) / ab1;  // Q+/Q- divide by ab1: one reciprocal
+  for (int x = threadIdx.x; x < n1; x += blockDim.x) arf[x] = g.area[fs.cells[x]] * (sizeof(R) == 8 ? rab1 : R(1));
   // the limiters' operands of tracer t0 + tz
   RowPlan<R, VK, GC> rp;
   rp.init(fs, ft.SC, n2, lk, L);
@@ -794,12 +800,12 @@ __global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameT
     // R+/R- of the thread's patch cell (its bounds and slots kept for
     // trcadv3), then of the ring-1 cells
     R hx[VK], hn[VK], tof[VK], tvf[VK];
-    if (on) limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, x, v, ab2, ab3, Rp, Rm, hx, hn, tof, tvf);
+    if (on) limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, x, v, ab2, ab3, rab1, Rp, Rm, hx, hn, tof, tvf);
     for (int it = threadIdx.x; it < (n1 - C) * GC; it += blockDim.x) {
       const int xe = C + it / GC, ve = (it % GC) * VK;
       if (ve >= lk) continue;
       R mx2[VK], mn2[VK], tof2[VK], tvf2[VK];
-      limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, xe, ve, ab2, ab3, Rp, Rm, mx2, mn2, tof2, tvf2);
+      limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, xe, ve, ab2, ab3, rab1, Rp, Rm, mx2, mn2, tof2, tvf2);
     }
     stage_wait();
     __syncthreads();
