@@ -1132,8 +1132,8 @@ int enqueue_step(fim_ctx* c, fim_state* st, StepIo* io = nullptr) {
   // no written data with it: edgvar3's layer-thickness edges beside edgvar1,
   // and pressure, Exner function and omega (cnuity5), dissip and momtum beside
   // the tracer transport.  A small grid's kernels do not fill the chip, so the
-  // branch hides behind the chain (glvl 5 / nvl 38: BR_SMALL); at glvl 8 they do and
-  // it costs nothing (BR_LARGE).  Per-kernel timing keeps one chain.
+  // branch hides behind the chain (glvl 5 / nvl 38: ~60 us of kernels); at glvl 8
+  // they do and it costs nothing.  Per-kernel timing keeps one chain.
   const bool branch = !io && !c->prof.on && c->aux;
   auto fork = [&]() -> int {
     CK(cudaEventRecord(c->ev_fork, c->stream), "step fork");

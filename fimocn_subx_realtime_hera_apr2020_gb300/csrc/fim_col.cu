@@ -1432,34 +1432,32 @@ int prepare_hybgen(int L) {
 }
 
 // ---------------------------------------------------------------- hystat --
-// hystat (hystat.F90:53-109): lane = column, 32 columns per warp.  The
-// column set-up reads each kHyChunk-level chunk of thickness, theta and
-// Exner function of the warp's columns into shared memory, then
-// every lane runs the reference's recursions up its own column (surface
-// pressure sum, Montgomery potential bottom-up, geopotential at the interface
-// above), in FP64 (FP64 build) or float-float (FP32-mixed build, which also
-// keeps the (hi, lo) Montgomery potential for the pressure gradient), and the
-// results leave through the same tiles.  The humidity floors and tracer x
-// thickness are k_hystat_trdp.  A chunk is kHyChunk levels; a load or store
-// instruction of the warp covers 32 / kHyChunk rows (columns).
-#ifndef FIM_HY_CHUNK
-#define FIM_HY_CHUNK 16
-#endif
-constexpr int kHyChunk = FIM_HY_CHUNK;
-constexpr int kHyRows = 32 / kHyChunk;
-template <typename R>
-constexpr int kHyWarps = sizeof(R) == 4 ? 4 : 2;
-template <typename R>
-__global__ void __launch_bounds__(32 * kHyWarps<R>) k_hystat(Grid<R> g, Strides s, const StepParams* __restrict__ sp,
+// hystat (hystat.F90:53-109), 32 columns a block.  The recursions up the
+// columns are the surface pressure sum (warp 0) and the Montgomery potential
+// (warp 1), lane = column over shared tiles in the reference's order, in FP64
+// (FP64 build) or float-float (FP32-mixed build, which also keeps the (hi, lo)
+// Montgomery potential for the pressure gradient).  What each level adds to the
+// potential, Exner(k) (theta(k) - theta(k-1)), is formed before and the
+// geopotential at each interface after with thread = (column, VK levels).  The
+// humidity floors and tracer x thickness are k_hystat_trdp.  One warp doing all of it for its 32 columns, 16 levels at a time, kept three warps an SM in
+// flight at glvl 5: HY_OLD
+constexpr int kHyCols = 32;
+constexpr int kHyBlock = 256;
+template <typename R, int VK>
+__global__ void __launch_bounds__(kHyBlock) k_hystat(Grid<R> g, Strides s, const StepParams* __restrict__ sp,
     R* __restrict__ ph3d, const R* __restrict__ ex3d, R* __restrict__ mp3d, const R* __restrict__ dp3d,
     const R* __restrict__ tr3d, R* __restrict__ psrf, R* __restrict__ ptdcy,
     float2* __restrict__ mpf, int bnd) {
-  __shared__ R tiles[kHyWarps<R>][3][32][kHyChunk + 1];
+  constexpr bool FFB = sizeof(R) == 4;
+  extern __shared__ __align__(16) unsigned char hysm[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int N = g.N, L = g.L, L1 = L + 1;
-  const int i0 = (blockIdx.x * kHyWarps<R> + wib) * 32;
-  if (i0 >= N) return;
-  const int ncol = N - i0 < 32 ? N - i0 : 32;
+  const int N = g.N, L = g.L, L1 = L + 1, LV = L / VK;
+  const int LS = L | 1;  // odd row stride: lane = column reads are conflict-free
+  R* const td = reinterpret_cast<R*>(hysm);  // thickness
+  R* const tm = td + kHyCols * LS;           // a level's term, then the potential
+  R* const tl = tm + kHyCols * LS;           // their low parts (FP32)
+  const int i0 = blockIdx.x * kHyCols;
+  const int ncol = N - i0 < kHyCols ? N - i0 : kHyCols;
   const size_t m = blockIdx.y;
   sp += m;
   if (!sp->active || (bnd && sp->its <= 1)) return;
@@ -1467,90 +1465,91 @@ __global__ void __launch_bounds__(32 * kHyWarps<R>) k_hystat(Grid<R> g, Strides 
   psrf += m * s.col; ptdcy += m * 2 * s.col;
   if (mpf) mpf += m * s.cell;
   const int its = sp->its - bnd;
-  const int i = i0 + lane;
-  const bool live = lane < ncol;
-  R (*tdp)[kHyChunk + 1] = tiles[wib][0];  // thickness in, Montgomery potential out
-  R (*tth)[kHyChunk + 1] = tiles[wib][1];  // theta in, low part of the Montgomery potential out (FP32)
-  R (*tex)[kHyChunk + 1] = tiles[wib][2];  // Exner function in, geopotential out
-  // the staging lanes: row (column) rr * kHyRows + lrow, level lk of the chunk
-  const int lrow = lane / kHyChunk, lk = lane - lrow * kHyChunk;
-  const R ph0 = live ? ph3d[(size_t)i * L1] : R(0);
-  const R exL = live ? ex3d[(size_t)i * L1 + L] : R(0);
-  const R work = live ? psrf[i] : R(0);
-  FF2 psf{0.f, 0.f}, mpff{0.f, 0.f};
-  double psd = 0.0, mpd = 0.0;
-  R thp = R(0);
-  for (int c0 = 0; c0 < L; c0 += kHyChunk) {
-    const int kk = c0 + lk;
-    const int nq = L - c0 < kHyChunk ? L - c0 : kHyChunk;
-#pragma unroll 8
-    for (int rr = 0; rr < 32 / kHyRows; rr++) {
-      const int r = rr * kHyRows + lrow;
-      if (r < ncol && kk < L) {
-        const size_t ic = (size_t)(i0 + r);
-        tdp[r][lk] = dp3d[ic * L + kk];
-        tth[r][lk] = tr3d[ic * L + kk];
-        tex[r][lk] = ex3d[ic * L1 + kk];
-      }
-    }
-    __syncwarp();
-    if (live) {
-      for (int q = 0; q < nq; q++) {
-        const int k = c0 + q;
-        const R d = tdp[lane][q], t = tth[lane][q], e = tex[lane][q];
-        if constexpr (sizeof(R) == 4) {
-          // float-float recursions (FP64-accurate on the FP32 pipes)
-          psf = ff_add(psf, FF2{d, 0.f});
-          FF2 term;
-          if (k == 0) {
-            term = ff_add(two_prod(e, t), FF2{ph0, 0.f});
-          } else {
-            tex[lane][q] = ff_add(mpff, ff_neg(two_prod(thp, e))).hi;  // geopotential at interface k
-            const FF2 dd = two_sum(t, -thp);
-            term = ff_add(two_prod(e, dd.hi), FF2{e * dd.lo, 0.f});
-          }
-          mpff = k == 0 ? term : ff_add(mpff, term);
-          tdp[lane][q] = mpff.hi;
-          tth[lane][q] = mpff.lo;
+  for (int it = threadIdx.x; it < ncol * LV; it += kHyBlock) {
+    const int r = it / LV, k = (it - r * LV) * VK;
+    const size_t c = (size_t)(i0 + r) * L + k, ci = (size_t)(i0 + r) * L1 + k;
+    R d[VK], t[VK], e[VK];
+    ldv<VK>(dp3d + c, d);
+    ldv<VK>(tr3d + c, t);
+    R tp = k > 0 ? tr3d[c - 1] : R(0);
+    FOR_V e[j] = ex3d[ci + j];
+    FOR_V {
+      const int o = r * LS + k + j;
+      td[o] = d[j];
+      if constexpr (FFB) {
+        FF2 term;
+        if (k + j == 0) {
+          term = ff_add(two_prod(e[j], t[j]), FF2{ph3d[ci], 0.f});
         } else {
-          psd += (double)d;
-          double term;
-          if (k == 0) {
-            term = (double)e * (double)t + (double)ph0;
-          } else {
-            tex[lane][q] = R(mpd - (double)thp * (double)e);
-            term = (double)e * ((double)t - (double)thp);
-          }
-          mpd = k == 0 ? term : mpd + term;
-          tdp[lane][q] = R(mpd);
+          const FF2 dd = two_sum(t[j], -tp);
+          term = ff_add(two_prod(e[j], dd.hi), FF2{e[j] * dd.lo, 0.f});
         }
-        thp = t;
+        tm[o] = term.hi;
+        tl[o] = term.lo;
+      } else {
+        tm[o] = k + j == 0 ? e[j] * t[j] + ph3d[ci] : e[j] * (t[j] - tp);
       }
+      tp = t[j];
     }
-    __syncwarp();
-#pragma unroll 8
-    for (int rr = 0; rr < 32 / kHyRows; rr++) {
-      const int r = rr * kHyRows + lrow;
-      if (r < ncol && kk < L) {
-        const size_t ic = (size_t)(i0 + r);
-        mp3d[ic * L + kk] = tdp[r][lk];
-        if (mpf) mpf[ic * L + kk] = make_float2((float)tdp[r][lk], (float)tth[r][lk]);
-        if (kk >= 1) ph3d[ic * L1 + kk] = tex[r][lk];
-      }
-    }
-    __syncwarp();
   }
-  if (live) {
-    R pn;
-    if constexpr (sizeof(R) == 4) {
-      ph3d[(size_t)i * L1 + L] = ff_add(mpff, ff_neg(two_prod(thp, exL))).hi;
-      pn = psf.hi;
-    } else {
-      ph3d[(size_t)i * L1 + L] = R(mpd - (double)thp * (double)exL);
-      pn = R(psd);
+  __syncthreads();
+  if (lane < ncol) {
+    if (wib == 0) {
+      const R* q = td + lane * LS;
+      R pn;
+      if constexpr (FFB) {
+        FF2 ps{0.f, 0.f};
+#pragma unroll 4
+        for (int k = 0; k < L; k++) ps = ff_add(ps, FF2{q[k], 0.f});
+        pn = ps.hi;
+      } else {
+        pn = R(0);
+#pragma unroll 4
+        for (int k = 0; k < L; k++) pn += q[k];
+      }
+      const int i = i0 + lane;
+      const R work = psrf[i];
+      psrf[i] = pn;
+      if (its > 0) ptdcy[(size_t)(its % 2) * N + i] = pn - work;
+    } else if (wib == 1) {
+      R* q = tm + lane * LS;
+      if constexpr (FFB) {
+        float* ql = (float*)tl + lane * LS;
+        FF2 mp{q[0], ql[0]};
+#pragma unroll 4
+        for (int k = 1; k < L; k++) {
+          mp = ff_add(mp, FF2{q[k], ql[k]});
+          q[k] = mp.hi;
+          ql[k] = mp.lo;
+        }
+      } else {
+        R mp = q[0];
+#pragma unroll 4
+        for (int k = 1; k < L; k++) {
+          mp = mp + q[k];
+          q[k] = mp;
+        }
+      }
     }
-    psrf[i] = pn;
-    if (its > 0) ptdcy[(size_t)(its % 2) * N + i] = pn - work;
+  }
+  __syncthreads();
+  for (int it = threadIdx.x; it < ncol * LV; it += kHyBlock) {
+    const int r = it / LV, k = (it - r * LV) * VK;
+    const size_t c = (size_t)(i0 + r) * L + k, ci = (size_t)(i0 + r) * L1 + k;
+    R t[VK], mo[VK];
+    ldv<VK>(tr3d + c, t);
+    FOR_V {
+      const int o = r * LS + k + j;
+      const R e1 = ex3d[ci + j + 1];  // the interface above
+      mo[j] = tm[o];
+      if constexpr (FFB) {
+        if (mpf) mpf[c + j] = make_float2(tm[o], tl[o]);
+        ph3d[ci + j + 1] = ff_add(FF2{tm[o], tl[o]}, ff_neg(two_prod(t[j], e1))).hi;
+      } else {
+        ph3d[ci + j + 1] = tm[o] - t[j] * e1;
+      }
+    }
+    stv<VK>(mp3d + c, mo);
   }
 }
 
@@ -1630,13 +1629,15 @@ constexpr int kGsSlots = kMaxT + 5;
 // and the partials are per (chunk, slot): the sums are deterministic and do
 // not depend on the grouping.
 constexpr int kGsGroup = 7;
-// Iterations of a block: 16 where that leaves at least four blocks an SM, fewer
-// for small grids (glvl 5 / nvl 38: 24 blocks of 16 took GS_OLD us, 380 of one
-// GS_NEW us).  A function of the grid alone: the sums do not depend on the
-// tracers or members beside them.
+// Iterations of a block: 16 where that leaves 1.5 blocks an SM, fewer for
+// small grids.  (A block's reduction takes ~60 FP64 operations a warp, so many
+// short blocks cost more than an idle SM: glvl 5 / nvl 38, one level a thread:
+// 760 blocks of two iterations 33 us, 380 of four 21 us.)
+// A function of the grid alone: the sums do not depend on the tracers or
+// members beside them.
 inline int gs_iters(long long NL, int vk) {
   int it = 16;
-  while (it > 1 && NL / ((long long)kBlock2 * vk * it) < 608) it /= 2;
+  while (it > 1 && NL / ((long long)kBlock2 * vk * it) < 228) it /= 2;
   return it;
 }
 inline int gs_chunks(long long NL, int vk) {
@@ -1919,11 +1920,20 @@ bool launch_hybgen(const Launch& l, const Grid<R>& g, const Strides& s, const Kn
 template <typename R>
 void launch_hystat(const Launch& l, const Grid<R>& g, const Strides& s, R* ph3d, const R* ex3d, R* mp3d,
                    const R* dp3d, R* tr3d, R* trdp, R* psrf, R* ptdcy, float2* mpf, bool trdp_done) {
-  dim3 gw(nblocks(g.N, 32 * kHyWarps<R>), l.members);
-  FIM_KBEGIN(l, "k_hystat");
-  k_hystat<R><<<gw, 32 * kHyWarps<R>, 0, l.stream>>>(g, s, l.sp, ph3d, ex3d, mp3d, dp3d, tr3d, psrf, ptdcy, mpf,
-                                                  l.boundary);
-  FIM_KEND(l);
+  {
+    const int vk = pick_vk<R>(g.L, {dp3d, tr3d, mp3d}, sizeof(R) == 8 ? 1 : 0);
+    const size_t smem = (size_t)(sizeof(R) == 4 ? 3 : 2) * kHyCols * (g.L | 1) * sizeof(R);
+    const dim3 grid(nblocks(g.N, kHyCols), l.members);
+    FIM_KBEGIN(l, "k_hystat");
+    FIM_VK_DISPATCH(R, vk, ({
+      if (smem > (size_t)48 * 1024)  // columns of more than 95 (FP64) or 127 levels
+        cudaFuncSetAttribute(k_hystat<R, VK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)((sizeof(R) == 4 ? 3 : 2) * kHyCols * (kMaxL | 1) * sizeof(R)));
+      k_hystat<R, VK><<<grid, kHyBlock, smem, l.stream>>>(g, s, l.sp, ph3d, ex3d, mp3d, dp3d, tr3d, psrf, ptdcy, mpf,
+                                                          l.boundary);
+    }));
+    FIM_KEND(l);
+  }
   if (trdp_done) return;  // the remap formed the floors and tracer x thickness
   const int vk = pick_vk<R>(g.L, {dp3d, tr3d, trdp});
   FIM_KBEGIN(l, "k_hystat_trdp");
