@@ -19,118 +19,188 @@ template <typename R> __device__ __forceinline__ R cmax(R a, R b) { return a > b
 template <typename R> __device__ __forceinline__ R cmin(R a, R b) { return a < b ? a : b; }
 template <typename R> __device__ __forceinline__ R cabs(R a) { return a < R(0) ? -a : a; }
 
+// FP64 comparisons on the integer pipe (fim_internal.h)
+__device__ __forceinline__ bool lt(float a, float b) { return a < b; }
+__device__ __forceinline__ bool lt(double a, double b) { return f64_key(a) < f64_key(b); }
+__device__ __forceinline__ double cmax(double a, double b) { return lt(b, a) ? a : b; }
+__device__ __forceinline__ double cmin(double a, double b) { return lt(a, b) ? a : b; }
+// a / b; FP64: b normal, reciprocal and one residual correction
+__device__ __forceinline__ float qdiv(float a, float b) { return a / b; }
+__device__ __forceinline__ double qdiv(double a, double b) { return f64_quot(a, b, f64_recip(b)); }
+// x / 10, rounded as the division (Markstein's correction; for this divisor the
+// rounded reciprocal gives the rounded quotient for every FP32 mantissa)
+__device__ __forceinline__ float tenth(float x) {
+  const float q = x * .1f;
+  return fmaf(fmaf(-10.f, q, x), .1f, q);
+}
+__device__ __forceinline__ double tenth(double x) { return f64_quot(x, 10., .1); }
+
 constexpr int kColBlock = 128;
 constexpr int kBlock2 = 256;
 inline unsigned nblocks(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 
 // ---------------------------------------------------------------- hybgen --
-// restp_1d (hybgen.F90:792-890).  The running minimum oldth is formed in
-// place in thold (the caller's column, not read again).  The new theta
-// column is targt except its two end layers (hybgen.F90:832-834), so it is
-// not stored: th0 and thL are its ends and tn(k) its layer k.
+// What regrid_1d takes from the target column alone, formed once a block: the
+// targets, the heat diffusion's factors (dffudt cnv^2 (th(k+1) - th(k-1)) / 2
+// and its floor .03 cnv, cnv = g / th(k)) and inflate's minimum layers.
 template <typename R, int ML>
-__device__ void restp_1d(R* thold, const R* pkold, int kold, R* pknew, const R* targt, int knew, int* bad) {
+struct RegTab {
+  R tg[ML], num[ML], fl[ML], d0[ML];
+  __device__ __forceinline__ void fill(const R* targt, const R* dpsig, int L) {
+    const R grv = R(kGrvity), dffudt = R(.1);
+    for (int k = threadIdx.x; k < L; k += blockDim.x) {
+      tg[k] = targt[k];
+      d0[k] = R(kRd) * dpsig[k] / R(kP1000);
+      if (k >= 1 && k <= L - 2) {
+        const R cnv = grv / targt[k];
+        num[k] = dffudt * cnv * cnv * R(.5) * (targt[k + 1] - targt[k - 1]);
+        fl[k] = R(.03) * cnv;
+      }
+    }
+  }
+};
+
+// restp_1d (hybgen.F90:792-890).  The running minimum oldth is formed in
+// place in thold (the caller's column, not read again), whose layers below
+// kmod are one already.  The new theta column is targt except its two end
+// layers (hybgen.F90:832-834), so it is not stored: th0 and thL are its ends
+// and tn(k) its layer k.
+template <typename R>
+__device__ void restp_1d(R* thold, int kmod, const R* pkold, int kold, R* pknew, const R* targt, int knew, int* bad) {
   R* oldth = thold;
-  for (int k = kold; k >= 2; k--) oldth[k - 2] = cmin(oldth[k - 1], oldth[k - 2]);
+  {
+    R up = oldth[kold - 1];
+    for (int k = kold - 2; k >= 0; k--) {
+      const R x = oldth[k];
+      if (k < kmod && !lt(up, x)) break;  // the column below is monotone
+      up = cmin(up, x);
+      oldth[k] = up;
+    }
+  }
   const R th0 = cmin(cmin(oldth[0], oldth[kold - 1]), targt[0]);
   const R thL = cmax(cmax(oldth[0], oldth[kold - 1]), targt[knew - 1]);
   auto tn = [&](int k) -> R { return k == 0 ? th0 : k == knew - 1 ? thL : targt[k]; };
   pknew[0] = pkold[0];
   pknew[knew] = pkold[kold];
   R colint = R(0), colscl = R(0), cloutt = R(0);
-  for (int k = 0; k < kold; k++) {
-    colint = colint + oldth[k] * (pkold[k + 1] - pkold[k]);
-    colscl = colscl + cabs(oldth[k] * (pkold[k + 1] - pkold[k]));
+  {
+    R p0 = pkold[0];
+#pragma unroll 4
+    for (int k = 0; k < kold; k++) {
+      const R p1 = pkold[k + 1], w = oldth[k] * (p1 - p0);
+      colint = colint + w;
+      colscl = colscl + cabs(w);
+      p0 = p1;
+    }
   }
   int ko = 0;
-  R tk = th0;
+  R tk = th0, prev = pknew[0], ok = oldth[0], pk = pkold[0];  // layer ko's theta and lower interface
   for (int k = 0; k < knew - 1; k++) {
     const R tk1 = tn(k + 1);
     R pinteg = R(0), tha, thb = tk;
     for (;;) {
       tha = thb;
-      thb = cmin(tk1, cmax(tk, oldth[ko]));
-      pinteg = pinteg + pkold[ko] * (thb - tha);
-      if (oldth[ko] < tk1) {
-        if (ko < kold - 1) { ko++; continue; }
+      thb = cmin(tk1, cmax(tk, ok));
+      pinteg = pinteg + pk * (thb - tha);
+      if (lt(ok, tk1)) {
+        if (ko < kold - 1) {
+          ko++;
+          ok = oldth[ko];
+          pk = pkold[ko];
+          continue;
+        }
         tha = thb;
         thb = tk1;
         pinteg = pinteg + pkold[kold] * (thb - tha);
       }
       break;
     }
-    pknew[k + 1] = pknew[k];
-    if (tk1 > tk) pknew[k + 1] = pinteg / (tk1 - tk);
-    cloutt = cloutt + tk * (pknew[k + 1] - pknew[k]);
+    R pn = prev;
+    if (lt(tk, tk1)) pn = qdiv(pinteg, tk1 - tk);
+    pknew[k + 1] = pn;
+    cloutt = cloutt + tk * (pn - prev);
+    prev = pn;
     tk = tk1;
   }
-  cloutt = cloutt + thL * (pknew[knew] - pknew[knew - 1]);
+  cloutt = cloutt + thL * (pknew[knew] - prev);
   if (cabs(cloutt - colint) > cmax(R(1.e-33), col_tol<R>(1.e-6) * colscl)) *bad = 1;
 }
 
-// equilb scenario 1 (hybgen.F90:1316-1363); in place on pres
+// equilb scenario 1 (hybgen.F90:1316-1363); in place on pres, the six
+// interfaces of a step kept as the loop moves up
 template <typename R>
 __device__ void equilb(const R* thet, R* pnew, int kk, R slak) {
   const R thin = R(kRd) / R(kP1000);
+  const R top = pnew[0] - thin;
+  R p0 = pnew[0], p1 = pnew[1], p2 = pnew[2], p3 = pnew[3], p4 = pnew[4];
   for (int k = 3; k <= kk - 2; k++) {
-    if (pnew[k - 3] > pnew[0] - thin) continue;
-    const R dp1 = pnew[k - 3] - pnew[k - 2];
-    const R dp2 = pnew[k - 2] - pnew[k - 1];
-    const R dp3 = pnew[k - 1] - pnew[k];
-    const R dp4 = pnew[k] - pnew[k + 1];
-    const R dp5 = pnew[k + 1] - pnew[k + 2];
-    const R th2 = thet[k - 2], th3 = thet[k - 1], th4 = thet[k];
-    if (dp2 > dp1 && dp4 > dp5) {
+    const R p5 = pnew[k + 2];
+    const R dp1 = p0 - p1, dp2 = p1 - p2, dp4 = p3 - p4, dp5 = p4 - p5;
+    if (!lt(top, p0) && lt(dp1, dp2) && lt(dp5, dp4)) {
+      const R dp3 = p2 - p3;
       const R goal = R(.5) * (dp3 + cmin(dp2, dp4));
-      if (dp2 > goal && dp4 > goal) {
+      if (lt(goal, dp2) && lt(goal, dp4)) {
         R dis3 = cmin(dp2 - goal, goal - dp3) * slak;
         R dis4 = cmin(dp4 - goal, goal - dp3) * slak;
+        const R th2 = thet[k - 2], th3 = thet[k - 1], th4 = thet[k];
         if (th3 > th2 && th4 > th3) {
           const R ratio = (th4 - th3) / (th3 - th2);
           if (ratio > R(1)) dis4 = dis3 / ratio;
           else dis3 = dis4 * ratio;
         }
-        pnew[k - 1] = pnew[k - 1] + dis3;
-        pnew[k] = pnew[k] - dis4;
+        p2 = p2 + dis3;
+        p3 = p3 - dis4;
+        pnew[k - 1] = p2;
+        pnew[k] = p3;
       }
     }
+    p0 = p1; p1 = p2; p2 = p3; p3 = p4; p4 = p5;
   }
 }
 
 template <typename R>
 __device__ __forceinline__ R cushn(R a, R b) {
   const R m = cmin(a, R(2) * b);
-  return R(.25) * (m * m) / b + cmax(a, R(2) * b) - b;
+  return qdiv(R(.25) * (m * m), b) + cmax(a, R(2) * b) - b;
 }
 
-// inflate (hybgen.F90:893-1007)
-template <typename R>
-__device__ void inflate(const Knobs& kn, const R* dpsig, int L, R psurf, R* exner) {
+// inflate (hybgen.F90:893-1007); d0(k) = rd dpsig(k) / p1000
+template <typename R, typename D0>
+__device__ void inflate(const Knobs& kn, D0 d0, int L, R psurf, R* exner) {
   const R thin = R(kRd) / R(kP1000);
   const R rd = R(kRd), p1000 = R(kP1000), cp = R(kCp);
   R dpsum = R(0);
   const R extop = cp * pow(R(kn.ptop) / p1000, rd / cp);
   const R top = R(.2);
   const R shrink = cmin(R(1), (psurf / p1000 - top) / (R(1) - top));
+  const R soft = rd * R(100) / p1000;
+  const R ex0 = exner[0];
+  R below = ex0;  // exner[k - 1]
   int last = 1;
   for (int k = 1; k <= L - 1; k++) {
-    R dp0 = rd * dpsig[k - 1] / p1000 * shrink;
+    R dp0 = d0(k - 1) * shrink;
     dpsum = dpsum + dp0;
     const R exold = exner[k];
+    R now = exold;
     if (k <= kn.kbl) {
       last = k + 1;
-      exner[k] = exner[k - 1] - dp0;
+      now = below - dp0;
+      exner[k] = now;
     } else {
       if (k > last) {
-        dp0 = dp0 / cmin(R(10), R(1.25) * ldexp(R(1), k - last));
-        dp0 = cmax(dp0, rd * R(100) / p1000);
+        // / min(10, 1.25 2^(k - last)): 2.5, 5, 10, 10, ... a tenth scaled exactly
+        const int n = k - last;
+        dp0 = tenth(dp0) * (n == 1 ? R(4) : n == 2 ? R(2) : R(1));
+        dp0 = cmax(dp0, soft);
       }
-      const R dp1 = cushn(cmax(R(0), exner[k - 1] - cmin(exold, exner[0] - dpsum)), dp0);
-      if (exner[k - 1] - dp1 < exold - thin) {
+      const R dp1 = cushn(cmax(R(0), below - cmin(exold, ex0 - dpsum)), dp0);
+      if (lt(below - dp1, exold - thin)) {
         if (k == last) last = k + 1;
-        exner[k] = cmax(extop, exner[k - 1] - dp1);
+        now = cmax(extop, below - dp1);
+        exner[k] = now;
       }
     }
+    below = now;
   }
   if (kn.thktop > 0.) {
     const R thk = R(kn.thktop);
@@ -147,22 +217,19 @@ __device__ void inflate(const Knobs& kn, const R* dpsig, int L, R psurf, R* exne
   }
 }
 
-// regrid_1d (hybgen.F90:207-512, hybrid-isentropic branch) for one column:
-// thcol (L) and excol (L+1) are overwritten; excol ends as the new Exner fcn.
+// regrid_1d (hybgen.F90:207-512, hybrid-isentropic branch) for one column.
+// thcol (L) comes as its running minimum from the top and excol (L+1) as its
+// running limit from the bottom (columns_in_min, columns_in_limit); both are
+// overwritten.  exnew ends as the new Exner function.
 template <typename R, int ML>
-__device__ void regrid_1d(const Knobs& kn, const R* targt, const R* dpsig, int L, int its, R* thcol, R* excol,
+__device__ void regrid_1d(const Knobs& kn, const RegTab<R, ML>& tab, int L, int its, R* thcol, R* excol, R* exnew,
                           R prcol0, int* bad) {
-  const R thin = R(kRd) / R(kP1000), tolrnce = R(0.001), dffudt = R(.1);
+  const R thin = R(kRd) / R(kP1000), tolrnce = R(0.001);
   const R eqlb_slak = R(.1) * R(its) / (R(10) + R(its));
-  // one local work array: the column's own excol serves as exwrk, thcol as
-  // restp_1d's oldth, the new theta column is targt but for its ends (which
-  // equilb does not read), and the heat fluxes are formed as the update runs
-  R exnew[ML + 1];
-  for (int k = 0; k < L; k++)
-    if (excol[k] < excol[k + 1] - thin) excol[k + 1] = excol[k];
-  for (int k = L - 2; k >= 0; k--) thcol[k] = cmin(thcol[k], thcol[k + 1]);
+  const R* targt = tab.tg;
   R* exwrk = excol;
   const R tt = targt[L - 1];
+  int kmod = L;  // lowest layer of thcol changed here
   for (int k = L; k >= 2; k--) {
     if (thcol[k - 1] <= tt + tolrnce) break;
     const R wgt1 = cmax(R(0), exwrk[k - 2] - exwrk[k - 1]);
@@ -171,43 +238,46 @@ __device__ void regrid_1d(const Knobs& kn, const R* targt, const R* dpsig, int L
     if (tr > tt - tolrnce) {
       exwrk[k - 1] = exwrk[L];
       for (int k1 = k - 1; k1 <= L; k1++) thcol[k1 - 1] = tr;
+      kmod = k - 2;
     } else {
       exwrk[k - 1] = cmin(exwrk[k - 2], cmax(exwrk[k], (exwrk[k - 1] * (thcol[k - 1] - thcol[k - 2]) +
                                                          exwrk[k] * (tt - thcol[k - 1])) /
                                                             (tt - thcol[k - 2])));
       for (int k1 = k; k1 <= L; k1++) thcol[k1 - 1] = tt;
+      kmod = k - 1;
       break;
     }
   }
-  restp_1d<R, ML>(thcol, exwrk, L, exnew, targt, L, bad);
-  const R grv = R(kGrvity);
-  // heatfx(j) of hybgen.F90's heat diffusion, from the work copy only (zero
-  // at j = 0 and nvl-1)
-  auto heatfx = [&](int j) -> R {
-    R h = R(0);
-    if (j >= 1 && j <= L - 2 && exwrk[j] < exwrk[0] - R(.01) && exwrk[j + 1] > exwrk[L] + R(.01)) {
-      const R cnv = grv / targt[j];
-      h = dffudt * cnv * cnv * R(.5) * (targt[j + 1] - targt[j - 1]) / cmax(R(.03) * cnv, exwrk[j] - exwrk[j + 1]);
-    }
-    return h;
-  };
+  restp_1d<R>(thcol, kmod, exwrk, L, exnew, targt, L, bad);
+  // heat diffusion (heatfx zero at the end layers and next to the column's
+  // ends) from the interfaces before the pass, whose neighbours stay in
+  // registers as the pass overwrites them
+  const R bot = exnew[0] - R(.01), top = exnew[L] + R(.01);
   for (int iter = 1; iter <= 3; iter++) {
-    for (int k = 0; k <= L; k++) exwrk[k] = exnew[k];
-    R hprev = R(0);  // heatfx(k - 1)
-    for (int k = 1; k <= L - 1; k++) {
-      const R hcur = heatfx(k);
-      if (exwrk[k] < exwrk[0] - R(.01) && exwrk[k] > exwrk[L] + R(.01))
-        exnew[k] = cmax(exwrk[k + 1], cmin(exwrk[k - 1], exwrk[k] + (hcur - hprev) / (targt[k] - targt[k - 1])));
-      hprev = hcur;
-    }
     bool event = false;
-    for (int k = 2; k <= L + 1; k++)
-      if (exnew[k - 1] > exnew[k - 2] + thin) event = true;
+    R hprev = R(0);                                        // heatfx(k - 1)
+    R lo = exnew[0], at = exnew[1], newlo = lo;            // old k - 1, old k, new k - 1
+#pragma unroll 2
+    for (int k = 1; k <= L - 1; k++) {
+      const R hi = exnew[k + 1];
+      R hcur = R(0);
+      if (k <= L - 2 && lt(at, bot) && lt(top, hi)) hcur = qdiv(tab.num[k], cmax(tab.fl[k], at - hi));
+      R now = at;
+      if (lt(at, bot) && lt(top, at)) {
+        now = cmax(hi, cmin(lo, at + qdiv(hcur - hprev, targt[k] - targt[k - 1])));
+        exnew[k] = now;
+      }
+      event = event || lt(newlo + thin, now);
+      hprev = hcur;
+      lo = at;
+      at = hi;
+      newlo = now;
+    }
+    event = event || lt(newlo + thin, at);
     if (!event) break;
   }
   equilb<R>(targt, exnew, L, eqlb_slak);  // reads layers 1..nvl-2 only
-  inflate<R>(kn, dpsig, L, prcol0, exnew);
-  for (int k = 0; k <= L; k++) excol[k] = exnew[k];
+  inflate<R>(kn, [&](int k) { return tab.d0[k]; }, L, prcol0, exnew);
 }
 
 // pcwise (hybgen.F90:1010-1279): 1-D PCM/PLM/PPM remap of yold from cell
@@ -343,18 +413,26 @@ __device__ bool pcwise(int kk, const R* xold, const R* yold, const R* xnew, R* y
 // lanes' column arrays through a 32 x 33 shared tile, 32 levels at a time, so
 // the global accesses run along k (128-byte rows) rather than one column per
 // lane.  n values of column i0 + lane start at src + (i0 + lane) * stride.
-template <typename R>
+// take(k, x) receives the levels upward (UP) or downward.
+template <bool UP, typename R, typename F>
 __device__ __forceinline__ void columns_in(const R* __restrict__ src, size_t stride, int n, int ncol, int i0,
-                                           int lane, R (*tile)[33], R* col) {
-  for (int c0 = 0; c0 < n; c0 += 32) {
+                                           int lane, R (*tile)[33], F take) {
+  const int nc = (n + 31) / 32;
+  for (int cc = 0; cc < nc; cc++) {
+    const int c0 = (UP ? cc : nc - 1 - cc) * 32;
     const int kk = c0 + lane;
 #pragma unroll 8
     for (int r = 0; r < 32; r++)
       if (r < ncol && kk < n) tile[r][lane] = src[(size_t)(i0 + r) * stride + kk];
     __syncwarp();
     const int m = n - c0 < 32 ? n - c0 : 32;
-    if (lane < ncol)
-      for (int q = 0; q < m; q++) col[c0 + q] = tile[lane][q];
+    if (lane < ncol) {
+#pragma unroll 4
+      for (int q = 0; q < m; q++) {
+        const int k = UP ? q : m - 1 - q;
+        take(c0 + k, tile[lane][k]);
+      }
+    }
     __syncwarp();
   }
 }
@@ -380,9 +458,12 @@ __global__ void __launch_bounds__(kColBlock) k_regrid(Grid<R> g, Strides s, Knob
     const R* __restrict__ ex3d, const R* __restrict__ pr3d, R* __restrict__ exsmo, int* __restrict__ flags,
     int bnd) {
   __shared__ R tiles[kColBlock / 32][32][33];
+  __shared__ RegTab<R, ML> tab;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int i0 = blockIdx.x * blockDim.x + wib * 32;
   const int N = g.N, L = g.L, L1 = L + 1;
+  tab.fill(targt, g.dpsig, L);
+  __syncthreads();
   if (i0 >= N) return;
   const int ncol = N - i0 < 32 ? N - i0 : 32;
   const int i = i0 + lane;
@@ -390,13 +471,22 @@ __global__ void __launch_bounds__(kColBlock) k_regrid(Grid<R> g, Strides s, Knob
   sp += m;
   if (!sp->active || (bnd && sp->its <= 1)) return;
   tr3d += m * s.tr; ex3d += m * s.intf; pr3d += m * s.intf; exsmo += m * s.intf;
-  R thcol[ML], excol[ML + 1];
-  columns_in(tr3d, (size_t)L, L, ncol, i0, lane, tiles[wib], thcol);
-  columns_in(ex3d, (size_t)L1, L1, ncol, i0, lane, tiles[wib], excol);
+  R thcol[ML], excol[ML + 1], exnew[ML + 1];
+  const R thin = R(kRd) / R(kP1000);
+  // theta's running minimum from the top; no interface above the one below it
+  R run = R(0);
+  columns_in<false>(tr3d, (size_t)L, L, ncol, i0, lane, tiles[wib], [&](int k, R x) {
+    run = k == L - 1 ? x : cmin(x, run);
+    thcol[k] = run;
+  });
+  columns_in<true>(ex3d, (size_t)L1, L1, ncol, i0, lane, tiles[wib], [&](int k, R x) {
+    run = k > 0 && lt(run, x - thin) ? run : x;
+    excol[k] = run;
+  });
   int bad = 0;
   if (lane < ncol)
-    regrid_1d<R, ML>(kn, targt, g.dpsig, L, sp->its - bnd, thcol, excol, pr3d[(size_t)i * L1], &bad);
-  columns_out(exsmo, (size_t)L1, L1, ncol, i0, lane, tiles[wib], excol);
+    regrid_1d<R, ML>(kn, tab, L, sp->its - bnd, thcol, excol, exnew, pr3d[(size_t)i * L1], &bad);
+  columns_out(exsmo, (size_t)L1, L1, ncol, i0, lane, tiles[wib], exnew);
   if (bad) atomicOr(flags + m, kFlagColumnIntegral);
 }
 
@@ -478,7 +568,8 @@ __global__ void __launch_bounds__(kColBlock) k_remap(Grid<R> g, Strides s, Knobs
     exnew[k] = exsmo[(size_t)i * L1 + k];
   }
   for (int k = 0; k <= L; k++) pk1col[k] = exold[k] * prcol[k] / cp;
-  if (kn.intfc_smooth > 0.) inflate<R>(kn, g.dpsig, L, prcol[0], exnew);
+  const R* dps = g.dpsig;
+  if (kn.intfc_smooth > 0.) inflate<R>(kn, [&](int k) { return rd * dps[k] / p1000; }, L, prcol[0], exnew);
   if (its > 0) {
     const R sl = R(kn.slak);
     for (int k = 0; k <= L; k++) exnew[k] = sl * exnew[k] + (R(1) - sl) * exold[k];
@@ -1004,6 +1095,9 @@ __global__ void __launch_bounds__(32 * kWarpsInflate) k_inflate(Grid<R> g, Strid
   extern __shared__ __align__(16) unsigned char smraw[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int N = g.N, L = g.L, L1 = L + 1;
+  __shared__ R d0[ML];
+  for (int k = threadIdx.x; k < L; k += blockDim.x) d0[k] = R(kRd) * g.dpsig[k] / R(kP1000);
+  __syncthreads();
   const int i0 = (blockIdx.x * kWarpsInflate + wib) * 32;
   if (i0 >= N) return;
   const int ncol = (N - i0 < 32) ? N - i0 : 32;
@@ -1011,9 +1105,11 @@ __global__ void __launch_bounds__(32 * kWarpsInflate) k_inflate(Grid<R> g, Strid
   if (!sp[m].active || (bnd && sp[m].its <= 1)) return;
   pr3d += m * s.intf; exn += m * s.intf;
   R* col = reinterpret_cast<R*>(smraw) + (size_t)wib * (32 * (ML + 1) + 1);
+#pragma unroll 8
   for (int q = lane; q < ncol * L1; q += 32) col[q] = exn[(size_t)i0 * L1 + q];
   __syncwarp();
-  if (lane < ncol) inflate<R>(kn, g.dpsig, L, pr3d[(size_t)(i0 + lane) * L1], col + lane * L1);
+  if (lane < ncol)
+    inflate<R>(kn, [&](int k) { return d0[k]; }, L, pr3d[(size_t)(i0 + lane) * L1], col + lane * L1);
   __syncwarp();
   for (int q = lane; q < ncol * L1; q += 32) exn[(size_t)i0 * L1 + q] = col[q];
 }
@@ -1439,8 +1535,10 @@ int prepare_hybgen(int L) {
 // Montgomery potential for the pressure gradient).  What each level adds to the
 // potential, Exner(k) (theta(k) - theta(k-1)), is formed before and the
 // geopotential at each interface after with thread = (column, VK levels).  The
-// humidity floors and tracer x thickness are k_hystat_trdp.  One warp doing all of it for its 32 columns, 16 levels at a time, kept three warps an SM in
-// flight at glvl 5: HY_OLD
+// humidity floors and tracer x thickness are k_hystat_trdp.  One warp doing
+// all of it for its 32 columns, 16 levels at a time, kept two warps an SM in
+// flight at glvl 5: 25 -> 11 us at glvl 5 / nvl 38, 137 -> 71 us at glvl 7 / nvl
+// 64, 0.47 -> 0.35 ms at glvl 8 (FP32), 36 -> 17 us in FP64 at glvl 5.
 constexpr int kHyCols = 32;
 constexpr int kHyBlock = 256;
 template <typename R, int VK>
