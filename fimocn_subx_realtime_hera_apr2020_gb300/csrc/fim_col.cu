@@ -10,6 +10,7 @@
 // deterministic partial buffer.
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "fim_internal.h"
 
@@ -65,9 +66,8 @@ struct RegTab {
 // kmod are one already.  The new theta column is targt except its two end
 // layers (hybgen.F90:832-834), so it is not stored: th0 and thL are its ends
 // and tn(k) its layer k.
-template <typename R>
-__device__ void restp_1d(R* thold, int kmod, const R* pkold, int kold, R* pknew, const R* targt, int knew, int* bad) {
-  R* oldth = thold;
+template <typename R, typename C>
+__device__ void restp_1d(C oldth, int kmod, C pkold, int kold, C pknew, const R* targt, int knew, int* bad) {
   {
     R up = oldth[kold - 1];
     for (int k = kold - 2; k >= 0; k--) {
@@ -128,8 +128,8 @@ __device__ void restp_1d(R* thold, int kmod, const R* pkold, int kold, R* pknew,
 
 // equilb scenario 1 (hybgen.F90:1316-1363); in place on pres, the six
 // interfaces of a step kept as the loop moves up
-template <typename R>
-__device__ void equilb(const R* thet, R* pnew, int kk, R slak) {
+template <typename R, typename C>
+__device__ void equilb(const R* thet, C pnew, int kk, R slak) {
   const R thin = R(kRd) / R(kP1000);
   const R top = pnew[0] - thin;
   R p0 = pnew[0], p1 = pnew[1], p2 = pnew[2], p3 = pnew[3], p4 = pnew[4];
@@ -165,8 +165,8 @@ __device__ __forceinline__ R cushn(R a, R b) {
 }
 
 // inflate (hybgen.F90:893-1007); d0(k) = rd dpsig(k) / p1000
-template <typename R, typename D0>
-__device__ void inflate(const Knobs& kn, D0 d0, int L, R psurf, R* exner) {
+template <typename R, typename D0, typename C>
+__device__ void inflate(const Knobs& kn, D0 d0, int L, R psurf, C exner) {
   const R thin = R(kRd) / R(kP1000);
   const R rd = R(kRd), p1000 = R(kP1000), cp = R(kCp);
   R dpsum = R(0);
@@ -217,17 +217,22 @@ __device__ void inflate(const Knobs& kn, D0 d0, int L, R psurf, R* exner) {
   }
 }
 
-// regrid_1d (hybgen.F90:207-512, hybrid-isentropic branch) for one column.
+// regrid_1d (hybgen.F90:207-512, hybrid-isentropic branch) for one column: a
+// serial chain of ~200 instructions a level, bound by its latency (small grids)
+// or issue and local memory (large ones).  What the target column decides
+// comes in tab, passes keep the neighbours they read in registers: 0.89 -> 0.62
+// ms at glvl 8 / nvl 64, 74 -> 41 us at glvl 5 / nvl 38 (with regrid_in_smem), FP64
+// glvl 6 0.87 -> 0.47 ms.
 // thcol (L) comes as its running minimum from the top and excol (L+1) as its
 // running limit from the bottom (columns_in_min, columns_in_limit); both are
 // overwritten.  exnew ends as the new Exner function.
-template <typename R, int ML>
-__device__ void regrid_1d(const Knobs& kn, const RegTab<R, ML>& tab, int L, int its, R* thcol, R* excol, R* exnew,
+template <typename R, int ML, typename C>
+__device__ void regrid_1d(const Knobs& kn, const RegTab<R, ML>& tab, int L, int its, C thcol, C excol, C exnew,
                           R prcol0, int* bad) {
   const R thin = R(kRd) / R(kP1000), tolrnce = R(0.001);
   const R eqlb_slak = R(.1) * R(its) / (R(10) + R(its));
   const R* targt = tab.tg;
-  R* exwrk = excol;
+  C exwrk = excol;
   const R tt = targt[L - 1];
   int kmod = L;  // lowest layer of thcol changed here
   for (int k = L; k >= 2; k--) {
@@ -436,9 +441,9 @@ __device__ __forceinline__ void columns_in(const R* __restrict__ src, size_t str
     __syncwarp();
   }
 }
-template <typename R>
+template <typename R, typename C>
 __device__ __forceinline__ void columns_out(R* __restrict__ dst, size_t stride, int n, int ncol, int i0, int lane,
-                                            R (*tile)[33], const R* col) {
+                                            R (*tile)[33], C col) {
   for (int c0 = 0; c0 < n; c0 += 32) {
     const int m = n - c0 < 32 ? n - c0 : 32;
     if (lane < ncol)
@@ -452,12 +457,20 @@ __device__ __forceinline__ void columns_out(R* __restrict__ dst, size_t stride, 
   }
 }
 
-template <typename R, int ML>
-__global__ void __launch_bounds__(kColBlock) k_regrid(Grid<R> g, Strides s, Knobs kn,
+// a lane's column of a warp's 32 in shared memory
+template <typename R>
+struct LaneCol {
+  R* p;
+  __device__ __forceinline__ R& operator[](int k) const { return p[k * 32]; }
+};
+
+template <typename R, int ML, bool SM>
+__global__ void __launch_bounds__(SM ? 32 : kColBlock) k_regrid(Grid<R> g, Strides s, Knobs kn,
     const StepParams* __restrict__ sp, const R* __restrict__ targt, const R* __restrict__ tr3d,
     const R* __restrict__ ex3d, const R* __restrict__ pr3d, R* __restrict__ exsmo, int* __restrict__ flags,
     int bnd) {
-  __shared__ R tiles[kColBlock / 32][32][33];
+  __shared__ R tiles[SM ? 1 : kColBlock / 32][32][33];
+  extern __shared__ __align__(16) unsigned char rgsm[];
   __shared__ RegTab<R, ML> tab;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int i0 = blockIdx.x * blockDim.x + wib * 32;
@@ -471,7 +484,19 @@ __global__ void __launch_bounds__(kColBlock) k_regrid(Grid<R> g, Strides s, Knob
   sp += m;
   if (!sp->active || (bnd && sp->its <= 1)) return;
   tr3d += m * s.tr; ex3d += m * s.intf; pr3d += m * s.intf; exsmo += m * s.intf;
-  R thcol[ML], excol[ML + 1], exnew[ML + 1];
+  R lth[SM ? 1 : ML], lex[SM ? 1 : ML + 1], lnw[SM ? 1 : ML + 1];
+  using C = std::conditional_t<SM, LaneCol<R>, R*>;
+  C thcol, excol, exnew;
+  if constexpr (SM) {
+    R* q = reinterpret_cast<R*>(rgsm) + lane;
+    thcol.p = q;
+    excol.p = q + 32 * L;
+    exnew.p = q + 32 * (L + L1);
+  } else {
+    thcol = lth;
+    excol = lex;
+    exnew = lnw;
+  }
   const R thin = R(kRd) / R(kP1000);
   // theta's running minimum from the top; no interface above the one below it
   R run = R(0);
@@ -569,7 +594,7 @@ __global__ void __launch_bounds__(kColBlock) k_remap(Grid<R> g, Strides s, Knobs
   }
   for (int k = 0; k <= L; k++) pk1col[k] = exold[k] * prcol[k] / cp;
   const R* dps = g.dpsig;
-  if (kn.intfc_smooth > 0.) inflate<R>(kn, [&](int k) { return rd * dps[k] / p1000; }, L, prcol[0], exnew);
+  if (kn.intfc_smooth > 0.) inflate<R>(kn, [&](int k) { return rd * dps[k] / p1000; }, L, prcol[0], (R*)exnew);
   if (its > 0) {
     const R sl = R(kn.slak);
     for (int k = 0; k <= L; k++) exnew[k] = sl * exnew[k] + (R(1) - sl) * exold[k];
@@ -1474,6 +1499,12 @@ inline int remap_vl(int L) { return L <= 32 ? 1 : L <= 64 ? 2 : 4; }
 template <typename R>
 inline bool remap_paired(int L) { return sizeof(R) == 4 && L > 32 && L <= 64; }
 
+inline int sm_count() {
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 // Columns a warp of k_remap_v takes in turn.  Many columns a warp amortise its
 // start (the first copies, the theta sweep); few leave small grids no nearly
 // empty last round of blocks.  FP64 (two blocks an SM by shared memory): the
@@ -1484,8 +1515,7 @@ inline bool remap_paired(int L) { return sizeof(R) == 4 && L > 32 && L <= 64; }
 // 6: 51, 4: 69; glvl 8 / nvl 64 8: 2.95 ms, 6: 3.01, 4: 3.12.
 template <typename R>
 int remap_columns(int N, int members, bool paired) {
-  int dev = 0, sms = 152;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const long long slots = sizeof(R) == 8 ? 2 * sms : sms;
   long long best = -1;
   int cols = kColsPerWarp;
@@ -1940,20 +1970,41 @@ __global__ void __launch_bounds__(kBlock2) k_prdp_from_ex(Grid<R> g, Strides s, 
 }
 
 
+// k_regrid's column arrays in shared memory, a warp a block, while every warp
+// of the launch fits the chip at once: the columns' serial chains then see
+// shared-memory latency (glvl 5 / nvl 38: 41 against 59 us, FP64 125 against 144).
+// Larger launches hide the latency of local memory behind more warps than
+// shared memory holds (glvl 6 / nvl 64 x 4 members: 181 against 298 us; glvl 8
+// 0.62 against 1.16 ms).
+template <typename R>
+bool regrid_in_smem(int N, int L, int members) {
+  const size_t block = 32 * (size_t)(3 * L + 2) * sizeof(R) + (32 * 33 + 4 * (L <= 64 ? 64 : kMaxL)) * sizeof(R) + 1024;
+  return (long long)nblocks(N, 32) * members <= (long long)sm_count() * (long long)(227 * 1024 / block);
+}
+
 template <typename R>
 bool launch_hybgen(const Launch& l, const Grid<R>& g, const Strides& s, const Knobs& kn, const HybgenScratch<R>& w,
                    const R* targt, R* us3d, R* vs3d, R* tr3d, R* sdot, R* ex3d, R* dp3d, R* pr3d, R* trdp) {
   bool trdp_done = false;
   dim3 gc(nblocks(g.N, kColBlock), l.members);
+  FIM_KBEGIN(l, "k_regrid");
+  const bool rsm = regrid_in_smem<R>(g.N, g.L, l.members);
+  const size_t rs = rsm ? (size_t)32 * (3 * g.L + 2) * sizeof(R) : 0;
+  const dim3 gr(nblocks(g.N, rsm ? 32 : kColBlock), l.members);
+#define FIM_REGRID(ML, SM)                                                                                    \
+  do {                                                                                                        \
+    if (rs > (size_t)24 * 1024)                                                                               \
+      cudaFuncSetAttribute(k_regrid<R, ML, SM>, cudaFuncAttributeMaxDynamicSharedMemorySize,                  \
+                           (int)(32 * (3 * ML + 2) * sizeof(R)));                                             \
+    k_regrid<R, ML, SM><<<gr, SM ? 32 : kColBlock, rs, l.stream>>>(g, s, kn, l.sp, targt, tr3d, ex3d, pr3d,   \
+                                                                   w.exsmo, l.flags, l.boundary);             \
+  } while (0)
   if (g.L <= 64) {
-    FIM_KBEGIN(l, "k_regrid");
-    k_regrid<R, 64><<<gc, kColBlock, 0, l.stream>>>(g, s, kn, l.sp, targt, tr3d, ex3d, pr3d, w.exsmo, l.flags,
-                                                     l.boundary);
-  } else {
-    FIM_KBEGIN(l, "k_regrid");
-    k_regrid<R, kMaxL><<<gc, kColBlock, 0, l.stream>>>(g, s, kn, l.sp, targt, tr3d, ex3d, pr3d, w.exsmo,
-                                                        l.flags, l.boundary);
-  }
+    if (rsm) FIM_REGRID(64, true);
+    else FIM_REGRID(64, false);
+  } else if (rsm) FIM_REGRID(kMaxL, true);
+  else FIM_REGRID(kMaxL, false);
+#undef FIM_REGRID
   FIM_KEND(l);
   const R* ex_in = w.exsmo;
   if (kn.intfc_smooth > 0.) {
