@@ -335,6 +335,7 @@ Launch make_launch(fim_ctx* c, int members) {
 }
 
 int push_sp(fim_ctx* c) {
+  for (auto& p : c->h_sp) p.narrow();
   // pageable source: the copy is staged before cudaMemcpyAsync returns
   CK(cudaMemcpyAsync(c->d_sp, c->h_sp.data(), sizeof(StepParams) * c->h_sp.size(), cudaMemcpyHostToDevice,
                      c->stream), "push step params");
@@ -1403,6 +1404,7 @@ int autotune_impl(fim_ctx* c, fim_state* st) {
     p.nf = (p.nf + 1) % 3;
     p.of = (p.of + 1) % 3;
     p.vof = (p.vof + 1) % 3;
+    p.narrow();
   }
   CK(cudaMemcpyAsync(c->d_sp, next.data(), sizeof(StepParams) * next.size(), cudaMemcpyHostToDevice, c->stream),
      "tune params");

@@ -1168,7 +1168,8 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
   ex3d += m * s.intf; dp3d += m * s.cell; pr3d += m * s.intf;
   if (trdp) trdp += m * s.tr;
   const int its = sp->its - bnd;
-  const R p1000 = R(kP1000), small = R(1.e-6);
+  const R p1000 = R(kP1000), small = R(1.e-6), sl = R(kn.slak);
+  const bool fill = kn.thktop == 0.;  // remap_1d's fill of thin layers
   // hystat's floors of tracers 2 and 3 (hystat.F90:90-93) when trdp is formed here
   const R qvmin = R(kQvmin), qwmin = R(kQwmin);
   const int hw = lane / WL, ls = lane - hw * WL;  // column in hand, lane within it
@@ -1250,7 +1251,6 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
         const R eo = S.exold[hw][k];
         R en = S.exnew[hw][k];
         if (its > 0) {
-          const R sl = R(kn.slak);
           en = sl * en + (R(1) - sl) * eo;
         }
         S.exnew[hw][k] = en;
@@ -1289,7 +1289,7 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
       ld_levels<R, VL, FULL>(&S.dpcol[hw][kb], L - kb, dpv);
 #pragma unroll
       for (int v = 0; v < VL; v++) {
-        qqv[v] = sizeof(R) == 4 || kn.thktop == 0. ? fdiv(R(1), dpv[v] + small) : R(0);
+        qqv[v] = sizeof(R) == 4 || fill ? fdiv(R(1), dpv[v] + small) : R(0);
       }
       __syncwarp();
     } else if (j == 1) {
@@ -1357,7 +1357,7 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
       if constexpr (NT == 3) {
         const bool bq = pcwise_v<R, VL, 3, WL, FULL>(L, ls, y, gp);
         bad |= valid && bq;
-        if (kn.thktop == 0.) fill_from_above<R, VL, 3, WL, FULL>(L, ls, y, dpv, qqv);
+        if (fill) fill_from_above<R, VL, 3, WL, FULL>(L, ls, y, dpv, qqv);
 #pragma unroll
         for (int h = 0; h < 3; h++)
           if (valid && o0 + h < F) {
@@ -1373,7 +1373,7 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
             for (int v = 0; v < VL; v++) t[0][v] = y[h][v];
             const bool bq = pcwise_v<R, VL, 1, WL, FULL>(L, ls, t, gp);
             bad |= valid && bq;
-            if (kn.thktop == 0.) fill_from_above<R, VL, 1, WL, FULL>(L, ls, t, dpv, qqv);
+            if (fill) fill_from_above<R, VL, 1, WL, FULL>(L, ls, t, dpv, qqv);
             if (valid) {
               if (trdp) tracer_out<R, VL>(o0 + h - 2, qvmin, qwmin, dpv, t[0], trdp, (size_t)N * L, i, L, kb, vec);
               store_levels<R, VL>(field(o0 + h, i), L, kb, vec, t[0]);

@@ -413,7 +413,7 @@ __device__ __forceinline__ void cnuity12_body(int bx, int by, const Grid<R>& g, 
   massfx += m * s.mf; dplo_tndcy += m * s.ab; antifx += m * s.edge; delp_lo += m * s.cell;
   p_plus += m * s.cell; p_mnus += m * s.cell;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
-  const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
+  const R ab1 = sp->template w1<R>(), ab2 = sp->template w2<R>(), ab3 = sp->template w3<R>();
   R* mfn = massfx + (size_t)nf * N * 6 * L;
   const int np = g.nprox[i];
   const R half = R(0.5);
@@ -499,7 +499,7 @@ __device__ __forceinline__ void cnuity3_body(int bx, int by, const Grid<R>& g, c
   delp_lo += m * s.cell; delp += m * s.cell; dp_tndcy += m * s.ab;
   p_plus += m * s.cell; p_mnus += m * s.cell; r_plus += m * s.cell; r_mnus += m * s.cell;
   const int of = sp->of, vof = sp->vof;
-  const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
+  const R ab1 = sp->template w1<R>(), ab2 = sp->template w2<R>(), ab3 = sp->template w3<R>();
   const R rab1 = R(1) / ab1;  // Q+/Q- divide by ab1: one reciprocal
   const R thshld = R(1.e-11);
   const size_t c = (size_t)i * L + k;
@@ -553,7 +553,7 @@ __device__ __forceinline__ void cnuity4_body(int bx, int by, const Grid<R>& g, c
   antifx += m * s.edge; r_plus += m * s.cell; r_mnus += m * s.cell; massfx += m * s.mf;
   dplo_tndcy += m * s.ab; dp_tndcy += m * s.ab; delp += m * s.cell;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
-  const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
+  const R ab1 = sp->template w1<R>(), ab2 = sp->template w2<R>(), ab3 = sp->template w3<R>();
   R* mfn = massfx + (size_t)nf * N * 6 * L;
   const size_t c = (size_t)i * L + k;
   R rp[VK], rm[VK], at[VK];
@@ -699,7 +699,7 @@ __global__ void __launch_bounds__(kC5Block, 4) k_cnuity5(Grid<R> g, Strides s,
   pres += m * s.intf; delp += m * s.cell; exner += m * s.intf; dp_tndcy += m * s.ab;
   omega += m * s.cell; lp_edg += m * s.edge; u += m * s.cell; v += m * s.cell;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
-  const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3), dt = R(sp->dt);
+  const R ab1 = sp->template w1<R>(), ab2 = sp->template w2<R>(), ab3 = sp->template w3<R>(), dt = sp->template step<R>();
   const R cp = R(kCp), p1000 = R(kP1000), rdt = R(1) / dt;
   const size_t NL = (size_t)N * L;
 #pragma unroll 2
@@ -855,7 +855,7 @@ __global__ void __launch_bounds__(kBlock) k_massadv_lim(Grid<R> g, Strides s, co
   u_edg += m * s.edge; v_edg += m * s.edge; dp_edg += m * s.edge; delp += m * s.cell; dp_tndcy += m * s.ab;
   qmin_out += m * s.cell; qmax_out += m * s.cell;
   const int of = sp->of, vof = sp->vof;
-  const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3), dt = R(sp->dt);
+  const R ab1 = sp->template w1<R>(), ab2 = sp->template w2<R>(), ab3 = sp->template w3<R>(), dt = sp->template step<R>();
   const size_t c = (size_t)i * L + k;
   const R gv = delp[c], rar = g.rarea[i];
   const int np = g.nprox[i];
@@ -1051,11 +1051,17 @@ __global__ void __launch_bounds__(kBlock) k_dissip(Grid<R> g, Strides s, const R
 
 // momtum1 (momtum_compute.F90:278-423, janjic=0) after adding the dissipation
 // increments (momtum.F90:130-139); one warp per column so the Rayleigh damping
-// of the top layers can read the updated top three levels.  Four blocks a
-// SM (64 registers, a few spilled) measured 1.77 ms at glvl 8 against 1.96
-// at three (80 registers).
-template <typename R, int NC>
-__global__ void __launch_bounds__(kBlock, 4) k_momtum1(Grid<R> g, Strides s, Knobs kn, const StepParams* __restrict__ sp,
+// of the top layers can read the updated top three levels.  A lane takes VK
+// consecutive levels (one chunk of 32 VK levels covers nvl 64 with two), so the
+// cell's tables and row addresses are formed once for both.  SPLIT: the
+// FP32-mixed step's form (mpf, tr0).  Bound by HBM: at glvl 8 / nvl 64 the step's
+// form takes 1.20 ms, 6,150 GB/s of its 44 words (one level a lane 1.57 ms; two
+// blocks an SM 1.32, four 1.34); the plain form at glvl 7 0.30 ms at four blocks
+// an SM (three 0.34; one level a lane 0.43).  FP64, one level a lane, is bound
+// by its operations: glvl 6 0.44 -> 0.32 ms with M + K - exm th formed once.
+template <typename R, int NC, int VK, bool SPLIT>
+__global__ void __launch_bounds__(kBlock, SPLIT ? 3 : 4) k_momtum1(Grid<R> g, Strides s, R rlthresh, R rleigh,
+    R rltaper, const StepParams* __restrict__ sp,
     R* __restrict__ u, R* __restrict__ v, const R* __restrict__ du, const R* __restrict__ dv,
     const R* __restrict__ exner, R* __restrict__ relvor, const R* __restrict__ u_edg, const R* __restrict__ v_edg,
     const R* __restrict__ trc_edg, const R* __restrict__ mont_edg, const R* __restrict__ uvsq_edg,
@@ -1074,41 +1080,68 @@ __global__ void __launch_bounds__(kBlock, 4) k_momtum1(Grid<R> g, Strides s, Kno
   uvsq_edg += m * s.edge; u_tndcy += m * s.ab; v_tndcy += m * s.ab;
   const bool have_d = du != nullptr;
   if (have_d) { du += m * s.cell; dv += m * s.cell; }
-  const bool split = mpf != nullptr;
-  if (split) { mpf += m * s.cell; tr0 += m * s.cell; }
+  if constexpr (SPLIT) { mpf += m * s.cell; tr0 += m * s.cell; }
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
-  const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
+  const R ab1 = sp->template w1<R>(), ab2 = sp->template w2<R>(), ab3 = sp->template w3<R>();
   const size_t NL = (size_t)N * L;
   const int np = g.nprox[i];
   const int* pr = g.prox + i * 6;
   const R rar = g.rarea[i], cor = g.corio[i];
-  // Loads use a clamped level and the six edge slots of every cell (a
+  // Loads use clamped levels and the six edge slots of every cell (a
   // pentagon's slot 5 and its prox entry are valid memory), so they carry no
   // branch and can be issued together; results and stores are masked.
-  R un[NC], vn[NC];
+  R un[NC][VK], vn[NC][VK];
 #pragma unroll
   for (int ch = 0; ch < NC; ch++) {
-    const int k = ch * 32 + lane;
-    const int kk = k < L ? k : L - 1;
+    const int k = (ch * 32 + lane) * VK;
+    const int kk = k < L ? k : L - VK;
     const size_t c = (size_t)i * L + kk;
-    R uu = u[c], vv = v[c];
-    if (have_d) { uu = uu + du[c]; vv = vv + dv[c]; }
-    const R exm = R(0.5) * (exner[(size_t)i * L1 + kk] + exner[(size_t)i * L1 + kk + 1]);
-    R pgfx = R(0), pgfy = R(0), rv = R(0);
-    if (!split) {
+    R uu[VK], vv[VK], exm[VK];
+    ldv<VK>(u + c, uu);
+    ldv<VK>(v + c, vv);
+    if (have_d) {
+      R a[VK], b[VK];
+      ldv<VK>(du + c, a);
+      ldv<VK>(dv + c, b);
+      FOR_V { uu[j] = uu[j] + a[j]; vv[j] = vv[j] + b[j]; }
+    }
+    {
+      const R* e = exner + (size_t)i * L1 + kk;
+      R lo = e[0];
+      FOR_V {
+        const R hi = e[j + 1];
+        exm[j] = R(0.5) * (lo + hi);
+        lo = hi;
+      }
+    }
+    R pgfx[VK], pgfy[VK], rv[VK];
+    FOR_V { pgfx[j] = R(0); pgfy[j] = R(0); rv[j] = R(0); }
+    if constexpr (!SPLIT) {
 #pragma unroll
       for (int e = 0; e < 6; e++) {
         const bool live = e < np;
         const R* svc = g.svc + (i * 6 + e) * 2;
         const R* sve = g.sve + (i * 6 + e) * 2;
         const size_t o = ((size_t)i * 6 + e) * L + kk;
-        const R mu = mont_edg[o] + uvsq_edg[o];
-        const R th = trc_edg[o];
-        const R ue = u_edg[o], ve = v_edg[o];
+        R mo[VK], kv[VK], th[VK], ue[VK], ve[VK];
+        ldv<VK>(mont_edg + o, mo);
+        ldv<VK>(uvsq_edg + o, kv);
+        ldv<VK>(trc_edg + o, th);
+        ldv<VK>(u_edg + o, ue);
+        ldv<VK>(v_edg + o, ve);
         if (live) {
-          pgfx = pgfx - mu * svc[1] + exm * th * svc[1];
-          pgfy = pgfy + mu * svc[0] - exm * th * svc[0];
-          rv = rv + (sve[0] * ue + sve[1] * ve);
+          FOR_V {
+            if constexpr (sizeof(R) == 8) {  // the fewest operations: (M + K - exm th) s
+              const R w = (mo[j] + kv[j]) - exm[j] * th[j];
+              pgfx[j] = pgfx[j] - w * svc[1];
+              pgfy[j] = pgfy[j] + w * svc[0];
+            } else {
+              const R mu = mo[j] + kv[j];
+              pgfx[j] = pgfx[j] - mu * svc[1] + exm[j] * th[j] * svc[1];
+              pgfy[j] = pgfy[j] + mu * svc[0] - exm[j] * th[j] * svc[0];
+            }
+            rv[j] = rv[j] + (sve[0] * ue[j] + sve[1] * ve[j]);
+          }
         }
       }
     } else {
@@ -1117,12 +1150,12 @@ __global__ void __launch_bounds__(kBlock, 4) k_momtum1(Grid<R> g, Strides s, Kno
       //   = sum_e (dM_e + K_e - exm dth_e) s_e + (M_c - exm th_c) sum_e s_e,
       // dM_e, dth_e the edge-minus-cell values (edgvar1's weights applied to
       // neighbour differences); the large cell term is formed in FP64.
-      const R thc = tr0[(size_t)i * L + kk];
-      R dth[6];
+      R thc[VK], dth[6][VK];
+      ldv<VK>(tr0 + c, thc);
 #pragma unroll
-      for (int j = 0; j < 6; j++) {
-        const R tn = tr0[(size_t)pr[j] * L + kk];
-        dth[j] = (j < np) ? tn - thc : R(0);
+      for (int q = 0; q < 6; q++) {
+        ldv<VK>(tr0 + (size_t)pr[q] * L + kk, dth[q]);
+        FOR_V dth[q][j] = (q < np) ? dth[q][j] - thc[j] : R(0);
       }
       const R divby6 = R(1) / R(6);
 #pragma unroll
@@ -1132,66 +1165,89 @@ __global__ void __launch_bounds__(kBlock, 4) k_momtum1(Grid<R> g, Strides s, Kno
         const R* sve = g.sve + (i * 6 + e) * 2;
         const size_t o = ((size_t)i * 6 + e) * L + kk;
         const int et = e == 0 ? np - 1 : e - 1, el = e == np - 1 ? 0 : e + 1;
-        R dte = R(0);
+        R mo[VK], kv[VK], ue[VK], ve[VK];
+        ldv<VK>(mont_edg + o, mo);
+        ldv<VK>(uvsq_edg + o, kv);
+        ldv<VK>(u_edg + o, ue);
+        ldv<VK>(v_edg + o, ve);
+        FOR_V {
+          R dte = R(0);
 #pragma unroll
-        for (int j = 0; j < 6; j++) {
-          if (j == e) dte = dte + R(2) * dth[j];
-          if (j == et || j == el) dte = dte + dth[j];
-        }
-        dte = dte * divby6;
-        const R mo = mont_edg[o], kv = uvsq_edg[o], ue = u_edg[o], ve = v_edg[o];
-        if (live) {
-          const R w = mo + kv - exm * dte;
-          pgfx = pgfx - w * svc[1];
-          pgfy = pgfy + w * svc[0];
-          rv = rv + (sve[0] * ue + sve[1] * ve);
+          for (int q = 0; q < 6; q++) {
+            if (q == e) dte = dte + R(2) * dth[q][j];
+            if (q == et || q == el) dte = dte + dth[q][j];
+          }
+          dte = dte * divby6;
+          if (live) {
+            const R w = mo[j] + kv[j] - exm[j] * dte;
+            pgfx[j] = pgfx[j] - w * svc[1];
+            pgfy[j] = pgfy[j] + w * svc[0];
+            rv[j] = rv[j] + (sve[0] * ue[j] + sve[1] * ve[j]);
+          }
         }
       }
       // Montgomery potential minus exner x theta, cancellation-free
-      const float2 mp = mpf[(size_t)i * L + kk];
-      const FF2 cf = ff_add(FF2{mp.x, mp.y}, ff_neg(two_prod(float(exm), float(thc))));
-      const R cell = R(cf.hi + cf.lo);
-      pgfx = pgfx - cell * g.svsum[i * 2 + 1];
-      pgfy = pgfy + cell * g.svsum[i * 2 + 0];
+      FOR_V {
+        const float2 mp = mpf[c + j];
+        const FF2 cf = ff_add(FF2{mp.x, mp.y}, ff_neg(two_prod(float(exm[j]), float(thc[j]))));
+        const R cell = R(cf.hi + cf.lo);
+        pgfx[j] = pgfx[j] - cell * g.svsum[i * 2 + 1];
+        pgfy[j] = pgfy[j] + cell * g.svsum[i * 2 + 0];
+      }
     }
-    pgfx = pgfx * rar;
-    pgfy = pgfy * rar;
-    rv = rv * rar;
-    const R uzeta = (cor + rv) * uu, vzeta = (cor + rv) * vv;
-    const R ut = pgfx + vzeta, vt = pgfy - uzeta;
-    uu = uu + ab1 * ut + ab2 * u_tndcy[(size_t)of * NL + c] + ab3 * u_tndcy[(size_t)vof * NL + c];
-    vv = vv + ab1 * vt + ab2 * v_tndcy[(size_t)of * NL + c] + ab3 * v_tndcy[(size_t)vof * NL + c];
-    un[ch] = uu;
-    vn[ch] = vv;
+    R ut[VK], vt[VK], uo[VK], uv[VK], vo[VK], vw[VK];
+    ldv<VK>(u_tndcy + (size_t)of * NL + c, uo);
+    ldv<VK>(u_tndcy + (size_t)vof * NL + c, uv);
+    ldv<VK>(v_tndcy + (size_t)of * NL + c, vo);
+    ldv<VK>(v_tndcy + (size_t)vof * NL + c, vw);
+    FOR_V {
+      pgfx[j] = pgfx[j] * rar;
+      pgfy[j] = pgfy[j] * rar;
+      rv[j] = rv[j] * rar;
+      const R uzeta = (cor + rv[j]) * uu[j], vzeta = (cor + rv[j]) * vv[j];
+      ut[j] = pgfx[j] + vzeta;
+      vt[j] = pgfy[j] - uzeta;
+      uu[j] = uu[j] + ab1 * ut[j] + ab2 * uo[j] + ab3 * uv[j];
+      vv[j] = vv[j] + ab1 * vt[j] + ab2 * vo[j] + ab3 * vw[j];
+      un[ch][j] = uu[j];
+      vn[ch][j] = vv[j];
+    }
     if (k < L) {
-      relvor[c] = rv;
-      u_tndcy[(size_t)nf * NL + c] = ut;
-      v_tndcy[(size_t)nf * NL + c] = vt;
-      if (k >= L - 3) { top[wib][L - 1 - k][0] = uu; top[wib][L - 1 - k][1] = vv; }
+      stv<VK>(relvor + c, rv);
+      stv<VK>(u_tndcy + (size_t)nf * NL + c, ut);
+      stv<VK>(v_tndcy + (size_t)nf * NL + c, vt);
+      FOR_V
+        if (k + j >= L - 3) { top[wib][L - 1 - k - j][0] = uu[j]; top[wib][L - 1 - k - j][1] = vv[j]; }
     }
   }
   __syncwarp();
   const R q1 = top[wib][0][0] * top[wib][0][0] + top[wib][0][1] * top[wib][0][1];
   const R q2 = top[wib][1][0] * top[wib][1][0] + top[wib][1][1] * top[wib][1][1];
   const R q3 = top[wib][2][0] * top[wib][2][0] + top[wib][2][1] * top[wib][2][1];
-  const R thr = R(kn.rlthresh);
-  R qq = rmax(rmax(q1, q2), q3) / (thr * thr);
-  const int ndamp = (int)(0.25 * L);
+  R qq = rmax(rmax(q1, q2), q3) / (rlthresh * rlthresh);
+  const int ndamp = L / 4;
   const bool damp = qq > R(1);
-  if (damp) qq = sqrt((qq - R(1)) * qq);
-  const R dtf = R(sp->dt) / R(86400.), rl = R(kn.rleigh), rt = R(kn.rltaper);
+  if (damp) {
+    qq = sqrt((qq - R(1)) * qq);
+    const R dtf = sp->template step<R>() / R(86400.);
+#pragma unroll
+    for (int ch = 0; ch < NC; ch++) {
+      FOR_V {
+        const int k = (ch * 32 + lane) * VK + j;
+        if (k >= L - 1 - ndamp) {
+          const R factor = R(1) - dtf * rleigh * qq * pow(R(2), rltaper * R(k + 1 - L));
+          un[ch][j] = un[ch][j] * factor;
+          vn[ch][j] = vn[ch][j] * factor;
+        }
+      }
+    }
+  }
 #pragma unroll
   for (int ch = 0; ch < NC; ch++) {
-    const int k = ch * 32 + lane;
+    const int k = (ch * 32 + lane) * VK;
     if (k < L) {
-      R uu = un[ch], vv = vn[ch];
-      if (damp && k >= L - 1 - ndamp) {
-        const R factor = R(1) - dtf * rl * qq * pow(R(2), rt * R(k + 1 - L));
-        uu = uu * factor;
-        vv = vv * factor;
-      }
-      u[(size_t)i * L + k] = uu;
-      v[(size_t)i * L + k] = vv;
+      stv<VK>(u + (size_t)i * L + k, un[ch]);
+      stv<VK>(v + (size_t)i * L + k, vn[ch]);
     }
   }
 }
@@ -1210,6 +1266,7 @@ __global__ void k_step_begin(StepParams* sp, int members) {
   if (p.its == 1) { p.ab1 = p.dt; p.ab2 = 0.; p.ab3 = 0.; }
   if (p.its == 2) { p.ab1 = p.dt * 1.5; p.ab2 = -p.dt * .5; p.ab3 = 0.; }
   if (p.its == 3) { p.ab1 = p.dt * 23. / 12.; p.ab2 = -p.dt * 16. / 12.; p.ab3 = p.dt * 5. / 12.; }
+  p.narrow();
   *sp = p;
 }
 
@@ -1331,14 +1388,32 @@ void launch_momtum(const Launch& l, const Grid<R>& g, const Strides& s, const Kn
   }
   dim3 gw(blocks_for((long long)g.N * 32), l.members);
   FIM_KBEGIN(l, "k_momtum1");
-  const int nc = (g.L + 31) / 32;
-#define FIM_MOMTUM1(NC)                                                                                        \
-  k_momtum1<R, NC><<<gw, kBlock, 0, l.stream>>>(g, s, kn, l.sp, u, v, du, dv, exner, relvor, u_edg, v_edg, trc_edg, \
-                                                 mont_edg, uvsq_edg, u_tndcy, v_tndcy, mpf, tr0)
-  if (nc == 1) FIM_MOMTUM1(1);
-  else if (nc == 2) FIM_MOMTUM1(2);
-  else if (nc == 3) FIM_MOMTUM1(3);
-  else FIM_MOMTUM1(4);
+  const int vm = pick_vk<R>(g.L, {u, v, du, dv, relvor, u_edg, v_edg, trc_edg, mont_edg, uvsq_edg, u_tndcy, v_tndcy,
+                                  tr0}, sizeof(R) == 8 ? 1 : 2);
+  const int nc = (g.L + 32 * vm - 1) / (32 * vm);
+#define FIM_MOMTUM1S(NC, VK, SPLIT)                                                                            \
+  k_momtum1<R, NC, VK, SPLIT><<<gw, kBlock, 0, l.stream>>>(g, s, R(kn.rlthresh), R(kn.rleigh), R(kn.rltaper), l.sp, u, \
+                                                            v, du, dv, exner, relvor, u_edg, v_edg, trc_edg, mont_edg, \
+                                                            uvsq_edg, u_tndcy, v_tndcy, mpf, tr0)
+#define FIM_MOMTUM1(NC, VK)                                                                                    \
+  do {                                                                                                         \
+    if constexpr (sizeof(R) == 4) {                                                                            \
+      if (mpf) FIM_MOMTUM1S(NC, VK, true);                                                                     \
+      else FIM_MOMTUM1S(NC, VK, false);                                                                        \
+    } else {                                                                                                   \
+      FIM_MOMTUM1S(NC, VK, false);                                                                             \
+    }                                                                                                          \
+  } while (0)
+  if (vm == 2) {
+    if constexpr (sizeof(R) == 4) {
+      if (nc == 1) FIM_MOMTUM1(1, 2);
+      else FIM_MOMTUM1(2, 2);
+    }
+  } else if (nc == 1) FIM_MOMTUM1(1, 1);
+  else if (nc == 2) FIM_MOMTUM1(2, 1);
+  else if (nc == 3) FIM_MOMTUM1(3, 1);
+  else FIM_MOMTUM1(4, 1);
+#undef FIM_MOMTUM1S
 #undef FIM_MOMTUM1
   FIM_KEND(l);
 }

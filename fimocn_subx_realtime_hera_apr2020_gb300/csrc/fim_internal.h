@@ -41,6 +41,20 @@ struct StepParams {
   // tracers the member transports (fim_member_set_tracers): the tracer
   // transport, the remap and the budget sums leave slots ntr.. as they are
   int ntr = 0x7fffffff;
+  // the weights and dt in FP32 (narrow(), wherever the doubles are set for the
+  // device): a conversion a thread costs the FP32 kernels 16 clocks of the FP64
+  // pipe a warp
+  float f1 = 0.f, f2 = 0.f, f3 = 0.f, fdt = 0.f;
+  __host__ __device__ void narrow() {
+    f1 = (float)ab1;
+    f2 = (float)ab2;
+    f3 = (float)ab3;
+    fdt = (float)dt;
+  }
+  template <typename R> __device__ __forceinline__ R w1() const { if constexpr (sizeof(R) == 4) return f1; else return ab1; }
+  template <typename R> __device__ __forceinline__ R w2() const { if constexpr (sizeof(R) == 4) return f2; else return ab2; }
+  template <typename R> __device__ __forceinline__ R w3() const { if constexpr (sizeof(R) == 4) return f3; else return ab3; }
+  template <typename R> __device__ __forceinline__ R step() const { if constexpr (sizeof(R) == 4) return fdt; else return dt; }
 };
 
 // device status bits

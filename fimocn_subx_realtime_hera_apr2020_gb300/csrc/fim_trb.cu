@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(kTB2) k_transp1(Grid<R> g, Strides s, const St
   cumufx += m * s.edge;
   massfx += m * s.mf;
   const size_t NE = (size_t)N * 6 * L;
-  const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
+  const R ab1 = sp->template w1<R>(), ab2 = sp->template w2<R>(), ab3 = sp->template w3<R>();
   const int np = g.nprox[i];
   for (int e = 0; e < np; e++) {
     const size_t o = ((size_t)i * 6 + e) * L + k;

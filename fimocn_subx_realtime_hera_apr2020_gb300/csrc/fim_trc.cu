@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(64 * GC, 8 / GC) k_trf_lo(Grid<R> g, Strides s
   if (!EV) load_coefs<R>(g, fs, hf, C, nre);
   const size_t NL = (size_t)N * L;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
-  const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
+  const R ab1 = sp->template w1<R>(), ab2 = sp->template w2<R>(), ab3 = sp->template w3<R>();
   const R* mfn = massfx + m * s.mf + (size_t)nf * 6 * NL;
   const R* te0 = trc_edg + m * s.tredg;  // EV: tracer t's at t * 6 NL; else theta's (edgvar1)
   // this step's tracer t: its frame, and the patch cells' AB3 slots of/vof
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameT
   __syncthreads();
   const size_t NL = (size_t)N * L;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
-  const R ab1 = R(sp->ab1), ab2 = R(sp->ab2), ab3 = R(sp->ab3);
+  const R ab1 = sp->template w1<R>(), ab2 = sp->template w2<R>(), ab3 = sp->template w3<R>();
   const R rab1 = R(1) / ab1;  // Q+/Q- divide by ab1: one reciprocal
   for (int x = threadIdx.x; x < n1; x += blockDim.x) arf[x] = g.area[fs.cells[x]] * (sizeof(R) == 8 ? rab1 : R(1));
   // the limiters' operands of tracer t0 + tz
