@@ -445,11 +445,20 @@ __device__ __forceinline__ void cnuity12_body(int bx, int by, const Grid<R>& g, 
     R dm[VK];
     ldv<VK>(dp_edg + o, de);
     ldv<VK>(dp_edg + ox, dm);
-    FOR_V de[j] = half * (de[j] + dm[j]);
+    if constexpr (sizeof(R) == 4) FOR_V de[j] = half * (de[j] + dm[j]);
     ldv<VK>(delp + (size_t)ipx * L + k, dx);
     FOR_V {
       const R vn = sv[1] * ue[j] - sv[0] * ve[j];
       const R vx = sx[1] * ux[j] - sx[0] * vx_[j];
+      if constexpr (sizeof(R) == 8) {  // the same, with half the FP64 operations
+        mf[j] = donor(vn, vx, dpi[j], dx[j]);
+        an[j] = fma(half * vn, de[j] + dm[j], -mf[j]);
+        if (live) {
+          sum[j] = sum[j] + mf[j];
+          split_sum(an[j], pp[j], pm[j]);
+        }
+        continue;
+      }
       const R flxhi = vn * de[j];
       mf[j] = half * ((vn + rabs(vn)) * dpi[j] - (vx + rabs(vx)) * dx[j]);
       const R a = flxhi - mf[j];
@@ -504,29 +513,39 @@ __device__ __forceinline__ void cnuity3_body(int bx, int by, const Grid<R>& g, c
   const R thshld = R(1.e-11);
   const size_t c = (size_t)i * L + k;
   const int* pr = g.prox + i * 6;
-  R dlo[VK], dc[VK], mx[VK], mn[VK];
+  R dlo[VK], dc[VK];
   ldv<VK>(delp_lo + c, dlo);
   ldv<VK>(delp + c, dc);
-  FOR_V { mx[j] = rmax(dlo[j], dc[j]); mn[j] = rmin(dlo[j], dc[j]); }
+  Bound<R> mx[VK], mn[VK];
+  FOR_V {
+    mx[j] = mn[j] = Bound<R>::of(dlo[j]);
+    const Bound<R> b = Bound<R>::of(dc[j]);
+    mx[j].up(b);
+    mn[j].down(b);
+  }
 #pragma unroll
   for (int e = 0; e < 6; e++) {
     R a[VK], b[VK];
     ldv<VK>(delp_lo + (size_t)pr[e] * L + k, a);
     ldv<VK>(delp + (size_t)pr[e] * L + k, b);
-    FOR_V { mx[j] = rmax(mx[j], rmax(a[j], b[j])); mn[j] = rmin(mn[j], rmin(a[j], b[j])); }
+    FOR_V {
+      const Bound<R> ba = Bound<R>::of(a[j]), bb = Bound<R>::of(b[j]);
+      mx[j].up(ba, bb);
+      mn[j].down(ba, bb);
+    }
   }
   R to[VK], tv[VK], pp[VK], pm[VK], rp[VK], rm[VK];
   ldv<VK>(dp_tndcy + (size_t)of * N * L + c, to);
   ldv<VK>(dp_tndcy + (size_t)vof * N * L + c, tv);
   ldv<VK>(p_plus + c, pp);
   ldv<VK>(p_mnus + c, pm);
-  const R ar = g.area[i];
+  const R ar = sizeof(R) == 8 ? g.area[i] * rab1 : g.area[i];
   FOR_V {
-    const R dpmax = rmax(R(0), mx[j]), dpmin = rmax(R(0), mn[j]);
-    const R q_plus = (dpmax - dlo[j] - (ab2 * rmin(R(0), to[j]) + ab3 * rmax(R(0), tv[j]))) * rab1 * ar;
-    const R q_mnus = (dlo[j] - dpmin + (ab2 * rmax(R(0), to[j]) + ab3 * rmin(R(0), tv[j]))) * rab1 * ar;
-    rp[j] = rmax(R(0), rmin(R(1), fdiv(q_plus, rmax(pp[j], thshld))));
-    rm[j] = rmax(R(0), rmin(R(1), fdiv(q_mnus, rmax(pm[j], thshld))));
+    const R dpmax = mx[j].at_least_zero(), dpmin = mn[j].at_least_zero();
+    const R q_plus = per_ab1(dpmax - dlo[j] - (ab2 * neg(to[j]) + ab3 * pos(tv[j])), rab1, ar);
+    const R q_mnus = per_ab1(dlo[j] - dpmin + (ab2 * pos(to[j]) + ab3 * neg(tv[j])), rab1, ar);
+    rp[j] = ratio01(q_plus, floor_at(pp[j], thshld));
+    rm[j] = ratio01(q_mnus, floor_at(pm[j], thshld));
   }
   stv<VK>(r_plus + c, rp);
   stv<VK>(r_mnus + c, rm);
@@ -570,7 +589,8 @@ __device__ __forceinline__ void cnuity4_body(int bx, int by, const Grid<R>& g, c
     ldv<VK>(r_plus + (size_t)px * L + k, rpx);
     ldv<VK>(r_mnus + (size_t)px * L + k, rmx);
     FOR_V {
-      const R clip = (a[j] >= R(0)) ? rmin(rm[j], rpx[j]) : rmin(rp[j], rmx[j]);
+      const bool in = negative(a[j]);
+      const R clip = min0(in ? rp[j] : rm[j], in ? rmx[j] : rpx[j]);
       const R ac = a[j] * clip;
       mf[j] = mf[j] + ac;
       at[j] = at[j] + ac;
@@ -990,7 +1010,7 @@ __global__ void __launch_bounds__(kBlock) k_dissip(Grid<R> g, Strides s, const R
   if (prep) { wu += m * s.cell; wv += m * s.cell; }
   const R thshld = R(1.e-11), two = R(2);
   const size_t c = (size_t)i * L + k;
-  R ui[VK], vi[VK], dpi[VK], factor[VK], dfl[VK], su[VK], sv[VK];
+  R ui[VK], vi[VK], dpi[VK], factor[VK], dfl[VK], dfl2[VK], su[VK], sv[VK];
   if (prep) {
     ldv<VK>(wu + c, ui);
     ldv<VK>(wv + c, vi);
@@ -1006,6 +1026,7 @@ __global__ void __launch_bounds__(kBlock) k_dissip(Grid<R> g, Strides s, const R
     dpi[j] = rmax(dpi[j], thshld);
     factor[j] = fdiv(rar, dpi[j]);
     dfl[j] = g.dfflen[k + j];
+    dfl2[j] = two * dfl[j];
     su[j] = R(0);
     sv[j] = R(0);
   }
@@ -1032,6 +1053,18 @@ __global__ void __launch_bounds__(kBlock) k_dissip(Grid<R> g, Strides s, const R
     }
     ldv<VK>(delp + cx, bx);
     const R sl = g.sideln[i * 6 + e];
+    if constexpr (sizeof(R) == 8) {
+      // the same with the factors gathered and the jumps formed in one chain
+      if (live) FOR_V {
+        const R b = floor_at(bx[j], thshld);
+        const R w = (dfl2[j] * sl) * f64_quot(dpi[j] * b, dpi[j] + b, f64_recip(dpi[j] + b)) * factor[j];
+        const R ju = cs[1] * ux[j] + sn[1] * vx[j] - cs[0] * ui[j] - sn[0] * vi[j];
+        const R jv = cs[1] * vx[j] - sn[1] * ux[j] - cs[0] * vi[j] + sn[0] * ui[j];
+        su[j] = su[j] + (cs[0] * ju - sn[0] * jv) * w;
+        sv[j] = sv[j] + (sn[0] * ju + cs[0] * jv) * w;
+      }
+      continue;
+    }
     FOR_V {
       const R uxy1 = cs[0] * ui[j] + sn[0] * vi[j], vxy1 = -sn[0] * ui[j] + cs[0] * vi[j];
       const R uxy2 = cs[1] * ux[j] + sn[1] * vx[j], vxy2 = -sn[1] * ux[j] + cs[1] * vx[j];
