@@ -19,6 +19,7 @@ namespace fim {
 template <typename R> __device__ __forceinline__ R cmax(R a, R b) { return a > b ? a : b; }
 template <typename R> __device__ __forceinline__ R cmin(R a, R b) { return a < b ? a : b; }
 template <typename R> __device__ __forceinline__ R cabs(R a) { return a < R(0) ? -a : a; }
+__device__ __forceinline__ double cabs(double a) { return fabs(a); }
 
 // FP64 comparisons on the integer pipe (fim_internal.h)
 __device__ __forceinline__ bool lt(float a, float b) { return a < b; }
@@ -858,7 +859,7 @@ __device__ __forceinline__ void lane_geo(int L, int lane, const R* xo, const R* 
     if (lv.in(v)) {
       fo = coord_thick(flip, xo, k);
       fn = coord_thick(flip, xn, k);
-      thin = thin || fo < fill_thin<R>();
+      thin = thin || lt(fo, fill_thin<R>());
     }
     G.fo[v] = fo;
     if constexpr (sizeof(R) == 4) G.rfo[v] = fdiv(R(1), fo + small);
@@ -866,19 +867,20 @@ __device__ __forceinline__ void lane_geo(int L, int lane, const R* xo, const R* 
     R nd = R(0), hh = R(0);
     if (lv.in(v) && !lv.first(v)) {
       const R d = flip ? (-xn[k]) - (-xo[k]) : xn[k] - xo[k];
-      if (d != R(0)) {
-        const R fl = coord_thick(flip, xo, d > R(0) ? k : k - 1);
-        if (fl > R(0)) {
-          const R dd = d > R(0) ? d : -d;
+      const bool down = lt(d, R(0)), rise = lt(R(0), d);
+      if (down || rise) {
+        const R fl = coord_thick(flip, xo, rise ? k : k - 1);
+        if (lt(R(0), fl)) {
+          const R dd = rise ? d : -d;
           const R dsl = cmin(fl, dd);
           const R dx = over(dsl, fl);
-          const R hx = d > R(0) ? dx - R(1) : R(1) - dx;
-          if (dsl != R(0)) {
+          const R hx = rise ? dx - R(1) : R(1) - dx;
+          if (lt(R(0), dsl)) {
             nd = -d;
             hh = R(.5) * hx;
           }
         }
-        if (d > R(0)) up |= 1u << v;
+        if (rise) up |= 1u << v;
       }
     }
     G.nd[v] = nd;
@@ -999,7 +1001,8 @@ __device__ __forceinline__ bool pcwise_v(int L, int lane, R (&y)[NF][VL], const 
       const bool up = (G.up >> v) & 1u;
       const R a = up ? yf[h][v] : (v > 0 ? yf[h][v - 1] : ym);
       const R b = up ? bk[v] : (v > 0 ? bk[v - 1] : bm);
-      fl[v] = G.nd[v] != R(0) ? G.nd[v] * (a + b * G.hh[v]) : R(0);
+      fl[v] = G.nd[v] * (a + b * G.hh[v]);
+      if (sizeof(R) == 4 && G.nd[v] == R(0)) fl[v] = R(0);
     }
     const R fnext = __shfl_down_sync(0xffffffffu, fl[0], 1, W);
     R after = R(0);
@@ -1450,14 +1453,14 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
       const R devilo = (tha - S.tg[k - 2]) * dplo;
       const R deviup = dev;
       R na = tha, nbv = thb;
-      if (deviup > R(0) && devilo < R(0)) {
+      if (lt(R(0), deviup) && lt(devilo, R(0))) {
         const R cc = cmin(deviup, -devilo);
-        na = tha + cc / dplo;
-        nbv = thb - cc / dpup;
-      } else if (deviup < R(0) && devilo > R(0)) {
+        na = tha + qdiv(cc, dplo);
+        nbv = thb - qdiv(cc, dpup);
+      } else if (lt(deviup, R(0)) && lt(R(0), devilo)) {
         const R cc = cmin(devilo, -deviup);
-        na = tha - cc / dplo;
-        nbv = thb + cc / dpup;
+        na = tha - qdiv(cc, dplo);
+        nbv = thb + qdiv(cc, dpup);
       }
       th[k - 1] = nbv;
       thb = na;

@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_edgvar1(Grid<R> g, Strides s, int
           vn = two * vn + cs[2] * vt - sn[2] * ut + cs[3] * vl - sn[3] * ul;
           const R sq = un * un + vn * vn;
           const R ms = (two * (m0[j] + mx[e][j]) + FIM_TRAIL(mx) + FIM_LEAD(mx)) * divby6;
-          const R q = sq > R(36) * eps * eps ? ms * inv_root(sq) : ms * (R(1) / (R(6) * eps));
+          const R q = ms * (f64_key(sq) > f64_key(R(36) * eps * eps) ? inv_root(sq) : R(1) / (R(6) * eps));
           ue[j] = un * q;
           ve[j] = vn * q;
         } else {
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_edgvar1(Grid<R> g, Strides s, int
   {
     const R divby6 = R(1) / R(6), half = R(0.5);
     const R* pm = pres + m * s.intf;
-    R p0[VK], pa[6][VK], pb[6][VK];
+    R p0[VK], pa[6][VK], pb[6][VK];  // FP64: pa the layer's sum
     FOR_V p0[j] = pm[(size_t)i * L1 + k + j] + pm[(size_t)i * L1 + k + j + 1];
 #pragma unroll
     for (int e = 0; e < 6; e++) {
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_edgvar1(Grid<R> g, Strides s, int
       R a = pe[0];
       FOR_V {
         const R b = pe[j + 1];
-        pa[e][j] = a;
+        pa[e][j] = sizeof(R) == 8 ? a + b : a;
         pb[e][j] = b;
         a = b;
       }
@@ -190,7 +190,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_edgvar1(Grid<R> g, Strides s, int
     for (int e = 0; e < 6; e++) {
       if (e == 5 && five) continue;
       R lp[VK];
-      FOR_V lp[j] = (p0[j] + pa[e][j] + pb[e][j] + half * (FIM_TRAIL(pa) + FIM_TRAIL(pb) + FIM_LEAD(pa) + FIM_LEAD(pb))) *
+      if constexpr (sizeof(R) == 8)
+        FOR_V lp[j] = (p0[j] + pa[e][j] + half * (FIM_TRAIL(pa) + FIM_LEAD(pa))) * divby6;
+      else
+        FOR_V lp[j] = (p0[j] + pa[e][j] + pb[e][j] + half * (FIM_TRAIL(pa) + FIM_TRAIL(pb) + FIM_LEAD(pa) + FIM_LEAD(pb))) *
                     divby6;
       stv<VK>(o + (size_t)e * L, lp);
     }
