@@ -37,7 +37,7 @@ UNIT = "cell-level-steps/s"
 WORDS = {
     # the fused step averages only the layer thickness in edgvar3; the
     # tracers' edge values are formed on chip by k_trf_lo/k_trf_hi
-    "k_edgvar1": lambda T: 41, "k_edgvar3_own": lambda T: 7, "k_edgvar3_avg": lambda T: 12,
+    "k_edgvar1": lambda T: 41, "k_edgvar3_own": lambda T: 7, "k_edgvar3_avg": lambda T: 12, "k_edgvar3_patch": lambda T: 7,
     # edgvar2 (hiOrderUVComp): speeds and gradient (u, v, 6+6 edge winds in,
     # 3 out), then the correction (3 + 12 in, 18 out)
     "k_edgvar2_grad": lambda T: 17, "k_edgvar2": lambda T: 33,
@@ -53,11 +53,11 @@ WORDS = {
     "k_cnuity12": lambda T: 37, "k_cnuity3": lambda T: 8, "k_cnuity4": lambda T: 26, "k_cnuity5": lambda T: 14,
     # cnuity1..4 as one persistent launch (--persistent): the three kernels' words
     "k_cnuity_coop": lambda T: 37 + 8 + 26,
-    "k_trcadv1": lambda T: 27 * T, "k_trcadv2": lambda T: 16 * T, "k_trcadv3": lambda T: 18 * T,
     "k_dissip": lambda T: 5, "k_del4prep": lambda T: 4, "k_momtum1": lambda T: 44,
     # in the step the remap also writes tracer x thickness (T words), which
     # k_hystat_trdp then leaves out
-    "k_regrid": lambda T: 3, "k_dffusn_lev": lambda T: 2, "k_remap": lambda T: 3 * T + 10, "k_inflate": lambda T: 2,
+    "k_regrid": lambda T: 3, "k_dffusn_lev": lambda T: 2, "k_smooth_inflate": lambda T: 2,
+    "k_remap": lambda T: 3 * T + 10,
     "k_hystat": lambda T: 7, "k_hystat_trdp": lambda T: 2 * T + 3, "k_globsum_levels": lambda T: T + 1,
 }
 

@@ -682,8 +682,8 @@ __global__ void __launch_bounds__(kColBlock) k_remap(Grid<R> g, Strides s, Knobs
 // ------------------------------------------ remap, warp per column, lane = levels --
 // remap_1d (hybgen.F90:515-700) for the default knobs: PLM pcwise with
 // one-layer migration (remap_optn = 2, miglim = 1).
-//  k_inflate: inflate, the one serial recursion of the column set-up, lane =
-//             column over 32 columns per warp staged in shared memory;
+//  k_smooth_inflate: the interface smoothing and inflate, the one serial
+//             recursion of the column set-up, of 32 columns a block;
 //  k_remap_v: each warp runs kColsPerWarp consecutive columns.  Lane l holds
 //             levels l*VL .. l*VL+VL-1 of the field in hand (u, v, tracers
 //             2..ntra in pressure, theta in p^(kappa+1)), so a field's column
@@ -705,7 +705,6 @@ __global__ void __launch_bounds__(kColBlock) k_remap(Grid<R> g, Strides s, Knobs
 // and held in registers; divisions by the coordinate thicknesses (fco +
 // small, fcn + small) become products with reciprocals.  Results differ from
 // the serial pcwise by rounding.
-constexpr int kWarpsInflate = 4;
 constexpr int kWarpsRemapV = 4;
 constexpr int kColsPerWarp = 8;  // at most; see remap_columns
 
@@ -1116,30 +1115,58 @@ __device__ __forceinline__ void tracer_out(int t, R qvmin, R qwmin, const R (&dp
   store_levels<R, VL>(trdp + (size_t)t * NL + (size_t)i * L, L, kb, vec, z);
 }
 
-// inflate (hybgen.F90:893-1007) of 32 columns per warp, lane = column
-template <typename R, int ML>
-__global__ void __launch_bounds__(32 * kWarpsInflate) k_inflate(Grid<R> g, Strides s, Knobs kn,
-    const StepParams* __restrict__ sp, const R* __restrict__ pr3d, R* __restrict__ exn, int bnd) {
+// dffusn_lev (k_dffusn_lev's arithmetic; none without interface smoothing) and
+// inflate (hybgen.F90:893-1007) of 32 columns a block: the smoothed interfaces
+// are formed into shared memory with thread = (column, interface), one warp
+// runs inflate up its columns, lane = column, and the result leaves as rows.
+// Two kernels moved the interfaces through memory in between.  A small grid
+// takes wide blocks (256 threads, glvl 5 / nvl 38: 25 -> 16 us, FP64 63 -> 53), one
+// of more than four blocks an SM narrow ones, whose serial warps are then more
+// of those resident (64 threads, glvl 8 / nvl 64: 0.40 -> 0.36 ms; 256: 0.54).
+constexpr int kInfCols = 32;
+constexpr int kInfBlock = 256;
+template <typename R>
+__global__ void __launch_bounds__(kInfBlock) k_smooth_inflate(Grid<R> g, Strides s, Knobs kn,
+    const StepParams* __restrict__ sp, int k1, int k2, const R* __restrict__ pr3d, const R* __restrict__ fld,
+    R* __restrict__ out, int bnd) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int N = g.N, L = g.L, L1 = L + 1;
-  __shared__ R d0[ML];
-  for (int k = threadIdx.x; k < L; k += blockDim.x) d0[k] = R(kRd) * g.dpsig[k] / R(kP1000);
-  __syncthreads();
-  const int i0 = (blockIdx.x * kWarpsInflate + wib) * 32;
-  if (i0 >= N) return;
-  const int ncol = (N - i0 < 32) ? N - i0 : 32;
+  const int N = g.N, L = g.L, L1 = L + 1, LS = L1 | 1;  // odd row stride: lane = column is conflict-free
+  R* const col = reinterpret_cast<R*>(smraw);           // [32][LS]
+  R* const d0 = col + kInfCols * LS;                    // rd dpsig / p1000 [L]
+  const int i0 = blockIdx.x * kInfCols;
+  const int ncol = N - i0 < kInfCols ? N - i0 : kInfCols;
   const size_t m = blockIdx.y;
-  if (!sp[m].active || (bnd && sp[m].its <= 1)) return;
-  pr3d += m * s.intf; exn += m * s.intf;
-  R* col = reinterpret_cast<R*>(smraw) + (size_t)wib * (32 * (ML + 1) + 1);
-#pragma unroll 8
-  for (int q = lane; q < ncol * L1; q += 32) col[q] = exn[(size_t)i0 * L1 + q];
-  __syncwarp();
-  if (lane < ncol)
-    inflate<R>(kn, [&](int k) { return d0[k]; }, L, pr3d[(size_t)(i0 + lane) * L1], col + lane * L1);
-  __syncwarp();
-  for (int q = lane; q < ncol * L1; q += 32) exn[(size_t)i0 * L1 + q] = col[q];
+  sp += m;
+  if (!sp->active || (bnd && sp->its <= 1)) return;
+  pr3d += m * s.intf; fld += m * s.intf; out += m * s.intf;
+  for (int k = threadIdx.x; k < L; k += blockDim.x) d0[k] = R(kRd) * g.dpsig[k] / R(kP1000);
+#pragma unroll 4
+  for (int q = threadIdx.x; q < ncol * L1; q += blockDim.x) {
+    const int r = q / L1, k = q - r * L1, i = i0 + r;
+    R v = fld[(size_t)i0 * L1 + q];
+    R x[6];
+#pragma unroll
+    for (int e = 0; e < 6; e++) x[e] = fld[(size_t)g.prox[i * 6 + e] * L1 + k];
+    if (k >= k1 && k <= k2) {
+      const int np = g.nprox[i];
+      R flxdv = R(0);
+#pragma unroll
+      for (int e = 0; e < 6; e++)
+        if (e < np) flxdv = flxdv + (v - x[e]) * g.sideln[i * 6 + e];
+      const R factor = -g.smoo[k] * g.rarea[i];
+      v = v + flxdv * factor;
+    }
+    col[r * LS + k] = v;
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < ncol)
+    inflate<R>(kn, [&](int k) { return d0[k]; }, L, pr3d[(size_t)(i0 + threadIdx.x) * L1], col + threadIdx.x * LS);
+  __syncthreads();
+#pragma unroll 4
+  for (int q = threadIdx.x; q < ncol * L1; q += blockDim.x) {
+    const int r = q / L1;
+    out[(size_t)i0 * L1 + q] = col[r * LS + (q - r * L1)];
+  }
 }
 
 // vec: every field column starts on a min(16, VL*sizeof(R))-byte boundary
@@ -1491,8 +1518,8 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
 
 template <typename R, int VL, int WL>
 size_t remap_v_smem() { return sizeof(RemapV<R, VL, 32 / WL>) * kWarpsRemapV; }
-template <typename R, int ML>
-size_t inflate_smem() { return sizeof(R) * (32 * (ML + 1) + 1) * kWarpsInflate; }
+template <typename R>
+size_t inflate_smem(int L) { return sizeof(R) * (kInfCols * (size_t)((L + 1) | 1) + L); }
 
 // levels per lane of k_remap_v
 inline int remap_vl(int L) { return L <= 32 ? 1 : L <= 64 ? 2 : 4; }
@@ -1549,14 +1576,9 @@ int prepare_hybgen(int L) {
   } else if (vl == 1) e = remap_v_attr<R, 1, 32>();
   else if (vl == 2) e = remap_v_attr<R, 2, 32>();
   else e = remap_v_attr<R, 4, 32>();
-  if (e == cudaSuccess) {
-    if (L <= 64)
-      e = cudaFuncSetAttribute(k_inflate<R, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)inflate_smem<R, 64>());
-    else
-      e = cudaFuncSetAttribute(k_inflate<R, kMaxL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)inflate_smem<R, kMaxL>());
-  }
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_smooth_inflate<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)inflate_smem<R>(kMaxL));
   return e == cudaSuccess ? 0 : (int)e;
 }
 
@@ -2010,28 +2032,26 @@ bool launch_hybgen(const Launch& l, const Grid<R>& g, const Strides& s, const Kn
 #undef FIM_REGRID
   FIM_KEND(l);
   const R* ex_in = w.exsmo;
-  if (kn.intfc_smooth > 0.) {
+  // Fortran levels kbl+2..nvl -> 0-based interfaces kbl+1..nvl-1
+  const int k1 = kn.kbl + 1, k2 = g.L - 1;
+  const bool plm1 = kn.remap_optn == 2 && kn.miglim == 1;
+  if (kn.intfc_smooth > 0. && plm1) {
+    FIM_KBEGIN(l, "k_smooth_inflate");
+    const unsigned nb = nblocks(g.N, kInfCols);
+    const int tb = (long long)nb * l.members <= 4ll * sm_count() ? kInfBlock : kInfBlock / 4;
+    k_smooth_inflate<R><<<dim3(nb, l.members), tb, inflate_smem<R>(g.L), l.stream>>>(
+        g, s, kn, l.sp, k1, k2, pr3d, w.exsmo, w.exsmo2, l.boundary);
+    FIM_KEND(l);
+    ex_in = w.exsmo2;
+  } else if (kn.intfc_smooth > 0.) {
+    // the remap of the other knobs inflates its columns itself
     dim3 gs(nblocks((long long)g.N * ((g.L + kDffK) / kDffK), kBlock2), l.members);
-    // Fortran levels kbl+2..nvl -> 0-based interfaces kbl+1..nvl-1
     FIM_KBEGIN(l, "k_dffusn_lev");
-    k_dffusn_lev<R><<<gs, kBlock2, 0, l.stream>>>(g, s, l.sp, l.boundary, kn.kbl + 1, g.L - 1, w.exsmo,
-                                                   w.exsmo2);
+    k_dffusn_lev<R><<<gs, kBlock2, 0, l.stream>>>(g, s, l.sp, l.boundary, k1, k2, w.exsmo, w.exsmo2);
     FIM_KEND(l);
     ex_in = w.exsmo2;
   }
-  if (kn.remap_optn == 2 && kn.miglim == 1) {
-    if (kn.intfc_smooth > 0.) {
-      // ex_in is the smoothing scratch here: inflate it in place
-      dim3 gi(nblocks(g.N, 32 * kWarpsInflate), l.members);
-      FIM_KBEGIN(l, "k_inflate");
-      if (g.L <= 64)
-        k_inflate<R, 64><<<gi, 32 * kWarpsInflate, inflate_smem<R, 64>(), l.stream>>>(g, s, kn, l.sp, pr3d,
-                                                                                      w.exsmo2, l.boundary);
-      else
-        k_inflate<R, kMaxL><<<gi, 32 * kWarpsInflate, inflate_smem<R, kMaxL>(), l.stream>>>(g, s, kn, l.sp, pr3d,
-                                                                                            w.exsmo2, l.boundary);
-      FIM_KEND(l);
-    }
+  if (plm1) {
     const int cpw = remap_columns<R>(g.N, l.members, remap_paired<R>(g.L));
     dim3 gw(nblocks(g.N, kWarpsRemapV * cpw), l.members);
     const bool paired = remap_paired<R>(g.L);
