@@ -253,24 +253,24 @@ int build_patches(fim_ctx* c, const std::vector<int>& prox, const std::vector<in
     if (--side < 1) return set_err(c, FIM_EINVAL, "tracer patches: a frame exceeds 255 cells");
   }
   FrameTab& f = c->ftab;
-  f.ntile = h.ntile; f.S2 = h.S2; f.S1 = h.S1; f.SC = h.SC; f.SE = h.SE; f.SR = h.SR;
+  std::vector<unsigned char> tab;
+  pack_frames(h, nprox.data(), &f, &tab);
   void* p;
   int rc;
-  if ((rc = dalloc(c, &p, h.cells.size() * sizeof(int)))) return rc;
-  CK(cudaMemcpy(p, h.cells.data(), h.cells.size() * sizeof(int), cudaMemcpyHostToDevice), "patch cells");
-  f.cells = (const int*)p;
-  if ((rc = dalloc(c, &p, h.nbr.size() * sizeof(uint32_t)))) return rc;
-  CK(cudaMemcpy(p, h.nbr.data(), h.nbr.size() * sizeof(uint32_t), cudaMemcpyHostToDevice), "patch neighbours");
-  f.nbr = (const uint2*)p;
+  if ((rc = dalloc(c, &p, tab.size()))) return rc;
+  CK(cudaMemcpy(p, tab.data(), tab.size(), cudaMemcpyHostToDevice), "patch tables");
+  f.tab = (const unsigned char*)p;
   if ((rc = dalloc(c, &p, h.cnt.size() * sizeof(int)))) return rc;
   CK(cudaMemcpy(p, h.cnt.data(), h.cnt.size() * sizeof(int), cudaMemcpyHostToDevice), "patch counts");
   f.cnt = (const int4*)p;
-  if ((rc = dalloc(c, &p, h.mir.size() * sizeof(uint16_t)))) return rc;
-  CK(cudaMemcpy(p, h.mir.data(), h.mir.size() * sizeof(uint16_t), cudaMemcpyHostToDevice), "patch mirrors");
-  f.mir = (const unsigned short*)p;
-  if ((rc = dalloc(c, &p, h.red.size() * sizeof(uint16_t)))) return rc;
-  CK(cudaMemcpy(p, h.red.data(), h.red.size() * sizeof(uint16_t), cudaMemcpyHostToDevice), "patch ring edges");
-  f.redge = (const unsigned short*)p;
+  if ((rc = dalloc(c, &p, (size_t)f.ntile * f.cstride * c->esz))) return rc;
+  f.coef = p;
+  // the kernel runs on the context's (non-blocking) stream: the table copies
+  // above have to be on the device
+  CK(cudaStreamSynchronize(0), "patch tables");
+  if (c->prec == FIM_PREC_F64) launch_patch_coefs<double>(c->stream, c->gd, f, (double*)p);
+  else launch_patch_coefs<float>(c->stream, c->gf, f, (float*)p);
+  CK(cudaGetLastError(), "patch coefficients");
   return FIM_OK;
 }
 

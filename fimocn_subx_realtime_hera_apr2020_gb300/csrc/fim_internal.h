@@ -600,11 +600,26 @@ struct FrameTab {
   // capacities: frame cells, interior + ring-1 cells, interior cells,
   // edge-value rows (6 per interior cell + ring edges), ring edges
   int S2 = 0, S1 = 0, SC = 0, SE = 0, SR = 0;
-  const int* cells = nullptr;            // [ntile][S2] cell index, frame order
-  const uint2* nbr = nullptr;            // [ntile][S1] frame-local index of prox slots 0..5, a byte each
   const int4* cnt = nullptr;             // [ntile] interior cells, + ring 1, + ring 2, ring edges
-  const unsigned short* mir = nullptr;   // [ntile][SC][6] edge-value row of the other side of each edge
-  const unsigned short* redge = nullptr; // [ntile][SR] ring edges: (frame-local cell << 3) | slot
+  // A patch's tables, as its block holds them in shared memory (copied 16
+  // bytes at a time): `bytes` of them a patch, the first `head` what
+  // k_trf_hi needs.  Laid out and resolved once, so that a block's set-up is
+  // a straight copy: gathering the tables, the coefficients and the flux rows
+  // through each other cost k_trf_lo the time of 1.5 tracers (FP32 at 655,362
+  // cells x 64 levels x 11 tracers, k_trf_lo 6.77 -> 6.28 ms and k_trf_hi
+  // 5.96 -> 5.85 ms; a step of 10,242 x 38 x 5 286 -> 260 us).  Byte offsets:
+  //   0    [S2] int            cell index, frame order
+  //   nbr  [S1] uint2          frame-local index of prox slots 0..5, a byte each
+  //   np   [S1] u8             nprox of the interior and ring-1 cells
+  //   mir  [SC][6] u16         edge-value row of the other side of each edge
+  //   red  [SR] u16            ring edges: (frame-local cell << 3) | slot
+  //   mfr  [SE] int            cell x 6 + slot of each edge-value row
+  const unsigned char* tab = nullptr;
+  int bytes = 0, head = 0, nbr = 0, np = 0, mir = 0, red = 0, mfr = 0;
+  // halved least-squares coefficients (of the context's precision): cstride
+  // values a patch, 36 per interior cell, then 6 per ring edge
+  const void* coef = nullptr;
+  int cstride = 0;
 };
 struct FrameHost {
   int ntile = 0, S2 = 0, S1 = 0, SC = 0, SE = 0, SR = 0;
@@ -644,6 +659,12 @@ int prepare_edges(const FrameTab& ft);
 template <typename R>
 void launch_edges_patch(const Launch&, const Grid<R>&, const Strides&, const FrameTab&, int nfields, const R* delp,
                         const R* tracr, R* dp_edg, R* trc_edg);
+// packs the patches' tables as FrameTab describes and sets its sizes and
+// offsets (not its pointers); edge-value rows of cells and slots follow proxs
+void pack_frames(const FrameHost& f, const int* nprox, FrameTab* tab, std::vector<unsigned char>* out);
+// fills coef (ntile x cstride values) from the grid's least-squares coefficients
+template <typename R>
+void launch_patch_coefs(cudaStream_t stream, const Grid<R>& g, const FrameTab& ft, R* coef);
 // one-time launch attributes (shared-memory size) of the tracer kernels for
 // these patches; returns a cudaError_t value
 template <typename R>

@@ -59,6 +59,8 @@ __device__ __forceinline__ void stage_copy(void* smem, const void* gmem) {
 }
 __device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+// all but the last group
+__device__ __forceinline__ void stage_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
 // Row of slot e of patch cell x in the edge-indexed shared arrays (edge
 // values, mass fluxes, antidiffusive fluxes): the slots of odd cells are
@@ -93,14 +95,14 @@ struct PatchLayout {
   template <typename R>
   __host__ __device__ static PatchLayout make(const FrameTab& f, int LK, bool hi, bool ev = false) {
     PatchLayout p{};
-    const size_t S2 = f.S2, S1 = f.S1, SC = f.SC, SE = f.SE, SR = f.SR;
+    const size_t S2 = f.S2, S1 = f.S1, SC = f.SC, SE = f.SE;
     size_t o = 0;
     if (!hi) {
       p.trs = o; o += 2 * S2 * LK;
       p.E = o; o += ev ? 0 : SE * LK;
       p.mf = o; o += SE * LK;
       p.ops = o; o += 2 * 3 * SC * LK;
-      p.hf = o; o += ev ? 0 : SC * 36 + SR * 6;
+      p.hf = o; o += ev ? 0 : (size_t)f.cstride;
     } else {
       p.TO = o; o += S2 * LK;
       p.TL = o; o += S2 * LK;
@@ -113,7 +115,7 @@ struct PatchLayout {
       p.dpf = o; o += S1 * LK;
       p.arf = o; o += S1;
     }
-    return p.tables<R>(f, o);
+    return p.tables<R>(hi ? f.head : f.bytes, o);
   }
   // edges: field frame x 2 buffers [S2][LK]; edge values [SE][LK];
   // least-squares coefficients as in lo
@@ -123,64 +125,75 @@ struct PatchLayout {
     size_t o = 0;
     p.trs = o; o += (size_t)2 * f.S2 * LK;
     p.E = o; o += (size_t)f.SE * LK;
-    p.hf = o; o += (size_t)f.SC * 36 + f.SR * 6;
-    return p.tables<R>(f, o);
+    p.hf = o; o += (size_t)f.cstride;
+    return p.tables<R>(f.bytes, o);
   }
   // the patch tables after o elements of R
   template <typename R>
-  __host__ __device__ PatchLayout tables(const FrameTab& f, size_t o) const {
+  __host__ __device__ PatchLayout tables(int nbytes, size_t o) const {
     PatchLayout p = *this;
     p.r_elems = o;
     size_t b = (o * sizeof(R) + 15) & ~(size_t)15;
     p.tab = b;
-    b += (size_t)f.S2 * 4 + f.S1 * 8 + f.SC * 6 * 2 + f.SR * 2 + f.S1;
+    b += (size_t)nbytes;
     p.bytes = (b + 15) & ~(size_t)15;
     return p;
   }
 };
 
 struct FrameSm {
-  int* cells;
-  uint2* nbr;
-  unsigned short* mir;
-  unsigned short* red;
-  unsigned char* np;  // nprox of the interior and ring-1 cells
+  const int* cells;
+  const uint2* nbr;
+  const unsigned char* np;  // nprox of the interior and ring-1 cells
+  const unsigned short* mir;
+  const unsigned short* red;
+  const int* mfr;
 };
 
-// the patch's tables into shared memory; callers synchronise before use
-template <typename R>
-__device__ __forceinline__ FrameSm load_tables(const Grid<R>& g, const FrameTab& ft, unsigned char* base,
-                                               size_t tab, int tile, int C, int n1, int n2, int nre) {
-  FrameSm t;
-  t.cells = reinterpret_cast<int*>(base + tab);
-  t.nbr = reinterpret_cast<uint2*>(t.cells + ft.S2);
-  t.mir = reinterpret_cast<unsigned short*>(t.nbr + ft.S1);
-  t.red = t.mir + ft.SC * 6;
-  t.np = reinterpret_cast<unsigned char*>(t.red + ft.SR);
-  const int* gc = ft.cells + (size_t)tile * ft.S2;
-  for (int x = threadIdx.x; x < n2; x += blockDim.x) t.cells[x] = gc[x];
-  for (int x = threadIdx.x; x < n1; x += blockDim.x) {
-    t.nbr[x] = ft.nbr[(size_t)tile * ft.S1 + x];
-    t.np[x] = (unsigned char)g.nprox[gc[x]];
-  }
-  for (int x = threadIdx.x; x < C * 6; x += blockDim.x) t.mir[x] = ft.mir[(size_t)tile * ft.SC * 6 + x];
-  for (int x = threadIdx.x; x < nre; x += blockDim.x) t.red[x] = ft.redge[(size_t)tile * ft.SR + x];
-  return t;
+// asynchronous copy of n bytes (a multiple of 16, both ends on 16 bytes)
+__device__ __forceinline__ void stage_bytes(void* dst, const void* src, int n) {
+  for (int q = threadIdx.x * 16; q < n; q += blockDim.x * 16)
+    stage_copy<16>(static_cast<unsigned char*>(dst) + q, static_cast<const unsigned char*>(src) + q);
 }
 
-// least-squares coefficients of the patch cells (all 36) and of the ring
-// edges (the row of the edge's slot), halved, into hf; needs the tables in
-// place.  The edge values are kept halved (exactly), so that the average of
-// an edge's two sides is one addition.
+// the patch's tables (the first n bytes of them) on their way into shared
+// memory; callers commit, wait and synchronise before use
+__device__ __forceinline__ FrameSm stage_tables(const FrameTab& ft, unsigned char* base, size_t tab, int tile, int n) {
+  unsigned char* q = base + tab;
+  stage_bytes(q, ft.tab + (size_t)tile * ft.bytes, n);
+  return {reinterpret_cast<const int*>(q), reinterpret_cast<const uint2*>(q + ft.nbr), q + ft.np,
+          reinterpret_cast<const unsigned short*>(q + ft.mir), reinterpret_cast<const unsigned short*>(q + ft.red),
+          reinterpret_cast<const int*>(q + ft.mfr)};
+}
+
+// halved least-squares coefficients of the patch cells (36 each) and of the
+// ring edges (the row of the edge's slot) on their way into hf.  The edge
+// values are kept halved (exactly), so that the average of an edge's two sides
+// is one addition.
 template <typename R>
-__device__ __forceinline__ void load_coefs(const Grid<R>& g, const FrameSm& fs, R* hf, int C, int nre) {
-  for (int q = threadIdx.x; q < C * 36; q += blockDim.x) {
-    const int x = q / 36;
-    hf[q] = R(0.5) * g.hfcoef[(size_t)fs.cells[x] * 36 + (q - x * 36)];
-  }
-  for (int q = threadIdx.x; q < nre * 6; q += blockDim.x) {
-    const int r = q / 6, code = fs.red[r];
-    hf[C * 36 + q] = R(0.5) * g.hfcoef[(size_t)fs.cells[code >> 3] * 36 + (code & 7) * 6 + (q - r * 6)];
+__device__ __forceinline__ void stage_coefs(const FrameTab& ft, R* hf, int tile, int C, int nre) {
+  stage_bytes(hf, static_cast<const R*>(ft.coef) + (size_t)tile * ft.cstride,
+              ((C * 36 + nre * 6) * (int)sizeof(R) + 15) & ~15);
+}
+
+template <typename R>
+__global__ void k_patch_coefs(Grid<R> g, FrameTab ft, R* __restrict__ coef) {
+  const int tile = blockIdx.x;
+  const unsigned char* q = ft.tab + (size_t)tile * ft.bytes;
+  const int* cells = reinterpret_cast<const int*>(q);
+  const unsigned short* red = reinterpret_cast<const unsigned short*>(q + ft.red);
+  const int4 cn = ft.cnt[tile];
+  R* out = coef + (size_t)tile * ft.cstride;
+  for (int a = threadIdx.x; a < ft.cstride; a += blockDim.x) {
+    R h = R(0);
+    if (a < cn.x * 36) {
+      const int x = a / 36;
+      h = g.hfcoef[(size_t)cells[x] * 36 + (a - x * 36)];
+    } else if (a < cn.x * 36 + cn.w * 6) {
+      const int b = a - cn.x * 36, r = b / 6, code = red[r];
+      h = g.hfcoef[(size_t)cells[code >> 3] * 36 + (code & 7) * 6 + (b - r * 6)];
+    }
+    out[a] = R(0.5) * h;
   }
 }
 
@@ -375,9 +388,13 @@ __global__ void __launch_bounds__(64 * GC, 8 / GC) k_trf_lo(Grid<R> g, Strides s
   R* const MF = sr + lay.mf;
   R* const ops = sr + lay.ops;
   R* const hf = sr + lay.hf;
-  const FrameSm fs = load_tables<R>(g, ft, fsm, lay.tab, tile, C, n1, n2, nre);
+  // the tables, then (arriving with the first operands) the coefficients
+  const FrameSm fs = stage_tables(ft, fsm, lay.tab, tile, ft.bytes);
+  stage_commit();
+  if (!EV) stage_coefs<R>(ft, hf, tile, C, nre);
+  stage_commit();
+  stage_wait1();
   __syncthreads();
-  if (!EV) load_coefs<R>(g, fs, hf, C, nre);
   const size_t NL = (size_t)N * L;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
   const R ab1 = sp->template w1<R>(), ab2 = sp->template w2<R>(), ab3 = sp->template w3<R>();
@@ -400,19 +417,7 @@ __global__ void __launch_bounds__(64 * GC, 8 / GC) k_trf_lo(Grid<R> g, Strides s
   // neighbour sides (tracer independent), with the first tracer's operands
   for (int it = threadIdx.x; it < (6 * C + nre) * GC; it += blockDim.x) {
     const int r = it / GC, v = (it - r * GC) * VK;
-    if (v >= lk) continue;
-    int cell, slot, row = r;
-    if (r < 6 * C) {
-      const int x = r / 6;
-      cell = fs.cells[x];
-      slot = r - x * 6;
-      row = erow(x, slot);
-    } else {
-      const int code = fs.red[r - 6 * C];
-      cell = fs.cells[code >> 3];
-      slot = code & 7;
-    }
-    stage_copy<VK * (int)sizeof(R)>(MF + row * LK + v, mfn + (cell * 6 + slot) * L + k0 + v);
+    if (v < lk) stage_copy<VK * (int)sizeof(R)>(MF + r * LK + v, mfn + fs.mfr[r] * L + k0 + v);
   }
   stage(t0, 0);
   CellItem<R, VK> ci;
@@ -619,7 +624,9 @@ __global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameT
   R* const tdb = sr + lay.tdb;
   R* const dpf = sr + lay.dpf;
   R* const arf = sr + lay.arf;
-  const FrameSm fs = load_tables<R>(g, ft, fsm, lay.tab, tile, C, n1, n2, nre);
+  const FrameSm fs = stage_tables(ft, fsm, lay.tab, tile, ft.head);
+  stage_commit();
+  stage_wait();
   __syncthreads();
   const size_t NL = (size_t)N * L;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
@@ -761,7 +768,11 @@ __global__ void __launch_bounds__(64 * GC, 3) k_edgvar3_patch(Grid<R> g, Strides
   R* const trs = sr + lay.trs;
   R* const E = sr + lay.E;
   R* const hf = sr + lay.hf;
-  const FrameSm fs = load_tables<R>(g, ft, fsm, lay.tab, tile, C, n1, n2, nre);
+  const FrameSm fs = stage_tables(ft, fsm, lay.tab, tile, ft.bytes);
+  stage_commit();
+  stage_coefs<R>(ft, hf, tile, C, nre);
+  stage_commit();
+  stage_wait1();
   __syncthreads();
   const size_t NL = (size_t)N * L;
   RowPlan<R, VK, GC> rp;
@@ -773,7 +784,6 @@ __global__ void __launch_bounds__(64 * GC, 3) k_edgvar3_patch(Grid<R> g, Strides
   };
   int f = blockIdx.z;
   stage(f, 0);
-  load_coefs<R>(g, fs, hf, C, nre);
   const int x = threadIdx.x / GC, v = (threadIdx.x - x * GC) * VK;
   const bool on = x < C && v < lk;
   const int i = on ? fs.cells[x] : 0, np = on ? fs.np[x] : 0;
@@ -1060,6 +1070,43 @@ int build_frames(int N, const int* prox, const int* proxs, const int* nprox, int
   return 0;
 }
 
+void pack_frames(const FrameHost& f, const int* nprox, FrameTab* tab, std::vector<unsigned char>* out) {
+  FrameTab& t = *tab;
+  t.ntile = f.ntile; t.S2 = f.S2; t.S1 = f.S1; t.SC = f.SC; t.SE = f.SE; t.SR = f.SR;
+  auto up = [](int n) { return (n + 15) & ~15; };
+  t.nbr = up(4 * f.S2);
+  t.np = t.nbr + up(8 * f.S1);
+  t.head = t.np + up(f.S1);
+  t.mir = t.head;
+  t.red = t.mir + up(12 * f.SC);
+  t.mfr = t.red + up(2 * f.SR);
+  t.bytes = t.mfr + up(4 * f.SE);
+  t.cstride = (f.SC * 36 + f.SR * 6 + 3) & ~3;
+  out->assign((size_t)f.ntile * t.bytes, 0);
+  for (int i = 0; i < f.ntile; i++) {
+    unsigned char* q = out->data() + (size_t)i * t.bytes;
+    const int* cells = &f.cells[(size_t)i * f.S2];
+    const int C = f.cnt[(size_t)i * 4], n1 = f.cnt[(size_t)i * 4 + 1], nre = f.cnt[(size_t)i * 4 + 3];
+    std::copy(cells, cells + f.S2, reinterpret_cast<int*>(q));
+    std::copy(&f.nbr[(size_t)i * f.S1 * 2], &f.nbr[(size_t)i * f.S1 * 2] + (size_t)f.S1 * 2,
+              reinterpret_cast<uint32_t*>(q + t.nbr));
+    for (int x = 0; x < n1; x++) q[t.np + x] = (unsigned char)nprox[cells[x]];
+    std::copy(&f.mir[(size_t)i * f.SC * 6], &f.mir[(size_t)i * f.SC * 6] + (size_t)f.SC * 6,
+              reinterpret_cast<uint16_t*>(q + t.mir));
+    const uint16_t* red = &f.red[(size_t)i * f.SR];
+    std::copy(red, red + f.SR, reinterpret_cast<uint16_t*>(q + t.red));
+    int* mfr = reinterpret_cast<int*>(q + t.mfr);
+    for (int x = 0; x < C; x++)
+      for (int e = 0; e < 6; e++) mfr[erow(x, e)] = cells[x] * 6 + e;
+    for (int r = 0; r < nre; r++) mfr[6 * C + r] = cells[red[r] >> 3] * 6 + (red[r] & 7);
+  }
+}
+
+template <typename R>
+void launch_patch_coefs(cudaStream_t stream, const Grid<R>& g, const FrameTab& ft, R* coef) {
+  k_patch_coefs<R><<<(unsigned)ft.ntile, 256, 0, stream>>>(g, ft, coef);
+}
+
 int check_frames(int N, const int* prox, const int* proxs, const int* nprox, const FrameHost& F) {
   std::vector<int> seen(N, 0);
   for (int t = 0; t < F.ntile; t++) {
@@ -1172,6 +1219,7 @@ int tune_tracers(const Launch& l, const Grid<R>& g, const Strides& s, const TrcF
   template void launch_tracers_fused<R>(const Launch&, const Grid<R>&, const Strides&,                       \
                                         const TrcFusedScratch<R>&, R*, R*, R*, R*, R*, const R*, const R*,   \
                                         const ChunkHook*);                                                    \
+  template void launch_patch_coefs<R>(cudaStream_t, const Grid<R>&, const FrameTab&, R*);                     \
   template int prepare_edges<R>(const FrameTab&);                                                             \
   template void launch_edges_patch<R>(const Launch&, const Grid<R>&, const Strides&, const FrameTab&, int,   \
                                       const R*, const R*, R*, R*);                                           \
