@@ -588,8 +588,16 @@ __device__ __forceinline__ void limiters(const FrameSm& fs, const R* TO, const R
 // Copies: the limiters' operands of tracer t (frames, slots, S+/S-) are
 // staged while the block clips tracer t-1; the clip's operands of tracer t
 // (fluxes, tendency, tracer x thickness) while it forms tracer t's limiters.
+//
+// Registers: the blocks an SM that the shared memory lets in at GC 4, two of
+// 98 KB with 16-byte rows a thread, more below (three at up to 80 registers
+// are as fast as four at 64).  Left to itself the compiler takes 80 and 64
+// and serialises the neighbour loads (FP32 glvl 7 / nvl 64 / 11 tracers 1.43
+// -> 1.41 ms, glvl 5 / nvl 38 / 5 tracers 66 -> 61 us, FP64 glvl 6 / nvl 64 /
+// 11 tracers 2.84 -> 2.78 ms; FP64 one level a thread at two blocks 252 us
+// against 239 at three).
 template <typename R, int VK, int GC>
-__global__ void __launch_bounds__(64 * GC) k_trf_hi(Grid<R> g, Strides s, FrameTab ft,
+__global__ void __launch_bounds__(64 * GC, VK * (int)sizeof(R) == 16 ? 8 / GC : 12 / GC) k_trf_hi(Grid<R> g, Strides s, FrameTab ft,
     const StepParams* __restrict__ sp, int t0, int nt, const R* __restrict__ trl_tdcy, const R* trcdp,
     R* __restrict__ trc_tdcy, const R* __restrict__ delp, const R* __restrict__ trold,
     const R* __restrict__ trcr_lo, const R* __restrict__ s_plus, const R* __restrict__ s_mnus,
