@@ -32,10 +32,11 @@
 // the tracer in place while the blocks of neighbouring patches still read it.
 //
 // Every value is formed from the same operands in the same order as in the
-// per-routine entries (k_edgvar3_own/_avg, then these kernels with EV), so the
-// fused step is bit-identical to the routine sequence.  nprox is 5 or 6 (checked when the
-// context is created), so only slot 5 of a cell can be missing: the tests
-// "e < nprox" are written (e < 5 || e < np) and cost nothing for slots 0..4.
+// per-routine entries (k_edgvar3_patch, or in FP64 k_edgvar3_own/_avg, then
+// these kernels with EV), so the fused step is bit-identical to the routine
+// sequence.  nprox is 5 or 6 (checked when the context is created), so only
+// slot 5 of a cell can be missing: the tests "e < nprox" are written
+// (e < 5 || e < np) and cost nothing for slots 0..4.
 #include "fim_internal.h"
 
 #include <algorithm>
@@ -359,8 +360,13 @@ struct CellItem {
 // loads its cell's six rows before it waits for the staged operands, and the
 // member's own tracer count does not apply.  EV = false forms them on chip
 // (theta's are edgvar1's).
+//
+// Two blocks an SM at GC 4, the shared memory's limit with 16-byte rows a
+// thread.  FP64 at one level a thread takes the three that fit then (80
+// registers: glvl 5 / nvl 37 / 5 tracers 273 -> 257 us); FP32 at two levels a
+// thread is slower there (59 -> 62 us).
 template <typename R, int VK, int GC, bool EV>
-__global__ void __launch_bounds__(64 * GC, 8 / GC) k_trf_lo(Grid<R> g, Strides s, FrameTab ft,
+__global__ void __launch_bounds__(64 * GC, sizeof(R) == 8 && VK == 1 ? 12 / GC : 8 / GC) k_trf_lo(Grid<R> g, Strides s, FrameTab ft,
     const StepParams* __restrict__ sp, int t0, int nt, const R* __restrict__ massfx, const R* __restrict__ trc_edg,
     const R* __restrict__ tracr, const R* __restrict__ trcdp, R* __restrict__ trl_tdcy, const R* __restrict__ delp,
     R* __restrict__ trcr_lo, R* __restrict__ s_plus, R* __restrict__ s_mnus, R* __restrict__ trold,
