@@ -487,8 +487,13 @@ __device__ __forceinline__ void cnuity12_body(int bx, int by, const Grid<R>& g, 
   stv<VK>(p_plus + c, pp);
   stv<VK>(p_mnus + c, pm);
 }
+// FP32 at four levels a thread: the three blocks an SM that 80 registers let
+// in (the compiler's own 72 also give three, with its loads serialised: glvl 7
+// / nvl 64 283 -> 255 us; two 294, four 322).  Narrower accesses keep the
+// compiler's choice (0): at two levels more registers make the kernel 3 us
+// faster alone and the step 4 us slower, its companion stream's blocks wait.
 template <typename R, int VK>
-__global__ void __launch_bounds__(kBlock) k_cnuity12(Grid<R> g, Strides s, const StepParams* __restrict__ sp,
+__global__ void __launch_bounds__(kBlock, VK == 4 ? 3 : 0) k_cnuity12(Grid<R> g, Strides s, const StepParams* __restrict__ sp,
     const R* __restrict__ u_edg, const R* __restrict__ v_edg, const R* __restrict__ dp_edg,
     const R* __restrict__ delp, R* __restrict__ massfx, R* __restrict__ dplo_tndcy, R* __restrict__ antifx,
     R* __restrict__ delp_lo, R* __restrict__ p_plus, R* __restrict__ p_mnus) {
