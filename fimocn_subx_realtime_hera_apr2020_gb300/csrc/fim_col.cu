@@ -1,10 +1,13 @@
 // Column kernels of the FIM dynamics step: hybgen (regrid_1d, dffusn_lev,
 // remap_1d with restp_1d, equilb, inflate, pcwise), hystat, globsum.
 //
-// hybgen's column logic is serial in k with data-dependent branches, so it
-// runs one thread per column over per-thread column arrays; the 1-ring
-// interface smoothing between regrid and remap is a (level, cell) stencil.
-// hystat's bottom-up Montgomery/geopotential recursion is a warp scan in FP64.
+// hybgen's regrid is serial in k with data-dependent branches, so k_regrid runs
+// one thread per column over column arrays (in shared memory while the grid
+// fits one round of warps, else local); the 1-ring interface smoothing and
+// inflate run in one kernel, 32 columns a block; the remap of the default
+// knobs takes whole columns a warp, that of the others a thread a column.
+// hystat runs 32 columns a block, its bottom-up Montgomery/geopotential
+// recursion with a lane a column over shared memory.
 // globsum accumulates per thread (FP64, or float-float compensated sums in the
 // FP32 build, whose error is that of an FP64 sum) and reduces per block into a
 // deterministic partial buffer.

@@ -2,11 +2,12 @@
 // cnuity1..5, del4prep/dissip/momtum1 (trcadv1..3: fim_trc.cu).
 //
 // Layout is the reference's (level index fastest), so one thread per
-// (level, cell) gives fully coalesced loads along k for own and neighbour
-// columns alike; a warp covers 32 consecutive levels of one cell and the grid
-// tables of that cell are warp-uniform (broadcast loads).  Kernels whose
-// result couples levels of one column (the cnuity5 pressure/omega scan and the
-// momtum1 Rayleigh damping) run one warp per column and scan with shuffles.
+// (level group, cell) gives fully coalesced loads along k for own and
+// neighbour columns alike; a warp covers consecutive levels of a cell and the
+// grid tables of that cell are broadcast loads.  Where levels of one column
+// are coupled, cnuity5 (pressure and omega sums) takes 32 columns a block and
+// sums with a lane a column over shared memory, and momtum1 (Rayleigh
+// damping) a warp a column.
 // Ensemble members map to gridDim.y; all members share the grid tables.
 //
 // Every kernel restates the arithmetic of the reference routine it names,
