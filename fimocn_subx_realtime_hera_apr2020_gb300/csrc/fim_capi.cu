@@ -271,6 +271,8 @@ int build_patches(fim_ctx* c, const std::vector<int>& prox, const std::vector<in
   if (c->prec == FIM_PREC_F64) launch_patch_coefs<double>(c->stream, c->gd, f, (double*)p);
   else launch_patch_coefs<float>(c->stream, c->gf, f, (float*)p);
   CK(cudaGetLastError(), "patch coefficients");
+  // the first kernels to read them may run on another stream
+  CK(cudaStreamSynchronize(c->stream), "patch coefficients");
   return FIM_OK;
 }
 

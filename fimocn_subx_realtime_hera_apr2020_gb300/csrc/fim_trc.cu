@@ -23,7 +23,7 @@
 // The per-routine trcadv runs the same two kernels with the caller's edge
 // values (EV): 38 words a cell-level and tracer at 16-byte accesses where one
 // thread a cell-level took about 60 at 4 (glvl 7, nvl 64, 11 tracers, FP32:
-// 8.04 -> 3.00 ms; FP64, glvl 5, nvl 37, 5 tracers: 0.82 -> 0.56 ms).
+// 8.04 -> 2.93 ms; FP64, glvl 5, nvl 37, 5 tracers: 0.82 -> 0.52 ms).
 //
 // The edge values (six per cell-level and tracer) and R+/R- never reach HBM:
 // per cell-level and tracer the pair reads and writes 32 words (10 of them
@@ -761,8 +761,9 @@ __global__ void __launch_bounds__(64 * GC, VK * (int)sizeof(R) == 16 ? 8 / GC : 
 // the own-side values and averaging them in a second pass (k_edgvar3_own,
 // k_edgvar3_avg) moves 19.  Held by the shared-memory pipe (77% busy: 1,400
 // wavefronts a patch, 16 levels and field), three blocks an SM (80 registers;
-// two 0.98 ms, four 0.91 ms): at glvl 7 / nvl 64, dp and 10 tracers, 0.89 ms
-// against 0.65 + 0.90 ms for the two passes.  blockIdx.z takes every
+// two 0.98 ms, four 0.91 ms, against 0.89): at glvl 7 / nvl 64, dp and 10
+// tracers, 0.84 ms (0.89 before the tables were packed) against 0.65 + 0.90 ms
+// for the two passes.  blockIdx.z takes every
 // gridDim.z-th field, so small grids fill the chip.
 template <typename R, int VK, int GC>
 __global__ void __launch_bounds__(64 * GC, 3) k_edgvar3_patch(Grid<R> g, Strides s, FrameTab ft, int nfields,
