@@ -61,11 +61,14 @@ __device__ __forceinline__ void ld4(const double* p, double (&r)[4]) {
 // A thread loads each of its cell's six neighbours once and keeps what the
 // three edges that see it share: the wind, the float-float difference of the
 // Montgomery potential, theta; in FP64, where operations bound the kernel,
-// also the wind's magnitude (a rotation keeps it; the FP32 build forms it from
-// the rotated components, because the thickness tendencies, differences of
-// large fluxes, show the last bit of the edge winds).  FP64 folds the edge
-// wind's common factors: with U, V six times the interpolated components and
-// M the interpolated magnitude, u m_2 / max(eps, m_1) = U M / sqrt(U^2 + V^2).
+// also the wind's speed.  The magnitude is that of the rotated components, and
+// the matrix (cs sn; -sn cs) scales every vector by sqrt(cs^2 + sn^2), so the
+// speeds enter with that factor (g.vw): tables in real*4, as a grid file holds
+// them, are off a rotation by 6e-8.  (The FP32 build forms it from the rotated
+// components, because the thickness tendencies, differences of large fluxes,
+// show the last bit of the edge winds.)  FP64 folds the edge wind's common
+// factors: with U, V six times the interpolated components and M the
+// interpolated magnitude, u m_2 / max(eps, m_1) = U M / sqrt(U^2 + V^2).
 // The winds and the scalars are formed one after the other, so their operands
 // share registers: 64 a thread, four blocks an SM (three: 1.53 ms, five,
 // spilling: 1.88 ms).  At glvl 8 / nvl 64 in FP32 1.41 ms, 4,880 GB/s of its
@@ -139,12 +142,14 @@ __global__ void __launch_bounds__(kBlock, 4) k_edgvar1(Grid<R> g, Strides s, int
       FOR_V {
         const R ut = FIM_TRAIL(ux), vt = FIM_TRAIL(vx), ul = FIM_LEAD(ux), vl = FIM_LEAD(vx);
         if constexpr (sizeof(R) == 8) {
+          R w[4];
+          ld4(g.vw + (i * 6 + e) * 4, w);
           R un = cs[0] * u0[j] + sn[0] * v0[j] + cs[1] * ux[e][j] + sn[1] * vx[e][j];
           R vn = cs[0] * v0[j] - sn[0] * u0[j] + cs[1] * vx[e][j] - sn[1] * ux[e][j];
           un = two * un + cs[2] * ut + sn[2] * vt + cs[3] * ul + sn[3] * vl;
           vn = two * vn + cs[2] * vt - sn[2] * ut + cs[3] * vl - sn[3] * ul;
           const R sq = un * un + vn * vn;
-          const R ms = (two * (m0[j] + mx[e][j]) + FIM_TRAIL(mx) + FIM_LEAD(mx)) * divby6;
+          const R ms = w[0] * m0[j] + w[1] * mx[e][j] + w[2] * FIM_TRAIL(mx) + w[3] * FIM_LEAD(mx);
           const R q = ms * (f64_key(sq) > f64_key(R(36) * eps * eps) ? inv_root(sq) : R(1) / (R(6) * eps));
           ue[j] = un * q;
           ve[j] = vn * q;
@@ -239,6 +244,21 @@ __global__ void __launch_bounds__(kBlock, 4) k_edgvar1(Grid<R> g, Strides s, int
 }
 #undef FIM_TRAIL
 #undef FIM_LEAD
+
+// g.vw; the first square's rounding is kept, so exact rotations give 1 / 3 and
+// 1 / 6 to the last bit
+template <typename R>
+__global__ void __launch_bounds__(kBlock) k_speed_weights(int n, const R* __restrict__ cs, const R* __restrict__ sn,
+                                                          R* __restrict__ vw) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  const R a = cs[q], b = sn[q], aa = a * a;
+  vw[q] = sqrt((fma(b, b, aa) + fma(a, a, -aa)) / R((q & 3) < 2 ? 9 : 36));
+}
+template <typename R>
+void launch_speed_weights(cudaStream_t stream, int N, const R* cs, const R* sn, R* vw) {
+  k_speed_weights<R><<<blocks_for((long long)N * 24), kBlock, 0, stream>>>(N * 24, cs, sn, vw);
+}
 
 // --------------------------------------------------------------------------
 // edgvar2 (edgvar2.F90:24-319, hiOrderUVComp; the MORE_VARS block is compiled
@@ -1467,6 +1487,7 @@ void launch_step_begin(const Launch& l, StepParams* sp) {
 }
 
 #define INSTANTIATE(R)                                                                                          \
+  template void launch_speed_weights<R>(cudaStream_t, int, const R*, const R*, R*);                           \
   template void launch_edgvar1<R>(const Launch&, const Grid<R>&, const Strides&, int, const R*, const R*,      \
                                   const R*, const R*, const R*, const R*, R*, R*, R*, R*, R*, R*, R*,          \
                                   const float2*, R*);                                                         \

@@ -84,6 +84,9 @@ struct Grid {
   const int* __restrict__ nprox;  // [N]
   const R* __restrict__ cs;       // [N*6*4]
   const R* __restrict__ sn;
+  // [N*6*4] sqrt(cs^2 + sn^2) x (2, 2, 1, 1) / 6, what edgvar1's magnitude
+  // takes of the four cells' speeds (FP64 contexts; else null)
+  const R* __restrict__ vw;
   const R* __restrict__ svc;      // sidevec_c [N*6*2]
   const R* __restrict__ sve;      // sidevec_e [N*6*2]
   const R* __restrict__ sideln;   // [N*6]
@@ -570,6 +573,9 @@ __device__ __forceinline__ float ff_diff(float2 x, float2 y) {
 // ---- launchers (instantiated for float and double) ----------------------
 // mpf (FP32-mixed step only, may be null): float-float copy (hi, lo) of the
 // Montgomery potential; mont_edg then holds the edge value minus the cell value.
+// fills Grid::vw on the device (N cells)
+template <typename R>
+void launch_speed_weights(cudaStream_t stream, int N, const R* cs, const R* sn, R* vw);
 template <typename R>
 void launch_edgvar1(const Launch&, const Grid<R>&, const Strides&, int hi_order, const R* u,
                     const R* v, const R* delp, const R* pres, const R* montg, const R* tracr,
