@@ -1412,9 +1412,7 @@ template <typename R>
 int autotune_impl(fim_ctx* c, fim_state* st) {
   std::vector<StepParams> next = c->h_sp;
   for (auto& p : next) {
-    p.nf = (p.nf + 1) % 3;
-    p.of = (p.of + 1) % 3;
-    p.vof = (p.vof + 1) % 3;
+    host_abstart(p, p.its + 1);  // the step's weights too: a zero ab1 gives limiters that are no numbers
     p.narrow();
   }
   CK(cudaMemcpyAsync(c->d_sp, next.data(), sizeof(StepParams) * next.size(), cudaMemcpyHostToDevice, c->stream),

@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_edgvar1(Grid<R> g, Strides s, int
           vn = two * vn + cs[2] * vt - sn[2] * ut + cs[3] * vl - sn[3] * ul;
           const R sq = un * un + vn * vn;
           const R ms = w[0] * m0[j] + w[1] * mx[e][j] + w[2] * FIM_TRAIL(mx) + w[3] * FIM_LEAD(mx);
-          const R q = ms * (f64_key(sq) > f64_key(R(36) * eps * eps) ? inv_root(sq) : R(1) / (R(6) * eps));
+          const R q = ms * (f64_lt(sq, R(36) * eps * eps) ? R(1) / (R(6) * eps) : inv_root(sq));
           ue[j] = un * q;
           ve[j] = vn * q;
         } else {
@@ -443,6 +443,7 @@ __device__ __forceinline__ void cnuity12_body(int bx, int by, const Grid<R>& g, 
   const R half = R(0.5);
   R dpi[VK], sum[VK], pp[VK], pm[VK];
   ldv<VK>(delp + (size_t)i * L + k, dpi);
+  bool rare = false;  // FP64: a flux needs plain_donor
   FOR_V { sum[j] = R(0); pp[j] = R(0); pm[j] = R(0); }
   if (np < 6) {
     R z[VK];
@@ -480,6 +481,7 @@ __device__ __forceinline__ void cnuity12_body(int bx, int by, const Grid<R>& g, 
         if (live) {
           sum[j] = sum[j] + mf[j];
           split_sum(an[j], pp[j], pm[j]);
+          rare |= donor_rare(vn, vx) | f64_odd(dx[j]);
         }
         continue;
       }
@@ -494,6 +496,30 @@ __device__ __forceinline__ void cnuity12_body(int bx, int by, const Grid<R>& g, 
     if (live) {
       stv<VK>(mfn + o, mf);
       stv<VK>(antifx + o, an);
+    }
+  }
+  if constexpr (sizeof(R) == 8) {
+    FOR_V rare |= f64_odd(dpi[j]) | sums_rare(pp[j], pm[j]);
+    if (rare) {
+      FOR_V { sum[j] = R(0); pp[j] = R(0); pm[j] = R(0); }
+#pragma unroll 1
+      for (int e = 0; e < np; e++) {
+        const int ipx = g.prox[i * 6 + e], edx = g.proxs[i * 6 + e];
+        const R* sv = g.sve + (i * 6 + e) * 2;
+        const R* sx = g.sve + (ipx * 6 + edx) * 2;
+        const size_t o = ((size_t)i * 6 + e) * L + k, ox = ((size_t)ipx * 6 + edx) * L + k;
+        FOR_V {
+          const R vn = sv[1] * u_edg[o + j] - sv[0] * v_edg[o + j];
+          const R vx = sx[1] * u_edg[ox + j] - sx[0] * v_edg[ox + j];
+          const R mf = plain_donor(vn, vx, dpi[j], delp[(size_t)ipx * L + k + j]);
+          const R a = fma(half * vn, dp_edg[o + j] + dp_edg[ox + j], -mf);
+          sum[j] = sum[j] + mf;
+          if (a <= R(0)) pp[j] = pp[j] - a;
+          else pm[j] = pm[j] + a;
+          mfn[o + j] = mf;
+          antifx[o + j] = a;
+        }
+      }
     }
   }
   const size_t c = (size_t)i * L + k;
@@ -569,12 +595,29 @@ __device__ __forceinline__ void cnuity3_body(int bx, int by, const Grid<R>& g, c
   ldv<VK>(p_plus + c, pp);
   ldv<VK>(p_mnus + c, pm);
   const R ar = sizeof(R) == 8 ? g.area[i] * rab1 : g.area[i];
+  bool rare = false;
   FOR_V {
     const R dpmax = mx[j].at_least_zero(), dpmin = mn[j].at_least_zero();
     const R q_plus = per_ab1(dpmax - dlo[j] - (ab2 * neg(to[j]) + ab3 * pos(tv[j])), rab1, ar);
     const R q_mnus = per_ab1(dlo[j] - dpmin + (ab2 * pos(to[j]) + ab3 * neg(tv[j])), rab1, ar);
     rp[j] = ratio01(q_plus, floor_at(pp[j], thshld));
     rm[j] = ratio01(q_mnus, floor_at(pm[j], thshld));
+    rare |= bounds_rare(mx[j], mn[j]) | ratio_rare(q_plus, q_mnus);
+  }
+  if (rare) {  // as the routine writes it
+    FOR_V {
+      R hi = rmax(dlo[j], dc[j]), lo = rmin(dlo[j], dc[j]);
+#pragma unroll 1
+      for (int e = 0; e < 6; e++) {
+        const R a = delp_lo[(size_t)pr[e] * L + k + j], b = delp[(size_t)pr[e] * L + k + j];
+        hi = rmax(hi, rmax(a, b));
+        lo = rmin(lo, rmin(a, b));
+      }
+      hi = rmax(R(0), hi);
+      lo = rmax(R(0), lo);
+      rp[j] = plain_ratio01(per_ab1(hi - dlo[j] - (ab2 * rmin(R(0), to[j]) + ab3 * rmax(R(0), tv[j])), rab1, ar), pp[j]);
+      rm[j] = plain_ratio01(per_ab1(dlo[j] - lo + (ab2 * rmax(R(0), to[j]) + ab3 * rmin(R(0), tv[j])), rab1, ar), pm[j]);
+    }
   }
   stv<VK>(r_plus + c, rp);
   stv<VK>(r_mnus + c, rm);
@@ -607,7 +650,13 @@ __device__ __forceinline__ void cnuity4_body(int bx, int by, const Grid<R>& g, c
   R rp[VK], rm[VK], at[VK];
   ldv<VK>(r_plus + c, rp);
   ldv<VK>(r_mnus + c, rm);
-  FOR_V at[j] = R(0);
+  FOR_V {
+    if (sizeof(R) == 8) {
+      rp[j] = own_limit(rp[j]);
+      rm[j] = own_limit(rm[j]);
+    }
+    at[j] = R(0);
+  }
   const int np = g.nprox[i];
   for (int e = 0; e < np; e++) {
     const int px = g.prox[i * 6 + e];
@@ -619,7 +668,8 @@ __device__ __forceinline__ void cnuity4_body(int bx, int by, const Grid<R>& g, c
     ldv<VK>(r_mnus + (size_t)px * L + k, rmx);
     FOR_V {
       const bool in = negative(a[j]);
-      const R clip = min0(in ? rp[j] : rm[j], in ? rmx[j] : rpx[j]);
+      const R own = in ? rp[j] : rm[j], other = in ? rmx[j] : rpx[j];
+      const R clip = sizeof(R) == 8 ? min0(own, other) : rmin(own, other);
       const R ac = a[j] * clip;
       mf[j] = mf[j] + ac;
       at[j] = at[j] + ac;

@@ -349,6 +349,18 @@ __device__ __forceinline__ long long f64_key(double x) {
   return b ^ ((b >> 63) & 0x7fffffffffffffffll);
 }
 __device__ __forceinline__ bool f64_neg(double x) { return __double2hiint(x) < 0; }
+// by the upper word: a NaN (quiet, as all arithmetic makes them); an infinity
+// or a NaN; negative and no NaN
+__device__ __forceinline__ bool f64_nan(double x) { return (__double2hiint(x) & 0x7fffffff) > 0x7ff00000; }
+__device__ __forceinline__ bool f64_odd(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
+__device__ __forceinline__ bool f64_below0(double x) {
+  return ((unsigned)__double2hiint(x) ^ 0x80000000u) <= 0x7ff00000u;
+}
+// a < b, false where either is a NaN (zeros are ordered by their signs)
+__device__ __forceinline__ bool f64_lt(double a, double b) {
+  const long long x = f64_key(a), y = f64_key(b);
+  return x < y && (int)(y >> 32) <= 0x7ff00000 && (int)(x >> 32) >= (int)0x800fffff;
+}
 // 1 / b, b normal and below 2^1000: one third-order step from the
 // approximation (its error cubed is below rounding)
 __device__ __forceinline__ double f64_recip(double b) {
@@ -427,21 +439,33 @@ __device__ __forceinline__ float pow_rd_cp(float x) { return pow(x, float(kRd) /
 
 // ---- flux limiters: bounds, signs and quotients ------------------------------
 // FP32 takes the min/max instructions; FP64 compares on the integer pipe and
-// divides with the fewest FP64 operations (above).  A NaN operand does not enter a bound or a
-// sign split here; it reaches the cell's result through the fluxes and the
-// AB3 sums, whose final clip (tmin/tmax) keeps it.
-// At glvl 6 / nvl 64 / 11 tracers this took the FP64 k_trf_lo from 9.56 to
-// 6.1 ms and k_trf_hi from 8.15 to 2.86 ms a step (FP32: 2% of k_trf_hi).
+// divides with the fewest FP64 operations (above).  At glvl 6 / nvl 64 / 11
+// tracers this took the FP64 k_trf_lo from 9.56 to 5.4 ms and k_trf_hi from
+// 8.15 to 2.86 ms a step (FP32: 2% of k_trf_hi).
+//
+// These forms hold for numbers.  What is not finite has to go where the
+// routines, written with a > b ? a : b, send it (a NaN in a tracer, a thickness
+// or a flux reaches the cells around it through fluxes and limiters), so every
+// item asks the _rare tests at its end and, if one says so, is formed again
+// as the routine writes it (plain_*).  One branch an item: the tests a level
+// cost 0-1 FP32 or ~6 integer instructions, where tests in every helper cost
+// the FP64 k_trf_lo 18%, k_trf_hi 19%, and the FP32 trcadv 5%.
+
+// max / min that keep a NaN of any value
+__device__ __forceinline__ float max_nan(float a, float b) { float r; asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float min_nan(float a, float b) { float r; asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float max_nan(float a, float b, float c) { float r; asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
+__device__ __forceinline__ float min_nan(float a, float b, float c) { float r; asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
 template <typename R> struct Bound;
 template <> struct Bound<float> {
   float v;
   __device__ __forceinline__ static Bound of(float x) { return {x}; }
-  __device__ __forceinline__ void up(Bound a) { v = fmaxf(v, a.v); }
-  __device__ __forceinline__ void down(Bound a) { v = fminf(v, a.v); }
+  __device__ __forceinline__ void up(Bound a) { v = max_nan(v, a.v); }
+  __device__ __forceinline__ void down(Bound a) { v = min_nan(v, a.v); }
   // with two values at once (three-input instructions)
-  __device__ __forceinline__ void up(Bound a, Bound b) { asm("max.f32 %0, %0, %1, %2;" : "+f"(v) : "f"(a.v), "f"(b.v)); }
-  __device__ __forceinline__ void down(Bound a, Bound b) { asm("min.f32 %0, %0, %1, %2;" : "+f"(v) : "f"(a.v), "f"(b.v)); }
-  __device__ __forceinline__ float at_least_zero() const { return fmaxf(v, 0.f); }
+  __device__ __forceinline__ void up(Bound a, Bound b) { v = max_nan(v, a.v, b.v); }
+  __device__ __forceinline__ void down(Bound a, Bound b) { v = min_nan(v, a.v, b.v); }
+  __device__ __forceinline__ float at_least_zero() const { return max_nan(v, 0.f); }
 };
 template <> struct Bound<double> {
   long long v;
@@ -452,23 +476,34 @@ template <> struct Bound<double> {
   __device__ __forceinline__ void down(Bound a, Bound b) { down(a); down(b); }
   __device__ __forceinline__ double at_least_zero() const { return __longlong_as_double(v > 0 ? v : 0); }
 };
+// upper and lower bound of a ring: some value is a NaN, or (FP64, whose one-
+// product fluxes leave it out) infinite
+__device__ __forceinline__ bool bounds_rare(Bound<float> up, Bound<float>) { return up.v != up.v; }
+__device__ __forceinline__ bool bounds_rare(Bound<double> up, Bound<double> down) {
+  return ((int)(up.v >> 32) >= 0x7ff00000) | ((int)(down.v >> 32) <= (int)0x800fffff);
+}
+template <typename R> __device__ __forceinline__ R plain_max(R a, R b) { return a > b ? a : b; }
+template <typename R> __device__ __forceinline__ R plain_min(R a, R b) { return a < b ? a : b; }
 
-// the positive / negative part of x
-__device__ __forceinline__ float pos(float x) { return fmaxf(x, 0.f); }
-__device__ __forceinline__ float neg(float x) { return fminf(x, 0.f); }
-__device__ __forceinline__ double pos(double x) { return __double2hiint(x) < 0 ? 0. : x; }
-__device__ __forceinline__ double neg(double x) { return __double2hiint(x) < 0 ? x : 0.; }
-// the smaller of two values >= 0
-__device__ __forceinline__ float min0(float a, float b) { return fminf(a, b); }
-__device__ __forceinline__ double min0(double a, double b) {
-  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+// the positive / negative part of x; a NaN in both
+__device__ __forceinline__ float pos(float x) { return max_nan(x, 0.f); }
+__device__ __forceinline__ float neg(float x) { return min_nan(x, 0.f); }
+__device__ __forceinline__ double pos(double x) { return f64_below0(x) ? 0. : x; }
+__device__ __forceinline__ double neg(double x) { return (unsigned)__double2hiint(x) > 0x7ff00000u ? x : 0.; }
+// own < other ? own : other of two cells' limiters (0 .. 1; a NaN comes sign
+// set from plain_ratio01), the cell's own through own_limit first
+__device__ __forceinline__ float own_limit(float r) { return r != r ? 2.f : r; }
+__device__ __forceinline__ double own_limit(double r) { return __double2hiint(r) < 0 ? 2. : r; }
+__device__ __forceinline__ float min0(float own, float other) { return min_nan(own, other); }
+__device__ __forceinline__ double min0(double own, double other) {
+  const long long x = __double_as_longlong(own), y = __double_as_longlong(other);
   return __longlong_as_double(x < y ? x : y);
 }
-// max(a, b) of values >= 0
+// a > b ? a : b, b > 0
 __device__ __forceinline__ float floor_at(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ double floor_at(double a, double b) {
   const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
-  return __longlong_as_double(x > y ? x : y);
+  return x > y && (int)(x >> 32) <= 0x7ff00000 ? a : b;
 }
 __device__ __forceinline__ bool negative(float x) { return x < 0.f; }
 __device__ __forceinline__ bool negative(double x) { return __double2hiint(x) < 0; }
@@ -480,22 +515,31 @@ __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-// low-order flux a tri - b trx of the two sides' outflows a, b >= 0.  The
-// two sides hold the same mass flux with opposite signs, up to rounding, so
-// one of the products is zero but for fluxes of a rounding error's size: FP64
-// forms the other one only.
+// low-order flux ((mf + |mf|) tri - (mfx + |mfx|) trx) / 2 of the two sides'
+// mass fluxes (plain_donor).  They are the same with opposite signs, up to
+// rounding, so one of the products is zero but for fluxes of a rounding error's
+// size: FP64 forms the other one only.  donor_rare: FP64 mass fluxes that are
+// not finite or are positive on both sides (FP32: not finite, asked by the
+// largest magnitude).
+template <typename R>
+__device__ __forceinline__ R plain_donor(R mf, R mfx, R tri, R trx) {
+  return mul_rn(R(0.5), fma_rn(mf + fabs(mf), tri, -mul_rn(mfx + fabs(mfx), trx)));
+}
 __device__ __forceinline__ float donor(float mf, float mfx, float tri, float trx) {
-  return fma_rn(pos(mf), tri, -mul_rn(pos(mfx), trx));
+  return fma_rn(fmaxf(mf, 0.f), tri, -mul_rn(fmaxf(mfx, 0.f), trx));
 }
 __device__ __forceinline__ double donor(double mf, double mfx, double tri, double trx) {
   const bool out = __double2hiint(mf) >= 0;
-  const double b = pos(mfx);
-  double lo = mul_rn(out ? mf : -b, out ? tri : trx);
-  if (out && __double_as_longlong(b) != 0ll) lo = fma_rn(mf, tri, -mul_rn(b, trx));
-  return lo;
+  const double b = negative(mfx) ? 0. : mfx;
+  return mul_rn(out ? mf : -b, out ? tri : trx);
+}
+__device__ __forceinline__ bool donor_rare(double mf, double mfx) {
+  const int a = __double2hiint(mf), b = __double2hiint(mfx);
+  return (max(a & 0x7fffffff, b & 0x7fffffff) >= 0x7ff00000) | ((a >= 0) & (__double_as_longlong(mfx) > 0ll));
 }
 
-// S+ -= min(0, a), S- += max(0, a); FP64: one addition, to the sum a's sign names
+// S+ -= min(0, a), S- += max(0, a); FP64: one addition, to the sum a's sign
+// names (sums_rare: one of them ended as a NaN)
 __device__ __forceinline__ void split_sum(float a, float& sp, float& sm) {
   sp = sp - neg(a);
   sm = sm + pos(a);
@@ -506,6 +550,8 @@ __device__ __forceinline__ void split_sum(double a, double& sp, double& sm) {
   sp = n ? t : sp;
   sm = n ? sm : t;
 }
+__device__ __forceinline__ bool sums_rare(float, float) { return false; }
+__device__ __forceinline__ bool sums_rare(double sp, double sm) { return f64_nan(sp) | f64_nan(sm); }
 
 // a / b with rb = 1 / b formed once; an FP64 result that is not finite is
 // divided as written
@@ -516,7 +562,8 @@ __device__ __forceinline__ double quot(double a, double b, double rb) {
   return q;
 }
 
-// max(0, min(1, a / b)), b > 0
+// max(0, min(1, a / b)), b > 0; ratio_rare: a NaN (FP32: or two infinities)
+// among the numerators of R+ and R-, or an infinite one (FP64)
 __device__ __forceinline__ float ratio01(float a, float b) { return __saturatef(__fdividef(a, b)); }
 __device__ __forceinline__ double ratio01(double a, double b) {
   const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
@@ -524,6 +571,16 @@ __device__ __forceinline__ double ratio01(double a, double b) {
   if (x >= y) return 1.;
   if (y >= 0x7e00000000000000ll) return a / b;
   return f64_quot(a, b, f64_recip(b));  // 0 < a < b
+}
+__device__ __forceinline__ bool ratio_rare(float a, float b) { return (a + b) != (a + b); }
+__device__ __forceinline__ bool ratio_rare(double a, double b) { return f64_odd(a) | f64_odd(b); }
+__device__ __forceinline__ float plain_ratio01(float a, float b) {
+  const float q = plain_max(0.f, plain_min(1.f, fdiv(a, plain_max(b, 1.e-11f))));
+  return q != q ? __int_as_float(0xffc00000) : q;
+}
+__device__ __forceinline__ double plain_ratio01(double a, double b) {
+  const double q = plain_max(0., plain_min(1., a / plain_max(b, 1.e-11)));
+  return q != q ? __longlong_as_double((long long)0xfff8000000000000ull) : q;
 }
 
 // q / ab1 x area: FP64 holds the factor once a cell; FP32 keeps two products

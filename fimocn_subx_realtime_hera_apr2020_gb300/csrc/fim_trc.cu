@@ -354,6 +354,65 @@ struct CellItem {
   }
 };
 
+// One level of a cell as the routines write it, for items that hold a value
+// that is not finite (or, in FP64, a mass flux positive on both sides).
+// trcadv1's bounds of frame cell x: T the tracer's frame at that level.
+template <typename R> struct UpDown { R up, down; };
+template <typename R, int LK>
+__device__ __forceinline__ UpDown<R> plain_bounds(const R* T, uint2 nb, int x) {
+  UpDown<R> b{T[x * LK], T[x * LK]};
+#pragma unroll 1
+  for (int e = 0; e < 6; e++) {
+    const R a = T[nb_at(nb, e) * LK];
+    b = {plain_max(b.up, a), plain_min(b.down, a)};
+  }
+  return {plain_max(R(0), b.up), plain_max(R(0), b.down)};
+}
+
+// fluxes, sums and bounds of patch cell x in trcadv1 and trcadv2; te: its six
+// edge values in memory (stride L), or null where they are E's; mir: its six
+// entries; anti: its antidiffusive fluxes (stride L)
+template <typename R> struct LoItem { R sum, sp, sm, hx, hn; };
+template <typename R, int LK>
+__device__ __noinline__ LoItem<R> plain_lo(const R* T, const R* MF, const R* E, const R* te,
+                                           const unsigned short* mir, uint2 nb, int x, int np, int L, R* anti) {
+  const UpDown<R> b = plain_bounds<R, LK>(T, nb, x);
+  LoItem<R> w{R(0), R(0), R(0), b.up, b.down};
+  const R tri = T[x * LK];
+#pragma unroll 1
+  for (int e = 0; e < np; e++) {
+    const R mf = MF[erow(x, e) * LK], mfx = MF[mir[e] * LK], trx = T[nb_at(nb, e) * LK];
+    const R tev = te ? te[e * L] : E[erow(x, e) * LK] + E[mir[e] * LK];
+    const R lo = plain_donor(mf, mfx, tri, trx);
+    const R a = fma_rn(mf, tev, -lo);
+    w.sum = w.sum + lo;
+    w.sp = w.sp - plain_min(R(0), a);
+    w.sm = w.sm + plain_max(R(0), a);
+    anti[e * L] = a;
+  }
+  return w;
+}
+
+// bounds and limiters of frame cell x in trcadv2 (ar: the cell's area, in FP64
+// over ab1)
+template <typename R> struct LimItem { R hx, hn, rp, rm; };
+template <typename R, int LK>
+__device__ __noinline__ LimItem<R> plain_limits(const R* TO, const R* TL, uint2 nb, int x, R dp, R tof, R tvf, R spl,
+                                                R smn, R ab2, R ab3, R rab1, R ar) {
+  const R lc = TL[x * LK];
+  UpDown<R> b = plain_bounds<R, LK>(TO, nb, x);
+  b = {plain_max(b.up, lc), plain_min(b.down, lc)};
+#pragma unroll 1
+  for (int e = 0; e < 6; e++) {
+    const R a = TL[nb_at(nb, e) * LK];
+    b = {plain_max(b.up, a), plain_min(b.down, a)};
+  }
+  b = {plain_max(R(0), b.up), plain_max(R(0), b.down)};
+  const R qp = per_ab1((b.up - lc) * dp - (ab2 * plain_min(R(0), tof) + ab3 * plain_max(R(0), tvf)), rab1, ar);
+  const R qm = per_ab1((lc - b.down) * dp + (ab2 * plain_max(R(0), tof) + ab3 * plain_min(R(0), tvf)), rab1, ar);
+  return {b.up, b.down, plain_ratio01(qp, spl), plain_ratio01(qm, smn)};
+}
+
 // trcadv1 + the S+/S- sums of trcadv2 + copy of the old tracer, per patch.
 // EV: the edge values of every tracer are the caller's (trc_edg of the
 // per-routine trcadv, or edgvar1's without hi_order_flux_comp); a thread
@@ -428,6 +487,7 @@ __global__ void __launch_bounds__(64 * GC, sizeof(R) == 8 && VK == 1 ? 12 / GC :
   stage(t0, 0);
   CellItem<R, VK> ci;
   ci.template load<GC>(g, s, fs, m, delp, C, k0, lk);
+  bool mf_rare = false;
   for (int tz = 0; tz < ntm; tz++) {
     const int t = t0 + tz, b = tz & 1;
     R ter[6][VK];  // EV: the edge values of the thread's cell, in flight over the wait
@@ -465,6 +525,18 @@ __global__ void __launch_bounds__(64 * GC, sizeof(R) == 8 && VK == 1 ? 12 / GC :
     if (!ci.on) continue;
     const int x = ci.x, v = ci.v, i = ci.i, c = ci.c;
     const uint2 nb = fs.nbr[x];
+    // a mass flux of the cell needs plain_donor: FP64 looks once, FP32 keeps the
+    // largest magnitude as the fluxes pass (one instruction each)
+    float top = 0.f;
+    if (sizeof(R) == 8 && tz == 0) {
+#pragma unroll
+      for (int e = 0; e < 6; e++) {
+        R a[VK], b[VK];
+        ldv<VK>(MF + erow(x, e) * LK + v, a);
+        ldv<VK>(MF + fs.mir[x * 6 + e] * LK + v, b);
+        FOR_V mf_rare |= (e < 5 || e < ci.np) & donor_rare(a[j], b[j]);
+      }
+    }
     R tri[VK], sumlo[VK], sp_[VK], sm_[VK];
     Bound<R> mx[VK], mn[VK];
     ldv<VK>(T + x * LK + v, tri);
@@ -495,12 +567,34 @@ __global__ void __launch_bounds__(64 * GC, sizeof(R) == 8 && VK == 1 ? 12 / GC :
         ldv<VK>(MF + erow(x, e) * LK + v, mfo);
         ldv<VK>(MF + fs.mir[x * 6 + e] * LK + v, mfm);
         FOR_V {
+          if constexpr (sizeof(R) == 4) top = max_nan(top, fabsf(mfo[j]), fabsf(mfm[j]));
           const R lo = donor(mfo[j], mfm[j], tri[j], trx[j]);
           anti[j] = fma_rn(mfo[j], tev[j], -lo);
           sumlo[j] = sumlo[j] + lo;
           split_sum(anti[j], sp_[j], sm_[j]);
         }
         stv<VK>(antifx + (m * nt + tz) * 6 * sc + (size_t)(i * 6 + e) * L + ci.k, anti);
+      }
+    }
+    const size_t q = (m * nt + tz) * sc + c;
+    R* const af = antifx + (m * nt + tz) * 6 * sc + (size_t)i * 6 * L + ci.k;
+    R hx[VK], hn[VK];
+    bool rare = mf_rare | !(top < __int_as_float(0x7f800000));
+    FOR_V {
+      hx[j] = mx[j].at_least_zero();
+      hn[j] = mn[j].at_least_zero();
+      rare |= bounds_rare(mx[j], mn[j]) | sums_rare(sp_[j], sm_[j]);
+    }
+    if (rare) {
+      const R* te = EV || t == 0 ? te0 + (EV ? (size_t)t * 6 * NL : (size_t)0) + (size_t)i * 6 * L + ci.k : nullptr;
+      FOR_V {
+        const LoItem<R> w = plain_lo<R, LK>(T + v + j, MF + v + j, E + v + j, te ? te + j : te, fs.mir + x * 6, nb, x,
+                                            ci.np, L, af + j);
+        sumlo[j] = w.sum;
+        sp_[j] = w.sp;
+        sm_[j] = w.sm;
+        hx[j] = w.hx;
+        hn[j] = w.hn;
       }
     }
     const R* o = ops + b * 3 * ft.SC * LK + x * LK + v;
@@ -510,11 +604,9 @@ __global__ void __launch_bounds__(64 * GC, sizeof(R) == 8 && VK == 1 ? 12 / GC :
     ldv<VK>(o, tlo);
     ldv<VK>(o + ft.SC * LK, tlv);
     ldv<VK>(o + 2 * ft.SC * LK, td);
-    const size_t q = (m * nt + tz) * sc + c;
     FOR_V {
       const R lo = td[j] + ab1 * tn[j] + ab2 * tlo[j] + ab3 * tlv[j];
-      const R hx = mx[j].at_least_zero(), hn = mn[j].at_least_zero();
-      out[j] = tmax(hn, tmin(hx, quot(lo, ci.dp[j], ci.rdp[j])));
+      out[j] = tmax(hn[j], tmin(hx[j], quot(lo, ci.dp[j], ci.rdp[j])));
     }
     stv<VK>(trcr_lo + q, out);
     stv<VK>(s_plus + q, sp_);
@@ -573,6 +665,7 @@ __device__ __forceinline__ void limiters(const FrameSm& fs, const R* TO, const R
   ldv<VK>(opq + 3 * S1 * LK + o, smn);
   ldv<VK>(dpf + o, dp);
   const R ar = arf[xe];
+  bool rare = false;
   FOR_V {
     hx[j] = mx[j].at_least_zero();
     hn[j] = mn[j].at_least_zero();
@@ -580,6 +673,17 @@ __device__ __forceinline__ void limiters(const FrameSm& fs, const R* TO, const R
     const R q_mnus = per_ab1((lc[j] - hn[j]) * dp[j] + (ab2 * pos(tof[j]) + ab3 * neg(tvf[j])), rab1, ar);
     rp[j] = ratio01(q_plus, floor_at(spl[j], thshld));
     rm[j] = ratio01(q_mnus, floor_at(smn[j], thshld));
+    rare |= bounds_rare(mx[j], mn[j]) | ratio_rare(q_plus, q_mnus);
+  }
+  if (rare) {
+    FOR_V {
+      const LimItem<R> w = plain_limits<R, LK>(TO + ve + j, TL + ve + j, nb, xe, dp[j], tof[j], tvf[j], spl[j],
+                                               smn[j], ab2, ab3, rab1, ar);
+      hx[j] = w.hx;
+      hn[j] = w.hn;
+      rp[j] = w.rp;
+      rm[j] = w.rm;
+    }
   }
   stv<VK>(Rp + o, rp);
   stv<VK>(Rm + o, rm);
@@ -719,7 +823,11 @@ __global__ void __launch_bounds__(64 * GC, VK * (int)sizeof(R) == 16 ? 8 / GC : 
     R rpc[VK], rmc[VK], at[VK];
     ldv<VK>(Rp + x * LK + v, rpc);
     ldv<VK>(Rm + x * LK + v, rmc);
-    FOR_V at[j] = R(0);
+    FOR_V {
+      rpc[j] = own_limit(rpc[j]);
+      rmc[j] = own_limit(rmc[j]);
+      at[j] = R(0);
+    }
 #pragma unroll
     for (int e = 0; e < 6; e++) {
       if (e < 5 || e < np) {
