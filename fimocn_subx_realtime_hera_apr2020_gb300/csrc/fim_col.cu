@@ -29,16 +29,13 @@ __device__ __forceinline__ bool lt(float a, float b) { return a < b; }
 __device__ __forceinline__ bool lt(double a, double b) { return f64_key(a) < f64_key(b); }
 __device__ __forceinline__ double cmax(double a, double b) { return lt(b, a) ? a : b; }
 __device__ __forceinline__ double cmin(double a, double b) { return lt(a, b) ? a : b; }
-// a / b; FP64: b normal, reciprocal and one residual correction
-__device__ __forceinline__ float qdiv(float a, float b) { return a / b; }
-__device__ __forceinline__ double qdiv(double a, double b) { return f64_quot(a, b, f64_recip(b)); }
 // x / 10, rounded as the division (Markstein's correction; for this divisor the
 // rounded reciprocal gives the rounded quotient for every FP32 mantissa)
 __device__ __forceinline__ float tenth(float x) {
   const float q = x * .1f;
   return fmaf(fmaf(-10.f, q, x), .1f, q);
 }
-__device__ __forceinline__ double tenth(double x) { return f64_quot(x, 10., .1); }
+__device__ __forceinline__ double tenth(double x) { return divide_by(x, 10., .1); }
 
 constexpr int kColBlock = 128;
 constexpr int kBlock2 = 256;
@@ -120,7 +117,7 @@ __device__ void restp_1d(C oldth, int kmod, C pkold, int kold, C pknew, const R*
       break;
     }
     R pn = prev;
-    if (lt(tk, tk1)) pn = qdiv(pinteg, tk1 - tk);
+    if (lt(tk, tk1)) pn = divide(pinteg, tk1 - tk);
     pknew[k + 1] = pn;
     cloutt = cloutt + tk * (pn - prev);
     prev = pn;
@@ -165,7 +162,7 @@ __device__ void equilb(const R* thet, C pnew, int kk, R slak) {
 template <typename R>
 __device__ __forceinline__ R cushn(R a, R b) {
   const R m = cmin(a, R(2) * b);
-  return qdiv(R(.25) * (m * m), b) + cmax(a, R(2) * b) - b;
+  return divide(R(.25) * (m * m), b) + cmax(a, R(2) * b) - b;
 }
 
 // inflate (hybgen.F90:893-1007); d0(k) = rd dpsig(k) / p1000
@@ -270,10 +267,10 @@ __device__ void regrid_1d(const Knobs& kn, const RegTab<R, ML>& tab, int L, int 
     for (int k = 1; k <= L - 1; k++) {
       const R hi = exnew[k + 1];
       R hcur = R(0);
-      if (k <= L - 2 && lt(at, bot) && lt(top, hi)) hcur = qdiv(tab.num[k], cmax(tab.fl[k], at - hi));
+      if (k <= L - 2 && lt(at, bot) && lt(top, hi)) hcur = divide(tab.num[k], cmax(tab.fl[k], at - hi));
       R now = at;
       if (lt(at, bot) && lt(top, at)) {
-        now = cmax(hi, cmin(lo, at + qdiv(hcur - hprev, targt[k] - targt[k - 1])));
+        now = cmax(hi, cmin(lo, at + divide(hcur - hprev, targt[k] - targt[k - 1])));
         exnew[k] = now;
       }
       event = event || lt(newlo + thin, now);
@@ -810,9 +807,8 @@ static_assert(sizeof(RemapV<float, 1, 1>) % 16 == 0 && sizeof(RemapV<double, 1, 
                   sizeof(RemapV<float, 4, 2>) % 16 == 0,
               "ring slots of consecutive warps stay 16-byte aligned");
 
-// x / cp, the division as the reference writes it
-__device__ __forceinline__ float by_cp(float x) { return x / float(kCp); }
-__device__ __forceinline__ double by_cp(double x) { return f64_quot(x, kCp, 1. / kCp); }
+template <typename R>
+__device__ __forceinline__ R by_cp(R x) { return divide_by(x, R(kCp), R(1) / R(kCp)); }
 
 // Level kb + v of a column of L levels held VL a lane by W lanes: with FULL the
 // column fills the lanes (L == W VL), so that the tests cost nothing but for
@@ -835,11 +831,10 @@ struct LaneGeo {
   bool thin;                   // (whole warp) some layer is thin enough for the fill to matter
 };
 
-// 1 / x and a / b of thicknesses (x > 0, at least 1e-22; 0 <= a <= b)
+// 1 / x and a / b of thicknesses
 __device__ __forceinline__ float recip(float x) { return fdiv(1.f, x); }
-__device__ __forceinline__ double recip(double x) { return f64_recip(x); }
 __device__ __forceinline__ float over(float a, float b) { return fdiv(a, b); }
-__device__ __forceinline__ double over(double a, double b) { return f64_quot(a, b, f64_recip(b)); }
+__device__ __forceinline__ double over(double a, double b) { return divide(a, b); }
 
 template <typename R>
 __device__ __forceinline__ R coord_thick(bool flip, const R* x, int k) {
@@ -1485,12 +1480,12 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
       R na = tha, nbv = thb;
       if (lt(R(0), deviup) && lt(devilo, R(0))) {
         const R cc = cmin(deviup, -devilo);
-        na = tha + qdiv(cc, dplo);
-        nbv = thb - qdiv(cc, dpup);
+        na = tha + divide(cc, dplo);
+        nbv = thb - divide(cc, dpup);
       } else if (lt(deviup, R(0)) && lt(R(0), devilo)) {
         const R cc = cmin(devilo, -deviup);
-        na = tha - qdiv(cc, dplo);
-        nbv = thb + qdiv(cc, dpup);
+        na = tha - divide(cc, dplo);
+        nbv = thb + divide(cc, dpup);
       }
       th[k - 1] = nbv;
       thb = na;

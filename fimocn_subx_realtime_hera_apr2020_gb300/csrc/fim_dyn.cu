@@ -760,10 +760,6 @@ __global__ void __launch_bounds__(kBlock) k_cnuity_coop(Grid<R> g, Strides s, co
                         flags);
 }
 
-// a / b with rb = 1 / b: FP32 divides as written
-__device__ __forceinline__ float quot_by(float a, float b, float) { return a / b; }
-__device__ __forceinline__ double quot_by(double a, double b, double rb) { return f64_quot(a, b, rb); }
-
 // cnuity5 (cnuity_compute.F90:408-445), 32 columns a block.  The layer
 // thickness and pressure tendency of every level are formed with thread =
 // (column, VK levels) into shared tiles; the top-down pressure sum (warp 0) and
@@ -820,7 +816,7 @@ __global__ void __launch_bounds__(kC5Block, 4) k_cnuity5(Grid<R> g, Strides s,
     }
     FOR_V {
       tp[r * LS + k + j] = d[j];
-      tw[r * LS + k + j] = quot_by(ab1 * tnf[j] + ab2 * tof[j] + ab3 * tvf[j], dt, rdt);
+      tw[r * LS + k + j] = divide_by(ab1 * tnf[j] + ab2 * tof[j] + ab3 * tvf[j], dt, rdt);
     }
   }
   __syncthreads();
@@ -882,7 +878,7 @@ __global__ void __launch_bounds__(kC5Block, 4) k_cnuity5(Grid<R> g, Strides s,
     FOR_V {
       const R pr = tp[r * LS + k + j];
       pres[(size_t)i * L1 + k + j] = pr;
-      exner[(size_t)i * L1 + k + j] = cp * pow_rd_cp(quot_by(pr, p1000, R(1) / R(kP1000)));
+      exner[(size_t)i * L1 + k + j] = cp * pow_rd_cp(divide_by(pr, p1000, R(1) / R(kP1000)));
       dpdx[j] = R(0);
       dpdy[j] = R(0);
     }

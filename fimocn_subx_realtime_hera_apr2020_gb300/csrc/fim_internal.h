@@ -375,6 +375,26 @@ __device__ __forceinline__ double f64_quot(double a, double b, double rb) {
   const double q = a * rb;
   return fma(fma(-b, q, a), rb, q);
 }
+// 1 / b and a / b of any operands: where b is zero or infinite, or a is, the
+// steps make NaNs of the approximation or the product, which are the result
+// then (selected on the integer pipe; a division as written in a branch cost
+// k_dissip 28% and k_regrid 45%).  FP32: as written.
+__device__ __forceinline__ double recip(double b) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+  const double e = fma(-b, r, 1.), s = fma(r, fma(e, e, e), r);
+  return f64_odd(e) ? r : s;
+}
+__device__ __forceinline__ double divide_by(double a, double b, double rb) {
+  const double q = a * rb, e = fma(-b, q, a), s = fma(e, rb, q);
+  return f64_odd(e) ? q : s;
+}
+__device__ __forceinline__ float divide_by(float a, float b, float) { return a / b; }
+__device__ __forceinline__ double divide(double a, double b) { return divide_by(a, b, recip(b)); }
+__device__ __forceinline__ float divide(float a, float b) { return a / b; }
+// the limiters' quotient: FP32 by the reciprocal
+__device__ __forceinline__ float quot(float a, float, float rb) { return a * rb; }
+__device__ __forceinline__ double quot(double a, double b, double rb) { return divide_by(a, b, rb); }
 // 1 / sqrt(x), x normal: one third-order step r (1 + e/2 + 3 e^2/8)
 __device__ __forceinline__ double f64_rsqrt(double x) {
   double r;
@@ -552,15 +572,6 @@ __device__ __forceinline__ void split_sum(double a, double& sp, double& sm) {
 }
 __device__ __forceinline__ bool sums_rare(float, float) { return false; }
 __device__ __forceinline__ bool sums_rare(double sp, double sm) { return f64_nan(sp) | f64_nan(sm); }
-
-// a / b with rb = 1 / b formed once; an FP64 result that is not finite is
-// divided as written
-__device__ __forceinline__ float quot(float a, float b, float rb) { return a * rb; }
-__device__ __forceinline__ double quot(double a, double b, double rb) {
-  double q = f64_quot(a, b, rb);
-  if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) q = a / b;
-  return q;
-}
 
 // max(0, min(1, a / b)), b > 0; ratio_rare: a NaN (FP32: or two infinities)
 // among the numerators of R+ and R-, or an infinite one (FP64)
