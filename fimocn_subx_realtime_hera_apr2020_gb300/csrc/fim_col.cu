@@ -24,9 +24,11 @@ template <typename R> __device__ __forceinline__ R cmin(R a, R b) { return a < b
 template <typename R> __device__ __forceinline__ R cabs(R a) { return a < R(0) ? -a : a; }
 __device__ __forceinline__ double cabs(double a) { return fabs(a); }
 
-// FP64 comparisons on the integer pipe (fim_internal.h)
+// FP64 comparisons on the integer pipe (fim_internal.h); false for NaNs, as <
 __device__ __forceinline__ bool lt(float a, float b) { return a < b; }
-__device__ __forceinline__ bool lt(double a, double b) { return f64_key(a) < f64_key(b); }
+__device__ __forceinline__ bool lt(double a, double b) { return f64_lt(a, b); }
+__device__ __forceinline__ bool nonzero(float a) { return a != 0.f; }
+__device__ __forceinline__ bool nonzero(double a) { return (__double_as_longlong(a) << 1) != 0ll; }
 __device__ __forceinline__ double cmax(double a, double b) { return lt(b, a) ? a : b; }
 __device__ __forceinline__ double cmin(double a, double b) { return lt(a, b) ? a : b; }
 // x / 10, rounded as the division (Markstein's correction; for this divisor the
@@ -716,7 +718,8 @@ __device__ __forceinline__ R fill_thin() { return R(1.2e-4); }
 // PLM slope of a layer from its filled value f and its neighbours' fm, fp
 __device__ __forceinline__ float plm_slope(float fm, float f, float fp) {
   const float b = ((fp - fm) * (fm + fp - 2.f * f) > 0.f) ? f - fm : fp - f;
-  return (f <= fminf(fm, fp) || f >= fmaxf(fm, fp)) ? 0.f : b;
+  // (a NaN is dropped from below and kept from above, as cmin and cmax do)
+  return (f <= fminf(fm, fp) || f >= fmaxf(fm, fp)) && fp == fp ? 0.f : b;
 }
 
 // FP64: monotonicity and the slope's sign by integer comparisons (a zero
@@ -729,7 +732,12 @@ __device__ __forceinline__ double plm_slope(double fm, double f, double fp) {
   const bool lower = c != 0. && f64_neg(c) == fall;
   return (lower ? f : fp) - (lower ? fm : f);
 }
-
+// the slope as pcwise writes it, for values that are not finite
+__device__ __forceinline__ float plain_slope(float fm, float f, float fp) { return plm_slope(fm, f, fp); }
+__device__ __forceinline__ double plain_slope(double fm, double f, double fp) {
+  const double b = (fp - fm) * (fm + fp - 2. * f) > 0. ? f - fm : fp - f;
+  return f <= plain_min(fm, fp) || f >= plain_max(fm, fp) ? 0. : b;
+}
 // asynchronous global -> shared copy of B = 4, 8 or 16 bytes
 template <int B>
 __device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
@@ -864,15 +872,15 @@ __device__ __forceinline__ void lane_geo(int L, int lane, const R* xo, const R* 
     R nd = R(0), hh = R(0);
     if (lv.in(v) && !lv.first(v)) {
       const R d = flip ? (-xn[k]) - (-xo[k]) : xn[k] - xo[k];
-      const bool down = lt(d, R(0)), rise = lt(R(0), d);
-      if (down || rise) {
+      const bool rise = lt(R(0), d);
+      if (nonzero(d)) {
         const R fl = coord_thick(flip, xo, rise ? k : k - 1);
         if (lt(R(0), fl)) {
           const R dd = rise ? d : -d;
           const R dsl = cmin(fl, dd);
           const R dx = over(dsl, fl);
           const R hx = rise ? dx - R(1) : R(1) - dx;
-          if (lt(R(0), dsl)) {
+          if (nonzero(dsl)) {
             nd = -d;
             hh = R(.5) * hx;
           }
@@ -980,42 +988,51 @@ __device__ __forceinline__ bool pcwise_v(int L, int lane, R (&y)[NF][VL], const 
   bool bad = false;
 #pragma unroll
   for (int h = 0; h < NF; h++) {
-    // PLM slopes (zero in the end layers)
     const R ym = __shfl_up_sync(0xffffffffu, yf[h][VL - 1], 1, W);
     const R yp = __shfl_down_sync(0xffffffffu, yf[h][0], 1, W);
-    R bk[VL];
+    R after;
+    // slopes, fluxes and new values; plain: of values that are not finite
+    auto advect = [&](bool plain) {
+      // PLM slopes (zero in the end layers)
+      R bk[VL];
 #pragma unroll
-    for (int v = 0; v < VL; v++) {
-      const R fm = v > 0 ? yf[h][v - 1] : ym;
-      const R fp = v < VL - 1 ? yf[h][v + 1] : yp;
-      bk[v] = lv.in(v) && !lv.first(v) && !lv.last(v) ? plm_slope(fm, yf[h][v], fp) : R(0);
-    }
-    // interface fluxes; one donor layer: vertfx = -dz * (fcdx * slab) / slab = -dz * fcdx
-    const R bm = __shfl_up_sync(0xffffffffu, bk[VL - 1], 1, W);
-    R fl[VL];
-#pragma unroll
-    for (int v = 0; v < VL; v++) {
-      const bool up = (G.up >> v) & 1u;
-      const R a = up ? yf[h][v] : (v > 0 ? yf[h][v - 1] : ym);
-      const R b = up ? bk[v] : (v > 0 ? bk[v - 1] : bm);
-      fl[v] = G.nd[v] * (a + b * G.hh[v]);
-      if (sizeof(R) == 4 && G.nd[v] == R(0)) fl[v] = R(0);
-    }
-    const R fnext = __shfl_down_sync(0xffffffffu, fl[0], 1, W);
-    R after = R(0);
-#pragma unroll
-    for (int v = 0; v < VL; v++) {
-      if (lv.in(v)) {
-        const R vn = !lv.last(v) ? (v < VL - 1 ? fl[v + 1] : fnext) : R(0);
-        const R amount = yf[h][v] * G.fo[v] - (vn - fl[v]);
-        after += amount;
-        y[h][v] = (amount + yf[h][v] * small) * G.rfn[v];
+      for (int v = 0; v < VL; v++) {
+        const R fm = v > 0 ? yf[h][v - 1] : ym;
+        const R fp = v < VL - 1 ? yf[h][v + 1] : yp;
+        bk[v] = !lv.in(v) || lv.first(v) || lv.last(v) ? R(0)
+                : plain ? plain_slope(fm, yf[h][v], fp) : plm_slope(fm, yf[h][v], fp);
       }
-    }
-    if (sizeof(R) == 8) {
+      // interface fluxes; one donor layer: vertfx = -dz * (fcdx * slab) / slab = -dz * fcdx
+      const R bm = __shfl_up_sync(0xffffffffu, bk[VL - 1], 1, W);
+      R fl[VL];
+#pragma unroll
+      for (int v = 0; v < VL; v++) {
+        const bool up = (G.up >> v) & 1u;
+        const R a = up ? yf[h][v] : (v > 0 ? yf[h][v - 1] : ym);
+        const R b = up ? bk[v] : (v > 0 ? bk[v - 1] : bm);
+        // (nothing passes an interface that stays, whatever lies beside it)
+        fl[v] = G.nd[v] * (a + b * G.hh[v]);
+        if (plain && G.nd[v] == R(0)) fl[v] = R(0);
+      }
+      const R fnext = __shfl_down_sync(0xffffffffu, fl[0], 1, W);
+      after = R(0);
+#pragma unroll
+      for (int v = 0; v < VL; v++) {
+        if (lv.in(v)) {
+          const R vn = !lv.last(v) ? (v < VL - 1 ? fl[v + 1] : fnext) : R(0);
+          const R amount = yf[h][v] * G.fo[v] - (vn - fl[v]);
+          after += amount;
+          y[h][v] = (amount + yf[h][v] * small) * G.rfn[v];
+        }
+      }
+    };
+    advect(sizeof(R) == 4);
+    if constexpr (sizeof(R) == 8) {
       R dif = bfore[h] - after, scl = colscl[h];
       warp_sum2<R, W>(lane, dif, scl);
-      bad |= cabs(dif) > cmax(R(1.e-33), col_tol<R>(1.e-11) * scl);
+      bad |= cabs(dif) > floor_at(col_tol<R>(1.e-11) * scl, R(1.e-33));
+      // (the same in every lane of the column; the warp's columns go together)
+      if (__any_sync(0xffffffffu, f64_odd(dif))) advect(true);
     }
   }
   return bad;
