@@ -39,6 +39,15 @@ __device__ __forceinline__ float tenth(float x) {
 }
 __device__ __forceinline__ double tenth(double x) { return divide_by(x, 10., .1); }
 
+// x / cp, and the pressure that belongs to an Exner function value.  Every kernel
+// forms it here, so an interface that has not moved since the initial
+// adjustment or the last remap keeps its pressure bit for bit, and the layer
+// thicknesses keep summing to the column's mass.
+template <typename R>
+__device__ __forceinline__ R by_cp(R x) { return divide_by(x, R(kCp), R(1) / R(kCp)); }
+template <typename R>
+__device__ __forceinline__ R pressure_of(R ex) { return R(kP1000) * pow_cp_rd(by_cp(ex)); }
+
 constexpr int kColBlock = 128;
 constexpr int kBlock2 = 256;
 inline unsigned nblocks(long long n, int b) { return (unsigned)((n + b - 1) / b); }
@@ -612,7 +621,7 @@ __global__ void __launch_bounds__(kColBlock) k_remap(Grid<R> g, Strides s, Knobs
       exnew[L - k] = cmax(exold[L], exnew[L - k]);
     }
   }
-  for (int k = L; k >= 0; k--) prnew[k] = p1000 * pow(exnew[k] / cp, cp / rd);
+  for (int k = L; k >= 0; k--) prnew[k] = pressure_of(exnew[k]);
   for (int k = 0; k < L; k++) dpcol[k] = prnew[k] - prnew[k + 1];
   for (int k = 0; k <= L; k++) pk1new[k] = exnew[k] * prnew[k] / cp;
   prnew[L] = prcol[L];
@@ -814,9 +823,6 @@ struct RemapV {
 static_assert(sizeof(RemapV<float, 1, 1>) % 16 == 0 && sizeof(RemapV<double, 1, 1>) % 16 == 0 &&
                   sizeof(RemapV<float, 4, 2>) % 16 == 0,
               "ring slots of consecutive warps stay 16-byte aligned");
-
-template <typename R>
-__device__ __forceinline__ R by_cp(R x) { return divide_by(x, R(kCp), R(1) / R(kCp)); }
 
 // Level kb + v of a column of L levels held VL a lane by W lanes: with FULL the
 // column fills the lanes (L == W VL), so that the tests cost nothing but for
@@ -1213,7 +1219,7 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
   ex3d += m * s.intf; dp3d += m * s.cell; pr3d += m * s.intf;
   if (trdp) trdp += m * s.tr;
   const int its = sp->its - bnd;
-  const R p1000 = R(kP1000), small = R(1.e-6), sl = R(kn.slak);
+  const R small = R(1.e-6), sl = R(kn.slak);
   const bool fill = kn.thktop == 0.;  // remap_1d's fill of thin layers
   // hystat's floors of tracers 2 and 3 (hystat.F90:90-93) when trdp is formed here
   const R qvmin = R(kQvmin), qwmin = R(kQwmin);
@@ -1308,11 +1314,8 @@ __global__ void __launch_bounds__(32 * kWarpsRemapV) k_remap_v(Grid<R> g, Stride
                               cmin(R(.0001) * S.exold[hw][k - 1] + R(.9999) * S.exold[hw][k - 2], S.exnew[hw][k - 1]));
       __syncwarp();
       for (int k = ls; k <= L; k += WL) {
-        // the reference's own operations: the pressures of unmoved
-        // interfaces then reproduce the old ones exactly, so the layer
-        // thicknesses keep summing to the unchanged column mass
         const R en = S.exnew[hw][k];
-        const R pn = p1000 * pow_cp_rd(by_cp(en));
+        const R pn = pressure_of(en);
         S.prnew[hw][k] = pn;
         S.pk1new[hw][k] = by_cp(en * pn);
       }
@@ -2000,11 +2003,10 @@ __global__ void __launch_bounds__(kBlock2) k_prdp_from_ex(Grid<R> g, Strides s, 
   const int i = gid / L1, k = gid - i * L1;
   const size_t m = blockIdx.y;
   ex3d += m * s.intf; pr3d += m * s.intf; dp3d += m * s.cell;
-  const R cp = R(kCp), rd = R(kRd), p1000 = R(kP1000);
-  const R p = p1000 * pow(ex3d[(size_t)i * L1 + k] / cp, cp / rd);
+  const R p = pressure_of(ex3d[(size_t)i * L1 + k]);
   pr3d[(size_t)i * L1 + k] = p;
   if (k < L) {
-    const R pu = p1000 * pow(ex3d[(size_t)i * L1 + k + 1] / cp, cp / rd);
+    const R pu = pressure_of(ex3d[(size_t)i * L1 + k + 1]);
     dp3d[(size_t)i * L + k] = p - pu;
   }
 }
