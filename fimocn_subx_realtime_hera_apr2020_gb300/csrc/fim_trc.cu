@@ -354,6 +354,31 @@ struct CellItem {
   }
 };
 
+// The AB3 weights of the slot a launch writes (nf) and of those it reads (of,
+// vof).  Where a caller's slots are the same one (fim_set_ab takes any), the
+// weights of the slots that are nf's go to the new tendency, as trcadv1 and 3
+// read it after they set it, and trcadv2's limiters see no old one (trcadv1
+// clears it): a block never reads a slot that another is writing.
+template <typename R>
+struct Ab3 {
+  R now, old, very_old;
+  __device__ __forceinline__ explicit Ab3(const StepParams& p)
+      : now(p.w1<R>()), old(p.w2<R>()), very_old(p.w3<R>()) {
+    if (p.of == p.nf) {
+      now = now + old;
+      old = R(0);
+    }
+    if (p.vof == p.nf) {
+      now = now + very_old;
+      very_old = R(0);
+    }
+  }
+};
+template <typename R>
+__device__ __forceinline__ void zero_rows(R* p, int n) {
+  for (int q = threadIdx.x; q < n; q += blockDim.x) p[q] = R(0);
+}
+
 // One level of a cell as the routines write it, for items that hold a value
 // that is not finite (or, in FP64, a mass flux positive on both sides).
 // trcadv1's bounds of frame cell x: T the tracer's frame at that level.
@@ -462,7 +487,7 @@ __global__ void __launch_bounds__(64 * GC, sizeof(R) == 8 && VK == 1 ? 12 / GC :
   __syncthreads();
   const size_t NL = (size_t)N * L;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
-  const R ab1 = sp->template w1<R>(), ab2 = sp->template w2<R>(), ab3 = sp->template w3<R>();
+  const Ab3<R> ab(*sp);
   const R* mfn = massfx + m * s.mf + (size_t)nf * 6 * NL;
   const R* te0 = trc_edg + m * s.tredg;  // EV: tracer t's at t * 6 NL; else theta's (edgvar1)
   // this step's tracer t: its frame, and the patch cells' AB3 slots of/vof
@@ -473,8 +498,8 @@ __global__ void __launch_bounds__(64 * GC, sizeof(R) == 8 && VK == 1 ? 12 / GC :
     rp.copy(trs + b * ft.S2 * LK, tracr + m * s.tr + (size_t)t * NL + k0, fs, ft.SC, n2, lk, L);
     const R* tl = trl_tdcy + m * s.trab + (size_t)t * 3 * NL + k0;
     R* o = ops + b * 3 * ft.SC * LK;
-    rp.copy(o, tl + (size_t)of * NL, fs, ft.SC, C, lk, L);
-    rp.copy(o + ft.SC * LK, tl + (size_t)vof * NL, fs, ft.SC, C, lk, L);
+    if (of != nf) rp.copy(o, tl + (size_t)of * NL, fs, ft.SC, C, lk, L);
+    if (vof != nf) rp.copy(o + ft.SC * LK, tl + (size_t)vof * NL, fs, ft.SC, C, lk, L);
     rp.copy(o + 2 * ft.SC * LK, trcdp + m * s.tr + (size_t)t * NL + k0, fs, ft.SC, C, lk, L);
     stage_commit();
   };
@@ -483,6 +508,10 @@ __global__ void __launch_bounds__(64 * GC, sizeof(R) == 8 && VK == 1 ? 12 / GC :
   for (int it = threadIdx.x; it < (6 * C + nre) * GC; it += blockDim.x) {
     const int r = it / GC, v = (it - r * GC) * VK;
     if (v < lk) stage_copy<VK * (int)sizeof(R)>(MF + r * LK + v, mfn + fs.mfr[r] * L + k0 + v);
+  }
+  for (int b = 0; b < 2; b++) {  // rows that no copy fills
+    if (of == nf) zero_rows(ops + b * 3 * ft.SC * LK, ft.SC * LK);
+    if (vof == nf) zero_rows(ops + (b * 3 + 1) * ft.SC * LK, ft.SC * LK);
   }
   stage(t0, 0);
   CellItem<R, VK> ci;
@@ -605,7 +634,7 @@ __global__ void __launch_bounds__(64 * GC, sizeof(R) == 8 && VK == 1 ? 12 / GC :
     ldv<VK>(o + ft.SC * LK, tlv);
     ldv<VK>(o + 2 * ft.SC * LK, td);
     FOR_V {
-      const R lo = td[j] + ab1 * tn[j] + ab2 * tlo[j] + ab3 * tlv[j];
+      const R lo = td[j] + ab.now * tn[j] + ab.old * tlo[j] + ab.very_old * tlv[j];
       out[j] = tmax(hn[j], tmin(hx[j], quot(lo, ci.dp[j], ci.rdp[j])));
     }
     stv<VK>(trcr_lo + q, out);
@@ -748,8 +777,8 @@ __global__ void __launch_bounds__(64 * GC, VK * (int)sizeof(R) == 16 ? 8 / GC : 
   __syncthreads();
   const size_t NL = (size_t)N * L;
   const int nf = sp->nf, of = sp->of, vof = sp->vof;
-  const R ab1 = sp->template w1<R>(), ab2 = sp->template w2<R>(), ab3 = sp->template w3<R>();
-  const R rab1 = R(1) / ab1;  // Q+/Q- divide by ab1: one reciprocal
+  const Ab3<R> ab(*sp);
+  const R rab1 = R(1) / sp->template w1<R>();  // Q+/Q- divide by ab1: one reciprocal
   for (int x = threadIdx.x; x < n1; x += blockDim.x) arf[x] = g.area[fs.cells[x]] * (sizeof(R) == 8 ? rab1 : R(1));
   // the limiters' operands of tracer t0 + tz
   RowPlan<R, VK, GC> rp;
@@ -759,8 +788,8 @@ __global__ void __launch_bounds__(64 * GC, VK * (int)sizeof(R) == 16 ? 8 / GC : 
     rp.copy(TO, trold + so, fs, ft.SC, n2, lk, L);
     rp.copy(TL, trcr_lo + so, fs, ft.SC, n2, lk, L);
     const R* tc = trc_tdcy + m * s.trab + (size_t)(t0 + tz) * 3 * NL + k0;
-    rp.copy(opq, tc + (size_t)of * NL, fs, ft.SC, n1, lk, L);
-    rp.copy(opq + ft.S1 * LK, tc + (size_t)vof * NL, fs, ft.SC, n1, lk, L);
+    if (of != nf) rp.copy(opq, tc + (size_t)of * NL, fs, ft.SC, n1, lk, L);
+    if (vof != nf) rp.copy(opq + ft.S1 * LK, tc + (size_t)vof * NL, fs, ft.SC, n1, lk, L);
     rp.copy(opq + 2 * ft.S1 * LK, s_plus + so, fs, ft.SC, n1, lk, L);
     rp.copy(opq + 3 * ft.S1 * LK, s_mnus + so, fs, ft.SC, n1, lk, L);
     stage_commit();
@@ -782,6 +811,8 @@ __global__ void __launch_bounds__(64 * GC, VK * (int)sizeof(R) == 16 ? 8 / GC : 
     stage_commit();
   };
   stage_rows<R, VK, GC>(dpf, delp + m * s.cell + k0, fs.cells, n1, lk, L);
+  if (of == nf) zero_rows(opq, ft.S1 * LK);  // rows that no copy fills
+  if (vof == nf) zero_rows(opq + ft.S1 * LK, ft.S1 * LK);
   stage_lim(0);
   const int x = threadIdx.x / GC, v = (threadIdx.x - x * GC) * VK;
   const bool on = x < C && v < lk;
@@ -805,12 +836,12 @@ __global__ void __launch_bounds__(64 * GC, VK * (int)sizeof(R) == 16 ? 8 / GC : 
     // R+/R- of the thread's patch cell (its bounds and slots kept for
     // trcadv3), then of the ring-1 cells
     R hx[VK], hn[VK], tof[VK], tvf[VK];
-    if (on) limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, x, v, ab2, ab3, rab1, Rp, Rm, hx, hn, tof, tvf);
+    if (on) limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, x, v, ab.old, ab.very_old, rab1, Rp, Rm, hx, hn, tof, tvf);
     for (int it = threadIdx.x; it < (n1 - C) * GC; it += blockDim.x) {
       const int xe = C + it / GC, ve = (it % GC) * VK;
       if (ve >= lk) continue;
       R mx2[VK], mn2[VK], tof2[VK], tvf2[VK];
-      limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, xe, ve, ab2, ab3, rab1, Rp, Rm, mx2, mn2, tof2, tvf2);
+      limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, xe, ve, ab.old, ab.very_old, rab1, Rp, Rm, mx2, mn2, tof2, tvf2);
     }
     stage_wait();
     __syncthreads();
@@ -852,7 +883,7 @@ __global__ void __launch_bounds__(64 * GC, VK * (int)sizeof(R) == 16 ? 8 / GC : 
     stv<VK>(trc_tdcy + m * s.trab + (size_t)t * 3 * NL + (size_t)nf * NL + c, tn);
     const size_t ob = m * out.mstride + (size_t)(t - out.tbase) * NL + c;
     FOR_V {
-      tdv[j] = tdv[j] + ab1 * tn[j] + ab2 * tof[j] + ab3 * tvf[j];
+      tdv[j] = tdv[j] + ab.now * tn[j] + ab.old * tof[j] + ab.very_old * tvf[j];
       const R q = sizeof(R) == 8 ? quot(tdv[j], dpk[j], rdp[j]) : fdiv(tdv[j], tmax(R(1.e-11), dp[j]));
       res[j] = tmax(hn[j], tmin(hx[j], q));
     }
