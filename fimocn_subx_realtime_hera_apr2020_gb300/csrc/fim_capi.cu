@@ -243,15 +243,19 @@ int index_tables(const fim_grid_desc* g, std::vector<int>& prox, std::vector<int
   return FIM_OK;
 }
 
-// The cell patches of the fused tracer kernels: 8 x 8 cells of a rhombus,
-// with the frame tables uploaded once per context.
+// The cell patches of the tracer and edge kernels: 8 x 8 cells of a rhombus,
+// with the frame tables uploaded once per context.  A pentagon's sixth prox
+// entry, which no edge uses but the one-ring bounds read, may be any cell: it
+// joins the frames of a context without high-order fluxes; the fused transport
+// takes the grids whose frames hold it already.
 int build_patches(fim_ctx* c, const std::vector<int>& prox, const std::vector<int>& proxs,
                   const std::vector<int>& nprox) {
   FrameHost h;
-  int side = 8;
-  while (build_frames(c->N, prox.data(), proxs.data(), nprox.data(), side, &h) != 0) {
-    if (--side < 1) return set_err(c, FIM_EINVAL, "tracer patches: a frame exceeds 255 cells");
-  }
+  int side = 8, bad;
+  while ((bad = build_frames(c->N, prox.data(), proxs.data(), nprox.data(), side, &h, !c->kn.hi_order)) != 0)
+    if (--side < 1)
+      return set_err(c, FIM_EINVAL, bad == 3 ? "tracer patches: a pentagon's sixth prox entry is not around it"
+                                             : "tracer patches: a frame exceeds 255 cells");
   FrameTab& f = c->ftab;
   std::vector<unsigned char> tab;
   pack_frames(h, nprox.data(), &f, &tab);
@@ -263,16 +267,24 @@ int build_patches(fim_ctx* c, const std::vector<int>& prox, const std::vector<in
   if ((rc = dalloc(c, &p, h.cnt.size() * sizeof(int)))) return rc;
   CK(cudaMemcpy(p, h.cnt.data(), h.cnt.size() * sizeof(int), cudaMemcpyHostToDevice), "patch counts");
   f.cnt = (const int4*)p;
-  if ((rc = dalloc(c, &p, (size_t)f.ntile * f.cstride * c->esz))) return rc;
-  f.coef = p;
-  // the kernel runs on the context's (non-blocking) stream: the table copies
+  // the kernels run on the context's (non-blocking) stream: the table copies
   // above have to be on the device
   CK(cudaStreamSynchronize(0), "patch tables");
-  if (c->prec == FIM_PREC_F64) launch_patch_coefs<double>(c->stream, c->gd, f, (double*)p);
-  else launch_patch_coefs<float>(c->stream, c->gf, f, (float*)p);
-  CK(cudaGetLastError(), "patch coefficients");
-  // the first kernels to read them may run on another stream
-  CK(cudaStreamSynchronize(c->stream), "patch coefficients");
+  // what forms edge values on chip reads the coefficients: the fused transport
+  // and the FP32 edgvar3
+  if (c->kn.hi_order || c->prec == FIM_PREC_F32) {
+    if ((rc = dalloc(c, &p, (size_t)f.ntile * f.cstride * c->esz))) return rc;
+    f.coef = p;
+    if (c->prec == FIM_PREC_F64) launch_patch_coefs<double>(c->stream, c->gd, f, (double*)p);
+    else launch_patch_coefs<float>(c->stream, c->gf, f, (float*)p);
+    CK(cudaGetLastError(), "patch coefficients");
+    // the first kernels to read them may run on another stream
+    CK(cudaStreamSynchronize(c->stream), "patch coefficients");
+  }
+  if (c->prec == FIM_PREC_F32) {
+    const int e = prepare_edges<float>(f);
+    if (e) return set_err(c, FIM_ECUDA, "edge kernel attributes", (cudaError_t)e);
+  }
   return FIM_OK;
 }
 
@@ -1543,7 +1555,6 @@ int fim_ctx_create(const fim_grid_desc* g, const fim_config* cfg, fim_ctx** out)
   if (!rc && c->prec == FIM_PREC_F32)
     rc = build_grid<float>(c, g, rarea, corio, grnd, dfflen, biharw, smoo, prox, proxs, nprox);
   if (!rc) rc = build_patches(c, prox, proxs, nprox);
-  if (!rc && c->prec == FIM_PREC_F32 && prepare_edges<float>(c->ftab)) rc = FIM_ECUDA;
   if (!rc) rc = dalloc(c, (void**)&c->d_sp, sizeof(StepParams) * c->M);
   if (!rc) rc = dalloc(c, (void**)&c->d_flags, sizeof(int) * c->M);
   if (!rc) {

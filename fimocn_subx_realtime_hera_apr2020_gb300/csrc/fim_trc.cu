@@ -1096,7 +1096,7 @@ void launch_edges_patch(const Launch& l, const Grid<R>& g, const Strides& s, con
 
 // ---- cell patches ---------------------------------------------------------
 
-int build_frames(int N, const int* prox, const int* proxs, const int* nprox, int side, FrameHost* F) {
+int build_frames(int N, const int* prox, const int* proxs, const int* nprox, int side, FrameHost* F, bool sixth) {
   if (side < 1 || side > 8) return 1;
   std::vector<std::vector<int>> tiles;
   // the reference's IJ numbering: north pole, 10 rhombi of sl x sl cells in
@@ -1160,7 +1160,7 @@ int build_frames(int N, const int* prox, const int* proxs, const int* nprox, int
       std::vector<int> add;
       for (int x = lo; x < hi; x++) {
         const int c = f.cells[x];
-        for (int e = 0; e < nprox[c]; e++) {
+        for (int e = 0; e < (sixth ? 6 : nprox[c]); e++) {
           const int n = prox[c * 6 + e];
           if (loc[n] == -1) { loc[n] = -2; add.push_back(n); }
         }
