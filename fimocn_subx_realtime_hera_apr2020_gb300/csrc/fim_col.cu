@@ -31,14 +31,6 @@ __device__ __forceinline__ bool nonzero(float a) { return a != 0.f; }
 __device__ __forceinline__ bool nonzero(double a) { return (__double_as_longlong(a) << 1) != 0ll; }
 __device__ __forceinline__ double cmax(double a, double b) { return lt(b, a) ? a : b; }
 __device__ __forceinline__ double cmin(double a, double b) { return lt(a, b) ? a : b; }
-// x / 10, rounded as the division (Markstein's correction; for this divisor the
-// rounded reciprocal gives the rounded quotient for every FP32 mantissa)
-__device__ __forceinline__ float tenth(float x) {
-  const float q = x * .1f;
-  return fmaf(fmaf(-10.f, q, x), .1f, q);
-}
-__device__ __forceinline__ double tenth(double x) { return divide_by(x, 10., .1); }
-
 // x / cp, and the pressure that belongs to an Exner function value.  Every kernel
 // forms it here, so an interface that has not moved since the initial
 // adjustment or the last remap keeps its pressure bit for bit, and the layer

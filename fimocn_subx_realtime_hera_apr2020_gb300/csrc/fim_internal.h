@@ -343,7 +343,9 @@ inline int pick_vk(int L, std::initializer_list<const void*> ptrs, int want = 0)
 // ones), so the FP64 build is bound by its FP64 operations.  Comparisons run
 // on the integer pipe (a double's bits, the magnitude of negative values
 // complemented, order as int64), reciprocals and powers by few steps from the
-// hardware's FP32-accurate approximations.
+// hardware's approximations (good to 2^-19).  Error bounds are relative and in
+// units of 2^-53, half a last place at most; tests/test_f64_arithmetic_gpu.py
+// holds each against 113-bit arithmetic.
 __device__ __forceinline__ long long f64_key(double x) {
   const long long b = __double_as_longlong(x);
   return b ^ ((b >> 63) & 0x7fffffffffffffffll);
@@ -361,8 +363,9 @@ __device__ __forceinline__ bool f64_lt(double a, double b) {
   const long long x = f64_key(a), y = f64_key(b);
   return x < y && (int)(y >> 32) <= 0x7ff00000 && (int)(x >> 32) >= (int)0x800fffff;
 }
-// 1 / b, b normal and below 2^1000: one third-order step from the
-// approximation (its error cubed is below rounding)
+// 1 / b, 2^-1000 < |b| < 2^1000: the approximation r and its residual e = 1 - b r
+// in the geometric series of 1 / (1 - e) to e^2 (the hyperpower iteration of
+// order three); the last rounding and e^3, 1.1 units
 __device__ __forceinline__ double f64_recip(double b) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
@@ -395,9 +398,18 @@ __device__ __forceinline__ float divide(float a, float b) { return a / b; }
 // the limiters' quotient: FP32 by the reciprocal
 __device__ __forceinline__ float quot(float a, float, float rb) { return a * rb; }
 __device__ __forceinline__ double quot(double a, double b, double rb) { return divide_by(a, b, rb); }
-// 1 / sqrt(x), x normal: one third-order step r (1 + e/2 + 3 e^2/8)
+// 1 / sqrt(x), x normal: the approximation r and e = 1 - x r^2 in the binomial
+// series of (1 - e)^(-1/2) to e^2 (an iteration of order three); 1.6 units,
+// where a root and a division have 2
 __device__ __forceinline__ double f64_rsqrt(double x) {
   double r;
+// x / 10, rounded as the division (Markstein's correction from the rounded
+// reciprocal)
+__device__ __forceinline__ float tenth(float x) {
+  const float q = x * .1f;
+  return fmaf(fmaf(-10.f, q, x), .1f, q);
+}
+__device__ __forceinline__ double tenth(double x) { return divide_by(x, 10., .1); }
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
   const double e = fma(-(x * r), r, 1.);
   return fma(r, e * fma(.375, e, .5), r);
@@ -422,8 +434,8 @@ __device__ __forceinline__ double f64_ln13(double x) {
 // x^(cp/rd) and x^(rd/cp), the Exner function's powers.  cp/rd = 3.5 + d and
 // rd/cp = 2/7 + d' with |d| < 1e-4, |d'| < 1e-5, so the root is taken by
 // Newton-type steps with its rounding kept in a second term, and x^d =
-// exp(d ln x) needs ln x to 1e-12 only.  About 40 FP64 operations and within
-// an ulp of the rounded power, where pow takes several times as many.
+// exp(d ln x) needs ln x to 1e-12 only.  About 40 FP64 operations, 1.2 and 2.6
+// units (pow: 2 last places), where pow takes several times as many.
 __device__ __forceinline__ double f64_expm1_small(double y) {  // |y| < 2e-3
   return fma(y * y, fma(y, fma(y, 1. / 24., 1. / 6.), .5), y);
 }
