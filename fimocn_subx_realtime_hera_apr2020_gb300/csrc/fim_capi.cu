@@ -282,7 +282,7 @@ int build_patches(fim_ctx* c, const std::vector<int>& prox, const std::vector<in
     CK(cudaStreamSynchronize(c->stream), "patch coefficients");
   }
   if (c->prec == FIM_PREC_F32) {
-    const int e = prepare_edges<float>(f);
+    const int e = prepare_edges(f);
     if (e) return set_err(c, FIM_ECUDA, "edge kernel attributes", (cudaError_t)e);
   }
   return FIM_OK;

@@ -730,7 +730,7 @@ __device__ __forceinline__ double plm_slope(double fm, double f, double fp) {
   const bool rise = km < k && k < kp, fall = km > k && k > kp;
   if (!rise && !fall) return 0.;
   const double c = fma(-2., f, fm + fp);
-  const bool lower = c != 0. && f64_neg(c) == fall;
+  const bool lower = c != 0. && negative(c) == fall;
   return (lower ? f : fp) - (lower ? fm : f);
 }
 // the slope as pcwise writes it, for values that are not finite
@@ -1539,12 +1539,6 @@ inline int remap_vl(int L) { return L <= 32 ? 1 : L <= 64 ? 2 : 4; }
 template <typename R>
 inline bool remap_paired(int L) { return sizeof(R) == 4 && L > 32 && L <= 64; }
 
-inline int sm_count() {
-  int dev = 0, sms = 152;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 // Columns a warp of k_remap_v takes in turn.  Many columns a warp amortise its
 // start (the first copies, the theta sweep); few leave small grids no nearly
 // empty last round of blocks.  FP64 (two blocks an SM by shared memory): the
@@ -1552,7 +1546,8 @@ inline int sm_count() {
 // glvl 6 / nvl 64 (8 columns 3.07 ms, 6: 2.81, 4: 2.90, 2: 2.98) and glvl 5 / nvl 38
 // (6: 0.59, 4: 0.60, 2: 0.55).  FP32: all blocks of a small grid are resident and
 // share their SM, blocks an SM times (columns + 3): glvl 5 / nvl 38 8: 62 us,
-// 6: 51, 4: 69; glvl 8 / nvl 64 8: 2.95 ms, 6: 3.01, 4: 3.12.
+// 6: 51, 4: 69; glvl 8 / nvl 64 8: 2.95 ms, 6: 3.01, 4: 3.12.  (Two columns a warp
+// would be taken by grids of a few hundred columns alone.)
 template <typename R>
 int remap_columns(int N, int members, bool paired) {
   const int sms = sm_count();
@@ -1796,8 +1791,9 @@ constexpr int kGsGroup = 7;
 // small grids.  (A block's reduction takes ~60 FP64 operations a warp, so many
 // short blocks cost more than an idle SM: glvl 5 / nvl 38, one level a thread:
 // 760 blocks of two iterations 33 us, 380 of four 21 us.)
-// A function of the grid alone: the sums do not depend on the tracers or
-// members beside them.
+// A function of the grid alone, the blocks a constant (1.5 of 152 SMs): the
+// order of the sums depends on neither the tracers or members beside them nor
+// the device.
 inline int gs_iters(long long NL, int vk) {
   int it = 16;
   while (it > 1 && NL / ((long long)kBlock2 * vk * it) < 228) it /= 2;

@@ -32,10 +32,6 @@ __device__ __forceinline__ bool cell_level(int N, int L, int& i, int& k) {
 
 inline unsigned blocks_for(long long n, int b = kBlock) { return (unsigned)((n + b - 1) / b); }
 
-// 1 / sqrt(x) of a squared speed
-__device__ __forceinline__ float inv_root(float x) { return rsqrtf(x); }
-__device__ __forceinline__ double inv_root(double x) { return f64_rsqrt(x); }
-
 // |(a, b)|: IEEE sqrt in FP64; x * rsqrt(x) in FP32, a few ulp from the
 // rounded root and about a third of its instructions
 __device__ __forceinline__ double vmag(double a, double b) { return sqrt(a * a + b * b); }
@@ -150,7 +146,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_edgvar1(Grid<R> g, Strides s, int
           vn = two * vn + cs[2] * vt - sn[2] * ut + cs[3] * vl - sn[3] * ul;
           const R sq = un * un + vn * vn;
           const R ms = w[0] * m0[j] + w[1] * mx[e][j] + w[2] * FIM_TRAIL(mx) + w[3] * FIM_LEAD(mx);
-          const R q = ms * (f64_lt(sq, R(36) * eps * eps) ? R(1) / (R(6) * eps) : inv_root(sq));
+          const R q = ms * (f64_lt(sq, R(36) * eps * eps) ? R(1) / (R(6) * eps) : f64_rsqrt(sq));
           ue[j] = un * q;
           ve[j] = vn * q;
         } else {
@@ -1401,20 +1397,21 @@ void launch_edgvar1(const Launch& l, const Grid<R>& g, const Strides& s, int hi_
 template <typename R>
 void launch_edgvar3(const Launch& l, const Grid<R>& g, const Strides& s, const R* delp, const R* tracr,
                     R* dp_edg, R* trc_edg, int nfields, const FrameTab& ft, bool average) {
-  if (sizeof(R) == 4 && average) {
-    launch_edges_patch<R>(l, g, s, ft, nfields, delp, tracr, dp_edg, trc_edg);
-    return;
+  if constexpr (sizeof(R) == 4) {
+    if (average) return launch_edges_patch(l, g, s, ft, nfields, delp, tracr, dp_edg, trc_edg);
   }
   const int vk = pick_vk<R>(g.L, {delp, tracr, dp_edg, trc_edg});
   FIM_KBEGIN(l, "k_edgvar3_own");
   FIM_VK_DISPATCH(R, vk, (k_edgvar3_own<R, VK><<<dim3(blocks_for((long long)g.N * (g.L / VK)), l.members, nfields),
                                                  kBlock, 0, l.stream>>>(g, s, delp, tracr, dp_edg, trc_edg)));
   FIM_KEND(l);
-  if (!average) return;
-  FIM_KBEGIN(l, "k_edgvar3_avg");
-  FIM_VK_DISPATCH(R, vk, (k_edgvar3_avg<R, VK><<<dim3(blocks_for((long long)g.N * (g.L / VK)), l.members, nfields),
-                                                 kBlock, 0, l.stream>>>(g, s, dp_edg, trc_edg)));
-  FIM_KEND(l);
+  if constexpr (sizeof(R) == 8) {
+    if (!average) return;
+    FIM_KBEGIN(l, "k_edgvar3_avg");
+    FIM_VK_DISPATCH(R, vk, (k_edgvar3_avg<R, VK><<<dim3(blocks_for((long long)g.N * (g.L / VK)), l.members, nfields),
+                                                   kBlock, 0, l.stream>>>(g, s, dp_edg, trc_edg)));
+    FIM_KEND(l);
+  }
 }
 
 template <typename R>

@@ -323,6 +323,13 @@ inline int pick_vk(int L, std::initializer_list<const void*> ptrs, int want = 0)
   return vk;
 }
 
+// streaming multiprocessors of the current device
+inline int sm_count() {
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 // run CALL with the compile-time constant VK equal to vk (4 only for float)
 #define FIM_VK_DISPATCH(R, vk, CALL)                          \
   do {                                                        \
@@ -350,7 +357,6 @@ __device__ __forceinline__ long long f64_key(double x) {
   const long long b = __double_as_longlong(x);
   return b ^ ((b >> 63) & 0x7fffffffffffffffll);
 }
-__device__ __forceinline__ bool f64_neg(double x) { return __double2hiint(x) < 0; }
 // by the upper word: a NaN (quiet, as all arithmetic makes them); an infinity
 // or a NaN; negative and no NaN
 __device__ __forceinline__ bool f64_nan(double x) { return (__double2hiint(x) & 0x7fffffff) > 0x7ff00000; }
@@ -373,7 +379,7 @@ __device__ __forceinline__ double f64_recip(double b) {
   return fma(r, fma(e, e, e), r);
 }
 // a / b with rb = 1 / b: the product and one residual correction (Markstein),
-// correctly rounded but for rare last-bit cases (finite results)
+// the division's result but for quotients next to half-way between two doubles
 __device__ __forceinline__ double f64_quot(double a, double b, double rb) {
   const double q = a * rb;
   return fma(fma(-b, q, a), rb, q);
@@ -395,6 +401,13 @@ __device__ __forceinline__ double divide_by(double a, double b, double rb) {
 __device__ __forceinline__ float divide_by(float a, float b, float) { return a / b; }
 __device__ __forceinline__ double divide(double a, double b) { return divide_by(a, b, recip(b)); }
 __device__ __forceinline__ float divide(float a, float b) { return a / b; }
+// x / 10, rounded as the division (Markstein's correction from the rounded
+// reciprocal)
+__device__ __forceinline__ float tenth(float x) {
+  const float q = x * .1f;
+  return fmaf(fmaf(-10.f, q, x), .1f, q);
+}
+__device__ __forceinline__ double tenth(double x) { return divide_by(x, 10., .1); }
 // the limiters' quotient: FP32 by the reciprocal
 __device__ __forceinline__ float quot(float a, float, float rb) { return a * rb; }
 __device__ __forceinline__ double quot(double a, double b, double rb) { return divide_by(a, b, rb); }
@@ -403,13 +416,6 @@ __device__ __forceinline__ double quot(double a, double b, double rb) { return d
 // where a root and a division have 2
 __device__ __forceinline__ double f64_rsqrt(double x) {
   double r;
-// x / 10, rounded as the division (Markstein's correction from the rounded
-// reciprocal)
-__device__ __forceinline__ float tenth(float x) {
-  const float q = x * .1f;
-  return fmaf(fmaf(-10.f, q, x), .1f, q);
-}
-__device__ __forceinline__ double tenth(double x) { return divide_by(x, 10., .1); }
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
   const double e = fma(-(x * r), r, 1.);
   return fma(r, e * fma(.375, e, .5), r);
@@ -741,11 +747,9 @@ void launch_edgvar3(const Launch&, const Grid<R>&, const Strides&, const R* delp
 // edgvar3 with the two-sided average on cell patches (fim_trc.cu; FP32: the
 // FP64 build is bound by its FP64 operations, which recomputing the ring
 // cells' sides would add to); prepare_edges: its one-time launch attributes
-template <typename R>
 int prepare_edges(const FrameTab& ft);
-template <typename R>
-void launch_edges_patch(const Launch&, const Grid<R>&, const Strides&, const FrameTab&, int nfields, const R* delp,
-                        const R* tracr, R* dp_edg, R* trc_edg);
+void launch_edges_patch(const Launch&, const Grid<float>&, const Strides&, const FrameTab&, int nfields,
+                        const float* delp, const float* tracr, float* dp_edg, float* trc_edg);
 // packs the patches' tables as FrameTab describes and sets its sizes and
 // offsets (not its pointers); edge-value rows of cells and slots follow proxs
 void pack_frames(const FrameHost& f, const int* nprox, FrameTab* tab, std::vector<unsigned char>* out);

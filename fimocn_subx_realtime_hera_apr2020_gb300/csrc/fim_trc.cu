@@ -981,7 +981,7 @@ void edges_launch(const Launch& l, const Grid<R>& g, const Strides& s, const Fra
   constexpr int GC = 4, LK = VK * GC;
   const unsigned nb = (unsigned)(ft.ntile * ((g.L + LK - 1) / LK));
   // enough blocks for two waves of three an SM, at most one field a block
-  const unsigned want = 912u / (nb * l.members) + 1u;
+  const unsigned want = 6u * (unsigned)sm_count() / (nb * l.members) + 1u;
   const unsigned nz = want < (unsigned)nfields ? want : (unsigned)nfields;
   k_edgvar3_patch<R, VK, GC><<<dim3(nb, l.members, nz), ft.SC * GC, PatchLayout::edges<R>(ft, LK).bytes, l.stream>>>(
       g, s, ft, nfields, delp, tracr, dp_edg, trc_edg);
@@ -1072,26 +1072,19 @@ int prepare_one(const FrameTab& ft) {
 
 }  // namespace
 
-template <typename R>
 int prepare_edges(const FrameTab& ft) {
-  cudaError_t e = cudaSuccess;
-  if constexpr (sizeof(R) == 4) {
-    e = allow_smem(k_edgvar3_patch<R, 1, 4>, PatchLayout::edges<R>(ft, 4).bytes);
-    if (e == cudaSuccess) e = allow_smem(k_edgvar3_patch<R, 2, 4>, PatchLayout::edges<R>(ft, 8).bytes);
-    if (e == cudaSuccess) e = allow_smem(k_edgvar3_patch<R, 4, 4>, PatchLayout::edges<R>(ft, 16).bytes);
-  }
+  cudaError_t e = allow_smem(k_edgvar3_patch<float, 1, 4>, PatchLayout::edges<float>(ft, 4).bytes);
+  if (e == cudaSuccess) e = allow_smem(k_edgvar3_patch<float, 2, 4>, PatchLayout::edges<float>(ft, 8).bytes);
+  if (e == cudaSuccess) e = allow_smem(k_edgvar3_patch<float, 4, 4>, PatchLayout::edges<float>(ft, 16).bytes);
   return (int)e;
 }
 
-template <typename R>
-void launch_edges_patch(const Launch& l, const Grid<R>& g, const Strides& s, const FrameTab& ft, int nfields,
-                        const R* delp, const R* tracr, R* dp_edg, R* trc_edg) {
-  if constexpr (sizeof(R) == 4) {
-    const int vk = pick_vk<R>(g.L, {delp, tracr, dp_edg, trc_edg});
-    FIM_KBEGIN(l, "k_edgvar3_patch");
-    FIM_VK_DISPATCH(R, vk, (edges_launch<R, VK>(l, g, s, ft, nfields, delp, tracr, dp_edg, trc_edg)));
-    FIM_KEND(l);
-  }
+void launch_edges_patch(const Launch& l, const Grid<float>& g, const Strides& s, const FrameTab& ft, int nfields,
+                        const float* delp, const float* tracr, float* dp_edg, float* trc_edg) {
+  const int vk = pick_vk<float>(g.L, {delp, tracr, dp_edg, trc_edg});
+  FIM_KBEGIN(l, "k_edgvar3_patch");
+  FIM_VK_DISPATCH(float, vk, (edges_launch<float, VK>(l, g, s, ft, nfields, delp, tracr, dp_edg, trc_edg)));
+  FIM_KEND(l);
 }
 
 // ---- cell patches ---------------------------------------------------------
@@ -1374,9 +1367,6 @@ int tune_tracers(const Launch& l, const Grid<R>& g, const Strides& s, const TrcF
                                         const TrcFusedScratch<R>&, R*, R*, R*, R*, R*, const R*, const R*,   \
                                         const ChunkHook*);                                                    \
   template void launch_patch_coefs<R>(cudaStream_t, const Grid<R>&, const FrameTab&, R*);                     \
-  template int prepare_edges<R>(const FrameTab&);                                                             \
-  template void launch_edges_patch<R>(const Launch&, const Grid<R>&, const Strides&, const FrameTab&, int,   \
-                                      const R*, const R*, R*, R*);                                           \
   template int prepare_tracers<R>(const FrameTab&);                                                           \
   template int tune_tracers<R>(const Launch&, const Grid<R>&, const Strides&, const TrcFusedScratch<R>&, R*, \
                                R*, R*, R*, R*, const R*, const R*, int*, int*, float*);
