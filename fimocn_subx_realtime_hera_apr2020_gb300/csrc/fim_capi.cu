@@ -303,13 +303,15 @@ int build_grid(fim_ctx* c, const fim_grid_desc* g, const std::vector<double>& ra
   { const R* t_; if ((rc = upload_conv<R>(c, g->cs, (size_t)N * 24, &t_))) return rc; G.cs = t_; }
   { const R* t_; if ((rc = upload_conv<R>(c, g->sn, (size_t)N * 24, &t_))) return rc; G.sn = t_; }
   G.vw = nullptr;
-  if (sizeof(R) == 8 && c->prec == FIM_PREC_F64) {
-    // on the stream of the table copies, before build_patches waits for it
-    void* p;
-    if ((rc = dalloc(c, &p, (size_t)N * 24 * sizeof(R)))) return rc;
-    launch_speed_weights<R>(0, N, G.cs, G.sn, (R*)p);
-    CK(cudaGetLastError(), "speed weights");
-    G.vw = (const R*)p;
+  if constexpr (sizeof(R) == 8) {
+    if (c->prec == FIM_PREC_F64) {
+      // on the stream of the table copies, before build_patches waits for it
+      void* p;
+      if ((rc = dalloc(c, &p, (size_t)N * 24 * sizeof(double)))) return rc;
+      launch_speed_weights(0, N, G.cs, G.sn, (double*)p);
+      CK(cudaGetLastError(), "speed weights");
+      G.vw = (const double*)p;
+    }
   }
   { const R* t_; if ((rc = upload_conv<R>(c, g->sidevec_c, (size_t)N * 12, &t_))) return rc; G.svc = t_; }
   { const R* t_; if ((rc = upload_conv<R>(c, g->sidevec_e, (size_t)N * 12, &t_))) return rc; G.sve = t_; }

@@ -243,17 +243,15 @@ __global__ void __launch_bounds__(kBlock, 4) k_edgvar1(Grid<R> g, Strides s, int
 
 // g.vw; the first square's rounding is kept, so exact rotations give 1 / 3 and
 // 1 / 6 to the last bit
-template <typename R>
-__global__ void __launch_bounds__(kBlock) k_speed_weights(int n, const R* __restrict__ cs, const R* __restrict__ sn,
-                                                          R* __restrict__ vw) {
+__global__ void __launch_bounds__(kBlock) k_speed_weights(int n, const double* __restrict__ cs,
+                                                          const double* __restrict__ sn, double* __restrict__ vw) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
-  const R a = cs[q], b = sn[q], aa = a * a;
-  vw[q] = sqrt((fma(b, b, aa) + fma(a, a, -aa)) / R((q & 3) < 2 ? 9 : 36));
+  const double a = cs[q], b = sn[q], aa = a * a;
+  vw[q] = sqrt((fma(b, b, aa) + fma(a, a, -aa)) / ((q & 3) < 2 ? 9. : 36.));
 }
-template <typename R>
-void launch_speed_weights(cudaStream_t stream, int N, const R* cs, const R* sn, R* vw) {
-  k_speed_weights<R><<<blocks_for((long long)N * 24), kBlock, 0, stream>>>(N * 24, cs, sn, vw);
+void launch_speed_weights(cudaStream_t stream, int N, const double* cs, const double* sn, double* vw) {
+  k_speed_weights<<<blocks_for((long long)N * 24), kBlock, 0, stream>>>(N * 24, cs, sn, vw);
 }
 
 // --------------------------------------------------------------------------
@@ -1530,7 +1528,6 @@ void launch_step_begin(const Launch& l, StepParams* sp) {
 }
 
 #define INSTANTIATE(R)                                                                                          \
-  template void launch_speed_weights<R>(cudaStream_t, int, const R*, const R*, R*);                           \
   template void launch_edgvar1<R>(const Launch&, const Grid<R>&, const Strides&, int, const R*, const R*,      \
                                   const R*, const R*, const R*, const R*, R*, R*, R*, R*, R*, R*, R*,          \
                                   const float2*, R*);                                                         \

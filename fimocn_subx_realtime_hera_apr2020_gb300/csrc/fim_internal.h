@@ -660,8 +660,7 @@ __device__ __forceinline__ float ff_diff(float2 x, float2 y) {
 // mpf (FP32-mixed step only, may be null): float-float copy (hi, lo) of the
 // Montgomery potential; mont_edg then holds the edge value minus the cell value.
 // fills Grid::vw on the device (N cells)
-template <typename R>
-void launch_speed_weights(cudaStream_t stream, int N, const R* cs, const R* sn, R* vw);
+void launch_speed_weights(cudaStream_t stream, int N, const double* cs, const double* sn, double* vw);
 template <typename R>
 void launch_edgvar1(const Launch&, const Grid<R>&, const Strides&, int hi_order, const R* u,
                     const R* v, const R* delp, const R* pres, const R* montg, const R* tracr,
