@@ -23,7 +23,7 @@
 // The per-routine trcadv runs the same two kernels with the caller's edge
 // values (EV): 38 words a cell-level and tracer at 16-byte accesses where one
 // thread a cell-level took about 60 at 4 (glvl 7, nvl 64, 11 tracers, FP32:
-// 8.04 -> 2.93 ms; FP64, glvl 5, nvl 37, 5 tracers: 0.82 -> 0.52 ms).
+// 8.04 -> 2.95 ms; FP64, glvl 5, nvl 37, 5 tracers: 0.82 -> 0.43 ms).
 //
 // The edge values (six per cell-level and tracer) and R+/R- never reach HBM:
 // per cell-level and tracer the pair reads and writes 32 words (10 of them
@@ -399,8 +399,8 @@ __device__ __forceinline__ UpDown<R> plain_bounds(const R* T, uint2 nb, int x) {
 // entries; anti: its antidiffusive fluxes (stride L)
 template <typename R> struct LoItem { R sum, sp, sm, hx, hn; };
 template <typename R, int LK>
-__device__ __noinline__ LoItem<R> plain_lo(const R* T, const R* MF, const R* E, const R* te,
-                                           const unsigned short* mir, uint2 nb, int x, int np, int L, R* anti) {
+__device__ __forceinline__ LoItem<R> plain_lo(const R* T, const R* MF, const R* E, const R* te,
+                                              const unsigned short* mir, uint2 nb, int x, int np, int L, R* anti) {
   const UpDown<R> b = plain_bounds<R, LK>(T, nb, x);
   LoItem<R> w{R(0), R(0), R(0), b.up, b.down};
   const R tri = T[x * LK];
@@ -416,6 +416,13 @@ __device__ __noinline__ LoItem<R> plain_lo(const R* T, const R* MF, const R* E, 
     anti[e * L] = a;
   }
   return w;
+}
+// the same as a call: at 16 bytes of levels a thread k_trf_lo is 1% faster with it,
+// at 8 it is 6% slower (glvl 5 / nvl 38 / 5 tracers 59.7 against 63.6 us)
+template <typename R, int LK>
+__device__ __noinline__ LoItem<R> plain_lo_call(const R* T, const R* MF, const R* E, const R* te,
+                                                const unsigned short* mir, uint2 nb, int x, int np, int L, R* anti) {
+  return plain_lo<R, LK>(T, MF, E, te, mir, nb, x, np, L, anti);
 }
 
 // bounds and limiters of frame cell x in trcadv2 (ar: the cell's area, in FP64
@@ -447,7 +454,8 @@ __device__ __noinline__ LimItem<R> plain_limits(const R* TO, const R* TL, uint2 
 //
 // Two blocks an SM at GC 4, the shared memory's limit with 16-byte rows a
 // thread.  FP64 at one level a thread takes the three that fit then (80
-// registers: glvl 5 / nvl 37 / 5 tracers 273 -> 257 us); FP32 at two levels a
+// registers: glvl 5 / nvl 37 / 5 tracers 273 -> 257 us when chosen, 184 us with
+// the present flux arithmetic); FP32 at two levels a
 // thread is slower there (59 -> 62 us).
 template <typename R, int VK, int GC, bool EV>
 __global__ void __launch_bounds__(64 * GC, sizeof(R) == 8 && VK == 1 ? 12 / GC : 8 / GC) k_trf_lo(Grid<R> g, Strides s, FrameTab ft,
@@ -617,8 +625,9 @@ __global__ void __launch_bounds__(64 * GC, sizeof(R) == 8 && VK == 1 ? 12 / GC :
     if (rare) {
       const R* te = EV || t == 0 ? te0 + (EV ? (size_t)t * 6 * NL : (size_t)0) + (size_t)i * 6 * L + ci.k : nullptr;
       FOR_V {
-        const LoItem<R> w = plain_lo<R, LK>(T + v + j, MF + v + j, E + v + j, te ? te + j : te, fs.mir + x * 6, nb, x,
-                                            ci.np, L, af + j);
+        constexpr auto plain = VK * sizeof(R) == 16 ? plain_lo_call<R, LK> : plain_lo<R, LK>;
+        const LoItem<R> w = plain(T + v + j, MF + v + j, E + v + j, te ? te + j : te, fs.mir + x * 6, nb, x, ci.np, L,
+                                  af + j);
         sumlo[j] = w.sum;
         sp_[j] = w.sp;
         sm_[j] = w.sm;
@@ -734,7 +743,8 @@ __device__ __forceinline__ void limiters(const FrameSm& fs, const R* TO, const R
 // and serialises the neighbour loads (FP32 glvl 7 / nvl 64 / 11 tracers 1.43
 // -> 1.41 ms, glvl 5 / nvl 38 / 5 tracers 66 -> 61 us, FP64 glvl 6 / nvl 64 /
 // 11 tracers 2.84 -> 2.78 ms; FP64 one level a thread at two blocks 252 us
-// against 239 at three).
+// against 239 at three; measured when chosen, the FP64 kernel has since come to
+// 2.53 ms and 212 us).
 template <typename R, int VK, int GC>
 __global__ void __launch_bounds__(64 * GC, VK * (int)sizeof(R) == 16 ? 8 / GC : 12 / GC) k_trf_hi(Grid<R> g, Strides s, FrameTab ft,
     const StepParams* __restrict__ sp, int t0, int nt, const R* __restrict__ trl_tdcy, const R* trcdp,
