@@ -69,7 +69,7 @@ __device__ __forceinline__ void ld4(const double* p, double (&r)[4]) {
 // share registers: 64 a thread, four blocks an SM (three: 1.53 ms, five,
 // spilling: 1.88 ms).  At glvl 8 / nvl 64 in FP32 1.41 ms, 4,880 GB/s of its
 // 41 words, where loading each neighbour for each of its edges took 1.98 ms;
-// glvl 6 in FP64 3.08 -> 1.81 ms.
+// glvl 6 in FP64 3.08 -> 1.70 ms.
 #define FIM_TRAIL(x) (e == 0 ? (five ? x[4][j] : x[5][j]) : x[e == 0 ? 0 : e - 1][j])
 #define FIM_LEAD(x) (e == 5 ? x[0][j] : e == 4 ? (five ? x[0][j] : x[5][j]) : x[e == 5 ? 0 : e + 1][j])
 // (2 (a + b) + c + d) / 6 on the live edges of a cell: x0 the cell's value, x
@@ -765,7 +765,7 @@ __global__ void __launch_bounds__(kBlock) k_cnuity_coop(Grid<R> g, Strides s, co
 // all three parts of its 32 columns, 32 levels at a time, left two to four warps
 // an SM in flight on small grids.  FP32, nvl 64: glvl 8 0.84 -> 0.44 ms (5,340
 // GB/s of its 14 words), glvl 5 / nvl 38 78 -> 14 us (4 levels a thread; one:
-// 0.65 ms and 18 us).  FP64, glvl 6: 0.70 -> 0.39 ms, with the power of
+// 0.65 ms and 18 us).  FP64, glvl 6: 0.70 -> 0.35 ms, with the power of
 // fim_internal.h; one level a thread, bound by the FP64 pipe.
 constexpr int kC5Cols = 32;
 constexpr int kC5Block = 256;
@@ -1157,7 +1157,7 @@ __global__ void __launch_bounds__(kBlock) k_dissip(Grid<R> g, Strides s, const R
 // consecutive levels (one chunk of 32 VK levels covers nvl 64 with two), so the
 // cell's tables and row addresses are formed once for both.  SPLIT: the
 // FP32-mixed step's form (mpf, tr0).  Bound by HBM: at glvl 8 / nvl 64 the step's
-// form takes 1.20 ms, 6,150 GB/s of its 44 words (one level a lane 1.57 ms; two
+// form takes 1.11 ms, 6,630 GB/s of its 44 words (one level a lane 1.57 ms; two
 // blocks an SM 1.32, four 1.34); the plain form at glvl 7 0.30 ms at four blocks
 // an SM (three 0.34; one level a lane 0.43).  FP64, one level a lane, is bound
 // by its operations: glvl 6 0.44 -> 0.32 ms with M + K - exm th formed once.
