@@ -661,7 +661,7 @@ __device__ __forceinline__ void cnuity4_body(int bx, int by, const Grid<R>& g, c
     ldv<VK>(r_plus + (size_t)px * L + k, rpx);
     ldv<VK>(r_mnus + (size_t)px * L + k, rmx);
     FOR_V {
-      const bool in = negative(a[j]);
+      const bool in = below0(a[j]);
       const R own = in ? rp[j] : rm[j], other = in ? rmx[j] : rpx[j];
       const R clip = sizeof(R) == 8 ? min0(own, other) : rmin(own, other);
       const R ac = a[j] * clip;

@@ -545,6 +545,9 @@ __device__ __forceinline__ double floor_at(double a, double b) {
 }
 __device__ __forceinline__ bool negative(float x) { return x < 0.f; }
 __device__ __forceinline__ bool negative(double x) { return __double2hiint(x) < 0; }
+// a < 0 of a number: a zero of either sign is not
+__device__ __forceinline__ bool below0(float a) { return a < 0.f; }
+__device__ __forceinline__ bool below0(double a) { return (int)((0ull - (unsigned long long)__double_as_longlong(a)) >> 32) > 0; }
 
 // products and sums whose contraction is pinned: the same value must come out
 // of every instantiation (the per-routine and the fused kernels, every shape)
@@ -591,8 +594,8 @@ __device__ __forceinline__ void split_sum(double a, double& sp, double& sm) {
 __device__ __forceinline__ bool sums_rare(float, float) { return false; }
 __device__ __forceinline__ bool sums_rare(double sp, double sm) { return f64_nan(sp) | f64_nan(sm); }
 
-// max(0, min(1, a / b)), b > 0; ratio_rare: a NaN (FP32: or two infinities)
-// among the numerators of R+ and R-, or an infinite one (FP64)
+// max(0, min(1, a / b)), b > 0; ratio_rare: a NaN or an infinity among the
+// numerators of R+ and R-
 __device__ __forceinline__ float ratio01(float a, float b) { return __saturatef(__fdividef(a, b)); }
 __device__ __forceinline__ double ratio01(double a, double b) {
   const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
@@ -601,7 +604,7 @@ __device__ __forceinline__ double ratio01(double a, double b) {
   if (y >= 0x7e00000000000000ll) return a / b;
   return f64_quot(a, b, f64_recip(b));  // 0 < a < b
 }
-__device__ __forceinline__ bool ratio_rare(float a, float b) { return (a + b) != (a + b); }
+__device__ __forceinline__ bool ratio_rare(float a, float b) { return !(fabsf(a + b) < __int_as_float(0x7f800000)); }
 __device__ __forceinline__ bool ratio_rare(double a, double b) { return f64_odd(a) | f64_odd(b); }
 __device__ __forceinline__ float plain_ratio01(float a, float b) {
   const float q = plain_max(0.f, plain_min(1.f, fdiv(a, plain_max(b, 1.e-11f))));

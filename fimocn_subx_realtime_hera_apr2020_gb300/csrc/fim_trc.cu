@@ -426,18 +426,26 @@ __device__ __noinline__ LoItem<R> plain_lo_call(const R* T, const R* MF, const R
 }
 
 // bounds and limiters of frame cell x in trcadv2 (ar: the cell's area, in FP64
-// over ab1)
+// over ab1).  routine: the bounds as trcadv1 and 2 form them one after the other;
+// else as the fused step does, old tracer and trcr_lo of a neighbour at a time
+// (in FP32 by the three-input instructions, which drop a NaN).
 template <typename R> struct LimItem { R hx, hn, rp, rm; };
+__device__ __forceinline__ float pair_max(float m, float a, float b) { return fmaxf(m, fmaxf(a, b)); }
+__device__ __forceinline__ float pair_min(float m, float a, float b) { return fminf(m, fminf(a, b)); }
+__device__ __forceinline__ double pair_max(double m, double a, double b) { return plain_max(m, plain_max(a, b)); }
+__device__ __forceinline__ double pair_min(double m, double a, double b) { return plain_min(m, plain_min(a, b)); }
 template <typename R, int LK>
 __device__ __noinline__ LimItem<R> plain_limits(const R* TO, const R* TL, uint2 nb, int x, R dp, R tof, R tvf, R spl,
-                                                R smn, R ab2, R ab3, R rab1, R ar) {
-  const R lc = TL[x * LK];
-  UpDown<R> b = plain_bounds<R, LK>(TO, nb, x);
+                                                R smn, R ab2, R ab3, R rab1, R ar, bool routine) {
+  const R lc = TL[x * LK], tc = TO[x * LK];
+  UpDown<R> b = {tc, tc};
+  if (routine) b = plain_bounds<R, LK>(TO, nb, x);
   b = {plain_max(b.up, lc), plain_min(b.down, lc)};
 #pragma unroll 1
   for (int e = 0; e < 6; e++) {
-    const R a = TL[nb_at(nb, e) * LK];
-    b = {plain_max(b.up, a), plain_min(b.down, a)};
+    const R a = TL[nb_at(nb, e) * LK], o = TO[nb_at(nb, e) * LK];
+    if (routine) b = {plain_max(b.up, a), plain_min(b.down, a)};
+    else b = {pair_max(b.up, o, a), pair_min(b.down, o, a)};
   }
   b = {plain_max(R(0), b.up), plain_max(R(0), b.down)};
   const R qp = per_ab1((b.up - lc) * dp - (ab2 * plain_min(R(0), tof) + ab3 * plain_max(R(0), tvf)), rab1, ar);
@@ -670,7 +678,7 @@ struct TrOut {
 // (clamped at zero) and the slots of/vof are returned for trcadv3
 template <typename R, int VK, int LK>
 __device__ __forceinline__ void limiters(const FrameSm& fs, const R* TO, const R* TL, const R* opq, const R* dpf,
-                                         const R* arf, int S1, int xe, int ve, R ab2, R ab3, R rab1,
+                                         const R* arf, int S1, int xe, int ve, R ab2, R ab3, R rab1, bool routine,
                                          R* Rp, R* Rm, R (&hx)[VK], R (&hn)[VK], R (&tof)[VK], R (&tvf)[VK]) {
   const R thshld = R(1.e-11);
   const uint2 nb = fs.nbr[xe];
@@ -716,7 +724,7 @@ __device__ __forceinline__ void limiters(const FrameSm& fs, const R* TO, const R
   if (rare) {
     FOR_V {
       const LimItem<R> w = plain_limits<R, LK>(TO + ve + j, TL + ve + j, nb, xe, dp[j], tof[j], tvf[j], spl[j],
-                                               smn[j], ab2, ab3, rab1, ar);
+                                               smn[j], ab2, ab3, rab1, ar, routine);
       hx[j] = w.hx;
       hn[j] = w.hn;
       rp[j] = w.rp;
@@ -846,12 +854,14 @@ __global__ void __launch_bounds__(64 * GC, VK * (int)sizeof(R) == 16 ? 8 / GC : 
     // R+/R- of the thread's patch cell (its bounds and slots kept for
     // trcadv3), then of the ring-1 cells
     R hx[VK], hn[VK], tof[VK], tvf[VK];
-    if (on) limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, x, v, ab.old, ab.very_old, rab1, Rp, Rm, hx, hn, tof, tvf);
+    if (on) limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, x, v, ab.old, ab.very_old, rab1, all, Rp, Rm, hx, hn, tof,
+                                   tvf);
     for (int it = threadIdx.x; it < (n1 - C) * GC; it += blockDim.x) {
       const int xe = C + it / GC, ve = (it % GC) * VK;
       if (ve >= lk) continue;
       R mx2[VK], mn2[VK], tof2[VK], tvf2[VK];
-      limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, xe, ve, ab.old, ab.very_old, rab1, Rp, Rm, mx2, mn2, tof2, tvf2);
+      limiters<R, VK, LK>(fs, TO, TL, opq, dpf, arf, ft.S1, xe, ve, ab.old, ab.very_old, rab1, all, Rp, Rm, mx2, mn2,
+                           tof2, tvf2);
     }
     stage_wait();
     __syncthreads();
@@ -878,7 +888,7 @@ __global__ void __launch_bounds__(64 * GC, VK * (int)sizeof(R) == 16 ? 8 / GC : 
         ldv<VK>(Rp + y * LK + v, rpx);
         ldv<VK>(Rm + y * LK + v, rmx);
         FOR_V {
-          const bool in = negative(a[j]);
+          const bool in = below0(a[j]);
           at[j] = fma_rn(a[j], min0(in ? rpc[j] : rmc[j], in ? rmx[j] : rpx[j]), at[j]);
         }
       }

@@ -50,6 +50,9 @@ BINARY(t_plain_ratio, double, plain_ratio01(x, y))
 BINARY(t_min0, double, min0(own_limit(x), y))
 BINARY(t_min0f, float, min0(own_limit(x), y))
 BINARY(t_ratiof, float, plain_ratio01(x, y))
+BINARY(t_rare, double, ratio_rare(x, y) ? 1. : 0.)
+BINARY(t_raref, float, ratio_rare(x, y) ? 1.f : 0.f)
+UNARY(t_below0, double, below0(x) ? 1. : 0.)
 UNARY(t_tenth, float, tenth(x))
 UNARY(t_tenthd, double, tenth(x))
 """
@@ -184,6 +187,14 @@ def test_limiter_quotients(lib):
         assert np.all(np.signbit(got[np.isnan(got)])), f  # min0 knows a NaN by its sign
         assert np.allclose(got[keep], q[keep], rtol=4e-7 if dt is np.float32 else 3e-16,
                            atol=1e-37 if dt is np.float32 else 0, equal_nan=True), f
+    # a numerator that is no number, or two that cancel or add to an infinity
+    with np.errstate(all="ignore"):
+        for f, dt in (("t_rare", np.float64), ("t_raref", np.float32)):
+            x, y = a.astype(dt), b.astype(dt)
+            rare = lib(f, x, y, dtype=dt) != 0
+            assert rare[~(np.isfinite(x) & np.isfinite(y))].all() and not rare[np.isfinite(x + y)].any(), f
+    x = np.concatenate([a[~np.isnan(a)], [0.0, -0.0]])  # (a NaN flux's limiters do not matter)
+    assert np.array_equal(lib("t_below0", x) != 0, x < 0)
     r = np.concatenate([rng.uniform(0, 1, 30), [0.0, 1.0], np.array([0xfff8 << 48], np.uint64).view(np.float64)])
     x, y = (v.ravel() for v in np.meshgrid(r, r))
     assert np.array_equal(np.nan_to_num(lib("t_min0", x, y), nan=7.5),
