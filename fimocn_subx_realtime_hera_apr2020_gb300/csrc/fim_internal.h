@@ -479,7 +479,7 @@ __device__ __forceinline__ float pow_rd_cp(float x) { return pow(x, float(kRd) /
 // FP32 takes the min/max instructions; FP64 compares on the integer pipe and
 // divides with the fewest FP64 operations (above).  At glvl 6 / nvl 64 / 11
 // tracers this took the FP64 k_trf_lo from 9.56 to 5.0 ms and k_trf_hi from
-// 8.15 to 2.53 ms a step (FP32: 2% of k_trf_hi).
+// 8.15 to 2.48 ms a step (FP32: 2% of k_trf_hi).
 //
 // These forms hold for numbers.  What is not finite has to go where the
 // routines, written with a > b ? a : b, send it (a NaN in a tracer, a thickness

@@ -752,7 +752,7 @@ __device__ __forceinline__ void limiters(const FrameSm& fs, const R* TO, const R
 // -> 1.41 ms, glvl 5 / nvl 38 / 5 tracers 66 -> 61 us, FP64 glvl 6 / nvl 64 /
 // 11 tracers 2.84 -> 2.78 ms; FP64 one level a thread at two blocks 252 us
 // against 239 at three; measured when chosen, the FP64 kernel has since come to
-// 2.53 ms and 212 us).
+// 2.48 ms and 212 us).
 template <typename R, int VK, int GC>
 __global__ void __launch_bounds__(64 * GC, VK * (int)sizeof(R) == 16 ? 8 / GC : 12 / GC) k_trf_hi(Grid<R> g, Strides s, FrameTab ft,
     const StepParams* __restrict__ sp, int t0, int nt, const R* __restrict__ trl_tdcy, const R* trcdp,
